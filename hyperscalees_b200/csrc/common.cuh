@@ -26,6 +26,8 @@ struct DeviceTables {
     uint64_t n_log_flips = 0, n_cos_flips = 0;
     // generator jump tables: entry k advances the state by 2^k steps
     uint64_t* jump_pow2 = nullptr;  // kJumpLevels matrices
+    // lane tables (see lane_jump): lane l goes 4 l or 16 l normals (two steps each) ahead
+    uint64_t *jump_lane4 = nullptr, *jump_lane16 = nullptr;
     // one int per device: kernels with bounded waits record here why they gave up
     int* status_word = nullptr;
 };

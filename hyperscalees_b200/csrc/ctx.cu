@@ -154,6 +154,22 @@ static int build_tables(DeviceTables& t) {
                              cudaMemcpyHostToDevice));
     }
 
+    for (int which = 0; which < 2; ++which) {
+        const int log2_steps = which == 0 ? 3 : 5;   // 4 or 16 normals
+        BitMat step = step_matrix(), m;
+        for (int k = 0; k < log2_steps; ++k) step = compose(step, step);
+        for (int j = 0; j < 64; ++j) m.col[j] = 1ull << j;   // identity
+        std::vector<uint64_t> host(kLaneWords);
+        for (int lane = 0; lane < 32; ++lane) {
+            for (int p = 0; p < 16; ++p)
+                for (int v = 0; v < 16; ++v) host[(size_t)(p * 16 + v) * 32 + lane] = m.apply((uint64_t)v << (4 * p));
+            m = compose(step, m);
+        }
+        uint64_t** dst = which == 0 ? &t.jump_lane4 : &t.jump_lane16;
+        HSES_CUDA(cudaMalloc(dst, host.size() * sizeof(uint64_t)));
+        HSES_CUDA(cudaMemcpy(*dst, host.data(), host.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));
+    }
+
     // candidates on the device, libm on the host
     uint32_t *d_bits = nullptr, *d_code = nullptr;
     HSES_CUDA(cudaMalloc(&d_bits, (size_t)kUnits * 4));

@@ -378,6 +378,7 @@ size_t hses_perturbed_linear_workspace_bytes(const hses_linear_args* g) {
     if (g->algo == HSES_ALGO_AUTO && small_path_supports(*g)) return small_path_workspace_bytes(*g);
     if ((g->algo == HSES_ALGO_AUTO || g->algo == HSES_ALGO_PAIR) && pair_path_supports(*g))
         return pair_path_workspace_bytes(*g);
+    if (g->algo == HSES_ALGO_AUTO && pack_path_supports(*g)) return pack_path_workspace_bytes(*g);
     if (g->algo == HSES_ALGO_TENSOR || g->algo == HSES_ALGO_PAIR || !g->perturb) return 0;
     return simt_scratch(*g, nullptr).bytes;
 }
@@ -456,6 +457,7 @@ int hses_perturbed_linear(hses_ctx* ctx, hses_stream stream, const hses_linear_a
     }
     if (g->algo == HSES_ALGO_PAIR || (g->algo == HSES_ALGO_AUTO && pair_ok))
         return run_pair_path(ctx, as_stream(stream), *g);
+    if (g->algo == HSES_ALGO_AUTO && pack_path_supports(*g)) return run_pack_path(ctx, as_stream(stream), *g);
     return run_simt(ctx, as_stream(stream), *g);
 }
 

@@ -23,6 +23,12 @@ bool small_path_supports(const hses_linear_args& g);
 size_t small_path_workspace_bytes(const hses_linear_args& g);
 int run_small_path(hses_ctx* ctx, cudaStream_t stream, const hses_linear_args& g);
 
+// Any other shape on the tensor cores (linear_pack.cu): rows packed per antithetic pair, ragged widths and
+// pitches, ranks up to 128.  Taken by HSES_ALGO_AUTO only.
+bool pack_path_supports(const hses_linear_args& g);
+size_t pack_path_workspace_bytes(const hses_linear_args& g);
+int run_pack_path(hses_ctx* ctx, cudaStream_t stream, const hses_linear_args& g);
+
 // Checks args.cache against the call and returns the cached raw factors of the call's
 // first pair: A rows (pair, a, rank) and B rows (pair, k, rank).
 int resolve_factor_cache(const hses_linear_args& g, const float** A, const float** B);

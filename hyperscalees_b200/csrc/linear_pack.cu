@@ -1,0 +1,944 @@
+// Tensor-core path of the perturbed linear layer (do_mm, hyperscalees-noiser/src/eggroll.rs:419-446,
+// + lif_step, snn.rs:53-65) for shapes that fit no tile: any number of rows, samples per member, inputs
+// and outputs, any pitch, ranks up to 128.  linear_tc.cu keeps the tile-aligned shapes.
+//
+// The rows of an antithetic pair (both members, all time steps) are packed next to each other and padded
+// to a multiple of 32 (64 or 128 for wide ranks), so that a 32-row slice of a 128-row tile always belongs
+// to one pair.  Both products of the rank-r term then run on the tensor cores as well: t = x·B is a
+// second, narrow product over the same x tiles (the B blocks of the tile's pairs side by side), and
+// t·(sA)ᵀ extends the K dimension of the main product (t in the columns of its own pair, zeros elsewhere),
+// so the epilogue only scales and stores.
+//
+//   launch 1  pack_split_w     rows of W: a power of two each, then fp16 hi + lo
+//   launch 2  pack_operands    x rows in packed order as fp16 hi + lo; the factors, regenerated from the
+//                              stream or read from a cache, as B (K-major fp16 hi + lo, fixed scale 2^11)
+//                              and A (three bf16 parts, scaled by s and by the scale of W's row)
+//   launch 3  linear_pack      persistent, ten warps: TMA producer, MMA issuer, eight epilogue warps
+// Products of x, W and B are hi*hi + hi*lo + lo*hi in fp16 (2^-21 relative residue); t and A are split into
+// three bf16 parts (24 bits, six products): bf16 has the exponent range of fp32, so that the rank-r term
+// can be accumulated on top of the main product in its scale.  No multicast, no cluster launch; every wait
+// is bounded.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
+#include "linear.cuh"
+#include "tc_common.cuh"
+
+namespace hses {
+
+namespace {
+
+using namespace tc;
+
+constexpr int PK_TILE = 128;       // rows per tile
+constexpr int PK_BK = 64;          // fp16 values per k-block (one 128-byte swizzle row)
+constexpr int PK_THREADS = 320;    // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
+constexpr int PK_MAX_STAGES = 6;
+constexpr int PK_SMEM_LIMIT = 232448;
+constexpr int PK_TR_PITCH = 17;    // staged 32 x 16 output block of an epilogue warp
+constexpr int PK_TR_BYTES = 8 * 32 * PK_TR_PITCH * 4;
+constexpr int PK_EXP_B = 11;       // B * 2^11: |normal| < 6 keeps it below 2^14
+constexpr int PK_SEG = 4096;       // normals of a factor segment
+
+// Which row of the call a packed row is.
+struct RowMap {
+    int packed;          // 0: row p is row p
+    int rp;              // padded rows per pair
+    int t_steps, bm;
+    int64_t n_pop;
+    int32_t first_thread, first_pair;
+    int64_t rows;        // packed rows in total
+};
+__device__ __forceinline__ bool map_row(const RowMap& m, int64_t p, int64_t& R, bool& odd) {
+    odd = false;
+    R = p;
+    if (p >= m.rows) return false;
+    if (!m.packed) return true;
+    const int32_t pair = (int32_t)(p / m.rp);
+    const int lr = (int)(p - (int64_t)pair * m.rp);
+    int64_t m_lo = (int64_t)(m.first_pair + pair) * 2 - m.first_thread, m_hi = m_lo + 2;
+    if (m_lo < 0) m_lo = 0;
+    if (m_hi > m.n_pop) m_hi = m.n_pop;
+    const int rps = (int)(m_hi - m_lo) * m.bm;
+    const int step = lr / rps, rr = lr - step * rps;
+    if (step >= m.t_steps) return false;
+    R = ((int64_t)step * m.n_pop + m_lo) * m.bm + rr;
+    odd = ((m.first_thread + m_lo + rr / m.bm) & 1) != 0;
+    return true;
+}
+
+// ------------------------------------------------------------------ operand preparation
+struct SplitJob {
+    const float* src;
+    int64_t stride;
+    int64_t rows;
+    int k, kp;           // values per row, row pitch of the operand (multiple of 8, padded with zeros)
+    int vec;             // rows are 16-byte aligned
+    __half *hi, *lo;
+    float* inv_scale;
+    int* lo_flag;
+};
+
+// values e .. e+3 of a row of k values; past the end: 0
+__device__ __forceinline__ float4 load4(const float* row, int e, int k, int vec) {
+    if (vec && e + 4 <= k) return __ldg(reinterpret_cast<const float4*>(row + e));
+    float4 v;
+    v.x = e < k ? __ldg(row + e) : 0.0f;
+    v.y = e + 1 < k ? __ldg(row + e + 1) : 0.0f;
+    v.z = e + 2 < k ? __ldg(row + e + 2) : 0.0f;
+    v.w = e + 3 < k ? __ldg(row + e + 3) : 0.0f;
+    return v;
+}
+// power of two that brings the largest magnitude m of a row into [2^13, 2^14); 1 for rows without one
+__device__ __forceinline__ int scale_exponent(float m) {
+    const int ex = (int)((__float_as_uint(m) >> 23) & 0xffu) - 127;
+    int e = 13 - ex;
+    if (ex <= -127 || ex >= 128) e = 0;
+    return max(-100, min(100, e));
+}
+__device__ __forceinline__ float warp_max(float m) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+    return m;
+}
+__device__ __forceinline__ float max4(float m, float4 v) {
+    return fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+}
+__device__ __forceinline__ void split4(float4 v, float s, uint2& h2, uint2& l2, uint32_t& nz) {
+    const float x0 = v.x * s, x1 = v.y * s, x2 = v.z * s, x3 = v.w * s;
+    const __half2 h01 = __floats2half2_rn(x0, x1), h23 = __floats2half2_rn(x2, x3);
+    const float2 b01 = __half22float2(h01), b23 = __half22float2(h23);
+    const __half2 l01 = __floats2half2_rn(x0 - b01.x, x1 - b01.y), l23 = __floats2half2_rn(x2 - b23.x, x3 - b23.y);
+    h2 = make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
+    l2 = make_uint2(*reinterpret_cast<const uint32_t*>(&l01), *reinterpret_cast<const uint32_t*>(&l23));
+    nz |= (l2.x | l2.y) & 0x7fff7fffu;   // a lo half of -0 is still zero
+}
+
+// One warp takes RPW rows at a time, NJ pieces of 128 values each in registers (NJ = 0: rows of any length,
+// read twice, the second time from L1 or L2).
+template <int NJ, int RPW>
+__device__ __forceinline__ void split_rows(const SplitJob& j, const RowMap& map, int64_t block) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t p0 = (block * (blockDim.x >> 5) + warp) * RPW;
+    uint32_t nz = 0;
+    const int n4 = j.kp >> 2;
+    if (NJ > 0) {
+        float4 v[RPW][NJ > 0 ? NJ : 1];
+        bool valid[RPW];
+#pragma unroll
+        for (int r = 0; r < RPW; ++r) {
+            int64_t R;
+            bool odd;
+            valid[r] = p0 + r < j.rows && map_row(map, p0 + r, R, odd);   // warp-uniform
+            const float* row = j.src + (size_t)(valid[r] ? R : 0) * j.stride;
+#pragma unroll
+            for (int i = 0; i < NJ; ++i)
+                v[r][i] = valid[r] ? load4(row, 4 * (lane + 32 * i), j.k, j.vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int r = 0; r < RPW; ++r) {
+            if (!valid[r]) continue;
+            float m = 0.0f;
+#pragma unroll
+            for (int i = 0; i < NJ; ++i) m = max4(m, v[r][i]);
+            const int e = scale_exponent(warp_max(m));
+            const float s = __uint_as_float((uint32_t)(127 + e) << 23);
+            if (lane == 0) j.inv_scale[p0 + r] = __uint_as_float((uint32_t)(127 - e) << 23);
+            uint2* dh = reinterpret_cast<uint2*>(j.hi + (size_t)(p0 + r) * j.kp);
+            uint2* dl = reinterpret_cast<uint2*>(j.lo + (size_t)(p0 + r) * j.kp);
+#pragma unroll
+            for (int i = 0; i < NJ; ++i) {
+                const int c = lane + 32 * i;
+                if (c < n4) {
+                    uint2 h2, l2;
+                    split4(v[r][i], s, h2, l2, nz);
+                    dh[c] = h2;
+                    dl[c] = l2;
+                }
+            }
+        }
+    } else {
+        int64_t R;
+        bool odd;
+        if (p0 >= j.rows || !map_row(map, p0, R, odd)) return;
+        const float* row = j.src + (size_t)R * j.stride;
+        float m = 0.0f;
+        for (int c = lane; c < n4; c += 32) m = max4(m, load4(row, 4 * c, j.k, j.vec));
+        const int e = scale_exponent(warp_max(m));
+        const float s = __uint_as_float((uint32_t)(127 + e) << 23);
+        if (lane == 0) j.inv_scale[p0] = __uint_as_float((uint32_t)(127 - e) << 23);
+        uint2* dh = reinterpret_cast<uint2*>(j.hi + (size_t)p0 * j.kp);
+        uint2* dl = reinterpret_cast<uint2*>(j.lo + (size_t)p0 * j.kp);
+        for (int c = lane; c < n4; c += 32) {
+            uint2 h2, l2;
+            split4(load4(row, 4 * c, j.k, j.vec), s, h2, l2, nz);
+            dh[c] = h2;
+            dl[c] = l2;
+        }
+    }
+    // one flag per call tells the product whether any lo half is non-zero (a set flag is not set again)
+    if (j.lo_flag && __any_sync(0xffffffffu, nz != 0) && lane == 0 && *reinterpret_cast<volatile int*>(j.lo_flag) == 0)
+        atomicOr(j.lo_flag, 1);
+}
+template <int NJ, int RPW>
+__global__ void __launch_bounds__(256) pack_split_kernel(SplitJob j, RowMap map) {
+    split_rows<NJ, RPW>(j, map, blockIdx.x);
+}
+
+struct FactorJob {
+    const float *cache_a, *cache_b;   // raw (pairs, a, r) and (pairs, k, r), or NULL: regenerate
+    const uint64_t *pow2, *lane_tab;
+    LibmCal cal;
+    uint64_t key;
+    int32_t true_epoch, first_pair;
+    int64_t pairs;
+    int r, r16, k, kp, a;
+    int row_a0, row_b0;               // first output-side and input-side row of a pair's stream block
+    int seg_b, seg_a;                 // rows per segment (multiples of 8)
+    int bn, n_chunks, kb;             // output columns per chunk, chunks, rank values per block of A's image
+    float base_sigma;
+    const float* col_scale;           // 2^-e of W's rows
+    __half *bhi, *blo;                // (pairs, r16, kp)
+    __nv_bfloat16* aimg;              // (pairs, chunk, r16 / kb, part 3, kb / 8, bn, 8)
+};
+
+// Segment `seg` of pair `p`: its normals into shared memory, 16 bytes per thread and trip, then to the operand
+// layout.  Regeneration: a warp takes 128 consecutive normals, its base state by powers of two (the same for all
+// lanes, so every table read is a broadcast), the lane's own state by one round of the lane table.
+__device__ __forceinline__ void factor_segment(const FactorJob& f, int64_t p, int seg, float* buf, double2* log_tab_s,
+                                               uint32_t* delta_s) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nseg_b = (f.k + f.seg_b - 1) / f.seg_b;
+    const bool is_b = seg < nseg_b;
+    const int row0 = is_b ? seg * f.seg_b : (seg - nseg_b) * f.seg_a;
+    const int nrows = is_b ? min(f.seg_b, f.k - row0) : min(f.seg_a, f.a - row0);
+    const int cnt = nrows * f.r;
+    if (f.cache_b) {
+        const float* src = is_b ? f.cache_b + ((size_t)p * f.k + row0) * f.r : f.cache_a + ((size_t)p * f.a + row0) * f.r;
+        if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+            for (int i = tid; i < cnt / 4; i += blockDim.x)
+                *reinterpret_cast<float4*>(buf + 4 * i) = __ldg(reinterpret_cast<const float4*>(src) + i);
+            for (int i = (cnt & ~3) + tid; i < cnt; i += blockDim.x) buf[i] = __ldg(src + i);
+        } else {
+            for (int i = tid; i < cnt; i += blockDim.x) buf[i] = __ldg(src + i);
+        }
+    } else {
+        LibmCal cal = f.cal;
+        for (int i = tid; i < 64; i += blockDim.x) log_tab_s[i] = cal.log_tab[i];
+        for (int i = tid; i < 256; i += blockDim.x) {
+            delta_s[i] = cal.log_delta[i];
+            delta_s[256 + i] = cal.cos_delta[i];
+        }
+        __syncthreads();
+        cal.log_tab = log_tab_s;
+        cal.log_delta = delta_s;
+        cal.cos_delta = delta_s + 256;
+        const uint64_t first = (uint64_t)f.r * (uint64_t)(row0 + (is_b ? f.row_b0 : f.row_a0));
+        const uint64_t s0 = noise_seed(f.key, f.true_epoch, f.first_pair + (int32_t)p) | 1ull;
+        for (int base = warp * 128; base < cnt; base += (blockDim.x >> 5) * 128) {
+            uint64_t s = lane_jump(f.lane_tab, jump_by(f.pow2, s0, 2ull * (first + (uint64_t)base)), lane);
+            float z[4];
+            next_normals4(s, cal, z);
+            *reinterpret_cast<float4*>(buf + base + 4 * lane) = make_float4(z[0], z[1], z[2], z[3]);
+        }
+    }
+    __syncthreads();
+    if (is_b) {
+        // eight consecutive k of one rank column per thread: 4 such pieces x 8 columns per warp
+        const int kend = min(f.kp - row0, f.seg_b);           // the padding of the last segment's rows is zero
+        const int ng = (kend + 7) >> 3;
+        const float sc = (float)(1 << PK_EXP_B);
+        for (int idx = tid; idx < ((ng + 3) & ~3) * f.r16; idx += blockDim.x) {
+            const int blk = idx >> 5, l = idx & 31;
+            const int qb = f.r16 >> 3;
+            const int q = (blk % qb) * 8 + (l & 7), g = (blk / qb) * 4 + (l >> 3);
+            if (g >= ng) continue;
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                v[j] = (q < f.r && g * 8 + j < nrows) ? buf[(g * 8 + j) * f.r + q] : 0.0f;
+            uint2 h0, h1, l0, l1;
+            uint32_t nz = 0;
+            split4(make_float4(v[0], v[1], v[2], v[3]), sc, h0, l0, nz);
+            split4(make_float4(v[4], v[5], v[6], v[7]), sc, h1, l1, nz);
+            const size_t o = ((size_t)p * f.r16 + q) * f.kp + row0 + g * 8;
+            *reinterpret_cast<uint4*>(f.bhi + o) = make_uint4(h0.x, h0.y, h1.x, h1.y);
+            *reinterpret_cast<uint4*>(f.blo + o) = make_uint4(l0.x, l0.y, l1.x, l1.y);
+        }
+    } else {
+        for (int idx = tid; idx < nrows * (f.r16 >> 3); idx += blockDim.x) {
+            const int g = idx / nrows, i = idx - g * nrows;   // rank piece, row of the segment
+            const int n = row0 + i, c = n / f.bn, nn = n - c * f.bn;
+            const uint32_t e = 254u - (__float_as_uint(__ldg(f.col_scale + n)) >> 23);   // exponent field of 2^+e
+            const float sc = __fmul_rn(f.base_sigma, __uint_as_float(e << 23)) * (1.0f / (1 << PK_EXP_B));
+            uint32_t w[3][4];
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {
+                float v[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int q = g * 8 + j + h;
+                    v[h] = q < f.r ? __fmul_rn(buf[i * f.r + q], sc) : 0.0f;
+                }
+#pragma unroll
+                for (int part = 0; part < 3; ++part) {
+                    const __nv_bfloat162 b = __floats2bfloat162_rn(v[0], v[1]);
+                    w[part][j >> 1] = *reinterpret_cast<const uint32_t*>(&b);
+                    v[0] -= __bfloat162float(b.x);
+                    v[1] -= __bfloat162float(b.y);
+                }
+            }
+            const int kblk = (g * 8) / f.kb, gi = g - kblk * (f.kb >> 3);
+            __nv_bfloat16* img = f.aimg + ((((size_t)p * f.n_chunks + c) * (f.r16 / f.kb) + kblk) * 3) * f.kb * f.bn;
+#pragma unroll
+            for (int part = 0; part < 3; ++part)
+                *reinterpret_cast<uint4*>(img + (size_t)part * f.kb * f.bn + ((size_t)gi * f.bn + nn) * 8) =
+                    make_uint4(w[part][0], w[part][1], w[part][2], w[part][3]);
+        }
+    }
+}
+
+// x rows and factors in one launch: the first x_blocks blocks split rows, the others take (pair, segment).
+template <int NJ, int RPW>
+__global__ void __launch_bounds__(256) pack_operands_kernel(SplitJob x, RowMap map, int64_t x_blocks, int segs, FactorJob f) {
+    __shared__ __align__(16) float buf[PK_SEG];
+    __shared__ double2 log_tab_s[64];
+    __shared__ uint32_t delta_s[512];
+    const int64_t b = blockIdx.x;
+    if (b < x_blocks) {
+        split_rows<NJ, RPW>(x, map, b);
+    } else {
+        const int64_t i = b - x_blocks;
+        factor_segment(f, i / segs, (int)(i % segs), buf, log_tab_s, delta_s);
+    }
+}
+
+// ----------------------------------------------------------------------------- product
+struct PackArgs {
+    RowMap map;
+    int64_t m_tiles;
+    int groups;            // column-chunk groups a tile's work is cut into
+    int n_chunks, bn, a, k_blocks;
+    int nt;                // columns of t in a tile: pairs per tile * r16
+    int r16, kb;
+    int rb;                // 32-row blocks per pair
+    int64_t pairs;
+    const __nv_bfloat16* aimg;
+    const float *row_scale, *col_scale;
+    const int* x_lo_flag;
+    int lif;
+    float leak, v_th, out_scale;
+    const float* out_scale_ptr;
+    float* out;
+    int64_t out_stride;
+    float* pot;
+    int stages, stage_bytes;
+    int staged_stores;     // room for the transposed store buffer
+    int* status;
+};
+
+// K-major operand without swizzle: 8-row x 16-byte core matrices, contiguous (128 bytes) along the rows,
+// `lbo` bytes apart along K
+__device__ __forceinline__ uint64_t make_plain_desc(const void* tile, uint32_t lbo) {
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_u32(tile) & 0x3FFFF) >> 4);
+    d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
+    d |= (uint64_t)(128 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    return d;
+}
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+
+template <bool PERT>
+__global__ void __launch_bounds__(PK_THREADS, 1)
+linear_pack_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_constant__ CUtensorMap tm_xlo,
+                   const __grid_constant__ CUtensorMap tm_whi, const __grid_constant__ CUtensorMap tm_wlo,
+                   const __grid_constant__ CUtensorMap tm_bhi, const __grid_constant__ CUtensorMap tm_blo,
+                   const PackArgs g) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    constexpr int X_BYTES = PK_TILE * PK_BK * 2;
+    const int w_bytes = g.bn * PK_BK * 2, b_bytes = g.nt * PK_BK * 2;
+    uint8_t* tpp = smem + (size_t)g.stages * g.stage_bytes;            // [part 3][nt / 8][128][8] bf16
+    const int part_bytes = g.nt * PK_TILE * 2;
+    float* tr = reinterpret_cast<float*>(tpp + (PERT ? 3 * part_bytes : 0));
+    __shared__ uint64_t full[PK_MAX_STAGES], empty[PK_MAX_STAGES], tfull[2], tempty[2], tacc, tready;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_flag_s;
+    volatile int* abort_flag = &abort_flag_s;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        abort_flag_s = 0;
+        for (int s = 0; s < g.stages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&tfull[b], 1);
+            mbar_init(&tempty[b], 256);
+        }
+        mbar_init(&tacc, 1);
+        mbar_init(&tready, 256);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(PERT ? 512 : 256)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;       // accumulators at columns 0 and 128, t at 256
+    const int64_t units = g.m_tiles * g.groups;
+    const int nkb = PERT ? g.r16 / g.kb : 1;
+    // pairs of tile mt: first one and count
+    auto pairs_of = [&](int64_t mt, int64_t& p0) {
+        p0 = (mt * 4) / g.rb;
+        const int64_t last = min((mt * 4 + 3) / (int64_t)g.rb, g.pairs - 1);
+        return (int)(last - p0) + 1;
+    };
+
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t it = 0;
+            bool ok = true;
+            const bool skip_xlo = *g.x_lo_flag == 0;
+            auto slot = [&](uint32_t bytes) -> uint8_t* {
+                const int s = it % g.stages;
+                ok = mbar_wait(&empty[s], ((it / g.stages) & 1) ^ 1, abort_flag, g.status, 1);
+                if (!ok) return nullptr;
+                mbar_expect_tx(&full[s], bytes);
+                return smem + (size_t)s * g.stage_bytes;
+            };
+            for (int64_t u = blockIdx.x; u < units && ok; u += gridDim.x) {
+                const int64_t mt = u / g.groups;
+                const int grp = (int)(u - mt * g.groups);
+                const int c0 = g.n_chunks * grp / g.groups, c1 = g.n_chunks * (grp + 1) / g.groups;
+                int64_t p0 = 0;
+                int nd = 0;
+                if (PERT) {
+                    nd = pairs_of(mt, p0);
+                    for (int kb = 0; kb < g.k_blocks; ++kb, ++it) {
+                        uint8_t* st = slot((skip_xlo ? 1 : 2) * X_BYTES + 2 * b_bytes);
+                        if (!ok) break;
+                        uint64_t* bar = &full[it % g.stages];
+                        tma_load_2d(st, &tm_xhi, kb * PK_BK, (int)(mt * PK_TILE), bar);
+                        if (!skip_xlo) tma_load_2d(st + X_BYTES, &tm_xlo, kb * PK_BK, (int)(mt * PK_TILE), bar);
+                        tma_load_2d(st + 2 * X_BYTES, &tm_bhi, kb * PK_BK, (int)(p0 * g.r16), bar);
+                        tma_load_2d(st + 2 * X_BYTES + b_bytes, &tm_blo, kb * PK_BK, (int)(p0 * g.r16), bar);
+                    }
+                }
+                for (int c = c0; c < c1 && ok; ++c) {
+                    for (int kb = 0; kb < g.k_blocks; ++kb, ++it) {
+                        uint8_t* st = slot((skip_xlo ? 1 : 2) * X_BYTES + 2 * w_bytes);
+                        if (!ok) break;
+                        uint64_t* bar = &full[it % g.stages];
+                        tma_load_2d(st, &tm_xhi, kb * PK_BK, (int)(mt * PK_TILE), bar);
+                        if (!skip_xlo) tma_load_2d(st + X_BYTES, &tm_xlo, kb * PK_BK, (int)(mt * PK_TILE), bar);
+                        tma_load_2d(st + 2 * X_BYTES, &tm_whi, kb * PK_BK, c * g.bn, bar);
+                        tma_load_2d(st + 2 * X_BYTES + w_bytes, &tm_wlo, kb * PK_BK, c * g.bn, bar);
+                    }
+                    if (PERT) {
+                        const uint32_t bytes = 3u * g.kb * g.bn * 2;
+                        for (int i = 0; i < nd * nkb && ok; ++i, ++it) {
+                            uint8_t* st = slot(bytes);
+                            if (!ok) break;
+                            const int d = i / nkb, kblk = i - d * nkb;
+                            const size_t img = (((size_t)(p0 + d) * g.n_chunks + c) * nkb + kblk) * 3 * g.kb * g.bn;
+                            bulk_load(st, g.aimg + img, bytes, &full[it % g.stages]);
+                        }
+                    }
+                }
+            }
+            if (!ok) {
+                // copies already issued still land in this CTA's shared memory: give them a bounded moment
+                for (int s = 0; s < g.stages; ++s)
+                    for (uint32_t i = 0; i < 4096; ++i) {
+                        if (mbar_try(&full[s], 0) || mbar_try(&full[s], 1)) break;
+                        __nanosleep(256);
+                    }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = make_idesc(g.bn), idesc_t = make_idesc(PERT ? g.nt : 16), idesc_u = make_idesc_bf16(g.bn);
+            uint32_t it = 0, acc_it = 0, unit_no = 0;
+            bool ok = true;
+            const bool skip_xlo = *g.x_lo_flag == 0;
+            auto arrive = [&]() -> uint8_t* {
+                const int s = it % g.stages;
+                ok = mbar_wait(&full[s], (it / g.stages) & 1, abort_flag, g.status, 3);
+                if (!ok) return nullptr;
+                tc_fence_after();
+                return smem + (size_t)s * g.stage_bytes;
+            };
+            // three fp16 passes over one k-block
+            auto three = [&](uint32_t d, uint8_t* st, int bytes, uint32_t id, bool first) {
+                const uint64_t dxh = make_smem_desc(st), dxl = make_smem_desc(st + X_BYTES);
+                const uint64_t dwh = make_smem_desc(st + 2 * X_BYTES), dwl = make_smem_desc(st + 2 * X_BYTES + bytes);
+#pragma unroll
+                for (int ks = 0; ks < PK_BK / 16; ++ks) {
+                    const uint64_t off = (uint64_t)(ks * 32 >> 4);
+                    const uint32_t acc = !(first && ks == 0);
+                    if (!skip_xlo) umma_f16(d, dxl + off, dwh + off, id, acc);
+                    umma_f16(d, dxh + off, dwl + off, id, skip_xlo ? acc : 1u);
+                    umma_f16(d, dxh + off, dwh + off, id, 1);
+                }
+            };
+            for (int64_t u = blockIdx.x; u < units && ok; u += gridDim.x, ++unit_no) {
+                const int64_t mt = u / g.groups;
+                const int grp = (int)(u - mt * g.groups);
+                const int c0 = g.n_chunks * grp / g.groups, c1 = g.n_chunks * (grp + 1) / g.groups;
+                int64_t p0 = 0;
+                int nd = 0;
+                if (PERT) {
+                    nd = pairs_of(mt, p0);
+                    for (int kb = 0; kb < g.k_blocks; ++kb, ++it) {
+                        uint8_t* st = arrive();
+                        if (!ok) break;
+                        three(tmem + 256, st, b_bytes, idesc_t, kb == 0);
+                        umma_commit(&empty[it % g.stages]);
+                    }
+                    if (!ok) break;
+                    umma_commit(&tacc);
+                }
+                for (int c = c0; c < c1 && ok; ++c, ++acc_it) {
+                    const int b = acc_it & 1;
+                    if (!mbar_wait(&tempty[b], ((acc_it >> 1) & 1) ^ 1, abort_flag, g.status, 2)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t d = tmem + (uint32_t)(b * 128);
+                    for (int kb = 0; kb < g.k_blocks; ++kb, ++it) {
+                        uint8_t* st = arrive();
+                        if (!ok) break;
+                        three(d, st, w_bytes, idesc, kb == 0);
+                        umma_commit(&empty[it % g.stages]);
+                    }
+                    if (PERT && ok) {
+                        if (c == c0 && !mbar_wait(&tready, unit_no & 1, abort_flag, g.status, 4)) { ok = false; break; }
+                        tc_fence_after();
+                        const uint32_t abytes = (uint32_t)g.kb * g.bn * 2;   // one part of an image block
+                        for (int i = 0; i < nd * nkb; ++i, ++it) {
+                            uint8_t* st = arrive();
+                            if (!ok) break;
+                            const int dd = i / nkb, kblk = i - dd * nkb;
+                            for (int ks = 0; ks < g.kb / 16; ++ks) {
+                                const int col8 = (dd * g.r16 + kblk * g.kb + ks * 16) >> 3;
+                                uint64_t dt[3], da[3];
+#pragma unroll
+                                for (int part = 0; part < 3; ++part) {
+                                    dt[part] = make_plain_desc(tpp + part * part_bytes + col8 * (PK_TILE * 16), PK_TILE * 16);
+                                    da[part] = make_plain_desc(st + part * abytes + ks * 2 * g.bn * 16, g.bn * 16);
+                                }
+                                umma_f16(d, dt[2], da[0], idesc_u, 1);
+                                umma_f16(d, dt[0], da[2], idesc_u, 1);
+                                umma_f16(d, dt[1], da[1], idesc_u, 1);
+                                umma_f16(d, dt[1], da[0], idesc_u, 1);
+                                umma_f16(d, dt[0], da[1], idesc_u, 1);
+                                umma_f16(d, dt[0], da[0], idesc_u, 1);
+                            }
+                            umma_commit(&empty[it % g.stages]);
+                        }
+                    }
+                    if (ok) umma_commit(&tfull[b]);
+                }
+            }
+        }
+    } else {
+        // ------------------------------------------------------------------------- epilogue
+        const int q4 = warp & 3, eh = (warp - 2) >> 2;      // TMEM quadrant, column half
+        const uint32_t lane_base = tmem + ((uint32_t)(q4 * 32) << 16);
+        const float gain = g.out_scale_ptr ? *g.out_scale_ptr : g.out_scale;
+        const bool wide = (reinterpret_cast<uintptr_t>(g.out) & 31) == 0 && (g.out_stride & 7) == 0 && (g.a & 7) == 0 &&
+                          (!g.pot || (reinterpret_cast<uintptr_t>(g.pot) & 31) == 0);
+        float* my_tr = tr + (warp - 2) * 32 * PK_TR_PITCH;
+        uint32_t acc_it = 0, unit_no = 0;
+        bool ok = true;
+        for (int64_t u = blockIdx.x; u < units && ok; u += gridDim.x, ++unit_no) {
+            const int64_t mt = u / g.groups;
+            const int grp = (int)(u - mt * g.groups);
+            const int c0 = g.n_chunks * grp / g.groups, c1 = g.n_chunks * (grp + 1) / g.groups;
+            const int64_t p = mt * PK_TILE + q4 * 32 + lane;
+            int64_t R;
+            bool odd;
+            const bool valid = map_row(g.map, p, R, odd);
+            const float rs = !valid ? 0.0f : g.row_scale ? g.row_scale[p] : 1.0f;
+            if (PERT) {
+                if (!mbar_wait(&tacc, unit_no & 1, abort_flag, g.status, 5)) { ok = false; break; }
+                tc_fence_after();
+                const int64_t p0 = (mt * 4) / g.rb;
+                const int d = (int)((mt * 4 + q4) / (int64_t)g.rb - p0);
+                for (int c8 = eh; c8 < g.nt / 8; c8 += 2) {
+                    uint32_t w[3][4];
+                    if (c8 * 8 >= d * g.r16 && c8 * 8 < (d + 1) * g.r16) {     // the columns of this slice's pair
+                        uint32_t acc[8];
+                        tmem_ld8(lane_base + 256 + c8 * 8, acc);
+#pragma unroll
+                        for (int j = 0; j < 8; j += 2) {
+                            float v0 = __uint_as_float(acc[j]), v1 = __uint_as_float(acc[j + 1]);
+                            if (odd) v0 = -v0, v1 = -v1;        // the odd member of a pair has A negated
+#pragma unroll
+                            for (int part = 0; part < 3; ++part) {
+                                const __nv_bfloat162 b = __floats2bfloat162_rn(v0, v1);
+                                w[part][j >> 1] = *reinterpret_cast<const uint32_t*>(&b);
+                                v0 -= __bfloat162float(b.x);
+                                v1 -= __bfloat162float(b.y);
+                            }
+                        }
+                    } else {
+#pragma unroll
+                        for (int part = 0; part < 3; ++part) w[part][0] = w[part][1] = w[part][2] = w[part][3] = 0u;
+                    }
+#pragma unroll
+                    for (int part = 0; part < 3; ++part)
+                        *reinterpret_cast<uint4*>(tpp + part * part_bytes + c8 * (PK_TILE * 16) + (q4 * 32 + lane) * 16) =
+                            make_uint4(w[part][0], w[part][1], w[part][2], w[part][3]);
+                }
+                fence_proxy_async();
+                tc_fence_before();
+                mbar_arrive(&tready);
+            }
+            for (int c = c0; c < c1 && ok; ++c, ++acc_it) {
+                const int b = acc_it & 1;
+                if (!mbar_wait(&tfull[b], (acc_it >> 1) & 1, abort_flag, g.status, 6)) { ok = false; break; }
+                tc_fence_after();
+                for (int cb = eh * 16; cb < g.bn; cb += 32) {
+                    const int n0 = c * g.bn + cb;
+                    if (n0 >= g.a) break;
+                    uint32_t acc[16];
+                    tmem_ld8_issue(lane_base + b * 128 + cb, *reinterpret_cast<uint32_t(*)[8]>(acc));
+                    tmem_ld8_issue(lane_base + b * 128 + cb + 8, *reinterpret_cast<uint32_t(*)[8]>(acc + 8));
+                    float cs[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) cs[j] = n0 + j < g.a ? __ldg(g.col_scale + n0 + j) : 0.0f;
+                    tmem_ld_wait();
+                    float v[16];     // the charge of a LIF step, or the scaled output
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        v[j] = __fmul_rn(__fmul_rn(__fmul_rn(__uint_as_float(acc[j]), rs), cs[j]), g.lif ? g.leak : gain);
+                    if (wide) {
+                        if (valid) {
+                            float* o = g.out + (size_t)R * g.out_stride + n0;
+                            float* q = g.pot ? g.pot + (size_t)R * g.out_stride + n0 : nullptr;
+#pragma unroll
+                            for (int h = 0; h < 16; h += 8) {
+                                if (n0 + h >= g.a) break;
+                                float s[8];
+#pragma unroll
+                                for (int j = 0; j < 8; ++j) s[j] = g.lif ? (v[h + j] >= g.v_th ? 1.0f : 0.0f) : v[h + j];
+                                if (q) {
+                                    *reinterpret_cast<float4*>(q + h) = make_float4(v[h], v[h + 1], v[h + 2], v[h + 3]);
+                                    *reinterpret_cast<float4*>(q + h + 4) = make_float4(v[h + 4], v[h + 5], v[h + 6], v[h + 7]);
+                                }
+                                asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o + h), "f"(s[0]),
+                                             "f"(s[1]), "f"(s[2]), "f"(s[3]), "f"(s[4]), "f"(s[5]), "f"(s[6]), "f"(s[7])
+                                             : "memory");
+                            }
+                        }
+                    } else if (g.staged_stores) {
+                        // rows that start anywhere: through shared memory, so that sixteen lanes write sixteen
+                        // neighbouring values of a row
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) my_tr[lane * PK_TR_PITCH + j] = v[j];
+                        __syncwarp();
+                        const int col = lane & 15;
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const int row = 2 * i + (lane >> 4);
+                            const int64_t Rr = __shfl_sync(0xffffffffu, R, row);
+                            const bool vr = __shfl_sync(0xffffffffu, (int)valid, row) != 0;
+                            const float x = my_tr[row * PK_TR_PITCH + col];
+                            if (vr && n0 + col < g.a) {
+                                const size_t o = (size_t)Rr * g.out_stride + n0 + col;
+                                if (g.pot) g.pot[o] = x;
+                                g.out[o] = g.lif ? (x >= g.v_th ? 1.0f : 0.0f) : x;
+                            }
+                        }
+                        __syncwarp();
+                    } else if (valid) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            if (n0 + j < g.a) {
+                                const size_t o = (size_t)R * g.out_stride + n0 + j;
+                                if (g.pot) g.pot[o] = v[j];
+                                g.out[o] = g.lif ? (v[j] >= g.v_th ? 1.0f : 0.0f) : v[j];
+                            }
+                    }
+                }
+                tc_fence_before();
+                mbar_arrive(&tempty[b]);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(PERT ? 512 : 256) : "memory");
+    }
+}
+
+// ------------------------------------------------------------------------------ host side
+struct PackPlan {
+    bool ok;
+    int rp, rb, r16, nt, kb, kp, bn, n_chunks, groups;
+    int64_t pairs, rows, m_tiles;
+    int stages, stage_bytes, staged, smem;
+    size_t o_xhi, o_xlo, o_whi, o_wlo, o_rs, o_cs, o_bhi, o_blo, o_aimg, o_flag, bytes;
+};
+
+PackPlan plan_pack(const hses_linear_args& g) {
+    PackPlan p{};
+    const int64_t rows_nat = (int64_t)g.t_steps * g.n_pop * g.bm;
+    p.kp = (g.k + 7) & ~7;
+    p.n_chunks = (g.a + 127) / 128;
+    p.bn = ((g.a + p.n_chunks - 1) / p.n_chunks + 15) & ~15;
+    p.n_chunks = (g.a + p.bn - 1) / p.bn;
+    p.rows = rows_nat;
+    p.rb = 1;
+    if (g.perturb) {
+        if (g.rank > 128) return p;
+        const int64_t R = (int64_t)2 * g.bm * g.t_steps;
+        p.r16 = g.rank <= 64 ? (g.rank + 15) & ~15 : 128;
+        // a tile holds the t columns of all its pairs, at most 128 of them
+        const int gran = p.r16 <= 32 ? 32 : p.r16 <= 64 ? 64 : 128;
+        const int64_t rp = (R + gran - 1) / gran * gran;
+        if (rp > (1 << 30)) return p;
+        p.rp = (int)rp;
+        p.rb = p.rp / 32;
+        const int nd = p.rp == 32 ? 4 : p.rp % 128 == 0 ? 1 : 2;
+        p.nt = nd * p.r16;
+        p.kb = std::min(p.r16, 64);
+        p.pairs = ((int64_t)g.first_thread + g.n_pop - 1) / 2 - g.first_thread / 2 + 1;
+        p.rows = p.pairs * p.rp;
+    }
+    if (p.rows >= (1ll << 31) - 256) return p;
+    p.m_tiles = (p.rows + PK_TILE - 1) / PK_TILE;
+    // work units: an m-tile's chunks in 1 .. n_chunks groups, the number that makes the last wave cheapest (a
+    // group repeats the tile's t product)
+    const int sms = plan_sm_count();
+    int64_t best = 0;
+    for (int gr = 1; gr <= p.n_chunks; ++gr) {
+        const int64_t waves = (p.m_tiles * gr + sms - 1) / sms;
+        const int64_t cost = waves * ((int64_t)((p.n_chunks + gr - 1) / gr) * (p.bn + 32) + p.nt);
+        if (gr == 1 || cost < best) {
+            best = cost;
+            p.groups = gr;
+        }
+    }
+    p.stage_bytes = 2 * PK_TILE * PK_BK * 2 + 2 * std::max(p.bn, p.nt) * PK_BK * 2;
+    const int fixed = 1024 + 3 * p.nt * PK_TILE * 2;
+    p.staged = PK_SMEM_LIMIT - 1024 - fixed - PK_TR_BYTES >= 2 * p.stage_bytes;
+    const int room = PK_SMEM_LIMIT - 1024 - fixed - (p.staged ? PK_TR_BYTES : 0);   // 1024: static shared memory
+    p.stages = std::min(PK_MAX_STAGES, room / p.stage_bytes);
+    if (p.stages < 2) return p;
+    p.smem = fixed + (p.staged ? PK_TR_BYTES : 0) + p.stages * p.stage_bytes;
+    size_t o = 0;
+    auto take = [&](size_t bytes) {
+        const size_t at = o;
+        o += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    const size_t nx = (size_t)p.rows * p.kp * 2, nw = (size_t)g.a * p.kp * 2;
+    p.o_xhi = take(nx);
+    p.o_xlo = take(nx);
+    p.o_whi = take(nw);
+    p.o_wlo = take(nw);
+    p.o_rs = take((size_t)p.rows * 4);
+    p.o_cs = take((size_t)g.a * 4);
+    p.o_flag = take(4);
+    if (g.perturb) {
+        const size_t nb = (size_t)p.pairs * p.r16 * p.kp * 2;
+        p.o_bhi = take(nb);
+        p.o_blo = take(nb);
+        p.o_aimg = take((size_t)p.pairs * p.n_chunks * p.r16 * 3 * p.bn * 2);
+    }
+    p.bytes = o + 256;   // the base is rounded up to 256 bytes
+    p.ok = p.bytes <= (24ull << 30);
+    return p;
+}
+
+int encode_rows(CUtensorMap* map, const void* base, int64_t rows, int cols, int box_rows) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) {
+        set_error("cuTensorMapEncodeTiled is not available from the driver");
+        return HSES_ERR_CUDA;
+    }
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+    cuuint32_t box[2] = {(cuuint32_t)PK_BK, (cuuint32_t)box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        set_error("cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
+        return HSES_ERR_CUDA;
+    }
+    return HSES_OK;
+}
+
+int vec_ok(const void* p, int64_t stride) { return ((uintptr_t)p & 15u) == 0 && stride % 4 == 0; }
+
+}  // namespace
+
+bool pack_path_supports(const hses_linear_args& g) {
+    if (g.n_groups > 1 || g.x_op != HSES_X_NONE || g.lif == 2) return false;
+    return plan_pack(g).ok;
+}
+
+size_t pack_path_workspace_bytes(const hses_linear_args& g) { return plan_pack(g).bytes; }
+
+int run_pack_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
+    const PackPlan p = plan_pack(g);
+    HSES_REQUIRE(g.workspace != nullptr && g.workspace_bytes >= p.bytes,
+                 "workspace too small; see hses_perturbed_linear_workspace_bytes");
+    uint8_t* ws = reinterpret_cast<uint8_t*>(((uintptr_t)g.workspace + 255) & ~(uintptr_t)255);
+    auto half_at = [&](size_t o) { return reinterpret_cast<__half*>(ws + o); };
+    int* flag = reinterpret_cast<int*>(ws + p.o_flag);
+    float* cs = reinterpret_cast<float*>(ws + p.o_cs);
+
+    RowMap map{};
+    map.packed = g.perturb ? 1 : 0;
+    map.rp = p.rp;
+    map.t_steps = g.t_steps;
+    map.bm = g.bm;
+    map.n_pop = g.n_pop;
+    map.first_thread = g.first_thread;
+    map.first_pair = g.first_thread / 2;
+    map.rows = p.rows;
+    RowMap plain{};
+    plain.rows = g.a;
+
+    const SplitJob jw{g.param, g.param_row_stride, g.a, g.k, p.kp, vec_ok(g.param, g.param_row_stride),
+                      half_at(p.o_whi), half_at(p.o_wlo), cs, nullptr};
+    SplitJob jx{g.x, g.x_row_stride, p.rows, g.k, p.kp, vec_ok(g.x, g.x_row_stride),
+                half_at(p.o_xhi), half_at(p.o_xlo), reinterpret_cast<float*>(ws + p.o_rs), flag};
+    // a caller-provided fp16 copy of an x that is exact in fp16 is the operand as it stands
+    const bool x_ready = !g.perturb && g.x_half != nullptr && ((uintptr_t)g.x_half & 15u) == 0 && p.kp == g.k;
+    HSES_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
+
+    FactorJob f{};
+    int segs = 0;
+    if (g.perturb) {
+        if (g.cache) {
+            int rc = resolve_factor_cache(g, &f.cache_a, &f.cache_b);
+            if (rc != HSES_OK) return rc;
+        }
+        f.pow2 = ctx->t.jump_pow2;
+        f.lane_tab = ctx->t.jump_lane4;
+        f.cal = ctx->cal();
+        f.key = g.key;
+        f.true_epoch = true_epoch_of(g.epoch, g.noise_reuse);
+        f.first_pair = map.first_pair;
+        f.pairs = p.pairs;
+        f.r = g.rank;
+        f.r16 = p.r16;
+        f.k = g.k;
+        f.kp = p.kp;
+        f.a = g.a;
+        f.row_a0 = g.factor_order == 1 ? 0 : g.k;
+        f.row_b0 = g.factor_order == 1 ? g.a : 0;
+        const int seg = std::max(8, std::min(512, PK_SEG / g.rank & ~7));
+        f.seg_a = f.seg_b = seg;
+        f.bn = p.bn;
+        f.n_chunks = p.n_chunks;
+        f.kb = p.kb;
+        f.base_sigma = g.sigma / sqrtf((float)g.rank);
+        f.col_scale = cs;
+        f.bhi = half_at(p.o_bhi);
+        f.blo = half_at(p.o_blo);
+        f.aimg = reinterpret_cast<__nv_bfloat16*>(ws + p.o_aimg);
+        segs = (g.k + seg - 1) / seg + (g.a + seg - 1) / seg;
+    }
+    auto prepare = [&](auto nj_c, auto rpw_c) -> int {
+        constexpr int NJ = decltype(nj_c)::value, RPW = decltype(rpw_c)::value;
+        {
+            HSES_KERNEL(ctx, st, "pack_split_w");
+            pack_split_kernel<NJ, RPW><<<(unsigned)((g.a + 8 * RPW - 1) / (8 * RPW)), 256, 0, st>>>(jw, plain);
+            HSES_LAUNCH_CHECK();
+        }
+        const int64_t xb = x_ready ? 0 : (p.rows + 8 * RPW - 1) / (8 * RPW), fb = p.pairs * segs;
+        HSES_REQUIRE(xb + fb < (1ll << 31), "too many rows");
+        if (g.perturb) {
+            HSES_KERNEL(ctx, st, "pack_operands");
+            pack_operands_kernel<NJ, RPW><<<(unsigned)(xb + fb), 256, 0, st>>>(jx, map, xb, segs, f);
+            HSES_LAUNCH_CHECK();
+        } else if (xb) {
+            HSES_KERNEL(ctx, st, "pack_split_x");
+            pack_split_kernel<NJ, RPW><<<(unsigned)xb, 256, 0, st>>>(jx, map);
+            HSES_LAUNCH_CHECK();
+        }
+        return HSES_OK;
+    };
+    using std::integral_constant;
+    // pieces of 128 values per row and rows in flight per warp: as many as the registers hold
+    int rc = p.kp <= 128    ? prepare(integral_constant<int, 1>{}, integral_constant<int, 8>{})
+             : p.kp <= 256  ? prepare(integral_constant<int, 2>{}, integral_constant<int, 4>{})
+             : p.kp <= 1024 ? prepare(integral_constant<int, 8>{}, integral_constant<int, 2>{})
+                            : prepare(integral_constant<int, 0>{}, integral_constant<int, 1>{});
+    if (rc != HSES_OK) return rc;
+
+    PackArgs a{};
+    a.map = map;
+    a.m_tiles = p.m_tiles;
+    a.groups = p.groups;
+    a.n_chunks = p.n_chunks;
+    a.bn = p.bn;
+    a.a = g.a;
+    a.k_blocks = (g.k + PK_BK - 1) / PK_BK;
+    a.nt = p.nt;
+    a.r16 = p.r16;
+    a.kb = p.kb;
+    a.rb = p.rb;
+    a.pairs = p.pairs;
+    a.aimg = f.aimg;
+    a.row_scale = x_ready ? nullptr : jx.inv_scale;
+    a.col_scale = cs;
+    a.x_lo_flag = flag;
+    a.lif = g.lif;
+    a.leak = g.lif ? 1.0f / g.tau_m : 0.0f;
+    a.v_th = g.v_th;
+    a.out_scale = g.out_scale;
+    a.out_scale_ptr = g.out_scale_ptr;
+    a.out = g.out;
+    a.out_stride = g.out_row_stride;
+    a.pot = g.lif ? g.potentials : nullptr;
+    a.stages = p.stages;
+    a.stage_bytes = p.stage_bytes;
+    a.staged_stores = p.staged;
+    a.status = ctx->t.status_word;
+    CUtensorMap mx, mxl, mw, mwl, mb, mbl;
+    const void* xhi = x_ready ? g.x_half : static_cast<const void*>(jx.hi);
+    rc = encode_rows(&mx, xhi, p.rows, p.kp, PK_TILE);
+    if (rc == HSES_OK) rc = encode_rows(&mxl, x_ready ? g.x_half : static_cast<const void*>(jx.lo), p.rows, p.kp, PK_TILE);
+    if (rc == HSES_OK) rc = encode_rows(&mw, jw.hi, g.a, p.kp, p.bn);
+    if (rc == HSES_OK) rc = encode_rows(&mwl, jw.lo, g.a, p.kp, p.bn);
+    mb = mw;
+    mbl = mwl;
+    if (rc == HSES_OK && g.perturb) rc = encode_rows(&mb, f.bhi, p.pairs * p.r16, p.kp, p.nt);
+    if (rc == HSES_OK && g.perturb) rc = encode_rows(&mbl, f.blo, p.pairs * p.r16, p.kp, p.nt);
+    if (rc != HSES_OK) return rc;
+    const int64_t units = p.m_tiles * p.groups;
+    const unsigned grid = (unsigned)std::min<int64_t>(units, ctx->sm_count);
+    HSES_KERNEL(ctx, st, "linear_pack");
+    if (g.perturb) {
+        HSES_CUDA(cudaFuncSetAttribute(linear_pack_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem));
+        linear_pack_kernel<true><<<grid, PK_THREADS, p.smem, st>>>(mx, mxl, mw, mwl, mb, mbl, a);
+    } else {
+        HSES_CUDA(cudaFuncSetAttribute(linear_pack_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem));
+        linear_pack_kernel<false><<<grid, PK_THREADS, p.smem, st>>>(mx, mxl, mw, mwl, mb, mbl, a);
+    }
+    HSES_LAUNCH_CHECK();
+    return HSES_OK;
+}
+
+}  // namespace hses

@@ -175,6 +175,17 @@ HSES_HD uint64_t jump_by(const uint64_t* __restrict__ tabs, uint64_t x, uint64_t
     return x;
 }
 
+// The 32 lanes of a warp from one common state to 32 equally spaced positions: the table holds, for every nibble
+// value of the common state, the images for all lanes side by side (16 x 16 x 32 words), so that one round of
+// coalesced reads does what up to log2(distance) dependent table lookups per lane would.
+constexpr int kLaneWords = 16 * 16 * 32;
+HSES_HD uint64_t lane_jump(const uint64_t* __restrict__ tab, uint64_t x, int lane) {
+    uint64_t r = 0;
+#pragma unroll
+    for (int p = 0; p < 16; ++p) r ^= tab[(p * 16 + (int)((x >> (4 * p)) & 15)) * 32 + lane];
+    return r;
+}
+
 // ---------------------------------------------------------------------------
 // libm-conformant logf / cosf on the 24-bit uniforms
 // ---------------------------------------------------------------------------
