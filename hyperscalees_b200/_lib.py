@@ -31,6 +31,7 @@ EXPORTS = [
     "hses_factor_cache_bytes", "hses_factor_cache_build", "hses_es_update_ex",
     "hses_population_grads_elems", "hses_population_grads", "hses_population_apply",
     "hses_convert_fitnesses_bs", "hses_vector_mul",
+    "hses_es_update_multi_workspace_bytes", "hses_es_update_multi", "hses_solver_step_multi",
     "hses_prng_normal_half", "hses_einsum_pair_workspace_bytes", "hses_einsum_pair", "hses_layer_norm", "hses_group_norm", "hses_token_shift_mix", "hses_relu_square", "hses_rate_encode",
     "hses_rwkv_mix_prepare", "hses_rwkv_mix_finish", "hses_token_shift_mix_multi",
     "hses_embedding", "hses_lif_rate", "hses_swish", "hses_add_inplace", "hses_token_fitness",
@@ -52,6 +53,11 @@ class UpdateArgs(C.Structure):
                 ("fitness", C.c_void_p), ("grad", C.c_void_p), ("workspace", C.c_void_p),
                 ("workspace_bytes", C.c_size_t), ("cache", C.POINTER(FactorCacheDesc)),
                 ("mode", C.c_int32), ("sign_factors", C.c_int32), ("algo", C.c_int32)]
+
+
+class UpdateItem(C.Structure):
+    _fields_ = [("key", C.c_uint64), ("a", C.c_int32), ("b", C.c_int32), ("grad", C.c_void_p),
+                ("cache", C.POINTER(FactorCacheDesc))]
 
 
 class LinearArgs(C.Structure):
@@ -155,6 +161,10 @@ def load():
     L.hses_es_update_static.argtypes = [vp, vp, u64, i32, i32, i32, i64, i64, i32, i32, i32, f32, vp, vp]
     L.hses_es_update_dense.argtypes = [vp, vp, u64, i32, i32, i32, i64, i64, i32, f32, vp, vp]
     L.hses_solver_step.argtypes = [vp, vp, C.POINTER(SolverDesc), i32, f32, vp, vp, vp, vp, i64]
+    L.hses_es_update_multi_workspace_bytes.restype = sz
+    L.hses_es_update_multi_workspace_bytes.argtypes = [C.POINTER(UpdateItem), i32, i32, i64]
+    L.hses_es_update_multi.argtypes = [vp, vp, C.POINTER(UpdateItem), i32, i32, i32, i32, i64, i64, i32, f32, i32, vp, vp, sz]
+    L.hses_solver_step_multi.argtypes = [vp, vp, C.POINTER(SolverDesc), i32, f32, i32, vp, vp, vp, vp, vp, vp]
     pm, pp = C.POINTER(SnnModelDesc), C.POINTER(PopArgs)
     L.hses_snn_forward_workspace_bytes.restype = sz
     L.hses_snn_forward_workspace_bytes.argtypes = [pm, pp]

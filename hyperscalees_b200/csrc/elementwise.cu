@@ -234,7 +234,7 @@ __global__ void zscore_kernel(const float* __restrict__ raw, int64_t n, int grou
 // ---------------------------------------------------------------------------
 // solver (noiser.rs:155-224)
 // ---------------------------------------------------------------------------
-constexpr int kSolverMulti = 12;
+constexpr int kSolverMulti = 48;
 struct SolverConsts {
     int kind;
     float lr, beta1, beta2, eps, wd;
@@ -301,21 +301,22 @@ __global__ void solver_kernel(SolverConsts c, float* __restrict__ p, const float
 // in tensor order.
 struct SolverMulti {
     int n;
-    float* p[kSolverMulti];
+    const float* src[kSolverMulti];   // parameters as they are
+    float* p[kSolverMulti];           // and as they become (may be the same tensor)
     float* m[kSolverMulti];
     float* v[kSolverMulti];
+    const float* g[kSolverMulti];
     int64_t len[kSolverMulti];
-    int64_t goff[kSolverMulti];
     int first_block[kSolverMulti + 1];
 };
-__global__ void solver_multi_kernel(SolverConsts c, SolverMulti d, const float* __restrict__ grads) {
+__global__ void solver_multi_kernel(SolverConsts c, const __grid_constant__ SolverMulti d) {
     int t = 0;
     while (t + 1 < d.n && (int)blockIdx.x >= d.first_block[t + 1]) ++t;
     const int64_t i = (int64_t)(blockIdx.x - d.first_block[t]) * blockDim.x + threadIdx.x;
     if (i >= d.len[t] || d.p[t] == nullptr) return;
     const bool adam = c.kind != HSES_SGD;
-    float mi = adam ? d.m[t][i] : 0.0f, vi = adam ? d.v[t][i] : 0.0f, pi = d.p[t][i];
-    solver_one(c, pi, grads[d.goff[t] + i], mi, vi);
+    float mi = adam ? d.m[t][i] : 0.0f, vi = adam ? d.v[t][i] : 0.0f, pi = d.src[t][i];
+    solver_one(c, pi, d.g[t][i], mi, vi);
     d.p[t][i] = pi;
     if (adam) {
         d.m[t][i] = mi;
@@ -590,19 +591,19 @@ int hses_vector_mul(hses_ctx* ctx, hses_stream stream, const float* a, const flo
 }  // extern "C"
 
 namespace hses {
-// One solver step over several parameter tensors whose gradients sit back to back in `grads`
-// (tensors with a NULL parameter pointer are skipped but still take their place in `grads`).
-int solver_step_multi(hses_ctx* ctx, cudaStream_t st, const hses_solver* solver, int32_t step, int n_tensors,
-                      float* const* params, float* const* m_bufs, float* const* v_bufs, const int64_t* lens,
-                      const float* grads) {
+// One solver step over several parameter tensors (tensors with a NULL parameter pointer are skipped).
+int solver_step_multi(hses_ctx* ctx, cudaStream_t st, const hses_solver* solver, int32_t step, float grad_scale, int n_tensors,
+                      const float* const* src, float* const* params, float* const* m_bufs, float* const* v_bufs,
+                      const int64_t* lens, const float* const* grads) {
     HSES_REQUIRE(solver->kind == HSES_SGD || solver->kind == HSES_ADAM || solver->kind == HSES_ADAMW,
                  "unknown solver kind");
     const bool moments = solver->kind != HSES_SGD;
     HSES_REQUIRE(!moments || step >= 1, "step is the counter after the increment (>= 1)");
+    HSES_REQUIRE(!moments || (m_bufs != nullptr && v_bufs != nullptr), "Adam needs moment buffers");
     SolverConsts c{};
     c.kind = solver->kind;
     c.lr = solver->lr;
-    c.grad_scale = 1.0f;
+    c.grad_scale = grad_scale;
     if (moments) {
         float t = (float)step;
         c.beta1 = solver->beta1;
@@ -614,26 +615,28 @@ int solver_step_multi(hses_ctx* ctx, cudaStream_t st, const hses_solver* solver,
         c.ibc1 = 1.0f / (1.0f - powf(solver->beta1, t));
         c.ibc2 = 1.0f / (1.0f - powf(solver->beta2, t));
     }
-    int64_t goff = 0;
     for (int t0 = 0; t0 < n_tensors; t0 += kSolverMulti) {
         SolverMulti d{};
         d.n = n_tensors - t0 < kSolverMulti ? n_tensors - t0 : kSolverMulti;
-        int blocks = 0;
+        int64_t blocks = 0;
         for (int t = 0; t < d.n; ++t) {
             d.p[t] = params[t0 + t];
+            d.src[t] = src ? src[t0 + t] : d.p[t];
             d.m[t] = moments ? m_bufs[t0 + t] : nullptr;
             d.v[t] = moments ? v_bufs[t0 + t] : nullptr;
-            HSES_REQUIRE(d.p[t] == nullptr || !moments || (d.m[t] != nullptr && d.v[t] != nullptr), "Adam needs moment buffers");
+            d.g[t] = grads[t0 + t];
             d.len[t] = lens[t0 + t];
-            d.goff[t] = goff;
-            goff += lens[t0 + t];
-            d.first_block[t] = blocks;
-            blocks += (int)((lens[t0 + t] + 255) / 256);
+            HSES_REQUIRE(d.len[t] >= 0, "len must be >= 0");
+            HSES_REQUIRE(d.p[t] == nullptr || (d.src[t] != nullptr && d.g[t] != nullptr), "NULL pointer");
+            HSES_REQUIRE(d.p[t] == nullptr || !moments || (d.m[t] != nullptr && d.v[t] != nullptr), "Adam needs moment buffers");
+            d.first_block[t] = (int)blocks;
+            blocks += (d.len[t] + 255) / 256;
         }
-        d.first_block[d.n] = blocks;
+        HSES_REQUIRE(blocks < (1ll << 31), "too many parameters for one launch");
+        d.first_block[d.n] = (int)blocks;
         if (blocks == 0) continue;
         HSES_KERNEL(ctx, st, "solver");
-        solver_multi_kernel<<<(unsigned)blocks, 256, 0, st>>>(c, d, grads);
+        solver_multi_kernel<<<(unsigned)blocks, 256, 0, st>>>(c, d);
         HSES_LAUNCH_CHECK();
     }
     return HSES_OK;
@@ -641,6 +644,14 @@ int solver_step_multi(hses_ctx* ctx, cudaStream_t st, const hses_solver* solver,
 }  // namespace hses
 
 extern "C" {
+
+int hses_solver_step_multi(hses_ctx* ctx, hses_stream stream, const hses_solver* solver, int32_t step, float grad_scale,
+                           int32_t n, const float* const* src, float* const* params, const float* const* grads,
+                           float* const* m, float* const* v, const int64_t* lens) {
+    HSES_REQUIRE(ctx != nullptr, "ctx is NULL");
+    HSES_REQUIRE(solver != nullptr && n >= 0 && params != nullptr && grads != nullptr && lens != nullptr, "NULL pointer");
+    return solver_step_multi(ctx, as_stream(stream), solver, step, grad_scale, n, src, params, m, v, lens, grads);
+}
 
 int hses_solver_step(hses_ctx* ctx, hses_stream stream, const hses_solver* solver, int32_t step,
                      float grad_scale, float* param, const float* grad, float* m, float* v,

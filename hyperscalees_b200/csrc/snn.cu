@@ -249,14 +249,26 @@ int hses_population_eval(hses_ctx* ctx, hses_stream stream, const hses_snn_model
     return hses_member_mean(ctx, stream, per_sample, p->n_pop, p->bm, raw_fitness);
 }
 
+// fitness | gradients of every parameter | scratch of the update
+static size_t grads_elems(const hses_snn_model* m) {
+    size_t n = 1;  // out_gain
+    for (int l = 0; l < m->n_layers; ++l) n += (size_t)m->dims[l + 1] * m->dims[l];
+    return n;
+}
+static std::vector<hses_update_item> update_items(const hses_snn_model* m, float* grads) {
+    std::vector<hses_update_item> items((size_t)m->n_layers);
+    for (int l = 0; l < m->n_layers; ++l) {
+        items[l] = hses_update_item{m->keys ? m->keys[l] : 0, m->dims[l + 1], m->dims[l], grads, nullptr};
+        if (grads) grads += (size_t)m->dims[l + 1] * m->dims[l];
+    }
+    return items;
+}
+
 size_t hses_population_update_workspace_bytes(const hses_snn_model* m, int32_t rank, int64_t n_total) {
     if (m == nullptr || m->n_layers < 1 || m->dims == nullptr || n_total < 2) return 0;
-    size_t grad = 0, upd = 0;
-    for (int l = 0; l < m->n_layers; ++l) {
-        grad = std::max(grad, (size_t)m->dims[l + 1] * m->dims[l]);
-        upd = std::max(upd, hses_es_update_workspace_bytes(m->dims[l + 1], m->dims[l], rank, n_total));
-    }
-    return (up64((size_t)n_total) + up64(grad)) * sizeof(float) + up64(upd);
+    const std::vector<hses_update_item> items = update_items(m, nullptr);
+    const size_t upd = hses_es_update_multi_workspace_bytes(items.data(), m->n_layers, rank, n_total);
+    return (up64((size_t)n_total) + up64(grads_elems(m))) * sizeof(float) + up64(upd);
 }
 
 int hses_population_update(hses_ctx* ctx, hses_stream stream, const hses_snn_model* m, float sigma, int32_t rank,
@@ -264,75 +276,22 @@ int hses_population_update(hses_ctx* ctx, hses_stream stream, const hses_snn_mod
                            uint64_t gain_key, const float* raw_fitness, int64_t n_total,
                            const hses_solver* solver, int32_t step, float* const* params, float* const* m_bufs,
                            float* const* v_bufs, void* workspace, size_t workspace_bytes) {
-    HSES_REQUIRE(ctx != nullptr, "ctx is NULL");
-    HSES_REQUIRE(m != nullptr && m->n_layers >= 1 && m->dims != nullptr && m->keys != nullptr, "bad model");
-    HSES_REQUIRE(raw_fitness != nullptr && solver != nullptr && params != nullptr, "NULL pointer");
-    HSES_REQUIRE(n_total >= 2 && n_total % 2 == 0, "the population must consist of whole antithetic pairs");
-    size_t need = hses_population_update_workspace_bytes(m, rank, n_total);
-    HSES_REQUIRE(workspace != nullptr && workspace_bytes >= need && ((uintptr_t)workspace & 255u) == 0,
-                 "workspace too small or not 256-byte aligned; see hses_population_update_workspace_bytes");
-    size_t grad_elems = 0;
-    for (int l = 0; l < m->n_layers; ++l) grad_elems = std::max(grad_elems, (size_t)m->dims[l + 1] * m->dims[l]);
-    float* fit = reinterpret_cast<float*>(workspace);
-    float* grad = fit + up64((size_t)n_total);
-    void* upd_ws = grad + up64(grad_elems);
-    size_t upd_bytes = workspace_bytes - (up64((size_t)n_total) + up64(grad_elems)) * sizeof(float);
-    int rc = hses_convert_fitnesses(ctx, stream, raw_fitness, n_total, group_size, fit, nullptr);
+    HSES_REQUIRE(solver != nullptr && params != nullptr, "NULL pointer");
+    HSES_REQUIRE(m != nullptr && m->n_layers >= 1 && m->dims != nullptr, "bad model");
+    HSES_REQUIRE(solver->kind == HSES_SGD || (m_bufs != nullptr && v_bufs != nullptr), "Adam needs moment buffers");
+    HSES_REQUIRE(n_total >= 2, "the population must consist of whole antithetic pairs");
+    float* grads = reinterpret_cast<float*>(workspace) + up64((size_t)n_total);
+    // a model without an out_gain parameter has no use for its gradient: the frozen form costs nothing
+    int rc = hses_population_grads(ctx, stream, m, sigma, rank, epoch, noise_reuse, group_size,
+                                   freeze_nonlora || params[m->n_layers] == nullptr, gain_key, raw_fitness, n_total, 0,
+                                   n_total, grads, workspace, workspace_bytes);
     if (rc != HSES_OK) return rc;
-    const bool moments = solver->kind != HSES_SGD;
-    HSES_REQUIRE(!moments || (m_bufs != nullptr && v_bufs != nullptr), "Adam needs moment buffers");
-    bool range_valid = false;
-    for (int l = 0; l < m->n_layers; ++l) {
-        int a = m->dims[l + 1], b = m->dims[l];
-        hses_update_args u{};
-        u.key = m->keys[l];
-        u.epoch = epoch;
-        u.noise_reuse = noise_reuse;
-        u.first_thread = 0;
-        u.n = n_total;
-        u.n_total = n_total;
-        u.rank = rank;
-        u.a = a;
-        u.b = b;
-        u.sigma = sigma;
-        u.fitness = fit;
-        u.grad = grad;
-        u.workspace = upd_ws;
-        u.workspace_bytes = upd_bytes;
-        u.mode = HSES_UPDATE_GRAD;
-        const hses_factor_cache* c = m->caches ? m->caches[l] : nullptr;
-        if (c && c->first_pair == 0 && c->n_pairs >= n_total / 2) u.cache = c;
-        // the layers share the fitness vector and the workspace: the pair-weight range that the
-        // first tensor-core layer leaves at the start of the workspace serves the following ones
-        bool took_tc = false;
-        rc = es_update_ex_impl(ctx, stream, &u, range_valid, &took_tc);
-        if (rc != HSES_OK) return rc;
-        range_valid = took_tc;
-        rc = hses_solver_step(ctx, stream, solver, step, 1.0f, params[l], grad, moments ? m_bufs[l] : nullptr,
-                              moments ? v_bufs[l] : nullptr, (int64_t)a * b);
-        if (rc != HSES_OK) return rc;
-    }
-    // out_gain: PARAM-class leaf of shape (1,1), dense noise (eggroll.rs:331-350); frozen -> zero gradient
-    if (params[m->n_layers] != nullptr) {
-        if (freeze_nonlora) {
-            HSES_CUDA(cudaMemsetAsync(grad, 0, sizeof(float), as_stream(stream)));
-        } else {
-            rc = hses_es_update_dense(ctx, stream, gain_key, epoch, noise_reuse, 0, n_total, n_total, 1, sigma, fit,
-                                      grad);
-            if (rc != HSES_OK) return rc;
-        }
-        rc = hses_solver_step(ctx, stream, solver, step, 1.0f, params[m->n_layers], grad,
-                              moments ? m_bufs[m->n_layers] : nullptr, moments ? v_bufs[m->n_layers] : nullptr, 1);
-        if (rc != HSES_OK) return rc;
-    }
-    return HSES_OK;
+    return hses_population_apply(ctx, stream, m, solver, step, params, m_bufs, v_bufs, grads);
 }
 
 size_t hses_population_grads_elems(const hses_snn_model* m) {
     if (m == nullptr || m->n_layers < 1 || m->dims == nullptr) return 0;
-    size_t n = 1;  // out_gain
-    for (int l = 0; l < m->n_layers; ++l) n += (size_t)m->dims[l + 1] * m->dims[l];
-    return n;
+    return grads_elems(m);
 }
 
 int hses_population_grads(hses_ctx* ctx, hses_stream stream, const hses_snn_model* m, float sigma, int32_t rank,
@@ -349,43 +308,23 @@ int hses_population_grads(hses_ctx* ctx, hses_stream stream, const hses_snn_mode
     size_t need = hses_population_update_workspace_bytes(m, rank, n_total);
     HSES_REQUIRE(workspace != nullptr && workspace_bytes >= need && ((uintptr_t)workspace & 255u) == 0,
                  "workspace too small or not 256-byte aligned; see hses_population_update_workspace_bytes");
-    size_t grad_elems = 0;
-    for (int l = 0; l < m->n_layers; ++l) grad_elems = std::max(grad_elems, (size_t)m->dims[l + 1] * m->dims[l]);
     float* fit = reinterpret_cast<float*>(workspace);
-    void* upd_ws = fit + up64((size_t)n_total) + up64(grad_elems);
-    size_t upd_bytes = workspace_bytes - (up64((size_t)n_total) + up64(grad_elems)) * sizeof(float);
+    const size_t head = up64((size_t)n_total) + up64(grads_elems(m));
+    void* upd_ws = fit + head;
+    size_t upd_bytes = workspace_bytes - head * sizeof(float);
     int rc = hses_convert_fitnesses(ctx, stream, raw_fitness, n_total, group_size, fit, nullptr);
     if (rc != HSES_OK) return rc;
-    float* g = grads;
-    bool range_valid = false;
+    std::vector<hses_update_item> items = update_items(m, grads);
     for (int l = 0; l < m->n_layers; ++l) {
-        int a = m->dims[l + 1], b = m->dims[l];
-        hses_update_args u{};
-        u.key = m->keys[l];
-        u.epoch = epoch;
-        u.noise_reuse = noise_reuse;
-        u.first_thread = first_thread;
-        u.n = n_local;
-        u.n_total = n_total;
-        u.rank = rank;
-        u.a = a;
-        u.b = b;
-        u.sigma = sigma;
-        u.fitness = fit + first_thread;
-        u.grad = g;
-        u.workspace = upd_ws;
-        u.workspace_bytes = upd_bytes;
-        u.mode = HSES_UPDATE_GRAD;
         const hses_factor_cache* c = m->caches ? m->caches[l] : nullptr;
         if (c && c->first_pair <= first_thread / 2 &&
             (int64_t)c->first_pair + c->n_pairs >= (int64_t)first_thread / 2 + n_local / 2)
-            u.cache = c;
-        bool took_tc = false;
-        rc = es_update_ex_impl(ctx, stream, &u, range_valid, &took_tc);
-        if (rc != HSES_OK) return rc;
-        range_valid = took_tc;
-        g += (size_t)a * b;
+            items[l].cache = c;
     }
+    rc = hses_es_update_multi(ctx, stream, items.data(), m->n_layers, epoch, noise_reuse, first_thread, n_local, n_total, rank,
+                              sigma, 0, fit + first_thread, upd_ws, upd_bytes);
+    if (rc != HSES_OK) return rc;
+    float* g = grads + grads_elems(m) - 1;
     // out_gain: PARAM-class leaf of shape (1,1), dense noise (eggroll.rs:331-350); frozen -> zero gradient
     if (freeze_nonlora) {
         HSES_CUDA(cudaMemsetAsync(g, 0, sizeof(float), as_stream(stream)));
@@ -407,9 +346,14 @@ int hses_population_apply(hses_ctx* ctx, hses_stream stream, const hses_snn_mode
     HSES_REQUIRE(!moments || (m_bufs != nullptr && v_bufs != nullptr), "Adam needs moment buffers");
     // every leaf in one launch: the step's cost is launches, not arithmetic
     std::vector<int64_t> lens((size_t)m->n_layers + 1);
-    for (int l = 0; l <= m->n_layers; ++l) lens[l] = l < m->n_layers ? (int64_t)m->dims[l + 1] * m->dims[l] : 1;
-    return solver_step_multi(ctx, as_stream(stream), solver, step, m->n_layers + 1, params, m_bufs, v_bufs,
-                             lens.data(), grads);
+    std::vector<const float*> g((size_t)m->n_layers + 1);
+    for (int l = 0; l <= m->n_layers; ++l) {
+        lens[l] = l < m->n_layers ? (int64_t)m->dims[l + 1] * m->dims[l] : 1;
+        g[l] = grads;
+        grads += lens[l];
+    }
+    return solver_step_multi(ctx, as_stream(stream), solver, step, 1.0f, m->n_layers + 1, nullptr, params, m_bufs, v_bufs,
+                             lens.data(), g.data());
 }
 
 }  // extern "C"

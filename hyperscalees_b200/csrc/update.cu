@@ -10,6 +10,7 @@
 // scratch (A pre-multiplied by the pair weight), a split-K fp32 GEMM writes
 // per-split partial sums, and a final pass adds the partials in a fixed order
 // so that every rank ends up with bit-identical gradients.
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -306,18 +307,28 @@ size_t hses_es_update_workspace_bytes(int32_t a, int32_t b, int32_t rank, int64_
         size_t tc = plan_update_tc(a, b, rank, n, true).bytes;
         if (tc > bytes) bytes = tc;
     }
-    return bytes;
+    const size_t multi = update_multi_workspace_bytes(&a, &b, 1, rank, n);
+    return multi > bytes ? multi : bytes;
 }
 
 int hses_es_update_ex(hses_ctx* ctx, hses_stream stream, const hses_update_args* args) {
-    return es_update_ex_impl(ctx, stream, args, false, nullptr);
+    return es_update_ex_impl(ctx, stream, args, false);
 }
 
 }  // extern "C"
 
-int hses::es_update_ex_impl(hses_ctx* ctx, hses_stream stream, const hses_update_args* args, bool reuse_range,
-                            bool* took_tc) {
-    if (took_tc) *took_tc = false;
+int hses::resolve_update_cache(const hses_factor_cache& c, uint64_t key, int32_t true_epoch, int rank, int a, int b,
+                               int32_t first_pair, int64_t pairs, const float** cache_a, const float** cache_b) {
+    HSES_REQUIRE(c.data != nullptr && c.key == key && c.true_epoch == true_epoch && c.rank == rank && c.a == a && c.b == b,
+                 "factor cache was built for another parameter, epoch bucket or shape");
+    HSES_REQUIRE(first_pair >= c.first_pair && first_pair + pairs <= c.first_pair + c.n_pairs,
+                 "factor cache does not cover these members");
+    *cache_a = c.data + (size_t)(first_pair - c.first_pair) * a * rank;
+    *cache_b = c.data + (size_t)c.n_pairs * a * rank + (size_t)(first_pair - c.first_pair) * b * rank;
+    return HSES_OK;
+}
+
+int hses::es_update_ex_impl(hses_ctx* ctx, hses_stream stream, const hses_update_args* args, bool reuse_range) {
     HSES_REQUIRE(ctx != nullptr, "ctx is NULL");
     HSES_REQUIRE(args != nullptr, "args is NULL");
     const hses_update_args& u = *args;
@@ -341,8 +352,21 @@ int hses::es_update_ex_impl(hses_ctx* ctx, hses_stream stream, const hses_update
         // wide factors on tile-aligned shapes: the contraction runs on the tensor cores
         float nf = (float)u.n_total;
         float sc = u.mode == HSES_UPDATE_GRAD ? -(base_sigma_tc * (1.0f / nf)) * sqrtf(nf) : base_sigma_tc;
-        if (took_tc) *took_tc = true;
         return run_update_tc(ctx, st, u, sc, reuse_range);
+    }
+    if (u.algo == HSES_ALGO_AUTO && a <= (1 << 20) && b <= (1 << 20)) {
+        const float nf = (float)u.n_total;
+        UpdateMultiItem item{u.key, a, b, nullptr, nullptr, u.grad};
+        if (u.cache) {
+            int rc = resolve_update_cache(*u.cache, u.key, true_epoch_of(u.epoch, u.noise_reuse), rank, a, b, u.first_thread / 2,
+                                          u.n / 2, &item.cache_a, &item.cache_b);
+            if (rc != HSES_OK) return rc;
+        }
+        const bool grad_mode = u.mode == HSES_UPDATE_GRAD;
+        const UpdateMultiCall call{u.epoch, u.noise_reuse, u.first_thread, u.n, rank, u.fitness,
+                                   grad_mode ? -(base_sigma_tc * (1.0f / nf)) * sqrtf(nf) : base_sigma_tc,
+                                   u.sign_factors, grad_mode ? 0 : 1, u.workspace, u.workspace_bytes};
+        return run_update_multi(ctx, st, &item, 1, call);
     }
     UpdatePlan p = plan_update(a, b, rank, u.n);
     HSES_REQUIRE(u.workspace != nullptr && u.workspace_bytes >= p.bytes,
@@ -355,14 +379,9 @@ int hses::es_update_ex_impl(hses_ctx* ctx, hses_stream stream, const hses_update
     const int32_t first_pair = u.first_thread / 2;
     dim3 grid((unsigned)((b + UN - 1) / UN), (unsigned)((a + UM - 1) / UM), (unsigned)p.splits);
     if (u.cache) {
-        const hses_factor_cache& c = *u.cache;
-        HSES_REQUIRE(c.data != nullptr && c.key == u.key && c.true_epoch == te && c.rank == rank &&
-                         c.a == a && c.b == b,
-                     "factor cache was built for another parameter, epoch bucket or shape");
-        HSES_REQUIRE(first_pair >= c.first_pair && first_pair + p.pairs <= c.first_pair + c.n_pairs,
-                     "factor cache does not cover these members");
-        const float* cA = c.data + (size_t)(first_pair - c.first_pair) * a * rank;
-        const float* cB = c.data + (size_t)c.n_pairs * a * rank + (size_t)(first_pair - c.first_pair) * b * rank;
+        const float *cA = nullptr, *cB = nullptr;
+        int rc = resolve_update_cache(*u.cache, u.key, te, rank, a, b, first_pair, p.pairs, &cA, &cB);
+        if (rc != HSES_OK) return rc;
         HSES_KERNEL(ctx, st, "update_gemm");
         update_gemm_kernel<<<grid, UT, 0, st>>>(cA, cB, p.pairs, rank, a, b, 0, u.fitness, u.sign_factors, partial);
         HSES_LAUNCH_CHECK();
@@ -423,6 +442,90 @@ int hses_es_update(hses_ctx* ctx, hses_stream stream, uint64_t key, int32_t epoc
     u.cache = nullptr;
     u.mode = HSES_UPDATE_GRAD;
     return hses_es_update_ex(ctx, stream, &u);
+}
+
+// Matrices whose rank the wide-rank contraction covers go there one by one, all others in common launches.
+size_t hses_es_update_multi_workspace_bytes(const hses_update_item* items, int32_t n_items, int32_t rank, int64_t n) {
+    if (items == nullptr || n_items < 1 || rank < 1 || n < 2) return 0;
+    size_t bytes = 0;
+    int a[kUpdateMulti], b[kUpdateMulti];
+    for (int32_t i0 = 0; i0 < n_items; i0 += kUpdateMulti) {
+        int cnt = 0;
+        for (int32_t i = i0; i < n_items && i < i0 + kUpdateMulti; ++i) {
+            if (items[i].a < 1 || items[i].b < 1) return 0;
+            if (update_tc_supports(items[i].a, items[i].b, rank)) {
+                bytes = std::max(bytes, hses_es_update_workspace_bytes(items[i].a, items[i].b, rank, n));
+            } else {
+                a[cnt] = items[i].a;
+                b[cnt++] = items[i].b;
+            }
+        }
+        if (cnt) bytes = std::max(bytes, update_multi_workspace_bytes(a, b, cnt, rank, n));
+    }
+    return bytes;
+}
+
+int hses_es_update_multi(hses_ctx* ctx, hses_stream stream, const hses_update_item* items, int32_t n_items, int32_t epoch,
+                         int32_t noise_reuse, int32_t first_thread, int64_t n, int64_t n_total, int32_t rank, float sigma,
+                         int32_t sign_factors, const float* fitness, void* workspace, size_t workspace_bytes) {
+    HSES_REQUIRE(ctx != nullptr, "ctx is NULL");
+    HSES_REQUIRE(items != nullptr && n_items >= 0 && fitness != nullptr, "NULL pointer");
+    HSES_REQUIRE(n > 0 && n % 2 == 0 && first_thread >= 0 && first_thread % 2 == 0,
+                 "members must form whole antithetic pairs");
+    HSES_REQUIRE(n_total >= 1 && noise_reuse >= 0, "n_total must be >= 1 and noise_reuse >= 0");
+    HSES_REQUIRE(rank >= 1 && rank <= 1024, "bad rank");
+    const float nf = (float)n_total, bs = sigma / sqrtf((float)rank);
+    UpdateMultiCall call{epoch, noise_reuse, first_thread, n, rank, fitness, -(bs * (1.0f / nf)) * sqrtf(nf), sign_factors, 0,
+                         workspace, workspace_bytes};
+    bool range_valid = false;
+    for (int32_t i = 0; i < n_items; ++i) {
+        const hses_update_item& it = items[i];
+        HSES_REQUIRE(it.a >= 1 && it.b >= 1 && it.a <= (1 << 20) && it.b <= (1 << 20) && it.grad != nullptr, "bad matrix");
+        if (!update_tc_supports(it.a, it.b, rank)) continue;
+        hses_update_args u{};
+        u.key = it.key;
+        u.epoch = epoch;
+        u.noise_reuse = noise_reuse;
+        u.first_thread = first_thread;
+        u.n = n;
+        u.n_total = n_total;
+        u.rank = rank;
+        u.a = it.a;
+        u.b = it.b;
+        u.sigma = sigma;
+        u.fitness = fitness;
+        u.grad = it.grad;
+        u.workspace = workspace;
+        u.workspace_bytes = workspace_bytes;
+        u.cache = it.cache;
+        u.mode = HSES_UPDATE_GRAD;
+        u.sign_factors = sign_factors;
+        // the matrices share the fitness vector and the workspace: the pair-weight range that the first one leaves at
+        // the start of the workspace serves the following ones
+        int rc = es_update_ex_impl(ctx, stream, &u, range_valid);
+        if (rc != HSES_OK) return rc;
+        range_valid = true;
+    }
+    UpdateMultiItem list[kUpdateMulti];
+    for (int32_t i0 = 0; i0 < n_items; i0 += kUpdateMulti) {
+        int cnt = 0;
+        for (int32_t i = i0; i < n_items && i < i0 + kUpdateMulti; ++i) {
+            const hses_update_item& it = items[i];
+            if (update_tc_supports(it.a, it.b, rank)) continue;
+            UpdateMultiItem& d = list[cnt++];
+            d = UpdateMultiItem{it.key, it.a, it.b, nullptr, nullptr, it.grad};
+            if (it.cache) {
+                int rc = resolve_update_cache(*it.cache, it.key, true_epoch_of(epoch, noise_reuse), rank, it.a, it.b,
+                                              first_thread / 2, n / 2, &d.cache_a, &d.cache_b);
+                if (rc != HSES_OK) return rc;
+            }
+        }
+        if (cnt) {
+            int rc = run_update_multi(ctx, as_stream(stream), list, cnt, call);
+            if (rc != HSES_OK) return rc;
+        }
+    }
+    return HSES_OK;
 }
 
 size_t hses_es_update_static_scratch_bytes(void) { return kStaticScratchBytes; }

@@ -377,14 +377,8 @@ int run_update_tc(hses_ctx* ctx, cudaStream_t st, const hses_update_args& u, flo
 
     const float *cA = nullptr, *cB = nullptr;
     if (u.cache) {
-        const hses_factor_cache& c = *u.cache;
-        HSES_REQUIRE(c.data != nullptr && c.key == u.key && c.true_epoch == te && c.rank == rank && c.a == a &&
-                         c.b == b,
-                     "factor cache was built for another parameter, epoch bucket or shape");
-        HSES_REQUIRE(first_pair >= c.first_pair && first_pair + p.pairs <= c.first_pair + c.n_pairs,
-                     "factor cache does not cover these members");
-        cA = c.data + (size_t)(first_pair - c.first_pair) * a * rank;
-        cB = c.data + (size_t)c.n_pairs * a * rank + (size_t)(first_pair - c.first_pair) * b * rank;
+        int rc = resolve_update_cache(*u.cache, u.key, te, rank, a, b, first_pair, p.pairs, &cA, &cB);
+        if (rc != HSES_OK) return rc;
     }
     if (!reuse_range) {
         HSES_KERNEL(ctx, st, "pair_weight_range");

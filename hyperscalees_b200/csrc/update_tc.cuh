@@ -21,8 +21,33 @@ UpdateTcPlan plan_update_tc(int a, int b, int rank, int64_t n, bool need_raw);
 // model share both), so it is not computed again
 int run_update_tc(hses_ctx* ctx, cudaStream_t stream, const hses_update_args& u, float scale,
                   bool reuse_range = false);
-// hses_es_update_ex with that option; *took_tc tells whether the tensor-core contraction ran
-int es_update_ex_impl(hses_ctx* ctx, hses_stream stream, const hses_update_args* args, bool reuse_range,
-                      bool* took_tc);
+// hses_es_update_ex with that option
+int es_update_ex_impl(hses_ctx* ctx, hses_stream stream, const hses_update_args* args, bool reuse_range);
+
+// The update of several matrices that share rank, fitness vector and members, for any rank, in one set of launches
+// (update_multi.cu).
+constexpr int kUpdateMulti = 48;
+struct UpdateMultiItem {
+    uint64_t key;
+    int a, b;
+    const float *cache_a, *cache_b;   // raw factors of the call's first pair, or NULL: regenerate
+    float* grad;                      // (a, b) dense
+};
+struct UpdateMultiCall {
+    int32_t epoch, noise_reuse, first_thread;
+    int64_t n;                        // members (whole pairs)
+    int rank;
+    const float* fitness;
+    float scale;                      // of the sum
+    int sign_factors;
+    int add_to_grad;                  // add to `grad` instead of writing it
+    void* workspace;
+    size_t workspace_bytes;
+};
+size_t update_multi_workspace_bytes(const int* a, const int* b, int n, int rank, int64_t members);
+int run_update_multi(hses_ctx* ctx, cudaStream_t stream, const UpdateMultiItem* items, int n, const UpdateMultiCall& call);
+// checks a cache descriptor against an update and returns the factors of its first pair
+int resolve_update_cache(const hses_factor_cache& c, uint64_t key, int32_t true_epoch, int rank, int a, int b, int32_t first_pair,
+                         int64_t pairs, const float** cache_a, const float** cache_b);
 
 }  // namespace hses

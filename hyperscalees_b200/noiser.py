@@ -10,6 +10,7 @@ device path is meant to be driven.
 from __future__ import annotations
 
 from dataclasses import dataclass, field
+from operator import attrgetter
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -26,6 +27,9 @@ class IterInfo:
     """noiser.rs:24-28."""
     epoch: int
     thread_id: int
+
+
+_THREAD_ID, _EPOCH = attrgetter("thread_id"), attrgetter("epoch")
 
 
 # ---------------------------------------------------------------------------
@@ -89,18 +93,16 @@ class Solver:
         kind = {"sgd": ops.SGD, "adam": ops.ADAM, "adamw": ops.ADAMW}[self.kind]
         if kind != ops.SGD:
             state.step += 1
-        out = []
-        for i, (p, g) in enumerate(zip(params, grads)):
-            q = p.detach().clone().contiguous()
-            m = v = None
-            if kind != ops.SGD:
-                m, v = state.moments[i].m, state.moments[i].v
-            ops.solver_step(kind, state.step, q, g.contiguous(), m, v, lr=self.lr, beta1=self.beta1,
-                            beta2=self.beta2, eps=self.eps,
-                            weight_decay=self.weight_decay if kind == ops.ADAMW else 0.0,
-                            grad_scale=grad_scale)
-            out.append(q)
-        return out
+        if len(params) == 0:
+            return []
+        m = v = None
+        if kind != ops.SGD:
+            m, v = [s.m for s in state.moments], [s.v for s in state.moments]
+        return ops.solver_step_multi(kind, state.step, [p.detach().contiguous() for p in params],
+                                     [g.contiguous() for g in grads], m, v, lr=self.lr, beta1=self.beta1,
+                                     beta2=self.beta2, eps=self.eps,
+                                     weight_decay=self.weight_decay if kind == ops.ADAMW else 0.0,
+                                     grad_scale=grad_scale)
 
 
 @dataclass
@@ -371,35 +373,40 @@ class EggRoll:
         """The per-parameter `-g*sqrt(N)` of do_update_with (eggroll.rs:384-404)."""
         n_total = len(iterinfos)
         infos = list(iterinfos)
-        contiguous = (n_total % 2 == 0 and infos[0].thread_id % 2 == 0 and all(
-            infos[i].thread_id == infos[0].thread_id + i and infos[i].epoch == infos[0].epoch
-            for i in range(n_total)))
+        # the usual numbering: thread ids first, first+1, ... of one epoch, whole antithetic pairs
+        first, epoch = infos[0].thread_id, infos[0].epoch
+        contiguous = (n_total % 2 == 0 and first % 2 == 0 and
+                      list(map(_THREAD_ID, infos)) == list(range(first, first + n_total)) and
+                      set(map(_EPOCH, infos)) == {epoch})
         if contiguous:
-            groups = {None: (infos[0].thread_id, fitnesses, infos[0].epoch)}
+            groups = {None: (first, fitnesses, epoch)}
         else:
             dense = _dense_fitness(fitnesses.detach().cpu().numpy(), infos, frozen.noise_reuse)
             nr = max(frozen.noise_reuse, 1)
             groups = {te: (lo, torch.as_tensor(vec, device=fitnesses.device), te * nr)
                       for te, (lo, vec) in dense.items()}
-        out = []
-        for p, key, cls in zip(params, base_keys, es_classes):
-            a, b = p.shape
-            total = None
-            for lo, vec, ep in groups.values():
-                if cls == MM_PARAM:
-                    g = ops.es_update(key, ep, frozen.noise_reuse, frozen.rank, a, b, noiser.sigma,
-                                      vec, first_thread=lo, n_total=n_total,
-                                      sign_factors=self.sign_factors)
+        out = [None] * len(params)
+        lora = [i for i, cls in enumerate(es_classes) if cls == MM_PARAM]
+        for lo, vec, ep in groups.values():
+            found = {}
+            if lora:   # every LoRA-noised matrix in one set of launches
+                gs = ops.es_update_multi([base_keys[i] for i in lora], [tuple(params[i].shape) for i in lora], ep,
+                                         frozen.noise_reuse, frozen.rank, noiser.sigma, vec, first_thread=lo,
+                                         n_total=n_total, sign_factors=self.sign_factors)
+                found = dict(zip(lora, gs))
+            for i, (p, key, cls) in enumerate(zip(params, base_keys, es_classes)):
+                a, b = p.shape
+                if i in found:
+                    g = found[i]
                 elif cls == PARAM and not frozen.freeze_nonlora:
                     g = ops.es_update_dense(key, ep, frozen.noise_reuse, (a, b), noiser.sigma, vec,
                                             first_thread=lo, n_total=n_total)
                 else:
                     g = torch.zeros((a, b), dtype=torch.float32, device=p.device)
-                if total is None:
-                    total = g
+                if out[i] is None:
+                    out[i] = g
                 else:
-                    ops.solver_step(ops.SGD, 0, total, g, lr=-1.0)  # total += g
-            out.append(total)
+                    ops.solver_step(ops.SGD, 0, out[i], g, lr=-1.0)  # total += g
         return out
 
     def do_updates(self, frozen: FrozenNoiserParams, noiser: NoiserParams,

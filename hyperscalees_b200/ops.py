@@ -397,6 +397,39 @@ def es_update(key: int, epoch: int, noise_reuse: int, rank: int, a: int, b: int,
     return out
 
 
+def _flat_like(shapes, device):
+    """One allocation, a dense tensor per shape (16-byte aligned each)."""
+    sizes = [math.prod(sh) for sh in shapes]
+    padded = [(n + 3) // 4 * 4 for n in sizes]
+    flat = torch.empty(sum(padded), dtype=torch.float32, device=device)
+    return [v[:n].view(sh) if n != m else v.view(sh)
+            for v, n, m, sh in zip(flat.split(padded), sizes, padded, shapes)]
+
+
+def es_update_multi(keys: Sequence[int], shapes: Sequence[Tuple[int, int]], epoch: int, noise_reuse: int, rank: int,
+                    sigma: float, fitness_: torch.Tensor, first_thread: int = 0, n_total: Optional[int] = None,
+                    caches: Optional[Sequence[Optional[FactorCache]]] = None, sign_factors: bool = False):
+    """es_update of several matrices (key and (a, b) each) that share members and fitness, in one set of launches."""
+    _check(fitness_, "fitness", ndim=1)
+    n, cnt = fitness_.numel(), len(keys)
+    grads = _flat_like(shapes, fitness_.device)
+    items = (_lib.UpdateItem * cnt)()
+    for it, key, (a, b), g in zip(items, keys, shapes, grads):
+        it.key, it.a, it.b, it.grad = key & _U64, a, b, g.data_ptr()
+    if caches is not None:
+        for it, c in zip(items, caches):
+            if c is not None:
+                it.cache = C.pointer(c.desc)
+    L = _lib.load()
+    need = int(L.hses_es_update_multi_workspace_bytes(items, cnt, rank, n))
+    ws = _workspace(fitness_.device, need)
+    ctx = get_context(fitness_.device)
+    _lib.check(L.hses_es_update_multi(ctx.handle, current_stream(), items, cnt, epoch, noise_reuse, first_thread, n,
+                                      n if n_total is None else n_total, rank, sigma, int(sign_factors),
+                                      fitness_.data_ptr(), ws.data_ptr() if ws is not None else None, need))
+    return grads
+
+
 def convert_fitnesses_bs(raw: torch.Tensor, group_size: int) -> torch.Tensor:
     """EggRollBS baseline-subtracted per-direction fitness (eggroll_bs.rs:226-250): (n,) -> (G,)."""
     _check(raw, "raw", ndim=1)
@@ -474,6 +507,28 @@ def solver_step(kind: int, step: int, param: torch.Tensor, grad: torch.Tensor,
     _lib.check(_lib.load().hses_solver_step(ctx.handle, current_stream(), C.byref(desc), step,
                                             grad_scale, _ptr(param), _ptr(grad), _ptr(m), _ptr(v),
                                             param.numel()))
+
+
+def solver_step_multi(kind: int, step: int, params: Sequence[torch.Tensor], grads: Sequence[torch.Tensor],
+                      m: Optional[Sequence[torch.Tensor]] = None, v: Optional[Sequence[torch.Tensor]] = None,
+                      lr: float = 0.01, beta1: float = 0.9, beta2: float = 0.999, eps: float = 1e-8,
+                      weight_decay: float = 0.0, grad_scale: float = 1.0):
+    """One optimizer step over contiguous parameter tensors in one launch; returns the updated copies (the moments
+    are updated in place)."""
+    n = len(params)
+    for t in list(params) + list(grads):
+        _check(t, "tensor")
+        if not t.is_contiguous():
+            raise ValueError("params and grads must be contiguous")
+    out = _flat_like([tuple(p.shape) for p in params], params[0].device)
+    arr = lambda ts: (C.c_void_p * n)(*[t.data_ptr() for t in ts])
+    lens = (C.c_int64 * n)(*[p.numel() for p in params])
+    desc = _lib.SolverDesc(kind, lr, beta1, beta2, eps, weight_decay)
+    ctx = get_context(params[0].device)
+    _lib.check(_lib.load().hses_solver_step_multi(
+        ctx.handle, current_stream(), C.byref(desc), step, grad_scale, n, arr(params), arr(out), arr(grads),
+        arr(m) if m is not None else None, arr(v) if v is not None else None, lens))
+    return out
 
 
 def base_sigma(sigma: float, rank: int) -> float:

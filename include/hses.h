@@ -347,6 +347,22 @@ typedef struct {
 } hses_update_args;
 int hses_es_update_ex(hses_ctx* ctx, hses_stream stream, const hses_update_args* args);
 
+/* ---- The gradients of several matrices that share members, rank and fitness vector (the MM leaves of a
+ *      model, do_updates_impl, eggroll.rs:508-528) in one set of launches: item i's gradient is what
+ *      hses_es_update gives for its key and shape.  cache: NULL or a factor cache of that parameter. --- */
+typedef struct {
+    uint64_t key;
+    int32_t a;
+    int32_t b;
+    float* grad; /* device (a,b) dense */
+    const hses_factor_cache* cache; /* host pointer or NULL */
+} hses_update_item;
+size_t hses_es_update_multi_workspace_bytes(const hses_update_item* items, int32_t n_items, int32_t rank, int64_t n);
+int hses_es_update_multi(hses_ctx* ctx, hses_stream stream, const hses_update_item* items /*host*/, int32_t n_items,
+                         int32_t epoch, int32_t noise_reuse, int32_t first_thread, int64_t n, int64_t n_total,
+                         int32_t rank, float sigma, int32_t sign_factors, const float* fitness /*device, n*/,
+                         void* workspace /*device*/, size_t workspace_bytes);
+
 /* ---- hses_es_update for callers that cannot hand over a workspace.  It has
  *      no counterpart in the reference.  Some hosts of this library never get
  *      to call cudaMalloc themselves: a plugin running inside another runtime's
@@ -411,6 +427,12 @@ typedef struct {
 int hses_solver_step(hses_ctx* ctx, hses_stream stream, const hses_solver* solver, int32_t step,
                      float grad_scale, float* param /*device*/, const float* grad /*device*/,
                      float* m /*device*/, float* v /*device*/, int64_t len);
+
+/* The same step for n tensors in one launch, from `src` (NULL: in place) into `params`; all arrays are HOST arrays of
+ * device pointers, tensors with a NULL parameter are skipped, m and v are NULL for SGD. */
+int hses_solver_step_multi(hses_ctx* ctx, hses_stream stream, const hses_solver* solver, int32_t step, float grad_scale,
+                           int32_t n, const float* const* src /*or NULL*/, float* const* params,
+                           const float* const* grads, float* const* m, float* const* v, const int64_t* lens);
 
 /* ---- SNN population step as two calls around the (optional) fitness all-gather.
  *      The model is the reference's SnnModel / TrainableVthSnn generalised to a list of layer

@@ -136,3 +136,31 @@ def test_tensor_core_update_tiny_and_huge_weights(hs):
         assert (tc - ref).abs().max().item() <= 2e-5 * ref.abs().max().item()
     z = ops.es_update(KEY, 0, 0, 64, 128, 64, 0.1, torch.zeros(32, device="cuda"), algo=ops.ALGO_TENSOR)
     assert torch.count_nonzero(z).item() == 0
+
+
+@pytest.mark.parametrize("rank,n", [(1, 2), (3, 46), (4, 256), (8, 66), (33, 10), (64, 6), (87, 12), (130, 4)])
+@pytest.mark.parametrize("cached,sign", [(False, False), (True, False), (False, True)])
+def test_multi_update_matches_general_kernel(hs, rank, n, cached, sign):
+    """Matrices of odd and even shapes in one set of launches against the fp32 kernel, one by one: ranks that divide
+    64 and ranks that do not, several row and column tiles, fewer pairs than a k-block holds."""
+    from hyperscalees_b200 import core, ops
+    shapes = [(10, 128), (1, 1), (130, 70), (16, 64), (128, 300), (257, 17)]
+    keys = [KEY + 13 * i for i in range(len(shapes))]
+    f = torch.randn(n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(n))
+    caches = [ops.FactorCache(k, 5, 2, rank, a, b, n // 2 + 1, 1) for k, (a, b) in zip(keys, shapes)] if cached else None
+    got = ops.es_update_multi(keys, shapes, 5, 2, rank, 0.2, f, first_thread=4, n_total=2 * n, caches=caches,
+                              sign_factors=sign)
+    for g, k, (a, b) in zip(got, keys, shapes):
+        want = ops.es_update(k, 5, 2, rank, a, b, 0.2, f, first_thread=4, n_total=2 * n, sign_factors=sign,
+                             algo=ops.ALGO_SIMT)
+        assert (g - want).abs().max().item() <= 2e-5 * want.abs().max().item()
+    assert core.get_context(0).device_status() == 0
+
+
+def test_multi_update_of_more_matrices_than_one_launch_holds(hs):
+    from hyperscalees_b200 import ops
+    f = torch.randn(20, device="cuda")
+    keys = [KEY + i for i in range(50)]
+    got = ops.es_update_multi(keys, [(6, 8)] * 50, 0, 0, 4, 0.1, f)
+    for k, g in zip(keys, got):
+        assert torch.equal(g, ops.es_update(k, 0, 0, 4, 6, 8, 0.1, f))
