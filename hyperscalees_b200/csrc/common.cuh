@@ -16,13 +16,13 @@ namespace hses {
 void set_error(const std::string& msg);
 
 struct DeviceTables {
-    // libm calibration
-    double2* log_tab = nullptr;
+    // the generator's tables (see NoiseCal)
+    float4* log_tab = nullptr;
+    float4* cos_tab = nullptr;
+    float* cos_width = nullptr;
     uint32_t* log_flip = nullptr;
     uint32_t* cos_flip = nullptr;
-    uint32_t* log_delta = nullptr;
-    uint32_t* cos_delta = nullptr;
-    float log_of_zero = 0.0f;
+    // inputs the host libm does not round correctly (reported by hses_ctx_calibration_info)
     uint64_t n_log_flips = 0, n_cos_flips = 0;
     // generator jump tables: entry k advances the state by 2^k steps
     uint64_t* jump_pow2 = nullptr;  // kJumpLevels matrices
@@ -86,16 +86,7 @@ struct hses_ctx {
     int sm_count = 0;
     hses::DeviceTables t;
     hses::Profiler prof;
-    hses::LibmCal cal() const {
-        hses::LibmCal c;
-        c.log_tab = t.log_tab;
-        c.log_flip = t.log_flip;
-        c.cos_flip = t.cos_flip;
-        c.log_delta = t.log_delta;
-        c.cos_delta = t.cos_delta;
-        c.log_of_zero = t.log_of_zero;
-        return c;
-    }
+    hses::NoiseCal cal() const { return {t.log_tab, t.cos_tab, t.cos_width, t.log_flip, t.cos_flip}; }
 };
 
 #define HSES_CUDA(call)                                                                   \
@@ -131,16 +122,42 @@ namespace hses {
 // Raw factors of `pairs` antithetic pairs starting at first_pair:
 // A (pairs, a, r) and B (pairs, b, r), row-major.  When pair_weight is given
 // (device, 2 floats per pair: the fitnesses of the even and the odd member),
-// A is multiplied by (f_even - f_odd).  With no_alloc the launch uses no table that
-// would have to be allocated on first use (slower row-to-row advance, same values).
+// A is multiplied by (f_even - f_odd).
 int launch_pair_factors(hses_ctx* ctx, cudaStream_t stream, uint64_t key, int32_t true_epoch,
                         int32_t first_pair, int64_t pairs, int rank, int a, int b,
-                        const float* pair_weight, float* A, float* B, bool no_alloc = false);
+                        const float* pair_weight, float* A, float* B);
 // One solver step (hses_solver_step's arithmetic) over several tensors in one launch, from `src` (NULL: in place) into
 // `params`; tensors with a NULL parameter skipped.
 int solver_step_multi(hses_ctx* ctx, cudaStream_t st, const hses_solver* solver, int32_t step, float grad_scale, int n_tensors,
                       const float* const* src, float* const* params, float* const* m_bufs, float* const* v_bufs,
                       const int64_t* lens, const float* const* grads);
+#if defined(__CUDACC__)
+// The normals pos0 .. pos0+cnt of the stream seeded by s0, made by the whole block: emit(offset, z) gets four at a time
+// (offset a multiple of four; the last four may run past cnt).  The states of runs of 512 (128 when there is little to
+// do) come from the power-of-two tables, one per thread side by side, those of a warp's lanes inside a run from a lane
+// table.  state_s: room for max(32, ceil(cnt / 512)) states; cal: staged (stage_cal), the call synchronises.
+constexpr int kStreamCoarse = 4096;   // from here on sixteen normals per thread and table round keep 256 threads busy
+template <class Emit>
+__device__ __forceinline__ void stream_fill(const NoiseCal& cal, const uint64_t* __restrict__ pow2,
+                                            const uint64_t* __restrict__ lane4, const uint64_t* __restrict__ lane16,
+                                            uint64_t s0, uint64_t pos0, int cnt, uint64_t* state_s, Emit emit) {
+    const bool coarse = cnt >= kStreamCoarse;
+    const int chn = coarse ? 16 : 4, run = 32 * chn, runs = (cnt + run - 1) / run, lane = threadIdx.x & 31;
+    for (int e = threadIdx.x; e < runs; e += blockDim.x) state_s[e] = jump_by(pow2, s0, 2ull * (pos0 + (uint64_t)e * run));
+    __syncthreads();
+    for (int e = threadIdx.x >> 5; e < runs; e += blockDim.x >> 5) {
+        const int off = e * run + lane * chn;
+        if (off >= cnt) continue;
+        uint64_t st = lane_jump(coarse ? lane16 : lane4, state_s[e], lane);
+#pragma unroll 1
+        for (int j = 0; j < chn && off + j < cnt; j += 4) {
+            float z[4];
+            normals4(st, cal, z);
+            emit(off + j, z);
+        }
+    }
+}
+#endif
 // lif_step (hyperscalees-models/src/snn.rs:53-65): charge, threshold, reset; returns the spike
 __device__ __forceinline__ float lif_update(float& v, float cur, float leak, float v_th, int reset) {
     float d = __fadd_rn(-v, cur);

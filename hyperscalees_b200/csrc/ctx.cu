@@ -78,6 +78,20 @@ __global__ void candidates_kernel(const double2* __restrict__ log_tab, int which
     code[i] = r.dist | ((r.alt < r.bits) ? 0x80000000u : 0u);
 }
 
+// the kernels' fp32 candidates of every 24-bit uniform
+__global__ void noise_candidates_kernel(const float4* __restrict__ log_tab, const float4* __restrict__ cos_tab, int which,
+                                        float* __restrict__ hi, float* __restrict__ lo) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= kUnits) return;
+    float h, l;
+    if (which == 0)
+        log_parts(i, log_tab[log_row(i)], h, l);
+    else
+        cos_parts(i, cos_tab[cos_row(i)], h, l);
+    hi[i] = h;
+    lo[i] = l;
+}
+
 int plan_sm_count() {
     static int cached = 0;
     if (cached > 0) return cached;
@@ -132,12 +146,6 @@ int get_hop_table(hses_ctx* ctx, uint64_t distance, const uint64_t** dev_tab) {
 }
 
 static int build_tables(DeviceTables& t) {
-    // log helper table
-    double host_tab[128];
-    build_log_table(host_tab);
-    HSES_CUDA(cudaMalloc(&t.log_tab, sizeof(host_tab)));
-    HSES_CUDA(cudaMemcpy(t.log_tab, host_tab, sizeof(host_tab), cudaMemcpyHostToDevice));
-
     HSES_CUDA(cudaMalloc(&t.status_word, sizeof(int)));
     HSES_CUDA(cudaMemset(t.status_word, 0, sizeof(int)));
 
@@ -170,43 +178,67 @@ static int build_tables(DeviceTables& t) {
         HSES_CUDA(cudaMemcpy(*dst, host.data(), host.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));
     }
 
-    // candidates on the device, libm on the host
+    // candidates on the device, libm on the host: the fp64 candidate for the count of inputs the host does not round
+    // correctly, the fp32 candidate for the kernels' bitmaps and filter widths
     uint32_t *d_bits = nullptr, *d_code = nullptr;
+    double2* d_log64 = nullptr;
     HSES_CUDA(cudaMalloc(&d_bits, (size_t)kUnits * 4));
     HSES_CUDA(cudaMalloc(&d_code, (size_t)kUnits * 4));
+    double host_tab[128];
+    build_log_table(host_tab);
+    HSES_CUDA(cudaMalloc(&d_log64, sizeof(host_tab)));
+    HSES_CUDA(cudaMemcpy(d_log64, host_tab, sizeof(host_tab), cudaMemcpyHostToDevice));
+    std::vector<float4> log_tab(kLogRows), cos_tab(kCosRows);
+    std::vector<float> cos_width(kCosRows);
+    build_noise_tables(log_tab.data(), cos_tab.data());
+    HSES_CUDA(cudaMalloc(&t.log_tab, log_tab.size() * sizeof(float4)));
+    HSES_CUDA(cudaMalloc(&t.cos_tab, cos_tab.size() * sizeof(float4)));
+    HSES_CUDA(cudaMalloc(&t.cos_width, cos_width.size() * sizeof(float)));
+    HSES_CUDA(cudaMemcpy(t.log_tab, log_tab.data(), log_tab.size() * sizeof(float4), cudaMemcpyHostToDevice));
+    HSES_CUDA(cudaMemcpy(t.cos_tab, cos_tab.data(), cos_tab.size() * sizeof(float4), cudaMemcpyHostToDevice));
     std::vector<uint32_t> h_bits(kUnits), h_code(kUnits);
-    CalibResult res[2];
-    for (int which = 0; which < 2; ++which) {
-        candidates_kernel<<<kUnits / 256, 256>>>(t.log_tab, which, d_bits, d_code);
+    std::string error;
+    for (int which = 0; which < 2 && error.empty(); ++which) {
+        CalibResult exact;
+        candidates_kernel<<<kUnits / 256, 256>>>(d_log64, which, d_bits, d_code);
         HSES_LAUNCH_CHECK();
         HSES_CUDA(cudaMemcpy(h_bits.data(), d_bits, (size_t)kUnits * 4, cudaMemcpyDeviceToHost));
         HSES_CUDA(cudaMemcpy(h_code.data(), d_code, (size_t)kUnits * 4, cudaMemcpyDeviceToHost));
         if (which == 0)
-            calibrate(h_bits.data(), h_code.data(), 1u, host_logf_u24, res[0]);
+            calibrate(h_bits.data(), h_code.data(), 1u, host_logf_u24, exact);
         else
-            calibrate(h_bits.data(), h_code.data(), 0u, host_cosf_u24, res[1]);
-        if (!res[which].error.empty()) {
-            set_error(res[which].error);
-            cudaFree(d_bits);
-            cudaFree(d_code);
-            return HSES_ERR_CALIBRATION;
-        }
+            calibrate(h_bits.data(), h_code.data(), 0u, host_cosf_u24, exact);
+        (which == 0 ? t.n_log_flips : t.n_cos_flips) = exact.n_flips;
+        error = exact.error;
+        if (!error.empty()) break;
+
+        NoiseCalResult res;
+        float *d_hi = reinterpret_cast<float*>(d_bits), *d_lo = reinterpret_cast<float*>(d_code);
+        float *h_hi = reinterpret_cast<float*>(h_bits.data()), *h_lo = reinterpret_cast<float*>(h_code.data());
+        noise_candidates_kernel<<<kUnits / 256, 256>>>(t.log_tab, t.cos_tab, which, d_hi, d_lo);
+        HSES_LAUNCH_CHECK();
+        HSES_CUDA(cudaMemcpy(h_hi, d_hi, (size_t)kUnits * 4, cudaMemcpyDeviceToHost));
+        HSES_CUDA(cudaMemcpy(h_lo, d_lo, (size_t)kUnits * 4, cudaMemcpyDeviceToHost));
+        if (which == 0)
+            calibrate_noise(h_hi, h_lo, kLogRows, log_row, host_logf_u24, res);
+        else
+            calibrate_noise(h_hi, h_lo, kCosRows, cos_row, host_cosf_u24, res);
+        error = res.error;
+        for (int r = 0; r < (which == 0 ? kLogRows : kCosRows); ++r)
+            (which == 0 ? log_tab[r].w : cos_width[r]) = res.width[r];
+        uint32_t** flip = which == 0 ? &t.log_flip : &t.cos_flip;
+        HSES_CUDA(cudaMalloc(flip, (size_t)kUnits / 8));
+        HSES_CUDA(cudaMemcpy(*flip, res.flip.data(), (size_t)kUnits / 8, cudaMemcpyHostToDevice));
     }
     HSES_CUDA(cudaFree(d_bits));
     HSES_CUDA(cudaFree(d_code));
-
-    uint32_t** flips[2] = {&t.log_flip, &t.cos_flip};
-    uint32_t** deltas[2] = {&t.log_delta, &t.cos_delta};
-    for (int which = 0; which < 2; ++which) {
-        HSES_CUDA(cudaMalloc(flips[which], (size_t)kUnits / 8));
-        HSES_CUDA(cudaMemcpy(*flips[which], res[which].flip.data(), (size_t)kUnits / 8,
-                             cudaMemcpyHostToDevice));
-        HSES_CUDA(cudaMalloc(deltas[which], 256 * 4));
-        HSES_CUDA(cudaMemcpy(*deltas[which], res[which].delta, 256 * 4, cudaMemcpyHostToDevice));
+    HSES_CUDA(cudaFree(d_log64));
+    if (!error.empty()) {
+        set_error(error);
+        return HSES_ERR_CALIBRATION;
     }
-    t.n_log_flips = res[0].n_flips;
-    t.n_cos_flips = res[1].n_flips;
-    t.log_of_zero = logf(1e-9f);
+    HSES_CUDA(cudaMemcpy(t.log_tab, log_tab.data(), log_tab.size() * sizeof(float4), cudaMemcpyHostToDevice));
+    HSES_CUDA(cudaMemcpy(t.cos_width, cos_width.data(), cos_width.size() * sizeof(float), cudaMemcpyHostToDevice));
     return HSES_OK;
 }
 

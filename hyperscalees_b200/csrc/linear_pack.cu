@@ -190,8 +190,8 @@ __global__ void __launch_bounds__(256) pack_split_kernel(SplitJob j, RowMap map)
 
 struct FactorJob {
     const float *cache_a, *cache_b;   // raw (pairs, a, r) and (pairs, k, r), or NULL: regenerate
-    const uint64_t *pow2, *lane_tab;
-    LibmCal cal;
+    const uint64_t *pow2, *lane4, *lane16;
+    NoiseCal cal;
     uint64_t key;
     int32_t true_epoch, first_pair;
     int64_t pairs;
@@ -205,12 +205,9 @@ struct FactorJob {
     __nv_bfloat16* aimg;              // (pairs, chunk, r16 / kb, part 3, kb / 8, bn, 8)
 };
 
-// Segment `seg` of pair `p`: its normals into shared memory, 16 bytes per thread and trip, then to the operand
-// layout.  Regeneration: a warp takes 128 consecutive normals, its base state by powers of two (the same for all
-// lanes, so every table read is a broadcast), the lane's own state by one round of the lane table.
-__device__ __forceinline__ void factor_segment(const FactorJob& f, int64_t p, int seg, float* buf, double2* log_tab_s,
-                                               uint32_t* delta_s) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// Segment `seg` of pair `p`: its normals into shared memory (from the cache, or stream_fill), then to the operand layout.
+__device__ __forceinline__ void factor_segment(const FactorJob& f, int64_t p, int seg, float* buf, CalTab& tab, uint64_t* state_s) {
+    const int tid = threadIdx.x;
     const int nseg_b = (f.k + f.seg_b - 1) / f.seg_b;
     const bool is_b = seg < nseg_b;
     const int row0 = is_b ? seg * f.seg_b : (seg - nseg_b) * f.seg_a;
@@ -226,24 +223,13 @@ __device__ __forceinline__ void factor_segment(const FactorJob& f, int64_t p, in
             for (int i = tid; i < cnt; i += blockDim.x) buf[i] = __ldg(src + i);
         }
     } else {
-        LibmCal cal = f.cal;
-        for (int i = tid; i < 64; i += blockDim.x) log_tab_s[i] = cal.log_tab[i];
-        for (int i = tid; i < 256; i += blockDim.x) {
-            delta_s[i] = cal.log_delta[i];
-            delta_s[256 + i] = cal.cos_delta[i];
-        }
-        __syncthreads();
-        cal.log_tab = log_tab_s;
-        cal.log_delta = delta_s;
-        cal.cos_delta = delta_s + 256;
+        NoiseCal cal = f.cal;
+        stage_cal(cal, tab);
         const uint64_t first = (uint64_t)f.r * (uint64_t)(row0 + (is_b ? f.row_b0 : f.row_a0));
-        const uint64_t s0 = noise_seed(f.key, f.true_epoch, f.first_pair + (int32_t)p) | 1ull;
-        for (int base = warp * 128; base < cnt; base += (blockDim.x >> 5) * 128) {
-            uint64_t s = lane_jump(f.lane_tab, jump_by(f.pow2, s0, 2ull * (first + (uint64_t)base)), lane);
-            float z[4];
-            next_normals4(s, cal, z);
-            *reinterpret_cast<float4*>(buf + base + 4 * lane) = make_float4(z[0], z[1], z[2], z[3]);
-        }
+        stream_fill(cal, f.pow2, f.lane4, f.lane16, noise_seed(f.key, f.true_epoch, f.first_pair + (int32_t)p) | 1ull, first, cnt,
+                    state_s, [&](int off, float (&z)[4]) {
+                        *reinterpret_cast<float4*>(buf + off) = make_float4(z[0], z[1], z[2], z[3]);
+                    });
     }
     __syncthreads();
     if (is_b) {
@@ -305,14 +291,14 @@ __device__ __forceinline__ void factor_segment(const FactorJob& f, int64_t p, in
 template <int NJ, int RPW>
 __global__ void __launch_bounds__(256) pack_operands_kernel(SplitJob x, RowMap map, int64_t x_blocks, int segs, FactorJob f) {
     __shared__ __align__(16) float buf[PK_SEG];
-    __shared__ double2 log_tab_s[64];
-    __shared__ uint32_t delta_s[512];
+    __shared__ CalTab tab;
+    __shared__ uint64_t state_s[32];
     const int64_t b = blockIdx.x;
     if (b < x_blocks) {
         split_rows<NJ, RPW>(x, map, b);
     } else {
         const int64_t i = b - x_blocks;
-        factor_segment(f, i / segs, (int)(i % segs), buf, log_tab_s, delta_s);
+        factor_segment(f, i / segs, (int)(i % segs), buf, tab, state_s);
     }
 }
 
@@ -834,7 +820,8 @@ int run_pack_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
             if (rc != HSES_OK) return rc;
         }
         f.pow2 = ctx->t.jump_pow2;
-        f.lane_tab = ctx->t.jump_lane4;
+        f.lane4 = ctx->t.jump_lane4;
+        f.lane16 = ctx->t.jump_lane16;
         f.cal = ctx->cal();
         f.key = g.key;
         f.true_epoch = true_epoch_of(g.epoch, g.noise_reuse);

@@ -87,7 +87,7 @@ struct TcArgs {
     const uint64_t* hop;  // generator advance from the end of one item of a warp to its next one
     const int* x_lo_flag; // 0 when every lo half of the split x is zero (x exactly representable in fp16)
     const float* cache_a; // cached raw A rows (pair, a, rank) from the call's first pair on, or NULL
-    LibmCal cal;
+    NoiseCal cal;
     int* status;
     // Ring slots (items) per TMEM quadrant and active generator warps per quadrant.  A slot must
     // always be written by the same generator warp and read by the same epilogue warp(s): waits
@@ -108,7 +108,7 @@ struct TcSmem {
     static constexpr int W_BYTES = BN * BK * 2;
     static constexpr int STAGE_BYTES = 2 * X_BYTES + 2 * W_BYTES;
     static constexpr int HOP_BYTES = 0;     // the hop table is read through L1;
-    static constexpr int TAB_BYTES = 1280;  // the logarithm's helper table and the thresholds as 2 x 128 bytes
+    static constexpr int TAB_BYTES = 1024;  // the generator's log table (its cosine table is read through L1)
     static constexpr int BAR_BYTES = 656;
     static constexpr int FIXED = STAGES * STAGE_BYTES + HOP_BYTES + TAB_BYTES + BAR_BYTES + 1024;
     static constexpr int LIMIT = 232448;  // 227 KB of dynamic shared memory per CTA
@@ -153,7 +153,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* stage_base = smem;
-    double2* log_tab_s = reinterpret_cast<double2*>(smem + S::STAGES * S::STAGE_BYTES + S::HOP_BYTES);
+    float4* log_tab_s = reinterpret_cast<float4*>(smem + S::STAGES * S::STAGE_BYTES + S::HOP_BYTES);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::STAGES * S::STAGE_BYTES + S::HOP_BYTES + S::TAB_BYTES);
     float* a_stage = reinterpret_cast<float*>(smem + S::STAGES * S::STAGE_BYTES + S::HOP_BYTES + S::TAB_BYTES +
                                               S::BAR_BYTES);
@@ -189,20 +189,9 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // small read-only tables go to shared memory: the epilogue's noise regeneration
-    // looks them up for every normal
-    if (RG > 0) {
-        for (int i = threadIdx.x; i < 64; i += NTHREADS) log_tab_s[i] = g.cal.log_tab[i];
-        // thresholds of the rounding filter as bytes (ceil(log2)), one per 1/128 of the input range
-        // (the larger of the two 1/256 thresholds): 256 bytes instead of 2 KB
-        uint8_t* thr_s = reinterpret_cast<uint8_t*>(log_tab_s + 64);
-        for (int i = threadIdx.x; i < 128; i += NTHREADS) {
-            const uint32_t tl = max(g.cal.log_delta[2 * i], g.cal.log_delta[2 * i + 1]);
-            const uint32_t tc_ = max(g.cal.cos_delta[2 * i], g.cal.cos_delta[2 * i + 1]);
-            thr_s[i] = pack_threshold_log2(tl);
-            thr_s[128 + i] = pack_threshold_log2(tc_);
-        }
-    }
+    // the smaller table goes to shared memory: the generators look it up for every normal
+    if (RG > 0)
+        for (int i = threadIdx.x; i < kLogRows; i += NTHREADS) log_tab_s[i] = g.cal.log_tab[i];
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "r"(2 * BN)
@@ -444,12 +433,8 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
         constexpr int RANK = RG * 4;
         const int gq = (warp - GEN_WARP0) & 3, gi = (warp - GEN_WARP0) >> 2;
         const int depth = g.ring_depth, GENS = g.gens;
-        LibmCal cal = g.cal;
+        NoiseCal cal = g.cal;
         cal.log_tab = log_tab_s;
-        cal.log_delta = reinterpret_cast<const uint32_t*>(log_tab_s + 64);                         // byte tables, see
-        cal.cos_delta = reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(log_tab_s + 64) + 128);  // next_normals4_t<true, 17>
-        LibmCal cal4 = g.cal;      // the one-at-a-time generator of ranks 1..3 reads the 32-bit thresholds
-        cal4.log_tab = log_tab_s;
         const int items_per_tile = g.a / IT::ROWS;
         const int n_local = lane % IT::ROWS, qoff = (lane / IT::ROWS) * IT::NPL;   // this lane's row and first rank index
         float* const lane_a = a_stage + (size_t)gq * depth * IT::SLOT_FLOATS + (lane / IT::ROWS) * IT::ROWS + n_local;
@@ -498,11 +483,11 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
                         z[0] = v[c4].x; z[1] = v[c4].y; z[2] = v[c4].z; z[3] = v[c4].w;
                     } else if (rt < 4) {
                         z[1] = z[2] = z[3] = 0.0f;
-                        z[0] = next_normal(a_state, cal4);
-                        if (rt > 1) z[1] = next_normal(a_state, cal4);
-                        if (rt > 2) z[2] = next_normal(a_state, cal4);
+                        z[0] = normal1(a_state, cal);
+                        if (rt > 1) z[1] = normal1(a_state, cal);
+                        if (rt > 2) z[2] = normal1(a_state, cal);
                     } else {
-                        next_normals4_t<true, 17>(a_state, cal, z);
+                        normals4(a_state, cal, z);
                     }
 #pragma unroll
                     for (int j = 0; j < 4; ++j) dst[(4 * c4 + j) * 32] = __fmul_rn(z[j], g.base_sigma);
@@ -606,7 +591,7 @@ constexpr int LT_ROWS = 64;
 constexpr int LT_KB = 256;
 template <int RANK_G>
 __global__ void __launch_bounds__(LT_THREADS, 2)
-lowrank_t_kernel(LibmCal cal, const uint64_t* __restrict__ pow2, const uint64_t* __restrict__ hop_kb,
+lowrank_t_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, const uint64_t* __restrict__ hop_kb,
                  uint64_t key, int32_t true_epoch, int32_t first_thread, const float* __restrict__ x,
                  int64_t x_stride, int t_steps, int64_t n_pop, int bm, int k, float* __restrict__ t,
                  __half* __restrict__ xhi, __half* __restrict__ xlo, float* __restrict__ inv_scale,
@@ -617,20 +602,12 @@ lowrank_t_kernel(LibmCal cal, const uint64_t* __restrict__ pow2, const uint64_t*
     constexpr int KSTEP = 4 * KQ;     // k covered by one pass of a warp
     __shared__ __align__(16) float bs[LT_KB * RANK];  // one block of B; reused for the k-part sums
     __shared__ uint64_t hop_s[kJumpWords];
-    __shared__ double2 log_tab_s[64];
-    __shared__ uint32_t delta_s[512];
+    __shared__ CalTab tab_s;
     __shared__ int64_t row_s[LT_ROWS];  // global row of each of this CTA's rows
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (!cache_b) {
         for (int i = tid; i < kJumpWords; i += LT_THREADS) hop_s[i] = hop_kb[i];
-        for (int i = tid; i < 64; i += LT_THREADS) log_tab_s[i] = cal.log_tab[i];
-        for (int i = tid; i < 256; i += LT_THREADS) {
-            delta_s[i] = cal.log_delta[i];
-            delta_s[256 + i] = cal.cos_delta[i];
-        }
-        cal.log_tab = log_tab_s;
-        cal.log_delta = delta_s;
-        cal.cos_delta = delta_s + 256;
+        stage_cal(cal, tab_s);
     }
     const int32_t first_pair = first_thread / 2;
     const int32_t pair = first_pair + blockIdx.x;
@@ -823,15 +800,15 @@ lowrank_t_kernel(LibmCal cal, const uint64_t* __restrict__ pow2, const uint64_t*
             const int pr = (tid / KSTEP) * KSTEP + (tid & 3) * KQ + ((tid % KSTEP) >> 2);
             if (rank_true < 4) {
                 float z[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                z[0] = next_normal(sb, cal);
-                if (rank_true > 1) z[1] = next_normal(sb, cal);
-                if (rank_true > 2) z[2] = next_normal(sb, cal);
+                z[0] = normal1(sb, cal);
+                if (rank_true > 1) z[1] = normal1(sb, cal);
+                if (rank_true > 2) z[2] = normal1(sb, cal);
                 *reinterpret_cast<float4*>(bs + pr * RANK) = make_float4(z[0], z[1], z[2], z[3]);
             } else {
 #pragma unroll 1
                 for (int q = 0; q < RANK; q += 4) {
                     float z[4];
-                    next_normals4(sb, cal, z);
+                    normals4(sb, cal, z);
                     *reinterpret_cast<float4*>(bs + pr * RANK + q) = make_float4(z[0], z[1], z[2], z[3]);
                 }
             }
@@ -912,7 +889,8 @@ __device__ __forceinline__ float4 apply_x_op(float4 v, int x_op) {
 // 32 apart, then read consecutive rows, eight of them covering all banks.
 template <int RANK_G, int NJ, int RPR, bool HALF>
 __global__ void __launch_bounds__(LT_THREADS, 2)
-lowrank_t_rows_kernel(LibmCal cal, const uint64_t* __restrict__ pow2,
+lowrank_t_rows_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, const uint64_t* __restrict__ lane4,
+                      const uint64_t* __restrict__ lane16,
                       uint64_t key, int32_t true_epoch, int32_t first_thread, const float* __restrict__ x,
                       int64_t x_stride, int t_steps, int64_t n_pop, int bm, int k, float* __restrict__ t,
                       __half* __restrict__ xhi, __half* __restrict__ xlo, float* __restrict__ inv_scale,
@@ -922,19 +900,12 @@ lowrank_t_rows_kernel(LibmCal cal, const uint64_t* __restrict__ pow2,
     constexpr int RP = 8 / RANK_G;    // rows of B per 128 bytes
     constexpr int ROWS_CTA = HALF ? 2 * LT_ROWS : LT_ROWS;   // x rows per CTA
     extern __shared__ __align__(16) float bsm[];   // ceil(k / 128) * 128 rows of RANK floats
-    __shared__ double2 log_tab_s[64];
-    __shared__ uint32_t delta_s[512];
+    __shared__ CalTab tab_s;
     __shared__ int64_t row_s[ROWS_CTA];
+    __shared__ uint64_t state_s[32];   // at most 16384 normals
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (!cache_b) {
-        for (int i = tid; i < 64; i += LT_THREADS) log_tab_s[i] = cal.log_tab[i];
-        for (int i = tid; i < 256; i += LT_THREADS) {
-            delta_s[i] = cal.log_delta[i];
-            delta_s[256 + i] = cal.cos_delta[i];
-        }
-        cal.log_tab = log_tab_s;
-        cal.log_delta = delta_s;
-        cal.cos_delta = delta_s + 256;
+        stage_cal(cal, tab_s);
     }
     const int32_t first_pair = first_thread / 2;
     const int32_t pair = first_pair + blockIdx.x;
@@ -979,30 +950,24 @@ lowrank_t_rows_kernel(LibmCal cal, const uint64_t* __restrict__ pow2,
             }
         }
     } else {
-        const int rpt = (k + LT_THREADS - 1) / LT_THREADS;   // rows per thread
-        const int kr0 = tid * rpt, kr1 = min(kr0 + rpt, k);
-        if (kr0 < k) {
-            uint64_t sb = noise_seed(key, true_epoch, pair) | 1ull;
-            sb = jump_by(pow2, sb, 2ull * (uint64_t)rank_true * (uint64_t)(row_b0 + kr0));   // row_b0: first input-side row
-#pragma unroll 1
-            for (int kr = kr0; kr < kr1; ++kr) {
-                const int p = stored_row(kr);
-                if (rank_true < 4) {
-                    float z[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                    z[0] = next_normal(sb, cal);
-                    if (rank_true > 1) z[1] = next_normal(sb, cal);
-                    if (rank_true > 2) z[2] = next_normal(sb, cal);
-                    bsm4[p] = make_float4(z[0], z[1], z[2], z[3]);
-                    continue;
-                }
-#pragma unroll 1
-                for (int c = 0; c < RANK_G; ++c) {
-                    float z[4];
-                    next_normals4(sb, cal, z);
-                    bsm4[p * RANK_G + ((c + p / RP) % RANK_G)] = make_float4(z[0], z[1], z[2], z[3]);
-                }
-            }
+        const uint64_t s0 = noise_seed(key, true_epoch, pair) | 1ull;
+        const uint64_t pos0 = (uint64_t)rank_true * (uint64_t)row_b0;   // row_b0: first input-side row
+        if (rank_true < 4) {
+            for (int kr = tid; kr < k; kr += LT_THREADS) bsm4[stored_row(kr)] = make_float4(0.f, 0.f, 0.f, 0.f);
+            __syncthreads();
         }
+        stream_fill(cal, pow2, lane4, lane16, s0, pos0, k * rank_true, state_s, [&](int off, float (&z)[4]) {
+            if (rank_true < 4) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int kr = (off + j) / rank_true;
+                    if (kr < k) bsm[stored_row(kr) * 4 + (off + j - kr * rank_true)] = z[j];
+                }
+            } else {
+                const int kr = off / RANK, c = (off - kr * RANK) >> 2, p = stored_row(kr);
+                bsm4[p * RANK_G + ((c + p / RP) % RANK_G)] = make_float4(z[0], z[1], z[2], z[3]);
+            }
+        });
     }
     __syncthreads();
 
@@ -1167,7 +1132,8 @@ lowrank_t_rows_kernel(LibmCal cal, const uint64_t* __restrict__ pow2,
 // the pieces.  The block kernel walks such a row four values per lane and trip.
 template <int RANK_G>
 __global__ void __launch_bounds__(LT_THREADS, 2)
-lowrank_t_long_kernel(LibmCal cal, const uint64_t* __restrict__ pow2,
+lowrank_t_long_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, const uint64_t* __restrict__ lane4,
+                      const uint64_t* __restrict__ lane16,
                       uint64_t key, int32_t true_epoch, int32_t first_thread, const float* __restrict__ x,
                       int64_t x_stride, int t_steps, int64_t n_pop, int bm, int k, float* __restrict__ t,
                       __half* __restrict__ xhi, __half* __restrict__ xlo, float* __restrict__ inv_scale,
@@ -1179,19 +1145,12 @@ lowrank_t_long_kernel(LibmCal cal, const uint64_t* __restrict__ pow2,
     constexpr int RP = 8 / RANK_G;    // rows of B per 128 bytes
     constexpr int ROWS_CTA = HALF ? 2 * LT_ROWS : LT_ROWS;   // x rows per CTA
     extern __shared__ __align__(16) float bsm[];   // ceil(k / 128) * 128 rows of RANK floats
-    __shared__ double2 log_tab_s[64];
-    __shared__ uint32_t delta_s[512];
+    __shared__ CalTab tab_s;
     __shared__ int64_t row_s[ROWS_CTA];
+    __shared__ uint64_t state_s[32];   // at most 16384 normals
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (!cache_b) {
-        for (int i = tid; i < 64; i += LT_THREADS) log_tab_s[i] = cal.log_tab[i];
-        for (int i = tid; i < 256; i += LT_THREADS) {
-            delta_s[i] = cal.log_delta[i];
-            delta_s[256 + i] = cal.cos_delta[i];
-        }
-        cal.log_tab = log_tab_s;
-        cal.log_delta = delta_s;
-        cal.cos_delta = delta_s + 256;
+        stage_cal(cal, tab_s);
     }
     const int32_t first_pair = first_thread / 2;
     const int32_t pair = first_pair + blockIdx.x;
@@ -1236,30 +1195,24 @@ lowrank_t_long_kernel(LibmCal cal, const uint64_t* __restrict__ pow2,
             }
         }
     } else {
-        const int rpt = (k + LT_THREADS - 1) / LT_THREADS;   // rows per thread
-        const int kr0 = tid * rpt, kr1 = min(kr0 + rpt, k);
-        if (kr0 < k) {
-            uint64_t sb = noise_seed(key, true_epoch, pair) | 1ull;
-            sb = jump_by(pow2, sb, 2ull * (uint64_t)rank_true * (uint64_t)(row_b0 + kr0));   // row_b0: first input-side row
-#pragma unroll 1
-            for (int kr = kr0; kr < kr1; ++kr) {
-                const int p = stored_row(kr);
-                if (rank_true < 4) {
-                    float z[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                    z[0] = next_normal(sb, cal);
-                    if (rank_true > 1) z[1] = next_normal(sb, cal);
-                    if (rank_true > 2) z[2] = next_normal(sb, cal);
-                    bsm4[p] = make_float4(z[0], z[1], z[2], z[3]);
-                    continue;
-                }
-#pragma unroll 1
-                for (int c = 0; c < RANK_G; ++c) {
-                    float z[4];
-                    next_normals4(sb, cal, z);
-                    bsm4[p * RANK_G + ((c + p / RP) % RANK_G)] = make_float4(z[0], z[1], z[2], z[3]);
-                }
-            }
+        const uint64_t s0 = noise_seed(key, true_epoch, pair) | 1ull;
+        const uint64_t pos0 = (uint64_t)rank_true * (uint64_t)row_b0;   // row_b0: first input-side row
+        if (rank_true < 4) {
+            for (int kr = tid; kr < k; kr += LT_THREADS) bsm4[stored_row(kr)] = make_float4(0.f, 0.f, 0.f, 0.f);
+            __syncthreads();
         }
+        stream_fill(cal, pow2, lane4, lane16, s0, pos0, k * rank_true, state_s, [&](int off, float (&z)[4]) {
+            if (rank_true < 4) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int kr = (off + j) / rank_true;
+                    if (kr < k) bsm[stored_row(kr) * 4 + (off + j - kr * rank_true)] = z[j];
+                }
+            } else {
+                const int kr = off / RANK, c = (off - kr * RANK) >> 2, p = stored_row(kr);
+                bsm4[p * RANK_G + ((c + p / RP) % RANK_G)] = make_float4(z[0], z[1], z[2], z[3]);
+            }
+        });
     }
     __syncthreads();
 
@@ -1678,7 +1631,7 @@ int run_tensor_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
         HSES_CUDA(cudaFuncSetAttribute(lowrank_t_rows_kernel<RG, NJ, RPR, HALF>,                              \
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));                  \
         lowrank_t_rows_kernel<RG, NJ, RPR, HALF><<<HALF ? lt_grid2 : lt_grid, LT_THREADS, b_bytes, st>>>(     \
-            ctx->cal(), ctx->t.jump_pow2, g.key, ta.true_epoch, g.first_thread, g.x, g.x_row_stride,          \
+            ctx->cal(), ctx->t.jump_pow2, ctx->t.jump_lane4, ctx->t.jump_lane16, g.key, ta.true_epoch, g.first_thread, g.x, g.x_row_stride, \
             g.t_steps, g.n_pop, g.bm, g.k, sc.t, sc.xhi, sc.xlo, sc.rs, cache_b, sc.lo_flag, one_pass, g.rank, \
             g.factor_order == 1 ? g.a : 0, reuse_split ? 1 : 0, groups, g.x_op);                                      \
     } while (0)
@@ -1707,7 +1660,7 @@ int run_tensor_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
         HSES_CUDA(cudaFuncSetAttribute(lowrank_t_long_kernel<RG>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                        65536));                                                               \
         lowrank_t_long_kernel<RG><<<lt_grid, LT_THREADS, b_bytes, st>>>(                                      \
-            ctx->cal(), ctx->t.jump_pow2, g.key, ta.true_epoch, g.first_thread, g.x, g.x_row_stride,          \
+            ctx->cal(), ctx->t.jump_pow2, ctx->t.jump_lane4, ctx->t.jump_lane16, g.key, ta.true_epoch, g.first_thread, g.x, g.x_row_stride, \
             g.t_steps, g.n_pop, g.bm, g.k, sc.t, sc.xhi, sc.xlo, sc.rs, cache_b, sc.lo_flag, one_pass, g.rank, \
             g.factor_order == 1 ? g.a : 0, reuse_split ? 1 : 0, 1, g.x_op);                                           \
     } while (0)

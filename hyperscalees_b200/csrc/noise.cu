@@ -11,19 +11,19 @@ namespace hses {
 // chunk with a jump of 2*kChunk*chunk_index generator steps.
 constexpr int kChunk = 16;
 
-__global__ void normal_fill_kernel(LibmCal cal, const uint64_t* __restrict__ pow2, uint64_t seed,
+__global__ void normal_fill_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, uint64_t seed,
                                    float* __restrict__ out, size_t n) {
     size_t chunk = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     size_t begin = chunk * kChunk;
     if (begin >= n) return;
     uint64_t s = jump_by(pow2, seed | 1ull, 2ull * begin);
     size_t end = begin + kChunk < n ? begin + kChunk : n;
-    for (size_t i = begin; i < end; ++i) out[i] = next_normal(s, cal);
+    for (size_t i = begin; i < end; ++i) out[i] = normal1(s, cal);
 }
 
 // One thread per (member, row of the (a+b, r) block).  Rows [0,b) are B, rows
 // [b,a+b) are A (eggroll.rs:98-101).
-__global__ void lora_factors_kernel(LibmCal cal, const uint64_t* __restrict__ pow2, uint64_t key,
+__global__ void lora_factors_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, uint64_t key,
                                     int32_t true_epoch, const int32_t* __restrict__ thread_ids,
                                     int32_t first_thread, int64_t n_members, int rank, int a, int b,
                                     float base_sigma, int layout, float* __restrict__ A,
@@ -41,7 +41,7 @@ __global__ void lora_factors_kernel(LibmCal cal, const uint64_t* __restrict__ po
     int dim = is_a ? a : b;
     float* dst = is_a ? A : B;
     for (int q = 0; q < rank; ++q) {
-        float z = next_normal(s, cal);
+        float z = normal1(s, cal);
         if (is_a) z = fmul(z, scale);
         size_t off = layout == HSES_LAYOUT_NAR
                          ? ((size_t)member * dim + m) * rank + q
@@ -50,7 +50,7 @@ __global__ void lora_factors_kernel(LibmCal cal, const uint64_t* __restrict__ po
     }
 }
 
-__global__ void dense_noise_kernel(LibmCal cal, const uint64_t* __restrict__ pow2, uint64_t key,
+__global__ void dense_noise_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, uint64_t key,
                                    int32_t true_epoch, const int32_t* __restrict__ thread_ids,
                                    int32_t first_thread, int64_t n_members, int len,
                                    float base_sigma, float* __restrict__ out) {
@@ -62,14 +62,14 @@ __global__ void dense_noise_kernel(LibmCal cal, const uint64_t* __restrict__ pow
     uint64_t s = noise_seed(key, true_epoch, tid / 2) | 1ull;
     s = jump_by(pow2, s, 2ull * (uint64_t)begin);
     int end = begin + kChunk < len ? begin + kChunk : len;
-    for (int i = begin; i < end; ++i) out[(size_t)member * len + i] = fmul(next_normal(s, cal), scale);
+    for (int i = begin; i < end; ++i) out[(size_t)member * len + i] = fmul(normal1(s, cal), scale);
 }
 
 // Dense-leaf update: block c owns elements [c*kChunk, (c+1)*kChunk); its
 // threads stride over the antithetic pairs, then reduce in a fixed order so
 // that every rank obtains the same bits.
 constexpr int kDenseThreads = 1024;  // few blocks (one per chunk of a leaf): all the parallelism is in the block
-__global__ void es_update_dense_kernel(LibmCal cal, const uint64_t* __restrict__ pow2, uint64_t key,
+__global__ void es_update_dense_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, uint64_t key,
                                        int32_t true_epoch, int32_t first_pair, int64_t n_pairs,
                                        int len, float sigma, float out_scale,
                                        const float* __restrict__ fitness, float* __restrict__ grad) {
@@ -86,7 +86,7 @@ __global__ void es_update_dense_kernel(LibmCal cal, const uint64_t* __restrict__
         s = jump_by(pow2, s, 2ull * (uint64_t)begin);
 #pragma unroll
         for (int i = 0; i < kChunk; ++i)
-            if (i < cnt) acc[i] = fmaf(w, next_normal(s, cal), acc[i]);
+            if (i < cnt) acc[i] = fmaf(w, normal1(s, cal), acc[i]);
     }
     for (int i = 0; i < cnt; ++i) {
         red[threadIdx.x] = acc[i];
@@ -100,80 +100,55 @@ __global__ void es_update_dense_kernel(LibmCal cal, const uint64_t* __restrict__
     }
 }
 
-// Pair-folded raw factors for the scratch-based paths (see common.cuh).  CTA (pair, chunk)
-// writes kPfBlocks blocks of 128 rows of the pair's (b + a, rank) normal block: a thread jumps
-// to its first row once and from then on hops 127 rows ahead after each row it has written.
-constexpr int kPfBlocks = 8;
-__global__ void __launch_bounds__(128)
-pair_factors_kernel(LibmCal cal, const uint64_t* __restrict__ pow2, const uint64_t* __restrict__ hop127,
-                    uint64_t key, int32_t true_epoch, int32_t first_pair, int64_t pairs, int rank, int a,
-                    int b, const float* __restrict__ pair_weight, float* __restrict__ A,
-                    float* __restrict__ B) {
-    // tables that every normal reads stay in shared memory
-    __shared__ double2 log_tab_s[64];
-    __shared__ uint32_t delta_s[512];
-    __shared__ uint64_t hop_s[kJumpWords];
-    for (int i = threadIdx.x; i < 64; i += blockDim.x) log_tab_s[i] = cal.log_tab[i];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-        delta_s[i] = cal.log_delta[i];
-        delta_s[256 + i] = cal.cos_delta[i];
-    }
-    // without a prebuilt hop table a thread advances with the per-context power-of-two tables instead
-    if (hop127)
-        for (int i = threadIdx.x; i < kJumpWords; i += blockDim.x) hop_s[i] = hop127[i];
-    __syncthreads();
-    cal.log_tab = log_tab_s;
-    cal.log_delta = delta_s;
-    cal.cos_delta = delta_s + 256;
-    const int64_t p = blockIdx.x;
-    int row = blockIdx.y * (128 * kPfBlocks) + threadIdx.x;
-    if (p >= pairs || row >= a + b) return;
-    uint64_t s = noise_seed(key, true_epoch, first_pair + (int32_t)p) | 1ull;
-    s = jump_by(pow2, s, 2ull * (uint64_t)rank * (uint64_t)row);
-    float w = 1.0f;
-    if (pair_weight) w = __fsub_rn(pair_weight[2 * p], pair_weight[2 * p + 1]);
-    for (int blk = 0; blk < kPfBlocks && row < a + b; ++blk, row += 128) {
-        const bool is_a = row >= b;
-        float* dst = is_a ? A + ((size_t)p * a + (row - b)) * rank : B + ((size_t)p * b + row) * rank;
-        const bool weigh = is_a && pair_weight;
-        if ((rank & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-            for (int q = 0; q < rank; q += 4) {
-                float z[4];
-                next_normals4(s, cal, z);
-                if (weigh) {
+// Pair-folded raw factors for the scratch-based paths (see common.cuh).  A pair's (b + a, rank) block is one run of the
+// stream; CTA (pair, piece) makes kPfPiece normals of it.  Bound by instruction issue (about a hundred per normal).
+constexpr int kPfPiece = 8192;
+__global__ void __launch_bounds__(256)
+pair_factors_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, const uint64_t* __restrict__ lane4,
+                    const uint64_t* __restrict__ lane16, uint64_t key, int32_t true_epoch, int32_t first_pair, int64_t na,
+                    int64_t nb, const float* __restrict__ pair_weight, float* __restrict__ A, float* __restrict__ B) {
+    __shared__ CalTab tab;
+    __shared__ uint64_t state_s[32];
+    stage_cal(cal, tab);
+    const int64_t p = blockIdx.x, e0 = (int64_t)blockIdx.y * kPfPiece;
+    const int cnt = (int)min((int64_t)kPfPiece, na + nb - e0);
+    const float w = pair_weight ? __fsub_rn(pair_weight[2 * p], pair_weight[2 * p + 1]) : 1.0f;
+    float* const dst_b = B + p * nb + e0;
+    float* const dst_a = A + p * na + (e0 - nb);
+    const int split = (int)min((int64_t)cnt, max((int64_t)0, nb - e0));   // values of this piece that belong to B
+    const bool vec = ((reinterpret_cast<uintptr_t>(dst_b) | reinterpret_cast<uintptr_t>(dst_a)) & 15) == 0 && (split & 3) == 0 &&
+                     (cnt & 3) == 0;
+    stream_fill(cal, pow2, lane4, lane16, noise_seed(key, true_epoch, first_pair + (int32_t)p) | 1ull, (uint64_t)e0, cnt, state_s,
+                [&](int off, float (&z)[4]) {
+                    if (vec) {
+                        const bool is_a = off >= split;
+                        if (is_a && pair_weight) {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) z[j] = __fmul_rn(z[j], w);
-                }
-                *reinterpret_cast<float4*>(dst + q) = make_float4(z[0], z[1], z[2], z[3]);
-            }
-        } else {
-            for (int q = 0; q < rank; ++q) {
-                float z = next_normal(s, cal);
-                dst[q] = weigh ? __fmul_rn(z, w) : z;
-            }
-        }
-        s = hop127 ? jump_apply(hop_s, s) : jump_by(pow2, s, 2ull * (uint64_t)rank * 127ull);
-    }
+                            for (int j = 0; j < 4; ++j) z[j] = __fmul_rn(z[j], w);
+                        }
+                        *reinterpret_cast<float4*>((is_a ? dst_a : dst_b) + off) = make_float4(z[0], z[1], z[2], z[3]);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            if (off + j < cnt) {
+                                if (off + j < split) dst_b[off + j] = z[j];
+                                else dst_a[off + j] = pair_weight ? __fmul_rn(z[j], w) : z[j];
+                            }
+                    }
+                });
 }
 
 int launch_pair_factors(hses_ctx* ctx, cudaStream_t stream, uint64_t key, int32_t true_epoch,
                         int32_t first_pair, int64_t pairs, int rank, int a, int b,
-                        const float* pair_weight, float* A, float* B, bool no_alloc) {
-    int rows = a + b;
-    int chunks = (rows + 128 * kPfBlocks - 1) / (128 * kPfBlocks);
-    HSES_REQUIRE(chunks <= 65535, "a + b too large");
+                        const float* pair_weight, float* A, float* B) {
+    const int64_t na = (int64_t)a * rank, nb = (int64_t)b * rank;
+    const int64_t pieces = (na + nb + kPfPiece - 1) / kPfPiece;
+    HSES_REQUIRE(pieces <= 65535, "a + b too large");
     HSES_REQUIRE(pairs >= 1 && pairs < (1ll << 31), "pair count out of range");
-    // the hop table of a rank is built (and allocated) on its first use; callers that must not
-    // allocate leave it out and the kernel advances with the context's power-of-two tables
-    const uint64_t* hop127 = nullptr;
-    if (!no_alloc) {
-        int rc = get_hop_table(ctx, 2ull * (uint64_t)rank * 127, &hop127);
-        if (rc != HSES_OK) return rc;
-    }
-    dim3 grid((unsigned)pairs, (unsigned)chunks);
+    dim3 grid((unsigned)pairs, (unsigned)pieces);
     HSES_KERNEL(ctx, stream, "pair_factors");
-    pair_factors_kernel<<<grid, 128, 0, stream>>>(ctx->cal(), ctx->t.jump_pow2, hop127, key, true_epoch,
-                                                  first_pair, pairs, rank, a, b, pair_weight, A, B);
+    pair_factors_kernel<<<grid, 256, 0, stream>>>(ctx->cal(), ctx->t.jump_pow2, ctx->t.jump_lane4, ctx->t.jump_lane16, key,
+                                                  true_epoch, first_pair, na, nb, pair_weight, A, B);
     HSES_LAUNCH_CHECK();
     return HSES_OK;
 }

@@ -14,9 +14,11 @@
 //      rounded to fp32;
 //   2. a per-context calibration that compares the candidate with the host
 //      libm over all 2^24 possible uniforms and records, one bit per input,
-//      where libm rounds to the other neighbour.  A cheap distance-to-midpoint
-//      test on the low 29 bits of the fp64 value filters out the ~90 % of
+//      where libm rounds to the other neighbour.  A cheap test filters out the
 //      inputs that cannot be affected before the bitmap is consulted.
+// The kernels run the same scheme on an fp32 candidate (NoiseCal below): a sum
+// hi + lo of two fp32 values, 2^-30 and better relative to the result, and two
+// roundings of it, hi + (lo +- c*hi), that differ for the few inputs in doubt.
 // The functions below compile for host and device so the candidate math can
 // be exercised on the CPU as well.
 #pragma once
@@ -33,6 +35,7 @@
 
 #if !defined(__CUDACC__)
 struct double2 { double x, y; };
+struct float4 { float x, y, z, w; };
 #endif
 
 namespace hses {
@@ -314,71 +317,173 @@ HSES_HD float next_normal(uint64_t& state, const LibmCal& cal) {
     return normal_from_draws(x1, x2, cal);
 }
 
-// Four consecutive normals of the stream.  Same values as four next_normal()
-// calls; the work is laid out as independent chains (eight generator steps, four
-// logarithms, four cosines, then all bitmap reads issued together without
-// branches) so that table and bitmap latencies overlap instead of adding up.
-// LOG2T: the two threshold tables are 256 bytes each holding ceil(log2(threshold)) (see
-// pack_thresholds_log2): a threshold rounded up only sends a few more candidates to the bitmap,
-// whose bit decides, so the values are the same; the tables then fit where 2 KB would not.
-// TSHIFT: the byte tables are indexed by input >> TSHIFT (16: 256 entries; 17: 128 entries, each the
-// larger of two neighbouring thresholds — again only a few more candidates for the bitmap).
-template <bool LOG2T, int TSHIFT = 16>
-HSES_HD void next_normals4_t(uint64_t& state, const LibmCal& cal, float (&out)[4]) {
-    uint32_t iu[4], ju[4];
-    uint64_t x = state;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        x = xs64_step(x);
-        iu[j] = (uint32_t)(x >> 40);
-        x = xs64_step(x);
-        ju[j] = (uint32_t)(x >> 40);
-    }
-    state = x;
-    Rounded rl[4], rc[4];
-    bool nl[4], nc[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        uint32_t i = iu[j] ? iu[j] : 1u;  // the zero uniform is replaced below
-        rl[j] = round_candidate(log_candidate(i, cal.log_tab));
-        if (LOG2T)
-            nl[j] = rl[j].dist < (1u << reinterpret_cast<const uint8_t*>(cal.log_delta)[i >> TSHIFT]);
-        else
-            nl[j] = rl[j].dist < cal.log_delta[i >> 16];
-        float theta = fmul(kTauF, (float)ju[j] * 5.9604644775390625e-08f);
-        rc[j] = round_candidate(cos_candidate(theta));
-        if (LOG2T)
-            nc[j] = rc[j].dist < (1u << reinterpret_cast<const uint8_t*>(cal.cos_delta)[ju[j] >> TSHIFT]);
-        else
-            nc[j] = rc[j].dist < cal.cos_delta[ju[j] >> 16];
-    }
-    uint32_t wl[4], wc[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        uint32_t i = iu[j] ? iu[j] : 1u;
-        wl[j] = nl[j] ? cal.log_flip[i >> 5] : 0u;
-        wc[j] = nc[j] ? cal.cos_flip[ju[j] >> 5] : 0u;
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        uint32_t i = iu[j] ? iu[j] : 1u;
-        // the bitmap's bit times the step to the other neighbour: a multiply-add (FMA pipe) instead of
-        // a compare and a select (integer pipe, the one that bounds this code)
-        uint32_t lb = rl[j].bits + (uint32_t)((int32_t)bit_of(wl[j], i) * rl[j].step);
-        uint32_t cb = rc[j].bits + (uint32_t)((int32_t)bit_of(wc[j], ju[j]) * rc[j].step);
-        float lg = iu[j] ? u2f(lb) : cal.log_of_zero;
-        out[j] = fmul(fsqrt(fmul(-2.0f, lg)), u2f(cb));
-    }
+// ---------------------------------------------------------------------------
+// The kernels' form: fp32 candidates.  fp64 operations and conversions share narrow pipes with each other and
+// with the tensor cores; here a normal is some 100 instructions, most of them on the full-rate fp32 pipe.
+// ---------------------------------------------------------------------------
+HSES_HD float ffma(float a, float b, float c) {
+#if defined(__CUDA_ARCH__)
+    return __fmaf_rn(a, b, c);
+#else
+    return fmaf(a, b, c);
+#endif
+}
+HSES_HD float fadd(float a, float b) {
+#if defined(__CUDA_ARCH__)
+    return __fadd_rn(a, b);
+#else
+    return a + b;
+#endif
+}
+HSES_HD float u2float(uint32_t v) {
+#if defined(__CUDA_ARCH__)
+    return __uint2float_rn(v);
+#else
+    return (float)v;
+#endif
+}
+HSES_HD float i2float(int32_t v) {
+#if defined(__CUDA_ARCH__)
+    return __int2float_rn(v);
+#else
+    return (float)v;
+#endif
 }
 
-HSES_HD void next_normals4(uint64_t& state, const LibmCal& cal, float (&out)[4]) {
-    next_normals4_t<false>(state, cal, out);
+constexpr int kLogRows = 64, kCosRows = 256;
+struct NoiseCal {
+    const float4* log_tab;      // kLogRows x {2^-24 / c, -log(1/c) high, low, filter width}
+    const float4* cos_tab;      // kCosRows x {t, cos t, sin t, low part of cos t}
+    const float* cos_width;     // kCosRows filter widths
+    const uint32_t* log_flip;   // 2^24 bits: which of the two roundings the host libm returns
+    const uint32_t* cos_flip;
+};
+// k * ln 2 in two parts; the factor 2^-23 undoes the scale of an exponent field read as an integer.  The high part
+// has 18 bits, like the table's, so that their sum is exact.
+constexpr float kLn2Hi = (float)(181704.0 / 262144.0 / 8388608.0);
+constexpr float kLn2Lo = (float)((0x1.62e42fefa39efp-1 - 181704.0 / 262144.0) / 8388608.0);
+constexpr float kUniform0 = 1e-9f * 16777216.0f;   // the reference raises u to 1e-9 (noiser.rs:471)
+
+// row of the log table an input uses
+HSES_HD int log_row(uint32_t i) {
+    float uf = u2float(i);
+    uf = uf > kUniform0 ? uf : kUniform0;
+    return (int)(((f2u(uf) - 0x4b400000u) >> 17) & 63u);
 }
-// ceil(log2(t)) of a 32-bit threshold as a byte (0 for t <= 1): dist < t implies dist < 2^byte
-HSES_HD uint8_t pack_threshold_log2(uint32_t t) {
-    uint8_t e = 0;
-    while (e < 31 && (1u << e) < t) ++e;
-    return e;
+// log(max(i 2^-24, 1e-9)) = hi + lo.  i = z 2^k with z in [0.75, 1.5) 2^24; the row's c divides z up to
+// r = z/c - 1, |r| < 2^-6 (rows 31 and 32 touch 1 and use c = 1: r is exact there).
+HSES_HD void log_parts(uint32_t i, const float4& e, float& hi, float& lo) {
+    float uf = u2float(i);
+    uf = uf > kUniform0 ? uf : kUniform0;
+    const uint32_t ix = f2u(uf), kb = (ix - 0x4b400000u) & 0xff800000u;
+    const float kf = i2float((int32_t)kb);
+    const float r = ffma(u2f(ix - kb), e.x, -1.0f);
+    const float th = ffma(kf, kLn2Hi, e.y), tl = ffma(kf, kLn2Lo, e.z);
+    hi = fadd(th, r);
+    const float er = fadd(r, -fadd(hi, -th));      // what the sum lost
+    float p = ffma(r, 0.2f, -0.25f);
+    p = ffma(r, p, 1.0f / 3.0f);
+    p = ffma(r, p, -0.5f);
+    lo = fadd(ffma(fmul(r, r), p, tl), er);
 }
+// cos of the fp32 product TAU * (j 2^-24) = hi + lo.  d = theta - t is exact, hi = cos t - d sin t rounded once, its
+// rounding error is recovered exactly, the rest is of second order.
+HSES_HD void cos_parts(uint32_t j, const float4& e, float& hi, float& lo) {
+    const float theta = fmul(u2float(j), kTauF * 5.9604644775390625e-08f);
+    const float d = fadd(theta, -e.x);
+    const float q = fmul(d, d);
+    const float inner = ffma(e.z, fmul(d, 1.0f / 6.0f), fmul(e.y, ffma(q, 1.0f / 24.0f, -0.5f)));
+    hi = ffma(-e.z, d, e.y);
+    const float res = ffma(-e.z, d, fadd(e.y, -hi));
+    lo = ffma(q, inner, fadd(res, e.w));
+}
+// the two roundings; they differ when the true value may lie on either side of a rounding boundary
+HSES_HD void roundings(float hi, float lo, float c, float& v0, float& v1) {
+    v0 = fadd(hi, ffma(hi, c, lo));
+    v1 = fadd(hi, ffma(hi, -c, lo));
+}
+HSES_HD int cos_row(uint32_t j) { return (int)(j >> 16); }
+
+#if defined(__CUDACC__)
+// sqrt of a normal, positive x, correctly rounded: one Newton step with an exact residual from an approximate
+// reciprocal root (Markstein, IBM J. Res. Dev. 34, 1990).  The argument is -2 log u, between 1e-7 and 42: none of the
+// special cases a general square root has to branch for.
+__device__ __forceinline__ float sqrt_residual(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    const float s = __fmul_rn(x, y);
+    return __fmaf_rn(__fmaf_rn(-s, s, x), __fmul_rn(0.5f, y), s);
+}
+// N consecutive normals (noiser.rs:470-477).  Laid out as independent chains — generator steps, logarithms, cosines,
+// then all bitmap reads together — so that table and bitmap latencies overlap instead of adding up.
+// The bitmap word's index i >> 5 is taken as the high half of a product: a shift would go to the integer pipe, which
+// bounds this code, the multiplier has room (223 -> 231 G normals/s).  The factor comes out of an opaque move, or the
+// compiler turns the product back into a shift.
+__device__ __forceinline__ uint32_t opaque(uint32_t v) {
+    uint32_t r;
+    asm("mov.b32 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
+}
+template <int N>
+__device__ __forceinline__ void normals(uint64_t& state, const NoiseCal& cal, float (&out)[N]) {
+    const uint32_t r5 = opaque(1u << 27);   // >> 5
+    uint32_t iu[N], ju[N];
+    uint64_t x = state;
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        x = xs64_step(x);
+        iu[n] = (uint32_t)(x >> 40);
+        x = xs64_step(x);
+        ju[n] = (uint32_t)(x >> 40);
+    }
+    state = x;
+    float l0[N], l1[N], c0[N], c1[N];
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        float hi, lo;
+        const float4 le = cal.log_tab[log_row(iu[n])];
+        log_parts(iu[n], le, hi, lo);
+        roundings(hi, lo, le.w, l0[n], l1[n]);
+        cos_parts(ju[n], cal.cos_tab[cos_row(ju[n])], hi, lo);
+        roundings(hi, lo, cal.cos_width[cos_row(ju[n])], c0[n], c1[n]);
+    }
+    uint32_t wl[N], wc[N];
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        wl[n] = l0[n] != l1[n] ? cal.log_flip[__umulhi(iu[n], r5)] : 0u;
+        wc[n] = c0[n] != c1[n] ? cal.cos_flip[__umulhi(ju[n], r5)] : 0u;
+    }
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        const float lg = (wl[n] & (1u << (iu[n] & 31u))) ? l1[n] : l0[n];
+        const float cs = (wc[n] & (1u << (ju[n] & 31u))) ? c1[n] : c0[n];
+        out[n] = __fmul_rn(sqrt_residual(__fmul_rn(-2.0f, lg)), cs);
+    }
+}
+__device__ __forceinline__ void normals4(uint64_t& state, const NoiseCal& cal, float (&out)[4]) { normals<4>(state, cal, out); }
+__device__ __forceinline__ float normal1(uint64_t& state, const NoiseCal& cal) {
+    float z[1];
+    normals<1>(state, cal, z);
+    return z[0];
+}
+// The candidate's tables in shared memory (6 KB); the caller synchronises.  Random rows of 16 bytes cost seven or
+// eight wavefronts a read, words three or four; with the width in the cosine rows (32-byte rows, half the banks) the
+// reads of a normal took 34 wavefronts and the L1 bounded the generator.
+struct CalTab {
+    float4 log_tab[kLogRows];
+    float4 cos_tab[kCosRows];
+    float cos_width[kCosRows];
+};
+__device__ __forceinline__ void stage_cal(NoiseCal& cal, CalTab& tab) {
+    for (int i = threadIdx.x; i < kLogRows; i += blockDim.x) tab.log_tab[i] = cal.log_tab[i];
+    for (int i = threadIdx.x; i < kCosRows; i += blockDim.x) {
+        tab.cos_tab[i] = cal.cos_tab[i];
+        tab.cos_width[i] = cal.cos_width[i];
+    }
+    cal.log_tab = tab.log_tab;
+    cal.cos_tab = tab.cos_tab;
+    cal.cos_width = tab.cos_width;
+}
+#endif
 
 }  // namespace hses

@@ -563,7 +563,7 @@ int hses_es_update_static(hses_ctx* ctx, hses_stream stream, uint64_t key, int32
     for (int64_t done = 0; done < p.pairs; done += p.chunk_pairs, ++chunk_idx) {
         int64_t cnt = p.pairs - done < p.chunk_pairs ? p.pairs - done : p.chunk_pairs;
         rc = launch_pair_factors(ctx, st, key, te, first_thread / 2 + (int32_t)done, cnt, rank, a, b,
-                                 fitness + 2 * done, wsA, wsB, /*no_alloc=*/true);
+                                 fitness + 2 * done, wsA, wsB);
         if (rc != HSES_OK) return rc;
         HSES_KERNEL(ctx, st, "update_gemm");
         // the first chunk overwrites the partial sums, so nothing left behind by an

@@ -43,12 +43,13 @@ struct UmMat {
     size_t part;                      // float offset of the partial sums
     int a, b, bn;                     // bn: columns per output tile
     int mt, nt;                       // row and column tiles
-    int gen0, gemm0, red0;            // first block of this matrix in each launch
+    int kb_a, kb_b;                   // k-blocks a CTA of update_operands makes of an A and of a B tile
+    int gen0, gen0_b, gemm0, red0;    // first block of this matrix in each launch (gen0_b: of its B tiles)
 };
 struct UmArgs {
     int n;
     const uint64_t *pow2, *lane4, *lane16;
-    LibmCal cal;
+    NoiseCal cal;
     int32_t true_epoch, first_pair;   // first_pair: of this chunk
     int64_t pair_off;                 // pairs of the call before this chunk
     int64_t pairs;                    // pairs of this chunk
@@ -87,127 +88,129 @@ __global__ void um_weight_range_kernel(const float* __restrict__ fitness, int64_
     }
 }
 
-// One operand tile.  Its normals are runs of consecutive stream values ("segments": the rows of the tile for one
-// pair, or, with rank > 64, 64 values of one row).  The segments' start states come from the power-of-two tables,
-// one segment per thread in parallel; from there a lane table spreads 32 threads over the segment.
+// The tiles of one row block in a few consecutive k-blocks, one after the other.  A tile's normals are runs of
+// consecutive stream values ("segments": the rows of the tile for one pair, or, with rank > 64, 64 values of one row).
+// The start states of all segments come from the power-of-two tables, one per thread side by side; from there a lane
+// table spreads 32 threads over a segment.
+constexpr int UM_STATES = 256;
+// values per start state and start states per segment of L values
+__host__ __device__ inline int um_run(int L) { return L >= 512 ? 512 : 128; }
+__host__ __device__ inline int um_starts(int L) { return (L + um_run(L) - 1) / um_run(L); }
+
 __global__ void __launch_bounds__(256) update_operands_kernel(const __grid_constant__ UmArgs g) {
     __shared__ __align__(16) float buf[UM_BUF];
-    __shared__ double2 log_tab_s[64];
-    __shared__ uint32_t delta_s[512];
-    __shared__ uint64_t seg_state[256];
+    __shared__ CalTab tab_s;
+    __shared__ uint64_t seg_state[UM_STATES];
     __shared__ float mul_s[64];
     const int tid = threadIdx.x;
     int i = 0;
     while (i + 1 < g.n && (int)blockIdx.x >= g.m[i + 1].gen0) ++i;
     const UmMat& m = g.m[i];
-    const int rel = (int)blockIdx.x - m.gen0, tiles = m.mt + m.nt;
-    const int64_t kb = rel / tiles;
-    const int s = rel - (int)kb * tiles;
-    const bool is_a = s < m.mt;
+    const bool is_a = (int)blockIdx.x < m.gen0_b;
+    const int rel = (int)blockIdx.x - (is_a ? m.gen0 : m.gen0_b), tiles = is_a ? m.mt : m.nt, kbn = is_a ? m.kb_a : m.kb_b;
+    const int s = rel % tiles;
+    const int64_t kb_lo = (int64_t)(rel / tiles) * kbn, kb_hi = min(kb_lo + kbn, g.kblks);
     const int dim = is_a ? m.a : m.b, step = is_a ? UM_ROWS : m.bn;
-    const int row0 = (is_a ? s : s - m.mt) * step, nrows = min(step, dim - row0);
+    const int row0 = s * step, nrows = min(step, dim - row0);
     const int r = g.r;
     const bool wide = r > 64;
-    const int64_t pair0 = wide ? kb / g.rkb : kb * g.pb;         // first pair of the tile (inside the chunk)
-    const int q0 = wide ? (int)(kb - pair0 * g.rkb) * 64 : 0;
-    const int npairs = wide ? 1 : (int)min((int64_t)g.pb, g.pairs - pair0);
-    const int nq = wide ? min(64, r - q0) : r;                   // rank values of the tile
-    const int nseg = wide ? nrows : npairs;
-    const int L = wide ? nq : nrows * r;                         // values per segment
+    const int max_seg = wide ? nrows : g.pb;
     const int LP = (((wide ? 64 : step * r) + 3) & ~3) + 4;      // pitch of a segment in shared memory
+    const int run = um_run(wide ? 64 : nrows * r), chn = run / 32;
+    const int cps = um_starts(wide ? 64 : nrows * r);
+    const int ns = max_seg * cps;                                // start states of a k-block
     const float* cache = is_a ? m.cache_a : m.cache_b;
-    if (tid < 64 && tid < npairs) {
-        float w = 1.0f;
-        if (is_a) {
-            const float* f = g.fitness + 2 * (pair0 + tid);
-            w = __fmul_rn(__fsub_rn(f[0], f[1]), ldexpf(1.0f, UM_EXP_A - *g.e_w));   // exact: a power of two
-        } else {
-            w = (float)(1 << UM_EXP_B);
-        }
-        mul_s[tid] = w;
-    }
-    if (cache) {
-        for (int sg = 0; sg < nseg; ++sg) {
-            const float* src = wide ? cache + ((size_t)(g.pair_off + pair0) * dim + row0 + sg) * r + q0
-                                    : cache + ((size_t)(g.pair_off + pair0 + sg) * dim + row0) * r;
-            if ((r & 3) == 0) {
-                for (int e = tid; e < L / 4; e += 256)
-                    *reinterpret_cast<float4*>(buf + sg * LP + 4 * e) = __ldg(reinterpret_cast<const float4*>(src) + e);
-            } else {
-                for (int e = tid; e < L; e += 256) buf[sg * LP + e] = __ldg(src + e);
-            }
-        }
-    } else {
-        LibmCal cal = g.cal;
-        for (int e = tid; e < 64; e += 256) log_tab_s[e] = cal.log_tab[e];
-        delta_s[tid] = cal.log_delta[tid];
-        delta_s[256 + tid] = cal.cos_delta[tid];
-        cal.log_tab = log_tab_s;
-        cal.log_delta = delta_s;
-        cal.cos_delta = delta_s + 256;
-        const bool coarse = L >= 512;                    // 16 normals per thread and table round, else 4
-        const int chn = coarse ? 16 : 4;
-        const int sub = chn * 32;                        // values a start state serves
-        const int cps = (L + sub - 1) / sub;             // start states per segment
-        const int ns = nseg * cps;                       // at most 128
-        for (int e = tid; e < ns; e += 256) {
-            const int sg = e / cps, c = e - sg * cps;
-            const int64_t pair = wide ? pair0 : pair0 + sg;
-            const uint64_t pos = (uint64_t)r * (uint64_t)((is_a ? m.b : 0) + row0 + (wide ? sg : 0)) + (uint64_t)q0 +
-                                 (uint64_t)c * sub;
+    const float sc_a = ldexpf(1.0f, UM_EXP_A - *g.e_w);
+    NoiseCal cal = g.cal;
+    if (!cache) {
+        stage_cal(cal, tab_s);
+        for (int e = tid; e < ns * (int)(kb_hi - kb_lo); e += 256) {
+            const int kr = e / ns, f = e - kr * ns, sg = f / cps, c = f - sg * cps;
+            const int64_t kb = kb_lo + kr;
+            const int64_t pair = wide ? kb / g.rkb : kb * g.pb + sg;
+            if (pair >= g.pairs) continue;
+            const uint64_t pos = (uint64_t)r * (uint64_t)((is_a ? m.b : 0) + row0 + (wide ? sg : 0)) +
+                                 (wide ? (uint64_t)(kb % g.rkb) * 64u : 0u) + (uint64_t)c * run;
             const uint64_t s0 = noise_seed(m.key, g.true_epoch, g.first_pair + (int32_t)pair) | 1ull;
             seg_state[e] = jump_by(g.pow2, s0, 2ull * pos);
         }
-        __syncthreads();
-        const int ppp = min(32, (min(L, sub) + chn - 1) / chn);   // pieces per start state
-        const uint64_t* tab = coarse ? g.lane16 : g.lane4;
-        for (int u = tid; u < ns * ppp; u += 256) {
-            const int e = ppp == 32 ? u >> 5 : u / ppp, piece = u - e * ppp;
-            const int sg = cps == 1 ? e : e / cps, c = e - sg * cps;
-            const int off = c * sub + piece * chn;
-            if (off >= L) continue;
-            uint64_t st = lane_jump(tab, seg_state[e], piece);
-            float* dst = buf + sg * LP + off;
-            for (int j = 0; j < chn && off + j < L; j += 4) {
-                float z[4];
-                next_normals4(st, cal, z);
-                *reinterpret_cast<float4*>(dst + j) = make_float4(z[0], z[1], z[2], z[3]);
-            }
-        }
     }
-    __syncthreads();
-    // eight consecutive K values of a row per thread; eight lanes fill a 128-byte row of the image
-    const int nr8 = is_a ? rows8(nrows) : min(m.bn, (nrows + 15) & ~15);
-    const int dim_pad = is_a ? rows8(m.a) : m.nt * m.bn;         // rows of the operand in a k-block's images
-    uint8_t* img = g.images + (is_a ? m.img_a : m.img_b) + (size_t)kb * dim_pad * 256 + (size_t)row0 * 256;
-    uint8_t* img_lo = img + (size_t)(is_a ? nr8 : m.bn) * 128;
-    for (int idx = tid; idx < nr8 * 8; idx += 256) {
-        const int row = idx >> 3, c = idx & 7;
-        float v[8];
-        int pp = wide ? 0 : (c * 8) / r, q = c * 8 - pp * r;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            float x = 0.0f;
-            if (row < nrows && pp < npairs && q < nq) {
-                x = wide ? buf[row * LP + q] : buf[pp * LP + row * r + q];
-                if (g.sign_factors) x = (float)sign_of(x);   // AltEggRoll contracts the sign patterns
-                x = __fmul_rn(x, mul_s[pp]);
+    for (int64_t kb = kb_lo; kb < kb_hi; ++kb) {
+        const int64_t pair0 = wide ? kb / g.rkb : kb * g.pb;     // first pair of the tile (inside the chunk)
+        const int q0 = wide ? (int)(kb - pair0 * g.rkb) * 64 : 0;
+        const int npairs = wide ? 1 : (int)min((int64_t)g.pb, g.pairs - pair0);
+        const int nq = wide ? min(64, r - q0) : r;               // rank values of the tile
+        const int nseg = wide ? nrows : npairs;
+        const int L = wide ? nq : nrows * r;                     // values per segment
+        __syncthreads();   // the states are there; the previous tile's values are no longer read
+        if (tid < npairs) {
+            const float* f = g.fitness + 2 * (pair0 + tid);
+            mul_s[tid] = is_a ? __fmul_rn(__fsub_rn(f[0], f[1]), sc_a) : (float)(1 << UM_EXP_B);   // sc_a: a power of two
+        }
+        if (cache) {
+            for (int sg = 0; sg < nseg; ++sg) {
+                const float* src = wide ? cache + ((size_t)(g.pair_off + pair0) * dim + row0 + sg) * r + q0
+                                        : cache + ((size_t)(g.pair_off + pair0 + sg) * dim + row0) * r;
+                if ((r & 3) == 0) {
+                    for (int e = tid; e < L / 4; e += 256)
+                        *reinterpret_cast<float4*>(buf + sg * LP + 4 * e) = __ldg(reinterpret_cast<const float4*>(src) + e);
+                } else {
+                    for (int e = tid; e < L; e += 256) buf[sg * LP + e] = __ldg(src + e);
+                }
             }
-            v[j] = x;
-            if (++q == r && !wide) q = 0, ++pp;
+        } else {
+            const uint64_t* states = seg_state + (int)(kb - kb_lo) * ns;
+            const int ppp = min(32, (min(L, run) + chn - 1) / chn);   // pieces per start state
+            const uint64_t* tab = chn == 16 ? g.lane16 : g.lane4;
+            for (int u = tid; u < nseg * cps * ppp; u += 256) {
+                const int e = ppp == 32 ? u >> 5 : u / ppp, piece = u - e * ppp;
+                const int sg = cps == 1 ? e : e / cps, c = e - sg * cps;
+                const int off = c * run + piece * chn;
+                if (off >= L) continue;
+                uint64_t st = lane_jump(tab, states[e], piece);
+                float* dst = buf + sg * LP + off;
+#pragma unroll 1
+                for (int j = 0; j < chn && off + j < L; j += 4) {
+                    float z[4];
+                    normals4(st, cal, z);
+                    *reinterpret_cast<float4*>(dst + j) = make_float4(z[0], z[1], z[2], z[3]);
+                }
+            }
         }
-        uint32_t h[4], l[4];
+        __syncthreads();
+        // eight consecutive K values of a row per thread; eight lanes fill a 128-byte row of the image
+        const int nr8 = is_a ? rows8(nrows) : min(m.bn, (nrows + 15) & ~15);
+        const int dim_pad = is_a ? rows8(m.a) : m.nt * m.bn;         // rows of the operand in a k-block's images
+        uint8_t* img = g.images + (is_a ? m.img_a : m.img_b) + (size_t)kb * dim_pad * 256 + (size_t)row0 * 256;
+        uint8_t* img_lo = img + (size_t)(is_a ? nr8 : m.bn) * 128;
+        for (int idx = tid; idx < nr8 * 8; idx += 256) {
+            const int row = idx >> 3, c = idx & 7;
+            float v[8];
+            int pp = wide ? 0 : (c * 8) / r, q = c * 8 - pp * r;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const __half2 hh = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
-            const float2 b = __half22float2(hh);
-            const __half2 ll = __floats2half2_rn(v[2 * j] - b.x, v[2 * j + 1] - b.y);
-            h[j] = *reinterpret_cast<const uint32_t*>(&hh);
-            l[j] = *reinterpret_cast<const uint32_t*>(&ll);
+            for (int j = 0; j < 8; ++j) {
+                float x = 0.0f;
+                if (row < nrows && pp < npairs && q < nq) {
+                    x = wide ? buf[row * LP + q] : buf[pp * LP + row * r + q];
+                    if (g.sign_factors) x = (float)sign_of(x);   // AltEggRoll contracts the sign patterns
+                    x = __fmul_rn(x, mul_s[pp]);
+                }
+                v[j] = x;
+                if (++q == r && !wide) q = 0, ++pp;
+            }
+            uint32_t h[4], l[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const __half2 hh = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
+                const float2 b = __half22float2(hh);
+                const __half2 ll = __floats2half2_rn(v[2 * j] - b.x, v[2 * j + 1] - b.y);
+                h[j] = *reinterpret_cast<const uint32_t*>(&hh);
+                l[j] = *reinterpret_cast<const uint32_t*>(&ll);
+            }
+            const int o = (row >> 3) * 1024 + (row & 7) * 128 + ((c ^ (row & 7)) << 4);
+            *reinterpret_cast<uint4*>(img + o) = make_uint4(h[0], h[1], h[2], h[3]);
+            *reinterpret_cast<uint4*>(img_lo + o) = make_uint4(l[0], l[1], l[2], l[3]);
         }
-        const int o = (row >> 3) * 1024 + (row & 7) * 128 + ((c ^ (row & 7)) << 4);
-        *reinterpret_cast<uint4*>(img + o) = make_uint4(h[0], h[1], h[2], h[3]);
-        *reinterpret_cast<uint4*>(img_lo + o) = make_uint4(l[0], l[1], l[2], l[3]);
     }
 }
 
@@ -217,11 +220,15 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                  : "memory");
 }
 
-// warp 0: copies, warp 1: MMAs, warps 2-5: partial sums out of TMEM
+// warp 0: copies, warp 1: MMAs, warps 2-5: sums.  The tensor core adds into its accumulator with truncation, an error
+// that grows with the chain: after UM_CHAIN k-blocks (24 MMAs) the MMAs go on in the other of two accumulators and the
+// warps add the finished one to fp32 sums in registers, one output row per thread.  One chain over 64 k-blocks left
+// gradients 2e-4 of their spread away from the fp32 kernel's.
+constexpr int UM_CHAIN = 2;
 __global__ void __launch_bounds__(192, 1) update_gemm_tc_kernel(const __grid_constant__ UmArgs g) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    __shared__ uint64_t full[UM_STAGES], empty[UM_STAGES], tfull;
+    __shared__ uint64_t full[UM_STAGES], empty[UM_STAGES], tfull[2], tempty[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag_s;
     volatile int* abort_flag = &abort_flag_s;
@@ -233,6 +240,7 @@ __global__ void __launch_bounds__(192, 1) update_gemm_tc_kernel(const __grid_con
     const int split = rel % g.splits, tile = rel / g.splits;
     const int nt = tile % m.nt, mt = tile / m.nt;
     const int64_t k_lo = g.kblks * split / g.splits, k_hi = g.kblks * (split + 1) / g.splits;
+    const uint32_t kn = (uint32_t)(k_hi - k_lo);
     const int arows = rows8(min(UM_ROWS, m.a - mt * UM_ROWS));
     const uint32_t a_bytes = (uint32_t)arows * 128, b_bytes = (uint32_t)m.bn * 128;
     if (threadIdx.x == 0) {
@@ -241,11 +249,14 @@ __global__ void __launch_bounds__(192, 1) update_gemm_tc_kernel(const __grid_con
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
-        mbar_init(&tfull, 1);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&tfull[b], 1);
+            mbar_init(&tempty[b], 128);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(128)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(256)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -259,14 +270,13 @@ __global__ void __launch_bounds__(192, 1) update_gemm_tc_kernel(const __grid_con
             const uint8_t* ia = g.images + m.img_a + (size_t)mt * UM_ROWS * 256;
             const uint8_t* ib = g.images + m.img_b + (size_t)nt * m.bn * 256;
             const size_t sa = (size_t)rows8(m.a) * 256, sb = (size_t)m.nt * m.bn * 256;
-            for (int64_t kb = k_lo; kb < k_hi; ++kb) {
-                const uint32_t it = (uint32_t)(kb - k_lo);
+            for (uint32_t it = 0; it < kn; ++it) {
                 const int s = it % UM_STAGES;
                 if (!mbar_wait(&empty[s], ((it / UM_STAGES) & 1) ^ 1, abort_flag, g.status, 11)) { ok = false; break; }
                 uint8_t* st = smem + (size_t)s * UM_STAGE_BYTES;
                 mbar_expect_tx(&full[s], 2 * a_bytes + 2 * b_bytes);
-                bulk_load(st, ia + kb * sa, 2 * a_bytes, &full[s]);                       // hi, then lo
-                bulk_load(st + 2 * UM_ROWS * 128, ib + kb * sb, 2 * b_bytes, &full[s]);
+                bulk_load(st, ia + (k_lo + it) * sa, 2 * a_bytes, &full[s]);              // hi, then lo
+                bulk_load(st + 2 * UM_ROWS * 128, ib + (k_lo + it) * sb, 2 * b_bytes, &full[s]);
             }
             if (!ok)
                 for (int s = 0; s < UM_STAGES; ++s)
@@ -278,11 +288,14 @@ __global__ void __launch_bounds__(192, 1) update_gemm_tc_kernel(const __grid_con
     } else if (warp == 1) {
         if (lane == 0) {
             const uint32_t idesc = make_idesc(m.bn);
-            bool ok = true;
-            for (int64_t kb = k_lo; kb < k_hi; ++kb) {
-                const uint32_t it = (uint32_t)(kb - k_lo);
+            for (uint32_t it = 0; it < kn; ++it) {
+                const uint32_t chain = it / UM_CHAIN, b = chain & 1;
+                if (it % UM_CHAIN == 0) {
+                    if (!mbar_wait(&tempty[b], ((chain >> 1) & 1) ^ 1, abort_flag, g.status, 14)) break;
+                    tc_fence_after();
+                }
                 const int s = it % UM_STAGES;
-                if (!mbar_wait(&full[s], (it / UM_STAGES) & 1, abort_flag, g.status, 12)) { ok = false; break; }
+                if (!mbar_wait(&full[s], (it / UM_STAGES) & 1, abort_flag, g.status, 12)) break;
                 tc_fence_after();
                 uint8_t* st = smem + (size_t)s * UM_STAGE_BYTES;
                 const uint64_t dah = make_smem_desc(st), dal = make_smem_desc(st + a_bytes);
@@ -290,43 +303,52 @@ __global__ void __launch_bounds__(192, 1) update_gemm_tc_kernel(const __grid_con
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks) {
                     const uint64_t off = (uint64_t)(ks * 32 >> 4);
-                    umma_f16(tmem, dal + off, dbh + off, idesc, (it | ks) != 0);
-                    umma_f16(tmem, dah + off, dbl + off, idesc, 1);
-                    umma_f16(tmem, dah + off, dbh + off, idesc, 1);
+                    umma_f16(tmem + b * 128, dal + off, dbh + off, idesc, (it % UM_CHAIN | ks) != 0);
+                    umma_f16(tmem + b * 128, dah + off, dbl + off, idesc, 1);
+                    umma_f16(tmem + b * 128, dah + off, dbh + off, idesc, 1);
                 }
                 umma_commit(&empty[s]);
+                if (it % UM_CHAIN == UM_CHAIN - 1 || it + 1 == kn) umma_commit(&tfull[b]);
             }
-            if (ok && k_hi > k_lo) umma_commit(&tfull);
         }
     } else {
         const int q4 = warp & 3;
-        bool have = k_hi > k_lo && mbar_wait(&tfull, 0, abort_flag, g.status, 13);
-        have = __all_sync(0xffffffffu, have);
-        tc_fence_after();
-        const int row = mt * UM_ROWS + q4 * 32 + lane, n0 = nt * m.bn;
-        float* dst = g.partial + m.part + ((size_t)split * m.a + (row < m.a ? row : 0)) * m.b;
-        if (mt * UM_ROWS + q4 * 32 < m.a) {                        // warp-uniform
-            for (int j0 = 0; j0 < m.bn && n0 + j0 < m.b; j0 += 8) {
-                uint32_t acc[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-                if (have) tmem_ld8(tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)j0, acc);
-                if (row < m.a) {
+        float sum[UM_ROWS];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const int n = n0 + j0 + j;
-                        if (n < m.b) {
-                            const float v = __uint_as_float(acc[j]);
-                            dst[n] = g.accumulate ? dst[n] + v : v;
-                        }
-                    }
+        for (int j = 0; j < UM_ROWS; ++j) sum[j] = 0.0f;
+        for (uint32_t chain = 0; chain * UM_CHAIN < kn; ++chain) {
+            const uint32_t b = chain & 1;
+            bool have = mbar_wait(&tfull[b], (chain >> 1) & 1, abort_flag, g.status, 13);
+            have = __all_sync(0xffffffffu, have);                  // the TMEM loads are warp-wide
+            if (!have) break;
+            tc_fence_after();
+#pragma unroll
+            for (int j0 = 0; j0 < UM_ROWS; j0 += 16) {
+                if (j0 < m.bn) {
+                    uint32_t acc[2][8];
+                    tmem_ld8_issue(tmem + ((uint32_t)(q4 * 32) << 16) + b * 128 + j0, acc[0]);
+                    tmem_ld8_issue(tmem + ((uint32_t)(q4 * 32) << 16) + b * 128 + j0 + 8, acc[1]);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) sum[j0 + j] = __fadd_rn(sum[j0 + j], __uint_as_float(acc[j >> 3][j & 7]));
                 }
             }
+            tc_fence_before();
+            mbar_arrive(&tempty[b]);
+        }
+        const int row = mt * UM_ROWS + q4 * 32 + lane, n0 = nt * m.bn;
+        if (row < m.a) {
+            float* dst = g.partial + m.part + ((size_t)split * m.a + row) * m.b;
+#pragma unroll
+            for (int j = 0; j < UM_ROWS; ++j)
+                if (j < m.bn && n0 + j < m.b) dst[n0 + j] = g.accumulate ? __fadd_rn(dst[n0 + j], sum[j]) : sum[j];
         }
     }
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256) : "memory");
     }
 }
 
@@ -461,10 +483,23 @@ int run_update_multi(hses_ctx* ctx, cudaStream_t st, const UpdateMultiItem* item
             img += (size_t)m.nt * m.bn * 256 * g.kblks;
             m.part = part;
             part += (size_t)p.splits * m.a * m.b;
+            // enough k-blocks per CTA that its set-up (tables, start states) is a small part of it, as long as the
+            // launch still has blocks for every SM; the states of all of them have room in shared memory
+            auto k_blocks_of = [&](int rows, int tiles) {
+                const int L = c.rank > 64 ? 64 : rows * c.rank;
+                const int ns = (c.rank > 64 ? rows : p.pb) * um_starts(L);
+                const int64_t want = std::max<int64_t>(1, 16384 / (64 * rows));
+                const int64_t fill = std::max<int64_t>(1, g.kblks * tiles * n / (4 * (int64_t)ctx->sm_count));
+                return (int)std::max<int64_t>(1, std::min({want, fill, (int64_t)(UM_STATES / ns)}));
+            };
+            m.kb_a = k_blocks_of(std::min(m.a, UM_ROWS), m.mt);
+            m.kb_b = k_blocks_of(std::min(m.b, m.bn), m.nt);
             m.gen0 = (int)gen;
             m.gemm0 = (int)gemm;
             m.red0 = (int)red;
-            gen += g.kblks * (m.mt + m.nt);
+            gen += (g.kblks + m.kb_a - 1) / m.kb_a * m.mt;
+            m.gen0_b = (int)gen;
+            gen += (g.kblks + m.kb_b - 1) / m.kb_b * m.nt;
             gemm += (int64_t)m.mt * m.nt * p.splits;
             red += ((int64_t)m.a * m.b + 31) / 32;
         }
