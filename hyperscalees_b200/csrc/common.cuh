@@ -158,6 +158,44 @@ __device__ __forceinline__ void stream_fill(const NoiseCal& cal, const uint64_t*
     }
 }
 #endif
+#if defined(__CUDACC__)
+__device__ __forceinline__ uint32_t poisson_seed(uint32_t idx, uint32_t mix) {
+    return 1000000007u * idx + mix + 0x9E3779B9u;
+}
+
+__device__ __forceinline__ uint32_t xs32(uint32_t x) {
+    x ^= x << 13;
+    x ^= x >> 17;
+    x ^= x << 5;
+    return x;
+}
+
+// The reference compares u = fl((k+1)/8388609) with p at every step, k being
+// the top 23 bits of the xorshift32 output.  fl(n/8388609) is monotone in n,
+// so "u < p" is "n < n*(p)" with n* the smallest n whose quotient reaches p.
+// n* is found once per element with exact divisions; the T steps are then
+// integer-only.
+__device__ __forceinline__ uint32_t poisson_threshold(float p) {
+    const float D = 8388609.0f;
+    float guess = __fmul_rn(p, D);
+    uint32_t c = guess >= 1.0f ? (guess < 8388609.0f ? (uint32_t)guess : 8388609u) : 1u;
+    while (c > 1u && __fdiv_rn((float)(c - 1u), D) >= p) --c;
+    while (c <= 8388608u && __fdiv_rn((float)c, D) < p) ++c;
+    return c;
+}
+// fitness of one sample (hyperscalees-envs/src/snn_mnist.rs:180-201)
+__device__ __forceinline__ float sample_fitness(const float* row, int classes, int label, int reward) {
+    float mx = row[0];
+    int arg = 0;
+    for (int c = 1; c < classes; ++c)
+        if (row[c] > mx) { mx = row[c]; arg = c; }
+    if (reward == HSES_REWARD_BINARY) return arg == label ? 1.0f : 0.0f;
+    float sum = 0.0f;
+    for (int c = 0; c < classes; ++c) sum = __fadd_rn(sum, expf(__fsub_rn(row[c], mx)));
+    const float picked = (label >= 0 && label < classes) ? row[label] : __int_as_float(0x7fc00000);
+    return __fsub_rn(__fsub_rn(picked, mx), logf(sum));
+}
+#endif
 // lif_step (hyperscalees-models/src/snn.rs:53-65): charge, threshold, reset; returns the spike
 __device__ __forceinline__ float lif_update(float& v, float cur, float leak, float v_th, int reset) {
     float d = __fadd_rn(-v, cur);

@@ -9,31 +9,6 @@ namespace hses {
 // ---------------------------------------------------------------------------
 // Poisson encode (poisson_encode_fused_oxide.rs:36-105)
 // ---------------------------------------------------------------------------
-// The reference compares u = fl((k+1)/8388609) with p at every step, k being
-// the top 23 bits of the xorshift32 output.  fl(n/8388609) is monotone in n,
-// so "u < p" is "n < n*(p)" with n* the smallest n whose quotient reaches p.
-// n* is found once per element with exact divisions; the T steps are then
-// integer-only.
-__device__ __forceinline__ uint32_t poisson_threshold(float p) {
-    const float D = 8388609.0f;
-    float guess = __fmul_rn(p, D);
-    uint32_t c = guess >= 1.0f ? (guess < 8388609.0f ? (uint32_t)guess : 8388609u) : 1u;
-    while (c > 1u && __fdiv_rn((float)(c - 1u), D) >= p) --c;
-    while (c <= 8388608u && __fdiv_rn((float)c, D) < p) ++c;
-    return c;
-}
-
-__device__ __forceinline__ uint32_t poisson_seed(uint32_t idx, uint32_t mix) {
-    return 1000000007u * idx + mix + 0x9E3779B9u;
-}
-
-__device__ __forceinline__ uint32_t xs32(uint32_t x) {
-    x ^= x << 13;
-    x ^= x >> 17;
-    x ^= x << 5;
-    return x;
-}
-
 // out_half (optional, dense rows of in_dim values): the same spikes as fp16 0/1, the operand
 // format of the tensor-core layer that follows, so that it need not convert them itself.
 template <int VEC>
@@ -161,20 +136,7 @@ __global__ void fitness_kernel(const float* __restrict__ logits, int64_t n, int 
                                float* __restrict__ out) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float* row = logits + (size_t)i * classes;
-    float mx = row[0];
-    int arg = 0;
-    for (int c = 1; c < classes; ++c)
-        if (row[c] > mx) { mx = row[c]; arg = c; }
-    int label = labels[i];
-    if (reward == HSES_REWARD_BINARY) {
-        out[i] = arg == label ? 1.0f : 0.0f;
-    } else {
-        float sum = 0.0f;
-        for (int c = 0; c < classes; ++c) sum = __fadd_rn(sum, expf(__fsub_rn(row[c], mx)));
-        float picked = (label >= 0 && label < classes) ? row[label] : __int_as_float(0x7fc00000);
-        out[i] = __fsub_rn(__fsub_rn(picked, mx), logf(sum));
-    }
+    out[i] = sample_fitness(logits + (size_t)i * classes, classes, labels[i], reward);
 }
 
 __global__ void member_mean_kernel(const float* __restrict__ x, int64_t n_pop, int bm,

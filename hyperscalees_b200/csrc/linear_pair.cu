@@ -58,13 +58,6 @@ struct PairArgs {
     int* status;
 };
 
-// plain (untiled) bulk copy global -> shared; both addresses 16-byte aligned, size a multiple of 16
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-
 // The pair's B and the matching columns of its x rows stream through a ring of PP_STAGES
 // shared-memory stages filled by the copy engine, two copies per pass: the B rows of a pass are
 // contiguous (one untiled bulk copy) and the pair's x rows are one box (columns, the pair's

@@ -8,6 +8,7 @@
 
 #include "common.cuh"
 #include "linear.cuh"
+#include "snn_layer.cuh"
 #include "update_tc.cuh"
 
 namespace hses {
@@ -99,6 +100,7 @@ extern "C" {
 
 size_t hses_snn_forward_workspace_bytes(const hses_snn_model* m, const hses_pop_args* p) {
     if (check_model(m, p) != HSES_OK) return 0;
+    if (snn_fused_supports(m, p)) return snn_fused_workspace_bytes(m, p);
     return plan_forward(m, p).bytes;
 }
 
@@ -195,7 +197,15 @@ static int snn_forward_impl(hses_ctx* ctx, hses_stream stream, const hses_snn_mo
 int hses_snn_forward(hses_ctx* ctx, hses_stream stream, const hses_snn_model* m, const hses_pop_args* p,
                      const float* spikes_in, int64_t in_stride, float* logits, void* workspace,
                      size_t workspace_bytes) {
-    return snn_forward_impl(ctx, stream, m, p, spikes_in, in_stride, nullptr, logits, workspace, workspace_bytes);
+    if (check_model(m, p) != HSES_OK || !snn_fused_supports(m, p))
+        return snn_forward_impl(ctx, stream, m, p, spikes_in, in_stride, nullptr, logits, workspace, workspace_bytes);
+    HSES_REQUIRE(ctx != nullptr, "ctx is NULL");
+    HSES_REQUIRE(m->weights != nullptr && m->weight_strides != nullptr, "weights are NULL");
+    HSES_REQUIRE(!p->perturb || m->keys != nullptr, "keys are NULL");
+    HSES_REQUIRE(spikes_in != nullptr && logits != nullptr, "NULL pointer");
+    HSES_REQUIRE(in_stride >= m->dims[0], "in_stride smaller than the input width");
+    return run_snn_fused(ctx, as_stream(stream), m, p, SnnInput{spikes_in, nullptr, in_stride, nullptr}, logits, SnnScore{},
+                         workspace, workspace_bytes);
 }
 
 // The encoder can hand the first layer an fp16 copy of the spikes when a dense fp16 row is a
@@ -204,6 +214,7 @@ static bool eval_writes_half(const hses_snn_model* m) { return m->n_layers > 1 &
 
 size_t hses_population_eval_workspace_bytes(const hses_snn_model* m, const hses_pop_args* p) {
     if (check_model(m, p) != HSES_OK) return 0;
+    if (snn_fused_supports(m, p)) return snn_fused_workspace_bytes(m, p);
     FwdPlan f = plan_forward(m, p);
     size_t in_stride = (size_t)(m->dims[0] + 3) / 4 * 4;
     size_t extra = up64((size_t)p->T * f.rows * in_stride) + up64(f.rows * (size_t)m->dims[m->n_layers]) +
@@ -224,13 +235,20 @@ int hses_population_eval(hses_ctx* ctx, hses_stream stream, const hses_snn_model
     size_t need = hses_population_eval_workspace_bytes(m, p);
     HSES_REQUIRE(workspace != nullptr && workspace_bytes >= need && ((uintptr_t)workspace & 255u) == 0,
                  "workspace too small or not 256-byte aligned; see hses_population_eval_workspace_bytes");
-    FwdPlan f = plan_forward(m, p);
     const int in = m->dims[0], classes = m->dims[m->n_layers];
     // the encoder writes with the pitch of its input; a dense copy of the images would cost a pass,
     // so the spike buffer simply takes the image pitch when it fits the reserved width
     size_t reserved = (size_t)(in + 3) / 4 * 4;
     HSES_REQUIRE((size_t)image_stride <= reserved || image_stride == in,
                  "image row stride must be the input width or its 4-element round-up");
+    if (snn_fused_supports(m, p)) {
+        HSES_REQUIRE(m->weights != nullptr && m->weight_strides != nullptr, "weights are NULL");
+        HSES_REQUIRE(!p->perturb || m->keys != nullptr, "keys are NULL");
+        HSES_REQUIRE(image_stride >= in, "image row stride smaller than the input width");
+        return run_snn_fused(ctx, as_stream(stream), m, p, SnnInput{nullptr, images, image_stride, seeds}, logits_out,
+                             SnnScore{labels, reward, raw_fitness}, workspace, workspace_bytes);
+    }
+    FwdPlan f = plan_forward(m, p);
     uint8_t* base = reinterpret_cast<uint8_t*>(workspace);
     float* spikes = reinterpret_cast<float*>(base + f.bytes);
     float* logits = spikes + up64((size_t)p->T * f.rows * reserved);

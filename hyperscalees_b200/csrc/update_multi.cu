@@ -214,12 +214,6 @@ __global__ void __launch_bounds__(256) update_operands_kernel(const __grid_const
     }
 }
 
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-
 // warp 0: copies, warp 1: MMAs, warps 2-5: sums.  The tensor core adds into its accumulator with truncation, an error
 // that grows with the chain: after UM_CHAIN k-blocks (24 MMAs) the MMAs go on in the other of two accumulators and the
 // warps add the finished one to fp32 sums in registers, one output row per thread.  One chain over 64 k-blocks left

@@ -85,6 +85,8 @@ class SnnMlp:
         perturbed with thread id first_thread + i (clean forward when frozen is None)."""
         T, n_pop, bm, _ = x.shape
         perturb = frozen is not None
+        if algo == ops.ALGO_AUTO and not want_hidden:
+            return self._forward_composite(x, frozen, noiser, base_keys, epoch, first_thread)
         kw = dict(n_pop=n_pop, bm=bm, perturb=perturb, algo=algo)
         if perturb:
             kw.update(sigma=noiser.sigma, rank=frozen.rank, epoch=epoch, first_thread=first_thread,
@@ -104,6 +106,38 @@ class SnnMlp:
         gain = float(self.out_gain.reshape(-1)[0].item())
         logits = ops.perturbed_linear(rate, self.weights[-1], t_steps=1, key=key, out_scale=gain, **kw)
         return (logits, hidden) if want_hidden else logits
+
+    def _forward_composite(self, x, frozen, noiser, base_keys, epoch, first_thread):
+        """One call of hses_snn_forward: the gain is read on the device, nothing waits for it."""
+        import ctypes as C
+        from . import _lib
+        from .core import current_stream, get_context
+        T, n_pop, bm, k = x.shape
+        ops._check(x, "x")
+        _, _, xs = ops._rows_2d(x, "x")
+        n = len(self.weights)
+        for w in self.weights:
+            ops._check(w, "param", ndim=2)
+            if w.shape[1] != k:
+                raise ValueError("param must be (a, k) with k = x's last dim")
+            k = w.shape[0]
+        perturb = frozen is not None
+        gain = self.out_gain.to(device=x.device, dtype=torch.float32)
+        keys = (C.c_uint64 * n)(*([int(v) & ((1 << 64) - 1) for v in base_keys[:n]] if perturb else [0] * n))
+        m = _lib.SnnModelDesc(n, (C.c_int32 * (n + 1))(x.shape[-1], *[w.shape[0] for w in self.weights]),
+                              (C.c_void_p * n)(*[w.data_ptr() for w in self.weights]),
+                              (C.c_int64 * n)(*[max(w.stride(0), w.shape[1]) for w in self.weights]), keys, 1.0,
+                              gain.data_ptr(), self.tau_m, (C.c_float * max(n - 1, 1))(*([self.v_th] * max(n - 1, 1))),
+                              self.reset_mode, None)
+        p = _lib.PopArgs(T, n_pop, bm, int(perturb), noiser.sigma if perturb else 0.0, frozen.rank if perturb else 1, epoch,
+                         first_thread, frozen.noise_reuse if perturb else 0)
+        L = _lib.load()
+        need = int(L.hses_snn_forward_workspace_bytes(C.byref(m), C.byref(p)))
+        ws = ops._workspace(x.device, need)
+        logits = torch.empty((n_pop * bm, self.weights[-1].shape[0]), dtype=torch.float32, device=x.device)
+        _lib.check(L.hses_snn_forward(get_context(x.device).handle, current_stream(), C.byref(m), C.byref(p), x.data_ptr(),
+                                      xs, logits.data_ptr(), ws.data_ptr() if ws is not None else None, need))
+        return logits
 
 
 class SnnModel(SnnMlp):
