@@ -28,7 +28,8 @@ namespace {
 using namespace tc;
 using namespace pack;
 
-constexpr int SL_THREADS = 320;          // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
+constexpr int SL_THREADS = 320;          // warp 0 TMA, warp 1 MMA, warps 2-9 scan; with noise also
+constexpr int SL_THREADS_T = 576;        // warps 10-17: t to operand layout
 constexpr int SL_MAX_STAGES = 6;
 constexpr int SL_SMEM_LIMIT = 232448;
 constexpr int kSnnMaxLayers = 8;         // hidden layers
@@ -131,7 +132,8 @@ __global__ void __launch_bounds__(256) snn_factors_kernel(const __grid_constant_
 
 // ------------------------------------------------------------------------- hidden layer
 struct LayerArgs {
-    int T, spt;              // steps, samples per tile (spt * T <= 128)
+    int T, spt;              // steps, samples per tile; (T - 1) * spt and spt rounded up to 8 fit `rows`
+    int rows;                // 128: two accumulators in turn; 192, 256: one, W and the factors read less often
     int64_t n;               // samples
     int64_t tiles;
     int ppt;                 // whole pairs per tile, or 0: tpp tiles inside a pair
@@ -168,7 +170,7 @@ struct Ring {
 };
 struct Scan {
     uint32_t y, u;           // TMEM address of sample 0's first step in the accumulators of the product and of the rank term
-    int T, cnt;              // samples of the tile
+    int T, spt, cnt;         // samples of the tile
     bool live;
     float cs, leak, v_th;
     const float* row_scale;  // of sample 0, step 0, or NULL
@@ -182,21 +184,14 @@ struct Scan {
 // these warps, and a loop over the steps: unrolled for a known T the same work was bound by fetching instructions.
 template <bool PERT, bool HARD>
 __device__ __forceinline__ void scan8(const Scan& c, int sb) {
-    uint32_t ny[8], nu[8], col[8];
+    uint32_t ny[8], nu[8];
     float v[8], sum[8];
     const int left = c.cnt - sb;                                // samples of this block, uniform
 #pragma unroll
-    for (int s = 0; s < 8; ++s) {
-        v[s] = sum[s] = 0.0f;
-        col[s] = c.y + (sb + min(s, left - 1)) * c.T;           // past the last sample: that one again, not stored
-    }
-    const uint32_t y_to_u = c.u - c.y;
-    auto load = [&](int t) {                                    // no branch here: these loads are for converged warps
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {
-            tmem_ld1_issue(col[s] + t, ny[s]);
-            if (PERT) tmem_ld1_issue(col[s] + t + y_to_u, nu[s]);
-        }
+    for (int s = 0; s < 8; ++s) v[s] = sum[s] = 0.0f;
+    auto load = [&](int t) {
+        tmem_ld8_issue(c.y + t * c.spt + sb, ny);
+        if (PERT) tmem_ld8_issue(c.u + t * c.spt + sb, nu);
     };
     load(0);
     unsigned short* out = c.out ? reinterpret_cast<unsigned short*>(c.out) + (int64_t)sb * c.T * c.out_pitch : nullptr;
@@ -241,7 +236,7 @@ __device__ __forceinline__ void scan8(const Scan& c, int sb) {
 }
 
 template <bool PERT>
-__global__ void __launch_bounds__(SL_THREADS, 1)
+__global__ void __launch_bounds__(PERT ? SL_THREADS_T : SL_THREADS, 1)
 snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_constant__ CUtensorMap tm_xlo,
                  const __grid_constant__ CUtensorMap tm_whi, const __grid_constant__ CUtensorMap tm_wlo,
                  const __grid_constant__ CUtensorMap tm_bhi, const __grid_constant__ CUtensorMap tm_blo,
@@ -250,10 +245,10 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t x_tx = (uint32_t)(g.spt * g.T) * 128;      // bytes a box of x brings
     const uint32_t w_tx = (uint32_t)g.bn * 128, b_bytes = (uint32_t)g.nt * 128;
-    constexpr int W_HI = SL_OPERAND, W_LO = 2 * SL_OPERAND, B_HI = 3 * SL_OPERAND;
-    uint8_t* tparts = smem + (size_t)g.stages * g.stage_bytes;   // t: [part 3][nt / 8][128][8] bf16
-    const int part_bytes = g.nt * 256;
-    __shared__ uint64_t full[SL_MAX_STAGES], empty[SL_MAX_STAGES], tfull[2], tempty[2], tacc, tready, ufree;
+    const int W_HI = g.rows * 128, W_LO = W_HI + SL_OPERAND, B_HI = W_LO + SL_OPERAND;
+    uint8_t* tparts = smem + (size_t)g.stages * g.stage_bytes;   // t: [part 3][nt / 8][rows][8] bf16
+    const int part_bytes = g.nt * g.rows * 2, bufs = !PERT || g.rows == 128 ? 2 : 1;
+    __shared__ uint64_t full[SL_MAX_STAGES], empty[SL_MAX_STAGES], tfull[2], tempty[2], tacc, tready;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag_s;
     volatile int* abort_flag = &abort_flag_s;
@@ -270,7 +265,6 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
         }
         mbar_init(&tacc, 1);
         mbar_init(&tready, 256);
-        mbar_init(&ufree, 256);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -282,8 +276,9 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_slot;                          // the product at columns 0 and 128, the rank term at 256, t from 384
-    const uint32_t tmem_u = tmem + 256, tmem_t = tmem + 384;
+    // Columns 0-255: accumulators of the product, `rows` each (without noise up to 511).  The same from 256: the rank term,
+    // whose columns hold t (a part of 128 columns per 128 rows) until it has been read.
+    const uint32_t tmem = tmem_slot;
     const int64_t units = g.tiles * g.groups;
     const bool x_lo = g.inexact != nullptr && *g.inexact != 0;
     const int x_parts = x_lo ? 2 : 1;                         // stages per k-block: (x_hi, W_hi, W_lo), then (x_lo, W_hi)
@@ -332,7 +327,7 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
                             uint8_t* st = slot(x_tx + (2 - part) * (w_tx + (with_t ? b_bytes : 0)));
                             if (!ok) break;
                             uint64_t* bar = &full[ring.s];
-                            tma_load_2d(st, part ? &tm_xlo : &tm_xhi, kb * 64, (int)(s0 * g.T), bar);
+                            tma_load_3d(st, part ? &tm_xlo : &tm_xhi, kb * 64, (int)s0, 0, bar);
                             tma_load_2d(st + W_HI, &tm_whi, kb * 64, c * g.bn, bar);
                             if (!part) tma_load_2d(st + W_LO, &tm_wlo, kb * 64, c * g.bn, bar);
                             if (with_t) {
@@ -362,12 +357,12 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
         }
     } else if (warp == 1) {
         // the whole warp runs the loop, so that addresses and descriptors are uniform; one lane issues
-        const int n16 = (g.spt * g.T + 15) & ~15;
+        const int n16 = (g.spt * g.T + 15) & ~15, t_halves = n16 > 128 ? 2 : 1;
         const uint32_t idesc = make_idesc(n16), idesc_u = make_idesc_bf16(n16);
         const uint32_t idesc_t = make_idesc(PERT ? 2 * g.nt : 16), idesc_tl = make_idesc(PERT ? g.nt : 16);
         const int tc_len = PERT ? (g.k_blocks + g.t_chains - 1) / g.t_chains : 1;
         const uint64_t desc0 = make_smem_desc(smem), desc_step = (uint64_t)(g.stage_bytes >> 4);
-        const uint64_t plain0 = make_plain_desc(smem, g.bn * 16), plain_t = make_plain_desc(tparts, 2048);
+        const uint64_t plain0 = make_plain_desc(smem, g.bn * 16), plain_t = make_plain_desc(tparts, g.rows * 16);
         const uint32_t abytes = (uint32_t)g.r16 * g.bn * 2;       // one part of an image
         uint32_t acc_it = 0, unit_no = 0;
         Ring ring{0, 0};
@@ -381,12 +376,13 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
             tile_of(mt, s0, cnt, p0, nd);
             for (int c = c0; c < c1 && ok; ++c, ++acc_it) {
                 const bool with_t = PERT && c == c0;
-                const int b = acc_it & 1;
-                ok = __all_sync(0xffffffffu, mbar_wait(&tempty[b], ((acc_it >> 1) & 1) ^ 1, abort_flag, g.status, 2));
+                const int b = bufs == 2 ? (int)(acc_it & 1) : 0;
+                const uint32_t ph = (bufs == 2 ? acc_it >> 1 : acc_it) & 1;
+                ok = __all_sync(0xffffffffu, mbar_wait(&tempty[b], ph ^ 1, abort_flag, g.status, 2));
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t d = tmem + (uint32_t)(b * 128);
-                uint32_t tc_col = tmem_t;                     // accumulator and k-blocks left of t's current sum
+                const uint32_t d = tmem + (uint32_t)(b * g.rows), tmem_u = d + 256;
+                uint32_t tc_col = tmem_u;                     // accumulator and k-blocks left of t's current sum
                 int tc_left = tc_len;
                 for (int kb = 0; kb < g.k_blocks && ok; ++kb)
                     for (int part = 0; part < x_parts; ++part, ring.next(g.stages)) {
@@ -405,10 +401,14 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
                             }
                             if (with_t) {
                                 // t: B's halves side by side, in sums of a few k-blocks each
+                                for (int h = 0; h < t_halves; ++h) {
+                                    const uint32_t col = tc_col + h * 128;
+                                    const uint64_t dxh = dx + h * (SL_OPERAND >> 4);
 #pragma unroll
-                                for (int ks = 0; ks < 4; ++ks)
-                                    umma_f16_warp(part ? tc_col + g.nt : tc_col, dx + 2 * ks, db + 2 * ks, part ? idesc_tl : idesc_t,
-                                             ks || part || tc_left != tc_len);
+                                    for (int ks = 0; ks < 4; ++ks)
+                                        umma_f16_warp(part ? col + g.nt : col, dxh + 2 * ks, db + 2 * ks, part ? idesc_tl : idesc_t,
+                                                      ks || part || tc_left != tc_len);
+                                }
                             }
                             umma_commit_warp(&empty[ring.s]);
                         }
@@ -424,15 +424,13 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
                         ok = __all_sync(0xffffffffu, mbar_wait(&tready, unit_no & 1, abort_flag, g.status, 4));
                         if (!ok) break;
                     }
-                    ok = __all_sync(0xffffffffu, mbar_wait(&ufree, (acc_it & 1) ^ 1, abort_flag, g.status, 7));
-                    if (!ok) break;
                     tc_fence_after();
                     for (int dd = 0; dd < nd; ++dd, ring.next(g.stages)) {
                         ok = __all_sync(0xffffffffu, mbar_wait(&full[ring.s], ring.ph, abort_flag, g.status, 3));
                         if (!ok) break;
                         tc_fence_after();
                         for (int ks = 0; ks < g.r16 / 16; ++ks) {
-                            const uint64_t dt = plain_t + (uint64_t)(((dd * g.r16 + ks * 16) >> 3) * 128);
+                            const uint64_t dt = plain_t + (uint64_t)(((dd * g.r16 + ks * 16) >> 3) * g.rows);
                             const uint64_t da = plain0 + ring.s * desc_step + (uint64_t)(ks * 2 * g.bn);
                             const uint32_t t1 = part_bytes >> 4, t2 = 2 * t1, a1 = abytes >> 4, a2 = 2 * a1;
                             {
@@ -452,70 +450,84 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
                 __syncwarp();
             }
         }
-    } else {
-        // ------------------------------------------------------------------------- epilogue
-        const int q4 = warp & 3, eh = (warp - 2) >> 2;        // TMEM quadrant; group: sample blocks eh, eh + 2, ..
-        const int gt = q4 * 32 + lane;                        // TMEM lane: a neuron of the chunk, or a row of t
-        const uint32_t lane_base = tmem + ((uint32_t)(q4 * 32) << 16);
-        const int sm = gt / g.T;                              // sample of row gt of t
+    } else if (PERT && warp >= 10) {
+        // ------------------------------------------------------- t to bf16 parts in shared memory
+        // more than 128 rows: each four warps take 128 of them; else every second piece of eight columns
+        const int q4 = warp & 3, eh = (warp - 10) >> 2;
+        const bool tall = g.spt * g.T > 128;
+        const int row = q4 * 32 + lane + (tall ? eh * 128 : 0), step = row / g.spt, sm = row - step * g.spt;
         uint32_t acc_it = 0, unit_no = 0;
+        for (int64_t u = blockIdx.x; u < units; u += gridDim.x, ++unit_no) {
+            const int64_t mt = u / g.groups;
+            const int grp = (int)(u - mt * g.groups);
+            int64_t s0, p0;
+            int cnt, nd;
+            tile_of(mt, s0, cnt, p0, nd);
+            const int b = bufs == 2 ? (int)(acc_it & 1) : 0;
+            acc_it += g.n_chunks * (grp + 1) / g.groups - g.n_chunks * grp / g.groups;
+            const uint32_t t0 = tmem + ((uint32_t)(q4 * 32) << 16) + 256 + b * g.rows + (tall ? eh * 128 : 0);
+            const int64_t s = s0 + sm;
+            const bool odd = ((s / g.bm) & 1) != 0;           // the odd member of a pair has A negated
+            const int d = step < g.T && sm < cnt ? (int)(s / g.spp - p0) : -1;
+            if (!__all_sync(0xffffffffu, mbar_wait(&tacc, unit_no & 1, abort_flag, g.status, 5))) break;
+            tc_fence_after();
+            for (int c8 = tall ? 0 : eh; c8 < g.nt / 8; c8 += tall ? 1 : 2) {
+                uint32_t w[3][4];
+                float tv[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) tv[j] = 0.0f;
+                for (int half = 1; half >= 0; --half)         // what B's lo half gave, then the rest
+                    for (int ch = 0; ch < g.t_chains; ++ch) {
+                        uint32_t v[8];
+                        tmem_ld8(t0 + (2 * ch + half) * g.nt + c8 * 8, v);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) tv[j] = __fadd_rn(tv[j], __uint_as_float(v[j]));
+                    }
+                const bool mine = c8 * 8 / g.r16 == d;        // only the columns of the row's own pair are not zero
+#pragma unroll
+                for (int j = 0; j < 8; j += 2) {
+                    float v0 = mine ? tv[j] : 0.0f, v1 = mine ? tv[j + 1] : 0.0f;
+                    if (odd) v0 = -v0, v1 = -v1;
+#pragma unroll
+                    for (int part = 0; part < 3; ++part) {
+                        const __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
+                        w[part][j >> 1] = *reinterpret_cast<const uint32_t*>(&h);
+                        v0 -= __bfloat162float(h.x);
+                        v1 -= __bfloat162float(h.y);
+                    }
+                }
+#pragma unroll
+                for (int part = 0; part < 3; ++part)
+                    if (row < g.rows) *reinterpret_cast<uint4*>(tparts + part * part_bytes + (c8 * g.rows + row) * 16) =
+                        make_uint4(w[part][0], w[part][1], w[part][2], w[part][3]);
+            }
+            fence_proxy_async();
+            tc_fence_before();
+            mbar_arrive(&tready);
+        }
+    } else {
+        // ----------------------------------------------------------------------------- scan
+        const int q4 = warp & 3, eh = (warp - 2) >> 2;        // TMEM quadrant; group: sample blocks eh, eh + 2, ..
+        const int gt = q4 * 32 + lane;                        // TMEM lane: a neuron of the chunk
+        const uint32_t lane_base = tmem + ((uint32_t)(q4 * 32) << 16);
+        uint32_t acc_it = 0;
         bool ok = true;
-        for (int64_t u = blockIdx.x; u < units && ok; u += gridDim.x, ++unit_no) {
+        for (int64_t u = blockIdx.x; u < units && ok; u += gridDim.x) {
             const int64_t mt = u / g.groups;
             const int grp = (int)(u - mt * g.groups);
             const int c0 = g.n_chunks * grp / g.groups, c1 = g.n_chunks * (grp + 1) / g.groups;
             int64_t s0, p0;
             int cnt, nd;
             tile_of(mt, s0, cnt, p0, nd);
-            if (PERT) {
-                // t to bf16 parts in shared memory; only the columns of the row's own pair are not zero
-                if (!mbar_wait(&tacc, unit_no & 1, abort_flag, g.status, 5)) { ok = false; break; }
-                tc_fence_after();
-                const int64_t s = s0 + sm;
-                const bool odd = ((s / g.bm) & 1) != 0;       // the odd member of a pair has A negated
-                const int d = sm < cnt ? (int)(s / g.spp - p0) : -1;
-                for (int c8 = eh; c8 < g.nt / 8; c8 += 2) {
-                    uint32_t w[3][4];
-                    float tv[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) tv[j] = 0.0f;
-                    for (int half = 1; half >= 0; --half)         // what B's lo half gave, then the rest
-                        for (int ch = 0; ch < g.t_chains; ++ch) {
-                            uint32_t v[8];
-                            tmem_ld8(lane_base + 384 + (2 * ch + half) * g.nt + c8 * 8, v);
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) tv[j] = __fadd_rn(tv[j], __uint_as_float(v[j]));
-                        }
-                    const bool mine = c8 * 8 / g.r16 == d;
-#pragma unroll
-                    for (int j = 0; j < 8; j += 2) {
-                        float v0 = mine ? tv[j] : 0.0f, v1 = mine ? tv[j + 1] : 0.0f;
-                        if (odd) v0 = -v0, v1 = -v1;
-#pragma unroll
-                        for (int part = 0; part < 3; ++part) {
-                            const __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
-                            w[part][j >> 1] = *reinterpret_cast<const uint32_t*>(&h);
-                            v0 -= __bfloat162float(h.x);
-                            v1 -= __bfloat162float(h.y);
-                        }
-                    }
-#pragma unroll
-                    for (int part = 0; part < 3; ++part)
-                        *reinterpret_cast<uint4*>(tparts + part * part_bytes + c8 * 2048 + gt * 16) =
-                            make_uint4(w[part][0], w[part][1], w[part][2], w[part][3]);
-                }
-                fence_proxy_async();
-                tc_fence_before();
-                mbar_arrive(&tready);
-            }
             for (int c = c0; c < c1; ++c, ++acc_it) {
-                const int b = acc_it & 1;
-                if (!mbar_wait(&tfull[b], (acc_it >> 1) & 1, abort_flag, g.status, 6)) { ok = false; break; }
+                const int b = bufs == 2 ? (int)(acc_it & 1) : 0;
+                ok = __all_sync(0xffffffffu, mbar_wait(&tfull[b], (bufs == 2 ? acc_it >> 1 : acc_it) & 1, abort_flag, g.status, 6));
+                if (!ok) break;
                 tc_fence_after();
                 const int n = c * g.bn + gt;
                 const bool live = gt < g.bn && n < g.a;
                 if (c * g.bn + q4 * 32 < g.a && q4 * 32 < g.bn) {
-                    const Scan sc{lane_base + b * 128, lane_base + 256, g.T, cnt, live, live ? __ldg(g.col_scale + n) : 0.0f,
+                    const Scan sc{lane_base + b * g.rows, lane_base + 256 + b * g.rows, g.T, g.spt, cnt, live, live ? __ldg(g.col_scale + n) : 0.0f,
                                   g.leak, g.v_th, x_lo ? g.row_scale + s0 * g.T : nullptr,
                                   g.out_half ? g.out_half + (size_t)s0 * g.T * g.out_pitch + n : nullptr, g.out_pitch,
                                   g.count ? g.count + (size_t)s0 * g.a + n : nullptr, g.a};
@@ -525,7 +537,6 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
                     }
                 }
                 tc_fence_before();
-                if (PERT) mbar_arrive(&ufree);
                 mbar_arrive(&tempty[b]);
             }
         }
@@ -576,7 +587,7 @@ __host__ __device__ inline size_t ro_floats(int h, int classes, int r, int rows)
 // and each member's mean.  A lane is a sample, a warp takes four columns at a time.  The whole is a chain of short phases,
 // so its time is their latencies: 24 us with a thread per sample and column, a divide per rate and a block per pair of 128
 // samples took 61.
-__global__ void __launch_bounds__(256) snn_readout_kernel(const __grid_constant__ ReadoutArgs g) {
+__global__ void __launch_bounds__(256, 4) snn_readout_kernel(const __grid_constant__ ReadoutArgs g) {
     extern __shared__ __align__(16) float sm[];
     __shared__ CalTab tab;
     __shared__ uint64_t state_s[64];
@@ -688,7 +699,7 @@ __global__ void __launch_bounds__(256) snn_readout_kernel(const __grid_constant_
 
 // ---------------------------------------------------------------------------- host side
 struct LayerPlan {
-    int spt, ppt, tpp, nt, r16, bn, n_chunks, groups, kp, ap, stages, stage_bytes, smem;
+    int rows, spt, ppt, tpp, nt, r16, bn, n_chunks, groups, kp, ap, stages, stage_bytes, smem;
     int64_t tiles;
     size_t o_whi, o_wlo, o_cs, o_bhi, o_blo, o_aimg;
 };
@@ -732,43 +743,58 @@ SnnPlan plan_snn(const hses_snn_model* m, const hses_pop_args* p) {
         q.n_chunks = (a + 127) / 128;
         q.bn = ((a + q.n_chunks - 1) / q.n_chunks + 15) & ~15;
         if (pert) q.r16 = (r + 15) & ~15;
-        // Samples per tile: as many as fit 128 rows, or fewer where that leaves SMs without a tile.  A tile costs its
-        // passes over k and its share of the scan; neurons of a chunk are scanned side by side, so narrow chunks save nothing.
+        // Samples per tile and groups of chunks: the cheapest by a model of the kernel in cycles (measured at 784 -> 128 and
+        // 128 -> 128, T = 8, rank 4).  Loads: 35 bytes per cycle reach an SM when all of them load; products: 8192 flop per
+        // cycle; the rank term's way through shared memory and back: 2600; scan: 20 per row.  Tiles of 128 rows overlap the
+        // scan with the next tile's products, taller ones read W less often.
         int64_t best = -1;
-        for (int cap = 128 / p->T; cap >= 1; cap -= std::max(1, cap / 8)) {
-            LayerPlan t = q;
-            t.tpp = 1;
-            t.ppt = 0;
-            if (pert) {
-                const int spp = 2 * p->bm;
-                if (spp <= cap) {
-                    t.ppt = (int)std::min<int64_t>({cap / spp, 64 / q.r16, s.pairs});
-                    t.spt = t.ppt * spp;
-                    t.tiles = (s.pairs + t.ppt - 1) / t.ppt;
+        for (int rows = 256; rows >= 128; rows -= 64)
+            for (int cap = rows / p->T; cap >= 1; cap -= std::max(1, cap / 16)) {
+                if ((p->T - 1) * cap + ((cap + 7) & ~7) > rows) continue;   // the scan reads eight columns at a time
+                LayerPlan t = q;
+                t.rows = rows;
+                t.tpp = 1;
+                t.ppt = 0;
+                if (pert) {
+                    const int spp = 2 * p->bm;
+                    if (spp <= cap) {
+                        t.ppt = (int)std::min<int64_t>({cap / spp, 64 / q.r16, s.pairs});
+                        t.spt = t.ppt * spp;
+                        t.tiles = (s.pairs + t.ppt - 1) / t.ppt;
+                    } else {
+                        t.tpp = (spp + cap - 1) / cap;
+                        t.spt = (spp + t.tpp - 1) / t.tpp;
+                        t.tiles = s.pairs * t.tpp;
+                    }
+                    t.nt = std::max(t.ppt, 1) * q.r16;
                 } else {
-                    t.tpp = (spp + cap - 1) / cap;
-                    t.spt = (spp + t.tpp - 1) / t.tpp;
-                    t.tiles = s.pairs * t.tpp;
+                    t.spt = cap;
+                    t.tiles = (s.n + cap - 1) / cap;
                 }
-                t.nt = std::max(t.ppt, 1) * q.r16;
-            } else {
-                t.spt = cap;
-                t.tiles = (s.n + cap - 1) / cap;
-            }
-            for (int gr = 1; gr <= q.n_chunks; ++gr) {
-                const int64_t waves = (t.tiles * gr + sms - 1) / sms;
-                const int64_t cost = waves * ((q.n_chunks + gr - 1) / gr) * (t.spt * p->T + 64 + 4 * ((k + 63) / 64));
-                if (best < 0 || cost < best) {
-                    best = cost;
-                    q = t;
-                    q.groups = gr;
+                const int used = t.spt * p->T;
+                if (used <= rows - 64 && rows > 128) continue;
+                t.stage_bytes = rows * 128 + 2 * SL_OPERAND + t.nt * 256;
+                const int fixed = 1024 + 3 * t.nt * rows * 2;
+                t.stages = std::min(SL_MAX_STAGES, (SL_SMEM_LIMIT - 1024 - fixed) / t.stage_bytes);
+                t.smem = fixed + t.stages * t.stage_bytes;
+                if (t.stages < 2) continue;
+                const int64_t load = ((int64_t)used * 128 + 2 * q.bn * 128 + t.nt * 256) / 35;
+                const int64_t mma = 4 * ((int64_t)used + (pert ? (used + 127) / 128 * std::max(32, t.nt) : 0));
+                const int64_t rank = pert ? 2600 + (int64_t)std::max(1, t.ppt) * q.r16 / 16 * 6 * used / 2 : 0;
+                const int64_t block = std::max(load, mma) + (t.stages == 2 ? std::min(load, mma) / 2 : 0);   // two hide less
+                const int64_t front = (k + 63) / 64 * block + rank, scan = 600 + 20 * (int64_t)used;
+                const int64_t chunk = pert && rows > 128 ? front + scan : std::max(front, scan);
+                for (int gr = 1; gr <= q.n_chunks; ++gr) {
+                    const int64_t waves = (t.tiles * gr + sms - 1) / sms;
+                    const int64_t cost = waves * ((q.n_chunks + gr - 1) / gr) * chunk + front + scan - chunk;
+                    if (best < 0 || cost < best) {
+                        best = cost;
+                        t.groups = gr;
+                        q = t;
+                    }
                 }
             }
-        }
-        q.stage_bytes = 3 * SL_OPERAND + q.nt * 256;
-        const int fixed = 1024 + 3 * q.nt * 256;
-        q.stages = std::min(SL_MAX_STAGES, (SL_SMEM_LIMIT - 1024 - fixed) / q.stage_bytes);
-        q.smem = fixed + q.stages * q.stage_bytes;
+        if (best < 0) return s;
         q.o_whi = take((size_t)a * q.kp * 2);
         q.o_wlo = take((size_t)a * q.kp * 2);
         q.o_cs = take((size_t)a * 4);
@@ -827,6 +853,26 @@ int encode_2d(CUtensorMap* map, const void* base, int64_t rows, int cols, int pi
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         set_error("cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
+        return HSES_ERR_CUDA;
+    }
+    return HSES_OK;
+}
+// spikes (n, T, k) with rows of `pitch` values; a box is 64 inputs of spt samples x T steps, step by step
+int encode_spikes(CUtensorMap* map, const void* base, int64_t n, int T, int k, int pitch, int spt) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) {
+        set_error("cuTensorMapEncodeTiled is not available from the driver");
+        return HSES_ERR_CUDA;
+    }
+    cuuint64_t dims[3] = {(cuuint64_t)k, (cuuint64_t)n, (cuuint64_t)T};
+    cuuint64_t strides[2] = {(cuuint64_t)pitch * 2 * (cuuint64_t)T, (cuuint64_t)pitch * 2};
+    cuuint32_t box[3] = {64, (cuuint32_t)spt, (cuuint32_t)T};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        set_error("cuTensorMapEncodeTiled (spikes) failed with code " + std::to_string((int)r));
         return HSES_ERR_CUDA;
     }
     return HSES_OK;
@@ -971,6 +1017,7 @@ int run_snn_fused(hses_ctx* ctx, cudaStream_t st, const hses_snn_model* m, const
         LayerArgs a{};
         a.T = p->T;
         a.spt = q.spt;
+        a.rows = q.rows;
         a.k_blocks = (m->dims[l] + 63) / 64;
         a.nt = q.nt;
         if (pert) {
@@ -1005,8 +1052,8 @@ int run_snn_fused(hses_ctx* ctx, cudaStream_t st, const hses_snn_model* m, const
         const void* x = l == 0 ? half_at(s.o_x) : half_at(s.o_h[(l - 1) & 1]);
         const int pitch = l == 0 ? kp0 : s.l[l - 1].ap;
         CUtensorMap mx, mxl, mw, mwl, mb, mbl;
-        int rc = encode_2d(&mx, x, rows, m->dims[l], pitch, q.spt * p->T);
-        if (rc == HSES_OK) rc = encode_2d(&mxl, l == 0 ? half_at(s.o_xlo) : x, rows, m->dims[l], pitch, q.spt * p->T);
+        int rc = encode_spikes(&mx, x, s.n, p->T, m->dims[l], pitch, q.spt);
+        if (rc == HSES_OK) rc = encode_spikes(&mxl, l == 0 ? half_at(s.o_xlo) : x, s.n, p->T, m->dims[l], pitch, q.spt);
         if (rc == HSES_OK) rc = encode_2d(&mw, half_at(q.o_whi), a.a, q.kp, q.kp, q.bn);
         if (rc == HSES_OK) rc = encode_2d(&mwl, half_at(q.o_wlo), a.a, q.kp, q.kp, q.bn);
         mb = mw;
@@ -1019,7 +1066,7 @@ int run_snn_fused(hses_ctx* ctx, cudaStream_t st, const hses_snn_model* m, const
         auto kernel = pert ? snn_layer_kernel<true> : snn_layer_kernel<false>;
         HSES_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, q.smem));
         HSES_KERNEL(ctx, st, "snn_layer");
-        kernel<<<grid, SL_THREADS, q.smem, st>>>(mx, mxl, mw, mwl, mb, mbl, a);
+        kernel<<<grid, pert ? SL_THREADS_T : SL_THREADS, q.smem, st>>>(mx, mxl, mw, mwl, mb, mbl, a);
         HSES_LAUNCH_CHECK();
     }
 

@@ -11,6 +11,7 @@ pytestmark = pytest.mark.gpu
     ([100, 33, 17, 10], 602, 1, 7, 5, 0),          # odd widths, packed pairs, a last tile with fewer of them
     ([64, 300, 130, 26], 6, 43, 3, 17, 1),         # a pair over several tiles, the last one short; two rank blocks
     ([70, 129, 5], 2, 1, 128, 64, 0),              # one sample per tile, T at its limit
+    ([784, 128, 64, 10], 400, 16, 8, 4, 1),        # tiles of 256 rows, several per CTA
     ([36, 16, 40, 24, 100], 10, 70, 5, 33, 1),     # three hidden layers, readout in slices
     ([784, 320, 10], 1, 500, 8, 0, 1),             # clean, one member
     ([31, 257, 64, 10], 7, 9, 9, 0, 0),            # clean, odd numbers of members and inputs
