@@ -170,17 +170,27 @@ __device__ __forceinline__ uint32_t xs32(uint32_t x) {
     return x;
 }
 
-// The reference compares u = fl((k+1)/8388609) with p at every step, k being
-// the top 23 bits of the xorshift32 output.  fl(n/8388609) is monotone in n,
-// so "u < p" is "n < n*(p)" with n* the smallest n whose quotient reaches p.
-// n* is found once per element with exact divisions; the T steps are then
-// integer-only.
-__device__ __forceinline__ uint32_t poisson_threshold(float p) {
+// The reference compares u = fl((k+1)/8388609) with p at every step, k being the top 23 bits of the xorshift32 output.
+// fl(n/D) is monotone in n, so a step spikes when k < q, q = the number of n >= 1 whose quotient stays below p; one
+// division per element finds it, and a step is a comparison of the raw state: k < q is state <= (q << 9) - 1.
+struct PoissonCell {
+    uint32_t x, last;
+};
+__device__ __forceinline__ PoissonCell poisson_cell(float p, uint32_t seed) {
     const float D = 8388609.0f;
-    float guess = __fmul_rn(p, D);
-    uint32_t c = guess >= 1.0f ? (guess < 8388609.0f ? (uint32_t)guess : 8388609u) : 1u;
-    while (c > 1u && __fdiv_rn((float)(c - 1u), D) >= p) --c;
-    while (c <= 8388608u && __fdiv_rn((float)c, D) < p) ++c;
+    uint32_t q = 0;                                // 0 .. 2^23
+    if (p >= 1.0f) {
+        q = 8388608u;
+    } else if (p > 0.0f) {
+        // below: the largest integer under pD = hi + lo.  Its quotient may reach p by rounding up; that of the integer
+        // before cannot, it is more than half a unit in the last place away
+        const float hi = __fmul_rn(p, D), lo = __fmaf_rn(p, D, -hi), f = floorf(hi);
+        const float below = hi > f || lo > 0.0f ? f : __fsub_rn(f, 1.0f);
+        if (below >= 1.0f) q = (uint32_t)below - (__fdiv_rn(below, D) >= p ? 1u : 0u);
+    }
+    PoissonCell c;
+    c.x = q ? seed : 1u;                           // a cell that never spikes: any state but 0, which stays as it is
+    c.last = q ? (q << 9) - 1u : 0u;
     return c;
 }
 // fitness of one sample (hyperscalees-envs/src/snn_mnist.rs:180-201)

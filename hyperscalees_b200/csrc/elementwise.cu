@@ -29,18 +29,15 @@ __global__ void poisson_kernel(const float* __restrict__ probs, int64_t batch, i
     } else {
         p[0] = probs[base];
     }
-    uint32_t x[VEC], thr[VEC];
+    PoissonCell c[VEC];
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-        x[i] = poisson_seed((uint32_t)(row * in_dim + col + i), mix);
-        thr[i] = poisson_threshold(p[i]);
-    }
+    for (int i = 0; i < VEC; ++i) c[i] = poisson_cell(p[i], poisson_seed((uint32_t)(row * in_dim + col + i), mix));
     for (int t = 0; t < T; ++t) {
         float s[VEC];
 #pragma unroll
         for (int i = 0; i < VEC; ++i) {
-            x[i] = xs32(x[i]);
-            s[i] = ((x[i] >> 9) + 1u) < thr[i] ? 1.0f : 0.0f;
+            c[i].x = xs32(c[i].x);
+            s[i] = c[i].x <= c[i].last ? 1.0f : 0.0f;
         }
         float* dst = out + (size_t)t * out_step + base;
         if constexpr (VEC == 4)

@@ -36,16 +36,17 @@ constexpr int kSnnMaxLayers = 8;         // hidden layers
 
 // ------------------------------------------------------------------------------- input
 // poisson_encode_fused_oxide.rs:36-105 (see poisson_kernel in elementwise.cu for the threshold), eight neighbouring
-// inputs of a row per thread, spikes as fp16 rows of kp values (the padding is zero), row sample * T + step.
+// inputs of a row per thread, spikes as fp16 rows of kp values (the padding is zero), row sample * T + step.  Bound by the
+// generator's integer work (8 steps of 784 inputs: 12 instructions a step).
 __global__ void __launch_bounds__(256)
 encode_half_kernel(const float* __restrict__ probs, int64_t batch, int in_dim, int64_t stride, int T, uint32_t mix,
                    __half* __restrict__ out, int kp) {
     const int groups = kp >> 3;
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= batch * groups) return;
-    const int64_t row = v / groups;
-    const int col = (int)(v - row * groups) * 8;
-    uint32_t x[8], thr[8];
+    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x, srow = v / (uint32_t)groups;   // batch * in_dim < 2^32
+    if (srow >= batch) return;
+    const int64_t row = srow;
+    const int col = (int)(v - srow * groups) * 8;
+    PoissonCell c[8];
     const bool vec = (reinterpret_cast<uintptr_t>(probs) & 15) == 0 && (stride & 3) == 0 && col + 8 <= in_dim;
     float p[8];
     if (vec) {
@@ -57,17 +58,14 @@ encode_half_kernel(const float* __restrict__ probs, int64_t batch, int in_dim, i
         for (int i = 0; i < 8; ++i) p[i] = col + i < in_dim ? __ldg(probs + row * stride + col + i) : 0.0f;
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        x[i] = poisson_seed((uint32_t)(row * in_dim + col + i), mix);
-        thr[i] = poisson_threshold(p[i]);
-    }
+    for (int i = 0; i < 8; ++i) c[i] = poisson_cell(p[i], poisson_seed((uint32_t)(row * in_dim + col + i), mix));
     for (int t = 0; t < T; ++t) {
         uint32_t w[4];
 #pragma unroll
         for (int i = 0; i < 8; i += 2) {
-            x[i] = xs32(x[i]);
-            x[i + 1] = xs32(x[i + 1]);
-            w[i >> 1] = (((x[i] >> 9) + 1u) < thr[i] ? 0x3C00u : 0u) | (((x[i + 1] >> 9) + 1u) < thr[i + 1] ? 0x3C000000u : 0u);
+            c[i].x = xs32(c[i].x);
+            c[i + 1].x = xs32(c[i + 1].x);
+            w[i >> 1] = (c[i].x <= c[i].last ? 0x3C00u : 0u) | (c[i + 1].x <= c[i + 1].last ? 0x3C000000u : 0u);
         }
         *reinterpret_cast<uint4*>(out + ((size_t)row * T + t) * kp + col) = make_uint4(w[0], w[1], w[2], w[3]);
     }
