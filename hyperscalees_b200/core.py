@@ -93,4 +93,9 @@ def get_context(device=None) -> Context:
 
 def current_stream(device=None) -> int:
     """Raw cudaStream_t of torch's current stream (0 means the legacy default stream)."""
-    return int(torch.cuda.current_stream(device).cuda_stream)
+    if device is None:
+        idx = torch.cuda.current_device()
+    else:
+        device = torch.device(device)
+        idx = torch.cuda.current_device() if device.index is None else device.index
+    return torch._C._cuda_getCurrentRawStream(idx)   # what torch.cuda.current_stream wraps in an object (4 us a call)

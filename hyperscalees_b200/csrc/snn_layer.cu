@@ -15,6 +15,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <array>
 #include <vector>
 
 #include "linear.cuh"
@@ -710,7 +711,7 @@ struct SnnPlan {
     size_t o_x, o_xlo, o_rs, o_h[2], o_rate, o_flag, o_per, bytes;
 };
 
-SnnPlan plan_snn(const hses_snn_model* m, const hses_pop_args* p) {
+SnnPlan make_plan(const hses_snn_model* m, const hses_pop_args* p) {
     SnnPlan s{};
     const int hidden = m->n_layers - 1;
     if (hidden < 1 || hidden > kSnnMaxLayers || p->T < 1 || p->T > 128) return s;
@@ -836,6 +837,29 @@ SnnPlan plan_snn(const hses_snn_model* m, const hses_pop_args* p) {
     return s;
 }
 
+// A step asks for its plan four times (the choice of path, sizes, the run): each thread keeps its last one.
+const SnnPlan& plan_snn(const hses_snn_model* m, const hses_pop_args* p) {
+    using Key = std::array<int64_t, kSnnMaxLayers + 12>;
+    thread_local Key last{};
+    thread_local SnnPlan plan{};
+    Key key{};
+    key[0] = m->n_layers;
+    for (int l = 0; l <= m->n_layers && l < kSnnMaxLayers + 3; ++l) key[1 + l] = m->dims[l];
+    int64_t* k = key.data() + kSnnMaxLayers + 4;
+    k[0] = p->T;
+    k[1] = p->n_pop;
+    k[2] = p->bm;
+    k[3] = p->perturb;
+    k[4] = p->rank;
+    k[5] = p->first_thread % 2;
+    k[6] = plan_sm_count();
+    if (key != last) {
+        plan = make_plan(m, p);
+        last = key;
+    }
+    return plan;
+}
+
 int encode_2d(CUtensorMap* map, const void* base, int64_t rows, int cols, int pitch, int box_rows) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) {
@@ -883,7 +907,7 @@ size_t snn_fused_workspace_bytes(const hses_snn_model* m, const hses_pop_args* p
 
 int run_snn_fused(hses_ctx* ctx, cudaStream_t st, const hses_snn_model* m, const hses_pop_args* p, const SnnInput& in,
                   float* logits, const SnnScore& score, void* workspace, size_t workspace_bytes) {
-    const SnnPlan s = plan_snn(m, p);
+    const SnnPlan& s = plan_snn(m, p);
     HSES_REQUIRE(s.ok, "shape not covered");
     HSES_REQUIRE(workspace != nullptr && workspace_bytes >= s.bytes, "workspace too small");
     HSES_REQUIRE(p->noise_reuse >= 0 && p->first_thread >= 0, "negative thread id or noise_reuse");

@@ -14,6 +14,7 @@ import numpy as np
 import torch
 
 from . import ops
+from .core import current_stream, get_context
 from .noiser import MM_PARAM, PARAM, FrozenNoiserParams, NoiserParams
 
 
@@ -111,7 +112,6 @@ class SnnMlp:
         """One call of hses_snn_forward: the gain is read on the device, nothing waits for it."""
         import ctypes as C
         from . import _lib
-        from .core import current_stream, get_context
         T, n_pop, bm, k = x.shape
         ops._check(x, "x")
         _, _, xs = ops._rows_2d(x, "x")
@@ -173,7 +173,6 @@ class PopulationStep:
                  reward: int = ops.REWARD_LOGLIK, cache: str = "off", n_total: Optional[int] = None):
         import ctypes as C
         from . import _lib
-        from .core import get_context
         self.C, self._lib, self.L = C, _lib, _lib.load()
         self.net, self.frozen, self.noiser = net, frozen, noiser
         self.keys = [int(k) & ((1 << 64) - 1) for k in base_keys]
@@ -185,7 +184,8 @@ class PopulationStep:
         self.moments = None
         if kind in ("adam", "adamw"):
             self.moments = ([torch.zeros_like(p) for p in self.params], [torch.zeros_like(p) for p in self.params])
-        self._ws = None
+        self._ws = self._desc = self._ptrs = None
+        self._need, self._need_update = {}, {}
         self.caches = None
         # "auto": generate every layer's factors once per epoch bucket (at the first eval of the
         # bucket) and let the forward pass and the update read them; with noise_reuse == 0 the
@@ -204,16 +204,22 @@ class PopulationStep:
             n_pairs = (self.first_thread + self.n_pop - 1) // 2 - first_pair + 1
         else:
             first_pair, n_pairs = 0, n_total // 2
+        self.drop_caches()
         self.caches = [ops.FactorCache(self.keys[l], epoch, self.frozen.noise_reuse, self.frozen.rank,
                                        w.shape[0], w.shape[1], n_pairs, first_pair, device=self.net.device)
                        for l, w in enumerate(self.net.weights)]
         return sum(c.data.numel() * 4 for c in self.caches)
 
     def drop_caches(self) -> None:
-        self.caches = None
+        self.caches = self._desc = None   # the descriptor holds on to them too
 
     def _model(self):
-        C, _lib = self.C, self._lib
+        """The model's descriptor; built anew when anything it names has changed."""
+        C, _lib, net = self.C, self._lib, self.net
+        now = ([(w.data_ptr(), w.stride(0)) for w in net.weights], list(self.keys), net.out_gain.data_ptr(), net.tau_m, net.v_th, net.reset_mode,
+               [id(c) for c in self.caches] if self.caches is not None else None)
+        if self._desc is not None and self._desc[0] == now:
+            return self._desc[1]
         n = len(self.net.weights)
         dims = (C.c_int32 * (n + 1))(*self.net.dims)
         wp = (C.c_void_p * n)(*[w.data_ptr() for w in self.net.weights])
@@ -225,18 +231,33 @@ class PopulationStep:
             cp = (C.POINTER(_lib.FactorCacheDesc) * n)(*[C.pointer(c.desc) for c in self.caches])
         m = _lib.SnnModelDesc(n, dims, wp, ws, keys, 1.0, self.net.out_gain.data_ptr(), self.net.tau_m, vth,
                               self.net.reset_mode, cp)
-        self._keep = (dims, wp, ws, keys, vth, cp)
+        self._desc = (now, m, (dims, wp, ws, keys, vth, cp, self.caches))
         return m
+
+    def _solver(self):
+        """The solver's descriptor and the pointer arrays of parameters and moments."""
+        C, sv = self.C, self.frozen.solver
+        kind = {"sgd": ops.SGD, "adam": ops.ADAM, "adamw": ops.ADAMW}[sv.kind]
+        desc = self._lib.SolverDesc(kind, sv.lr, sv.beta1, sv.beta2, sv.eps, sv.weight_decay if kind == ops.ADAMW else 0.0)
+        if kind != ops.SGD:
+            self.noiser.opt_state.step += 1
+        ptr = [t.data_ptr() for ts in [self.params] + list(self.moments or ()) for t in ts]
+        if self._ptrs is None or self._ptrs[0] != ptr:
+            n = len(self.params)
+            arr = C.c_void_p * n
+            arrays = [arr(*ptr[i:i + n]) for i in range(0, len(ptr), n)]
+            self._ptrs = (ptr, arrays + [None] * (3 - len(arrays)))
+        return desc, self._ptrs[1]
 
     def _args(self, epoch: int, perturb: bool = True):
         return self._lib.PopArgs(self.T, self.n_pop, self.bm, int(perturb), self.noiser.sigma, self.frozen.rank,
                                  epoch, self.first_thread, self.frozen.noise_reuse)
 
-    def _scratch(self, nbytes: int) -> torch.Tensor:
+    def _scratch(self, nbytes: int) -> int:
+        """Address of that much scratch."""
         if self._ws is None or self._ws.numel() < nbytes + 256:
             self._ws = torch.empty(nbytes + 256, dtype=torch.uint8, device=self.net.device)
-        off = (-self._ws.data_ptr()) % 256
-        return self._ws[off:off + nbytes]
+        return (self._ws.data_ptr() + 255) // 256 * 256
 
     def eval(self, images: torch.Tensor, labels: torch.Tensor, seeds: Sequence[int], epoch: int = 0,
              want_logits: bool = False, perturb: bool = True):
@@ -250,17 +271,20 @@ class PopulationStep:
                 self.build_caches(epoch, self.n_total)
                 self._cache_bucket = bucket
         m, p = self._model(), self._args(epoch, perturb)
-        need = int(self.L.hses_population_eval_workspace_bytes(C.byref(m), C.byref(p)))
+        shape = (perturb, p.rank, p.T, p.n_pop, p.bm, p.first_thread, self.caches is None)
+        need = self._need.get(shape)
+        if need is None:
+            need = int(self.L.hses_population_eval_workspace_bytes(C.byref(m), C.byref(p)))
+            self._need = {shape: need}
         ws = self._scratch(need)
         raw = torch.empty(self.n_pop, dtype=torch.float32, device=images.device)
         logits = torch.empty((self.n_pop * self.bm, self.net.dims[-1]), dtype=torch.float32,
                              device=images.device) if want_logits else None
         sd = (C.c_uint32 * 4)(*[int(s) & 0xFFFFFFFF for s in seeds])
-        from .core import current_stream
         self._lib.check(self.L.hses_population_eval(
             self.ctx.handle, current_stream(), C.byref(m), C.byref(p), images.data_ptr(),
             images.stride(0), labels.data_ptr(), sd, self.reward, raw.data_ptr(),
-            logits.data_ptr() if want_logits else None, ws.data_ptr(), need))
+            logits.data_ptr() if want_logits else None, ws, need))
         return (raw, logits) if want_logits else raw
 
     def update_sharded(self, raw_fitness: torch.Tensor, epoch: int = 0, gain_key: Optional[int] = None,
@@ -281,12 +305,11 @@ class PopulationStep:
         if getattr(self, "_grads", None) is None or self._grads.numel() != elems:
             self._grads = torch.empty(elems, dtype=torch.float32, device=self.net.device)
         gk = self.keys[len(self.net.weights)] if gain_key is None else gain_key
-        from .core import current_stream
         self._lib.check(self.L.hses_population_grads(
             self.ctx.handle, current_stream(), C.byref(m), self.noiser.sigma, self.frozen.rank, epoch,
             self.frozen.noise_reuse, self.frozen.group_size, int(self.frozen.freeze_nonlora),
             C.c_uint64(gk & ((1 << 64) - 1)), raw_fitness.data_ptr(), n_total, self.first_thread, self.n_pop,
-            self._grads.data_ptr(), ws.data_ptr(), need))
+            self._grads.data_ptr(), ws, need))
         if reduce_fn is not None:
             reduce_fn(self._grads)
         elif comm is not None:
@@ -294,17 +317,7 @@ class PopulationStep:
                 comm.allreduce_grads(self._grads)
         elif dist.is_initialized() and dist.get_world_size(group) > 1:
             dist.all_reduce(self._grads, op=dist.ReduceOp.SUM, group=group)
-        sv = self.frozen.solver
-        kind = {"sgd": ops.SGD, "adam": ops.ADAM, "adamw": ops.ADAMW}[sv.kind]
-        desc = self._lib.SolverDesc(kind, sv.lr, sv.beta1, sv.beta2, sv.eps, sv.weight_decay if kind == ops.ADAMW else 0.0)
-        if kind != ops.SGD:
-            self.noiser.opt_state.step += 1
-        n = len(self.params)
-        pp = (C.c_void_p * n)(*[t.data_ptr() for t in self.params])
-        mp = vp = None
-        if self.moments is not None:
-            mp = (C.c_void_p * n)(*[t.data_ptr() for t in self.moments[0]])
-            vp = (C.c_void_p * n)(*[t.data_ptr() for t in self.moments[1]])
+        desc, (pp, mp, vp) = self._solver()
         self._lib.check(self.L.hses_population_apply(
             self.ctx.handle, current_stream(), C.byref(m), C.byref(desc), self.noiser.opt_state.step, pp, mp, vp,
             self._grads.data_ptr()))
@@ -314,26 +327,19 @@ class PopulationStep:
         C = self.C
         m = self._model()
         n_total = raw_fitness.numel()
-        need = int(self.L.hses_population_update_workspace_bytes(C.byref(m), self.frozen.rank, n_total))
+        shape = ("update", self.frozen.rank, n_total)
+        need = self._need_update.get(shape)
+        if need is None:
+            need = int(self.L.hses_population_update_workspace_bytes(C.byref(m), self.frozen.rank, n_total))
+            self._need_update = {shape: need}
         ws = self._scratch(need)
-        sv = self.frozen.solver
-        kind = {"sgd": ops.SGD, "adam": ops.ADAM, "adamw": ops.ADAMW}[sv.kind]
-        desc = self._lib.SolverDesc(kind, sv.lr, sv.beta1, sv.beta2, sv.eps, sv.weight_decay if kind == ops.ADAMW else 0.0)
-        if kind != ops.SGD:
-            self.noiser.opt_state.step += 1
-        n = len(self.params)
-        pp = (C.c_void_p * n)(*[t.data_ptr() for t in self.params])
-        mp = vp = None
-        if self.moments is not None:
-            mp = (C.c_void_p * n)(*[t.data_ptr() for t in self.moments[0]])
-            vp = (C.c_void_p * n)(*[t.data_ptr() for t in self.moments[1]])
+        desc, (pp, mp, vp) = self._solver()
         gk = self.keys[len(self.net.weights)] if gain_key is None else gain_key
-        from .core import current_stream
         self._lib.check(self.L.hses_population_update(
             self.ctx.handle, current_stream(), C.byref(m), self.noiser.sigma, self.frozen.rank, epoch,
             self.frozen.noise_reuse, self.frozen.group_size, int(self.frozen.freeze_nonlora),
             C.c_uint64(gk & ((1 << 64) - 1)), raw_fitness.data_ptr(), n_total, C.byref(desc),
-            self.noiser.opt_state.step, pp, mp, vp, ws.data_ptr(), need))
+            self.noiser.opt_state.step, pp, mp, vp, ws, need))
 
 
 class ChannelMixing:

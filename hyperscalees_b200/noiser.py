@@ -10,7 +10,6 @@ device path is meant to be driven.
 from __future__ import annotations
 
 from dataclasses import dataclass, field
-from operator import attrgetter
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -27,9 +26,6 @@ class IterInfo:
     """noiser.rs:24-28."""
     epoch: int
     thread_id: int
-
-
-_THREAD_ID, _EPOCH = attrgetter("thread_id"), attrgetter("epoch")
 
 
 # ---------------------------------------------------------------------------
@@ -376,8 +372,7 @@ class EggRoll:
         # the usual numbering: thread ids first, first+1, ... of one epoch, whole antithetic pairs
         first, epoch = infos[0].thread_id, infos[0].epoch
         contiguous = (n_total % 2 == 0 and first % 2 == 0 and
-                      list(map(_THREAD_ID, infos)) == list(range(first, first + n_total)) and
-                      set(map(_EPOCH, infos)) == {epoch})
+                      [i.thread_id for i in infos if i.epoch == epoch] == list(range(first, first + n_total)))
         if contiguous:
             groups = {None: (first, fitnesses, epoch)}
         else:

@@ -171,12 +171,11 @@ def _workspace(device: torch.device, nbytes: int) -> Optional[torch.Tensor]:
     handed back to the allocator tied to the stream whose kernels may still be using it."""
     if nbytes == 0:
         return None
-    stream = torch.cuda.current_stream(device)
-    slot = (device, stream.cuda_stream)
+    slot = (device, current_stream(device))
     buf = _workspaces.get(slot)
     if buf is None or buf.numel() < nbytes:
         if buf is not None:
-            buf.record_stream(stream)
+            buf.record_stream(torch.cuda.current_stream(device))
         buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
         _workspaces[slot] = buf
     return buf
