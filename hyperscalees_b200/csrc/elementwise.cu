@@ -15,6 +15,7 @@ template <int VEC>
 __global__ void poisson_kernel(const float* __restrict__ probs, int64_t batch, int in_dim,
                                int64_t stride, int T, uint32_t mix, float* __restrict__ out,
                                __half* __restrict__ out_half) {
+    chain_begin();
     int64_t vec_per_row = in_dim / VEC;
     int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= batch * vec_per_row) return;
@@ -151,6 +152,7 @@ __global__ void member_mean_kernel(const float* __restrict__ x, int64_t n_pop, i
 constexpr int kZThreads = 1024;
 __global__ void zscore_kernel(const float* __restrict__ raw, int64_t n, int group_size,
                               float* __restrict__ out, float* __restrict__ stats) {
+    chain_begin();
     __shared__ float s_sum[kZThreads];
     __shared__ float s_sq[kZThreads];
     float a = 0.0f, b = 0.0f;
@@ -269,6 +271,7 @@ struct SolverMulti {
     int first_block[kSolverMulti + 1];
 };
 __global__ void solver_multi_kernel(SolverConsts c, const __grid_constant__ SolverMulti d) {
+    chain_begin();
     int t = 0;
     while (t + 1 < d.n && (int)blockIdx.x >= d.first_block[t + 1]) ++t;
     const int64_t i = (int64_t)(blockIdx.x - d.first_block[t]) * blockDim.x + threadIdx.x;
@@ -423,12 +426,12 @@ int hses_poisson_encode_dual(hses_ctx* ctx, hses_stream stream, const float* pro
     if (vec) {
         int64_t total = batch * (in_dim / 4);
         HSES_KERNEL(ctx, as_stream(stream), "poisson_encode");
-        poisson_kernel<4><<<(unsigned)((total + 255) / 256), 256, 0, as_stream(stream)>>>(
+        chain_launch(poisson_kernel<4>, (unsigned)((total + 255) / 256), 256, 0, as_stream(stream),
             probs, batch, in_dim, row_stride, T, mix, out, reinterpret_cast<__half*>(out_half));
     } else {
         int64_t total = batch * in_dim;
         HSES_KERNEL(ctx, as_stream(stream), "poisson_encode");
-        poisson_kernel<1><<<(unsigned)((total + 255) / 256), 256, 0, as_stream(stream)>>>(
+        chain_launch(poisson_kernel<1>, (unsigned)((total + 255) / 256), 256, 0, as_stream(stream),
             probs, batch, in_dim, row_stride, T, mix, out, reinterpret_cast<__half*>(out_half));
     }
     HSES_LAUNCH_CHECK();
@@ -511,7 +514,7 @@ int hses_convert_fitnesses(hses_ctx* ctx, hses_stream stream, const float* raw, 
     HSES_REQUIRE(group_size == 0 || n % group_size == 0, "n must be a multiple of group_size");
     HSES_REQUIRE(raw != nullptr && out != nullptr, "NULL pointer");
     HSES_KERNEL(ctx, as_stream(stream), "zscore");
-    zscore_kernel<<<1, kZThreads, 0, as_stream(stream)>>>(raw, n, group_size, out, stats);
+    chain_launch(zscore_kernel, 1, kZThreads, 0, as_stream(stream), raw, n, group_size, out, stats);
     HSES_LAUNCH_CHECK();
     return HSES_OK;
 }
@@ -595,7 +598,7 @@ int solver_step_multi(hses_ctx* ctx, cudaStream_t st, const hses_solver* solver,
         d.first_block[d.n] = (int)blocks;
         if (blocks == 0) continue;
         HSES_KERNEL(ctx, st, "solver");
-        solver_multi_kernel<<<(unsigned)blocks, 256, 0, st>>>(c, d);
+        chain_launch(solver_multi_kernel, (unsigned)blocks, 256, 0, st, c, d);
         HSES_LAUNCH_CHECK();
     }
     return HSES_OK;

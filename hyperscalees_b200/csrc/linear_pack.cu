@@ -43,7 +43,9 @@ constexpr int PK_TR_PITCH = 17;    // staged 32 x 16 output block of an epilogue
 constexpr int PK_TR_BYTES = 8 * 32 * PK_TR_PITCH * 4;
 
 template <int NJ, int RPW>
-__global__ void __launch_bounds__(256) pack_split_kernel(SplitJob j, RowMap map) {
+__global__ void __launch_bounds__(256) pack_split_kernel(SplitJob j, RowMap map, int* clear) {
+    chain_begin();
+    if (clear && blockIdx.x == 0 && threadIdx.x == 0) *clear = 0;
     split_rows<NJ, RPW>(j, map, blockIdx.x);
 }
 
@@ -54,7 +56,9 @@ __global__ void __launch_bounds__(256) pack_operands_kernel(SplitJob x, RowMap m
     __shared__ CalTab tab;
     __shared__ uint64_t state_s[32];
     const int64_t b = blockIdx.x;
+    chain_next();
     if (b < x_blocks) {
+        chain_wait();
         split_rows<NJ, RPW>(x, map, b);
     } else {
         const int64_t i = b - x_blocks;
@@ -118,6 +122,7 @@ linear_pack_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_cons
         mbar_init(&tready, 256);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    chain_wait();                          // before the allocation: a waiting block holds no tensor memory
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
                      "r"(PERT ? 512 : 256)
@@ -127,6 +132,7 @@ linear_pack_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    chain_next();
     const uint32_t tmem = tmem_slot;       // accumulators at columns 0 and 128, t at 256
     const int64_t units = g.m_tiles * g.groups;
     const int nkb = PERT ? g.r16 / g.kb : 1;
@@ -554,7 +560,6 @@ int run_pack_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
                 half_at(p.o_xhi), half_at(p.o_xlo), reinterpret_cast<float*>(ws + p.o_rs), flag};
     // a caller-provided fp16 copy of an x that is exact in fp16 is the operand as it stands
     const bool x_ready = !g.perturb && g.x_half != nullptr && ((uintptr_t)g.x_half & 15u) == 0 && p.kp == g.k;
-    HSES_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
 
     FactorJob f{};
     int segs = 0;
@@ -594,18 +599,18 @@ int run_pack_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
         constexpr int NJ = decltype(nj_c)::value, RPW = decltype(rpw_c)::value;
         {
             HSES_KERNEL(ctx, st, "pack_split_w");
-            pack_split_kernel<NJ, RPW><<<(unsigned)((g.a + 8 * RPW - 1) / (8 * RPW)), 256, 0, st>>>(jw, plain);
+            chain_launch(pack_split_kernel<NJ, RPW>, (unsigned)((g.a + 8 * RPW - 1) / (8 * RPW)), 256, 0, st, jw, plain, flag);
             HSES_LAUNCH_CHECK();
         }
         const int64_t xb = x_ready ? 0 : (p.rows + 8 * RPW - 1) / (8 * RPW), fb = p.pairs * segs;
         HSES_REQUIRE(xb + fb < (1ll << 31), "too many rows");
         if (g.perturb) {
             HSES_KERNEL(ctx, st, "pack_operands");
-            pack_operands_kernel<NJ, RPW><<<(unsigned)(xb + fb), 256, 0, st>>>(jx, map, xb, segs, f);
+            chain_launch(pack_operands_kernel<NJ, RPW>, (unsigned)(xb + fb), 256, 0, st, jx, map, xb, segs, f);
             HSES_LAUNCH_CHECK();
         } else if (xb) {
             HSES_KERNEL(ctx, st, "pack_split_x");
-            pack_split_kernel<NJ, RPW><<<(unsigned)xb, 256, 0, st>>>(jx, map);
+            chain_launch(pack_split_kernel<NJ, RPW>, (unsigned)xb, 256, 0, st, jx, map, nullptr);
             HSES_LAUNCH_CHECK();
         }
         return HSES_OK;
@@ -663,10 +668,10 @@ int run_pack_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
     HSES_KERNEL(ctx, st, "linear_pack");
     if (g.perturb) {
         HSES_CUDA(cudaFuncSetAttribute(linear_pack_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem));
-        linear_pack_kernel<true><<<grid, PK_THREADS, p.smem, st>>>(mx, mxl, mw, mwl, mb, mbl, a);
+        chain_launch(linear_pack_kernel<true>, grid, PK_THREADS, p.smem, st, mx, mxl, mw, mwl, mb, mbl, a);
     } else {
         HSES_CUDA(cudaFuncSetAttribute(linear_pack_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem));
-        linear_pack_kernel<false><<<grid, PK_THREADS, p.smem, st>>>(mx, mxl, mw, mwl, mb, mbl, a);
+        chain_launch(linear_pack_kernel<false>, grid, PK_THREADS, p.smem, st, mx, mxl, mw, mwl, mb, mbl, a);
     }
     HSES_LAUNCH_CHECK();
     return HSES_OK;

@@ -74,6 +74,7 @@ __global__ void es_update_dense_kernel(NoiseCal cal, const uint64_t* __restrict_
                                        int len, float sigma, float out_scale,
                                        const float* __restrict__ fitness, float* __restrict__ grad) {
     __shared__ float red[kDenseThreads];
+    chain_begin();
     int begin = blockIdx.x * kChunk;
     int cnt = len - begin < kChunk ? len - begin : kChunk;
     float acc[kChunk];
@@ -260,7 +261,7 @@ int hses_es_update_dense(hses_ctx* ctx, hses_stream stream, uint64_t key, int32_
     float out_scale = -(1.0f / nf) * sqrtf(nf);
     int blocks = (len + kChunk - 1) / kChunk;
     HSES_KERNEL(ctx, as_stream(stream), "es_update_dense");
-    es_update_dense_kernel<<<blocks, kDenseThreads, 0, as_stream(stream)>>>(
+    chain_launch(es_update_dense_kernel, blocks, kDenseThreads, 0, as_stream(stream),
         ctx->cal(), ctx->t.jump_pow2, key, true_epoch_of(epoch, noise_reuse), first_thread / 2,
         n / 2, len, sigma, out_scale, fitness, grad);
     HSES_LAUNCH_CHECK();

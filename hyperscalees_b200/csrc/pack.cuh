@@ -184,6 +184,7 @@ __device__ __forceinline__ void factor_segment(const FactorJob& f, int64_t p, in
     const int nrows = is_b ? min(f.seg_b, f.k - row0) : min(f.seg_a, f.a - row0);
     const int cnt = nrows * f.r;
     if (f.cache_b) {
+        chain_wait();
         const float* src = is_b ? f.cache_b + ((size_t)p * f.k + row0) * f.r : f.cache_a + ((size_t)p * f.a + row0) * f.r;
         if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
             for (int i = tid; i < cnt / 4; i += blockDim.x)
@@ -200,6 +201,7 @@ __device__ __forceinline__ void factor_segment(const FactorJob& f, int64_t p, in
                     state_s, [&](int off, float (&z)[4]) {
                         *reinterpret_cast<float4*>(buf + off) = make_float4(z[0], z[1], z[2], z[3]);
                     });
+        chain_wait();   // the normals need nothing of the kernels before
     }
     __syncthreads();
     if (is_b) {

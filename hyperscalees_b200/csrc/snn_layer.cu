@@ -42,6 +42,7 @@ constexpr int kSnnMaxLayers = 8;         // hidden layers
 __global__ void __launch_bounds__(256)
 encode_half_kernel(const float* __restrict__ probs, int64_t batch, int in_dim, int64_t stride, int T, uint32_t mix,
                    __half* __restrict__ out, int kp) {
+    chain_begin();
     const int groups = kp >> 3;
     const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x, srow = v / (uint32_t)groups;   // batch * in_dim < 2^32
     if (srow >= batch) return;
@@ -76,6 +77,7 @@ encode_half_kernel(const float* __restrict__ probs, int64_t batch, int in_dim, i
 __global__ void __launch_bounds__(256)
 spikes_half_kernel(const float* __restrict__ src, int64_t n, int T, int k, int64_t stride, __half* __restrict__ out, int kp,
                    int* __restrict__ inexact) {
+    chain_begin();
     const int groups = kp >> 3;
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= n * T * groups) return;
@@ -95,6 +97,7 @@ spikes_half_kernel(const float* __restrict__ src, int64_t n, int T, int k, int64
 // only when the flag is set: the input once more, every row scaled and split into hi + lo
 template <int NJ, int RPW>
 __global__ void __launch_bounds__(256) split_if_inexact_kernel(SplitJob j, RowMap map) {
+    chain_begin();
     if (*j.lo_flag == 0) return;
     for (int64_t b = blockIdx.x; b * (blockDim.x >> 5) * RPW < j.rows; b += gridDim.x) split_rows<NJ, RPW>(j, map, b);
 }
@@ -103,9 +106,12 @@ struct SplitJobs {
     int n;
     SplitJob j[kSnnMaxLayers];
     int block0[kSnnMaxLayers + 1];
+    int* clear;              // the input's flag, or NULL
 };
 template <int NJ, int RPW>
 __global__ void __launch_bounds__(256) snn_split_w_kernel(const __grid_constant__ SplitJobs jobs) {
+    chain_begin();
+    if (jobs.clear && blockIdx.x == 0 && threadIdx.x == 0) *jobs.clear = 0;
     int i = 0;
     while (i + 1 < jobs.n && (int)blockIdx.x >= jobs.block0[i + 1]) ++i;
     RowMap map{};
@@ -123,6 +129,7 @@ __global__ void __launch_bounds__(256) snn_factors_kernel(const __grid_constant_
     __shared__ __align__(16) float buf[PK_SEG];
     __shared__ CalTab tab;
     __shared__ uint64_t state_s[32];
+    chain_next();                                             // factor_segment waits
     int i = 0;
     while (i + 1 < jobs.n && (int64_t)blockIdx.x >= jobs.block0[i + 1]) ++i;
     const int64_t rel = blockIdx.x - jobs.block0[i];
@@ -266,6 +273,7 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
         mbar_init(&tready, 256);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    chain_wait();                                             // before the allocation: a waiting block holds no tensor memory
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
                      "r"(512)
@@ -275,6 +283,7 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    chain_next();
     // Columns 0-255: accumulators of the product, `rows` each (without noise up to 511).  The same from 256: the rank term,
     // whose columns hold t (a part of 128 columns per 128 rows) until it has been read.
     const uint32_t tmem = tmem_slot;
@@ -597,6 +606,7 @@ __global__ void __launch_bounds__(256, 4) snn_readout_kernel(const __grid_consta
     float* xs = as + ((r * C + 3) & ~3);                      // [rows][hp]
     float* ys = xs + g.rows * hp;                             // [rows][jp]
     float* fs = ys + g.rows * jp;                             // [rows]
+    chain_begin();
     const int64_t p = r ? blockIdx.x / g.slices : 0;
     const int64_t s_lo = r ? p * 2 * g.bm + (int64_t)(blockIdx.x - p * g.slices) * g.spb : (int64_t)blockIdx.x * g.spb;
     const int64_t s_hi = min(s_lo + g.spb, r ? (p + 1) * 2 * g.bm : g.n);
@@ -920,44 +930,12 @@ int run_snn_fused(hses_ctx* ctx, cudaStream_t st, const hses_snn_model* m, const
     const int32_t te = true_epoch_of(p->epoch, p->noise_reuse);
     int* flag = reinterpret_cast<int*>(ws + s.o_flag);
 
-    // ---- input spikes ----
     const int k0 = m->dims[0], kp0 = s.l[0].kp;
-    if (in.images) {
-        HSES_REQUIRE((double)s.n * k0 < 4294967296.0, "batch*in_dim must fit the 32-bit element index of the reference stream");
-        const uint32_t mix = in.seeds[0] ^ in.seeds[1] ^ in.seeds[2] ^ in.seeds[3];
-        const int64_t total = s.n * (kp0 / 8);
-        HSES_KERNEL(ctx, st, "encode_half");
-        encode_half_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(in.images, s.n, k0, in.stride, p->T, mix, half_at(s.o_x),
-                                                                           kp0);
-        HSES_LAUNCH_CHECK();
-    } else {
-        HSES_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
-        const int64_t total = rows * (kp0 / 8);
-        {
-            HSES_KERNEL(ctx, st, "spikes_half");
-            spikes_half_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(in.spikes, s.n, p->T, k0, in.stride, half_at(s.o_x), kp0,
-                                                                               flag);
-            HSES_LAUNCH_CHECK();
-        }
-        RowMap map{};
-        map.rows = rows;
-        map.packed = 2;
-        map.t_steps = p->T;
-        map.n_pop = s.n;
-        const int vec = ((uintptr_t)in.spikes & 15u) == 0 && in.stride % 4 == 0;
-        const SplitJob j{in.spikes, in.stride, rows, k0, kp0, vec, half_at(s.o_x), half_at(s.o_xlo), float_at(s.o_rs), flag};
-        HSES_KERNEL(ctx, st, "split_if_inexact");
-        if (kp0 <= 1024)
-            split_if_inexact_kernel<8, 2><<<4 * ctx->sm_count, 256, 0, st>>>(j, map);
-        else
-            split_if_inexact_kernel<0, 1><<<4 * ctx->sm_count, 256, 0, st>>>(j, map);
-        HSES_LAUNCH_CHECK();
-    }
-
-    // ---- weights and factors of every hidden layer ----
+    // ---- weights of every hidden layer ----
     {
         SplitJobs jobs{};
         jobs.n = hidden;
+        jobs.clear = in.images ? nullptr : flag;
         int widest = 0, blocks = 0;
         for (int l = 0; l < hidden; ++l) widest = std::max(widest, s.l[l].kp);
         const int rpb = widest <= 1024 ? 16 : 8;   // rows per block
@@ -971,11 +949,44 @@ int run_snn_fused(hses_ctx* ctx, cudaStream_t st, const hses_snn_model* m, const
         }
         HSES_KERNEL(ctx, st, "snn_split_w");
         if (widest <= 1024)
-            snn_split_w_kernel<8, 2><<<(unsigned)blocks, 256, 0, st>>>(jobs);
+            chain_launch(snn_split_w_kernel<8, 2>, (unsigned)blocks, 256, 0, st, jobs);
         else
-            snn_split_w_kernel<0, 1><<<(unsigned)blocks, 256, 0, st>>>(jobs);
+            chain_launch(snn_split_w_kernel<0, 1>, (unsigned)blocks, 256, 0, st, jobs);
         HSES_LAUNCH_CHECK();
     }
+    // ---- input spikes ----
+    if (in.images) {
+        HSES_REQUIRE((double)s.n * k0 < 4294967296.0, "batch*in_dim must fit the 32-bit element index of the reference stream");
+        const uint32_t mix = in.seeds[0] ^ in.seeds[1] ^ in.seeds[2] ^ in.seeds[3];
+        const int64_t total = s.n * (kp0 / 8);
+        HSES_KERNEL(ctx, st, "encode_half");
+        chain_launch(encode_half_kernel, (unsigned)((total + 255) / 256), 256, 0, st, in.images, s.n, k0, in.stride, p->T, mix, half_at(s.o_x),
+                                                                           kp0);
+        HSES_LAUNCH_CHECK();
+    } else {
+        const int64_t total = rows * (kp0 / 8);
+        {
+            HSES_KERNEL(ctx, st, "spikes_half");
+            chain_launch(spikes_half_kernel, (unsigned)((total + 255) / 256), 256, 0, st, in.spikes, s.n, p->T, k0, in.stride, half_at(s.o_x), kp0,
+                                                                               flag);
+            HSES_LAUNCH_CHECK();
+        }
+        RowMap map{};
+        map.rows = rows;
+        map.packed = 2;
+        map.t_steps = p->T;
+        map.n_pop = s.n;
+        const int vec = ((uintptr_t)in.spikes & 15u) == 0 && in.stride % 4 == 0;
+        const SplitJob j{in.spikes, in.stride, rows, k0, kp0, vec, half_at(s.o_x), half_at(s.o_xlo), float_at(s.o_rs), flag};
+        HSES_KERNEL(ctx, st, "split_if_inexact");
+        if (kp0 <= 1024)
+            chain_launch(split_if_inexact_kernel<8, 2>, 4 * ctx->sm_count, 256, 0, st, j, map);
+        else
+            chain_launch(split_if_inexact_kernel<0, 1>, 4 * ctx->sm_count, 256, 0, st, j, map);
+        HSES_LAUNCH_CHECK();
+    }
+
+    // ---- factors of every hidden layer ----
     if (pert) {
         FactorJobs jobs{};
         jobs.n = hidden;
@@ -1028,7 +1039,7 @@ int run_snn_fused(hses_ctx* ctx, cudaStream_t st, const hses_snn_model* m, const
         }
         HSES_REQUIRE(blocks < (1ll << 31), "too many pairs");
         HSES_KERNEL(ctx, st, "snn_factors");
-        snn_factors_kernel<<<(unsigned)blocks, 256, 0, st>>>(jobs);
+        chain_launch(snn_factors_kernel, (unsigned)blocks, 256, 0, st, jobs);
         HSES_LAUNCH_CHECK();
     }
 
@@ -1088,7 +1099,7 @@ int run_snn_fused(hses_ctx* ctx, cudaStream_t st, const hses_snn_model* m, const
         auto kernel = pert ? snn_layer_kernel<true> : snn_layer_kernel<false>;
         HSES_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, q.smem));
         HSES_KERNEL(ctx, st, "snn_layer");
-        kernel<<<grid, pert ? SL_THREADS_T : SL_THREADS, q.smem, st>>>(mx, mxl, mw, mwl, mb, mbl, a);
+        chain_launch(kernel, grid, pert ? SL_THREADS_T : SL_THREADS, q.smem, st, mx, mxl, mw, mwl, mb, mbl, a);
         HSES_LAUNCH_CHECK();
     }
 
@@ -1143,7 +1154,7 @@ int run_snn_fused(hses_ctx* ctx, cudaStream_t st, const hses_snn_model* m, const
         const int64_t blocks = pert ? s.pairs * s.ro_slices : (s.n + s.ro_spb - 1) / s.ro_spb;
         HSES_CUDA(cudaFuncSetAttribute(snn_readout_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, s.ro_smem));
         HSES_KERNEL(ctx, st, "snn_readout");
-        snn_readout_kernel<<<(unsigned)blocks, 256, s.ro_smem, st>>>(o);
+        chain_launch(snn_readout_kernel, (unsigned)blocks, 256, s.ro_smem, st, o);
         HSES_LAUNCH_CHECK();
     }
     if (o.per_sample) return hses_member_mean(ctx, reinterpret_cast<hses_stream>(st), o.per_sample, p->n_pop, p->bm, score.raw_fitness);

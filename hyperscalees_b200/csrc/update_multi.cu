@@ -69,6 +69,7 @@ __device__ __forceinline__ int rows8(int n) { return (n + 7) & ~7; }
 __device__ __forceinline__ int sign_of(float v) { return v > 0.0f ? 1 : v < 0.0f ? -1 : 0; }
 
 __global__ void um_weight_range_kernel(const float* __restrict__ fitness, int64_t pairs, int* __restrict__ e_out) {
+    chain_begin();
     __shared__ float red[32];
     float m = 0.0f;
     for (int64_t p = threadIdx.x; p < pairs; p += blockDim.x) {
@@ -120,7 +121,8 @@ __global__ void __launch_bounds__(256) update_operands_kernel(const __grid_const
     const int cps = um_starts(wide ? 64 : nrows * r);
     const int ns = max_seg * cps;                                // start states of a k-block
     const float* cache = is_a ? m.cache_a : m.cache_b;
-    const float sc_a = ldexpf(1.0f, UM_EXP_A - *g.e_w);
+    chain_next();
+    if (cache) chain_wait();
     NoiseCal cal = g.cal;
     if (!cache) {
         stage_cal(cal, tab_s);
@@ -143,10 +145,6 @@ __global__ void __launch_bounds__(256) update_operands_kernel(const __grid_const
         const int nseg = wide ? nrows : npairs;
         const int L = wide ? nq : nrows * r;                     // values per segment
         __syncthreads();   // the states are there; the previous tile's values are no longer read
-        if (tid < npairs) {
-            const float* f = g.fitness + 2 * (pair0 + tid);
-            mul_s[tid] = is_a ? __fmul_rn(__fsub_rn(f[0], f[1]), sc_a) : (float)(1 << UM_EXP_B);   // sc_a: a power of two
-        }
         if (cache) {
             for (int sg = 0; sg < nseg; ++sg) {
                 const float* src = wide ? cache + ((size_t)(g.pair_off + pair0) * dim + row0 + sg) * r + q0
@@ -176,6 +174,12 @@ __global__ void __launch_bounds__(256) update_operands_kernel(const __grid_const
                     *reinterpret_cast<float4*>(dst + j) = make_float4(z[0], z[1], z[2], z[3]);
                 }
             }
+        }
+        chain_wait();      // the normals need nothing of the kernels before
+        if (tid < npairs) {
+            const float* f = g.fitness + 2 * (pair0 + tid);
+            const float sc_a = ldexpf(1.0f, UM_EXP_A - *g.e_w);   // a power of two
+            mul_s[tid] = is_a ? __fmul_rn(__fsub_rn(f[0], f[1]), sc_a) : (float)(1 << UM_EXP_B);
         }
         __syncthreads();
         // eight consecutive K values of a row per thread; eight lanes fill a 128-byte row of the image
@@ -249,6 +253,7 @@ __global__ void __launch_bounds__(192, 1) update_gemm_tc_kernel(const __grid_con
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    chain_wait();          // before the allocation: a waiting block holds no tensor memory
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(256)
                      : "memory");
@@ -257,6 +262,7 @@ __global__ void __launch_bounds__(192, 1) update_gemm_tc_kernel(const __grid_con
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    chain_next();
     const uint32_t tmem = tmem_slot;
     if (warp == 0) {
         if (lane == 0) {
@@ -349,6 +355,7 @@ __global__ void __launch_bounds__(192, 1) update_gemm_tc_kernel(const __grid_con
 // Eight warps per 32 elements: warp w adds the splits w, w + 8, .. in index order, then the eight sums are added in
 // warp order: a fixed order, the same bits on every rank.
 __global__ void __launch_bounds__(256) update_multi_reduce_kernel(const __grid_constant__ UmArgs g) {
+    chain_begin();
     __shared__ float part[8][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int i = 0;
@@ -450,7 +457,7 @@ int run_update_multi(hses_ctx* ctx, cudaStream_t st, const UpdateMultiItem* item
                                    UM_STAGES * UM_STAGE_BYTES + 1024));
     {
         HSES_KERNEL(ctx, st, "pair_weight_range");
-        um_weight_range_kernel<<<1, 1024, 0, st>>>(c.fitness, p.pairs, const_cast<int*>(g.e_w));
+        chain_launch(um_weight_range_kernel, 1, 1024, 0, st, c.fitness, p.pairs, const_cast<int*>(g.e_w));
         HSES_LAUNCH_CHECK();
     }
     for (int64_t done = 0; done < p.pairs; done += p.chunk_pairs) {
@@ -500,18 +507,18 @@ int run_update_multi(hses_ctx* ctx, cudaStream_t st, const UpdateMultiItem* item
         HSES_REQUIRE(gen < (1ll << 31) && gemm < (1ll << 31) && red < (1ll << 31), "too many tiles");
         {
             HSES_KERNEL(ctx, st, "update_operands");
-            update_operands_kernel<<<(unsigned)gen, 256, 0, st>>>(g);
+            chain_launch(update_operands_kernel, (unsigned)gen, 256, 0, st, g);
             HSES_LAUNCH_CHECK();
         }
         {
             HSES_KERNEL(ctx, st, "update_gemm_tc");
-            update_gemm_tc_kernel<<<(unsigned)gemm, 192, UM_STAGES * UM_STAGE_BYTES + 1024, st>>>(g);
+            chain_launch(update_gemm_tc_kernel, (unsigned)gemm, 192, UM_STAGES * UM_STAGE_BYTES + 1024, st, g);
             HSES_LAUNCH_CHECK();
         }
         if (done + p.chunk_pairs >= p.pairs) {
             g.add_to_grad = c.add_to_grad;
             HSES_KERNEL(ctx, st, "update_reduce");
-            update_multi_reduce_kernel<<<(unsigned)red, 256, 0, st>>>(g);
+            chain_launch(update_multi_reduce_kernel, (unsigned)red, 256, 0, st, g);
             HSES_LAUNCH_CHECK();
         }
     }
