@@ -89,20 +89,24 @@ __global__ void um_weight_range_kernel(const float* __restrict__ fitness, int64_
     }
 }
 
-// The tiles of one row block in a few consecutive k-blocks, one after the other.  A tile's normals are runs of
-// consecutive stream values ("segments": the rows of the tile for one pair, or, with rank > 64, 64 values of one row).
-// The start states of all segments come from the power-of-two tables, one per thread side by side; from there a lane
-// table spreads 32 threads over a segment.
+// The tiles of one row block in a few consecutive k-blocks.  Their normals are runs of consecutive stream values
+// ("segments": the rows of the tile for one pair, or, with rank > 64, 64 values of one row).  The start states of all
+// segments come from the power-of-two tables, one per thread side by side; from there a lane table gives the start of
+// every piece of a segment.  Narrow matrices take several k-blocks at a time, up to 8704 values: one k-block of 16 rows at
+// a time left most threads with a piece of four values and the lane table's 16 reads for it (430 us for 62 M normals of
+// 33 matrices, two thirds of it the generator).  Bound by the generator's instruction issue.
 constexpr int UM_STATES = 256;
-// values per start state and start states per segment of L values
-__host__ __device__ inline int um_run(int L) { return L >= 512 ? 512 : 128; }
-__host__ __device__ inline int um_starts(int L) { return (L + um_run(L) - 1) / um_run(L); }
+constexpr int UM_GROUP = 16;                         // k-blocks at a time, at most
+__host__ __device__ inline int um_pitch(int L) { return ((L + 3) & ~3) + 4; }
+// values per start state: pieces of 16 or, where that leaves threads without one, of 4; start states per segment
+__host__ __device__ inline int um_run(int L, int values) { return L >= 512 || (L >= 64 && values >= 4096) ? 512 : 128; }
+__host__ __device__ inline int um_starts(int L, int run) { return (L + run - 1) / run; }
 
-__global__ void __launch_bounds__(256) update_operands_kernel(const __grid_constant__ UmArgs g) {
+__global__ void __launch_bounds__(256, 4) update_operands_kernel(const __grid_constant__ UmArgs g) {
     __shared__ __align__(16) float buf[UM_BUF];
     __shared__ CalTab tab_s;
     __shared__ uint64_t seg_state[UM_STATES];
-    __shared__ float mul_s[64];
+    __shared__ float mul_s[64 * UM_GROUP];
     const int tid = threadIdx.x;
     int i = 0;
     while (i + 1 < g.n && (int)blockIdx.x >= g.m[i + 1].gen0) ++i;
@@ -115,11 +119,10 @@ __global__ void __launch_bounds__(256) update_operands_kernel(const __grid_const
     const int row0 = s * step, nrows = min(step, dim - row0);
     const int r = g.r;
     const bool wide = r > 64;
-    const int max_seg = wide ? nrows : g.pb;
-    const int LP = (((wide ? 64 : step * r) + 3) & ~3) + 4;      // pitch of a segment in shared memory
-    const int run = um_run(wide ? 64 : nrows * r), chn = run / 32;
-    const int cps = um_starts(wide ? 64 : nrows * r);
-    const int ns = max_seg * cps;                                // start states of a k-block
+    const int seg_len = wide ? 64 : nrows * r, segs = wide ? nrows : g.pb, LP = um_pitch(seg_len);
+    const int group = wide ? 1 : max(1, min(min(UM_GROUP, kbn), UM_BUF / (segs * LP)));   // k-blocks made at a time
+    const int run = um_run(seg_len, group * segs * seg_len), chn = run / 32, cps = um_starts(seg_len, run);
+    const int ns = segs * cps;                  // start states of a k-block
     const float* cache = is_a ? m.cache_a : m.cache_b;
     chain_next();
     if (cache) chain_wait();
@@ -137,14 +140,20 @@ __global__ void __launch_bounds__(256) update_operands_kernel(const __grid_const
             seg_state[e] = jump_by(g.pow2, s0, 2ull * pos);
         }
     }
-    for (int64_t kb = kb_lo; kb < kb_hi; ++kb) {
-        const int64_t pair0 = wide ? kb / g.rkb : kb * g.pb;     // first pair of the tile (inside the chunk)
+    // eight consecutive K values of a row per thread; eight lanes fill a 128-byte row of the image
+    const int nr8 = is_a ? rows8(nrows) : min(m.bn, (nrows + 15) & ~15);
+    const int dim_pad = is_a ? rows8(m.a) : m.nt * m.bn;         // rows of the operand in a k-block's images
+    const int lo_ofs = (is_a ? nr8 : m.bn) * 128;
+    const int c8 = tid & 7, pp0 = wide ? 0 : c8 * 8 / r, q_first = c8 * 8 - pp0 * r;
+    for (int64_t kb = kb_lo; kb < kb_hi; kb += group) {
+        const int gk = (int)min((int64_t)group, kb_hi - kb);
+        const int64_t pair0 = wide ? kb / g.rkb : kb * g.pb;     // first pair of the tiles (inside the chunk)
         const int q0 = wide ? (int)(kb - pair0 * g.rkb) * 64 : 0;
-        const int npairs = wide ? 1 : (int)min((int64_t)g.pb, g.pairs - pair0);
+        const int npairs = wide ? 1 : (int)min((int64_t)gk * g.pb, g.pairs - pair0);
         const int nq = wide ? min(64, r - q0) : r;               // rank values of the tile
         const int nseg = wide ? nrows : npairs;
         const int L = wide ? nq : nrows * r;                     // values per segment
-        __syncthreads();   // the states are there; the previous tile's values are no longer read
+        __syncthreads();   // the states are there; the previous tiles' values are no longer read
         if (cache) {
             for (int sg = 0; sg < nseg; ++sg) {
                 const float* src = wide ? cache + ((size_t)(g.pair_off + pair0) * dim + row0 + sg) * r + q0
@@ -176,44 +185,56 @@ __global__ void __launch_bounds__(256) update_operands_kernel(const __grid_const
             }
         }
         chain_wait();      // the normals need nothing of the kernels before
-        if (tid < npairs) {
-            const float* f = g.fitness + 2 * (pair0 + tid);
+        for (int i = tid; i < npairs; i += 256) {
+            const float* f = g.fitness + 2 * (pair0 + i);
             const float sc_a = ldexpf(1.0f, UM_EXP_A - *g.e_w);   // a power of two
-            mul_s[tid] = is_a ? __fmul_rn(__fsub_rn(f[0], f[1]), sc_a) : (float)(1 << UM_EXP_B);
+            mul_s[i] = is_a ? __fmul_rn(__fsub_rn(f[0], f[1]), sc_a) : (float)(1 << UM_EXP_B);
         }
         __syncthreads();
-        // eight consecutive K values of a row per thread; eight lanes fill a 128-byte row of the image
-        const int nr8 = is_a ? rows8(nrows) : min(m.bn, (nrows + 15) & ~15);
-        const int dim_pad = is_a ? rows8(m.a) : m.nt * m.bn;         // rows of the operand in a k-block's images
-        uint8_t* img = g.images + (is_a ? m.img_a : m.img_b) + (size_t)kb * dim_pad * 256 + (size_t)row0 * 256;
-        uint8_t* img_lo = img + (size_t)(is_a ? nr8 : m.bn) * 128;
-        for (int idx = tid; idx < nr8 * 8; idx += 256) {
-            const int row = idx >> 3, c = idx & 7;
+        uint8_t* img0 = g.images + (is_a ? m.img_a : m.img_b) + (size_t)kb * dim_pad * 256 + (size_t)row0 * 256;
+        int row = tid >> 3, j = 0;                               // row and k-block of the group
+        while (row >= nr8) row -= nr8, ++j;
+        while (j < gk) {
             float v[8];
-            int pp = wide ? 0 : (c * 8) / r, q = c * 8 - pp * r;
+            if (!wide && (r & 7) == 0) {                         // eight values of one pair
+                const int pp = j * g.pb + pp0;
+                const bool live = row < nrows && pp < npairs && pp0 < g.pb;
+                const float* src = buf + pp * LP + row * r + q_first;
+                const float4 x = live ? *reinterpret_cast<const float4*>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 y = live ? *reinterpret_cast<const float4*>(src + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float w = live ? mul_s[pp] : 0.0f;
+                v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w, v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                float x = 0.0f;
-                if (row < nrows && pp < npairs && q < nq) {
-                    x = wide ? buf[row * LP + q] : buf[pp * LP + row * r + q];
-                    if (g.sign_factors) x = (float)sign_of(x);   // AltEggRoll contracts the sign patterns
-                    x = __fmul_rn(x, mul_s[pp]);
+                for (int k = 0; k < 8; ++k) v[k] = __fmul_rn(g.sign_factors ? (float)sign_of(v[k]) : v[k], w);
+            } else {
+                int pl = pp0, q = q_first;                       // pair of the k-block, rank value
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int pp = j * g.pb + pl;
+                    float x = 0.0f;
+                    if (row < nrows && pl < g.pb && pp < npairs && q < nq) {
+                        x = wide ? buf[row * LP + q] : buf[pp * LP + row * r + q];
+                        if (g.sign_factors) x = (float)sign_of(x);   // AltEggRoll contracts the sign patterns
+                        x = __fmul_rn(x, mul_s[pp]);
+                    }
+                    v[k] = x;
+                    if (++q == r && !wide) q = 0, ++pl;
                 }
-                v[j] = x;
-                if (++q == r && !wide) q = 0, ++pp;
             }
             uint32_t h[4], l[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const __half2 hh = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
+            for (int k = 0; k < 4; ++k) {
+                const __half2 hh = __floats2half2_rn(v[2 * k], v[2 * k + 1]);
                 const float2 b = __half22float2(hh);
-                const __half2 ll = __floats2half2_rn(v[2 * j] - b.x, v[2 * j + 1] - b.y);
-                h[j] = *reinterpret_cast<const uint32_t*>(&hh);
-                l[j] = *reinterpret_cast<const uint32_t*>(&ll);
+                const __half2 ll = __floats2half2_rn(v[2 * k] - b.x, v[2 * k + 1] - b.y);
+                h[k] = *reinterpret_cast<const uint32_t*>(&hh);
+                l[k] = *reinterpret_cast<const uint32_t*>(&ll);
             }
-            const int o = (row >> 3) * 1024 + (row & 7) * 128 + ((c ^ (row & 7)) << 4);
-            *reinterpret_cast<uint4*>(img + o) = make_uint4(h[0], h[1], h[2], h[3]);
-            *reinterpret_cast<uint4*>(img_lo + o) = make_uint4(l[0], l[1], l[2], l[3]);
+            uint8_t* img = img0 + (size_t)j * dim_pad * 256 + (row >> 3) * 1024 + (row & 7) * 128 + ((c8 ^ (row & 7)) << 4);
+            *reinterpret_cast<uint4*>(img) = make_uint4(h[0], h[1], h[2], h[3]);
+            *reinterpret_cast<uint4*>(img + lo_ofs) = make_uint4(l[0], l[1], l[2], l[3]);
+            row += 32;
+            while (row >= nr8) row -= nr8, ++j;
         }
     }
 }
@@ -488,7 +509,7 @@ int run_update_multi(hses_ctx* ctx, cudaStream_t st, const UpdateMultiItem* item
             // launch still has blocks for every SM; the states of all of them have room in shared memory
             auto k_blocks_of = [&](int rows, int tiles) {
                 const int L = c.rank > 64 ? 64 : rows * c.rank;
-                const int ns = (c.rank > 64 ? rows : p.pb) * um_starts(L);
+                const int ns = (c.rank > 64 ? rows : p.pb) * um_starts(L, L >= 512 ? 512 : 128);
                 const int64_t want = std::max<int64_t>(1, 16384 / (64 * rows));
                 const int64_t fill = std::max<int64_t>(1, g.kblks * tiles * n / (4 * (int64_t)ctx->sm_count));
                 return (int)std::max<int64_t>(1, std::min({want, fill, (int64_t)(UM_STATES / ns)}));
