@@ -28,6 +28,24 @@ class IterInfo:
     thread_id: int
 
 
+_range: List[int] = []   # 0, 1, 2, ..: as long as the largest population seen
+
+
+def _contiguous(infos: List[IterInfo]) -> bool:
+    """The usual numbering: thread ids first, first+1, ... of one epoch, whole antithetic pairs."""
+    first, epoch, n = infos[0].thread_id, infos[0].epoch, len(infos)
+    global _range
+    if n % 2 or first % 2 or infos[-1].thread_id != first + n - 1:
+        return False
+    if len(_range) < first + n <= 1 << 20:
+        _range = list(range(first + n))
+    want = _range[first:first + n] if 0 <= first and first + n <= len(_range) else list(range(first, first + n))
+    return [i.thread_id for i in infos if i.epoch == epoch] == want
+
+
+_SOLVERS = {"sgd": ops.SGD, "adam": ops.ADAM, "adamw": ops.ADAMW}
+
+
 # ---------------------------------------------------------------------------
 # Solver (noiser.rs:42-244)
 # ---------------------------------------------------------------------------
@@ -86,7 +104,7 @@ class Solver:
             norm = float(np.sqrt(np.float32(sq)))
             scale = self.max_norm / norm if (norm > self.max_norm and norm > 0.0) else 1.0
             return self.inner.update(params, grads, state, grad_scale=scale)
-        kind = {"sgd": ops.SGD, "adam": ops.ADAM, "adamw": ops.ADAMW}[self.kind]
+        kind = _SOLVERS[self.kind]
         if kind != ops.SGD:
             state.step += 1
         if len(params) == 0:
@@ -369,12 +387,8 @@ class EggRoll:
         """The per-parameter `-g*sqrt(N)` of do_update_with (eggroll.rs:384-404)."""
         n_total = len(iterinfos)
         infos = list(iterinfos)
-        # the usual numbering: thread ids first, first+1, ... of one epoch, whole antithetic pairs
-        first, epoch = infos[0].thread_id, infos[0].epoch
-        contiguous = (n_total % 2 == 0 and first % 2 == 0 and
-                      [i.thread_id for i in infos if i.epoch == epoch] == list(range(first, first + n_total)))
-        if contiguous:
-            groups = {None: (first, fitnesses, epoch)}
+        if _contiguous(infos):
+            groups = {None: (infos[0].thread_id, fitnesses, infos[0].epoch)}
         else:
             dense = _dense_fitness(fitnesses.detach().cpu().numpy(), infos, frozen.noise_reuse)
             nr = max(frozen.noise_reuse, 1)
@@ -411,6 +425,18 @@ class EggRoll:
         advances noiser.opt_state."""
         if len(params) == 0:
             return []
+        sv, state = frozen.solver, noiser.opt_state
+        infos = list(iterinfos)
+        if (type(self).grads is EggRoll.grads and sv.kind in _SOLVERS and all(c == MM_PARAM for c in es_classes) and
+                _contiguous(infos)):
+            if sv.kind != "sgd":
+                state.step += 1
+            adam = sv.kind != "sgd"
+            return ops.es_update_step_multi(
+                base_keys, params, infos[0].epoch, frozen.noise_reuse, frozen.rank, noiser.sigma, fitnesses,
+                (_SOLVERS[sv.kind], sv.lr, sv.beta1, sv.beta2, sv.eps, sv.weight_decay if sv.kind == "adamw" else 0.0),
+                state.step, [s.m for s in state.moments] if adam else None, [s.v for s in state.moments] if adam else None,
+                first_thread=infos[0].thread_id, n_total=len(infos), sign_factors=self.sign_factors)
         grads = self.grads(frozen, noiser, params, base_keys, fitnesses, iterinfos, es_classes)
         return frozen.solver.update(params, grads, noiser.opt_state)
 

@@ -396,25 +396,36 @@ def es_update(key: int, epoch: int, noise_reuse: int, rank: int, a: int, b: int,
     return out
 
 
+def _offsets(shapes):
+    """Where tensors of these shapes lie in one buffer of floats, 16-byte aligned each; the last is its size."""
+    out = [0]
+    for sh in shapes:
+        out.append(out[-1] + (math.prod(sh) + 3) // 4 * 4)
+    return out
+
+
 def _flat_like(shapes, device):
-    """One allocation, a dense tensor per shape (16-byte aligned each)."""
-    sizes = [math.prod(sh) for sh in shapes]
-    padded = [(n + 3) // 4 * 4 for n in sizes]
-    flat = torch.empty(sum(padded), dtype=torch.float32, device=device)
-    return [v[:n].view(sh) if n != m else v.view(sh)
-            for v, n, m, sh in zip(flat.split(padded), sizes, padded, shapes)]
+    """One allocation, a dense tensor per shape."""
+    offs = _offsets(shapes)
+    flat = torch.empty(offs[-1], dtype=torch.float32, device=device)
+    return [flat.as_strided(sh, (sh[1], 1), o) if len(sh) == 2 else flat[o:o + math.prod(sh)].view(sh)
+            for sh, o in zip(shapes, offs)]
 
 
 def es_update_multi(keys: Sequence[int], shapes: Sequence[Tuple[int, int]], epoch: int, noise_reuse: int, rank: int,
                     sigma: float, fitness_: torch.Tensor, first_thread: int = 0, n_total: Optional[int] = None,
                     caches: Optional[Sequence[Optional[FactorCache]]] = None, sign_factors: bool = False):
     """es_update of several matrices (key and (a, b) each) that share members and fitness, in one set of launches."""
+    grads = _flat_like(shapes, fitness_.device)
+    _es_update_into([g.data_ptr() for g in grads], keys, shapes, epoch, noise_reuse, rank, sigma, fitness_, first_thread,
+                    n_total, caches, sign_factors)
+    return grads
+
+
+def _es_update_into(ptrs, keys, shapes, epoch, noise_reuse, rank, sigma, fitness_, first_thread, n_total, caches, sign_factors):
     _check(fitness_, "fitness", ndim=1)
     n, cnt = fitness_.numel(), len(keys)
-    grads = _flat_like(shapes, fitness_.device)
-    items = (_lib.UpdateItem * cnt)()
-    for it, key, (a, b), g in zip(items, keys, shapes, grads):
-        it.key, it.a, it.b, it.grad = key & _U64, a, b, g.data_ptr()
+    items = (_lib.UpdateItem * cnt)(*[(key & _U64, a, b, g) for key, (a, b), g in zip(keys, shapes, ptrs)])
     if caches is not None:
         for it, c in zip(items, caches):
             if c is not None:
@@ -426,7 +437,21 @@ def es_update_multi(keys: Sequence[int], shapes: Sequence[Tuple[int, int]], epoc
     _lib.check(L.hses_es_update_multi(ctx.handle, current_stream(), items, cnt, epoch, noise_reuse, first_thread, n,
                                       n if n_total is None else n_total, rank, sigma, int(sign_factors),
                                       fitness_.data_ptr(), ws.data_ptr() if ws is not None else None, need))
-    return grads
+
+
+def es_update_step_multi(keys: Sequence[int], params: Sequence[torch.Tensor], epoch: int, noise_reuse: int, rank: int,
+                         sigma: float, fitness_: torch.Tensor, solver: Sequence, step: int,
+                         m: Optional[Sequence[torch.Tensor]], v: Optional[Sequence[torch.Tensor]], first_thread: int = 0,
+                         n_total: Optional[int] = None, sign_factors: bool = False):
+    """es_update_multi and solver_step_multi over its gradients, which stay in one buffer that nobody else sees (a view per
+    matrix and its checks took longer on the host than the kernels).  solver: (kind, lr, beta1, beta2, eps, weight_decay)."""
+    params = [p.detach().contiguous() for p in params]
+    shapes = [tuple(p.shape) for p in params]
+    offs = _offsets(shapes)
+    flat = torch.empty(offs[-1], dtype=torch.float32, device=fitness_.device)
+    ptrs = [flat.data_ptr() + 4 * o for o in offs[:-1]]
+    _es_update_into(ptrs, keys, shapes, epoch, noise_reuse, rank, sigma, fitness_, first_thread, n_total, None, sign_factors)
+    return _solver_step_multi(solver, step, 1.0, params, shapes, ptrs, m, v)
 
 
 def convert_fitnesses_bs(raw: torch.Tensor, group_size: int) -> torch.Tensor:
@@ -514,19 +539,29 @@ def solver_step_multi(kind: int, step: int, params: Sequence[torch.Tensor], grad
                       weight_decay: float = 0.0, grad_scale: float = 1.0):
     """One optimizer step over contiguous parameter tensors in one launch; returns the updated copies (the moments
     are updated in place)."""
-    n = len(params)
-    for t in list(params) + list(grads):
+    for t in grads:
         _check(t, "tensor")
         if not t.is_contiguous():
             raise ValueError("params and grads must be contiguous")
-    out = _flat_like([tuple(p.shape) for p in params], params[0].device)
-    arr = lambda ts: (C.c_void_p * n)(*[t.data_ptr() for t in ts])
-    lens = (C.c_int64 * n)(*[p.numel() for p in params])
-    desc = _lib.SolverDesc(kind, lr, beta1, beta2, eps, weight_decay)
+    return _solver_step_multi((kind, lr, beta1, beta2, eps, weight_decay), step, grad_scale, params,
+                              [tuple(p.shape) for p in params], [g.data_ptr() for g in grads], m, v)
+
+
+def _solver_step_multi(solver, step, grad_scale, params, shapes, grad_ptrs, m, v):
+    n = len(params)
+    for t in params:
+        _check(t, "tensor")
+        if not t.is_contiguous():
+            raise ValueError("params and grads must be contiguous")
+    out = _flat_like(shapes, params[0].device)
+    arr = C.c_void_p * n
+    ptrs = lambda ts: arr(*[t.data_ptr() for t in ts]) if ts is not None else None
+    lens = (C.c_int64 * n)(*[math.prod(sh) for sh in shapes])
+    desc = _lib.SolverDesc(*solver)
     ctx = get_context(params[0].device)
     _lib.check(_lib.load().hses_solver_step_multi(
-        ctx.handle, current_stream(), C.byref(desc), step, grad_scale, n, arr(params), arr(out), arr(grads),
-        arr(m) if m is not None else None, arr(v) if v is not None else None, lens))
+        ctx.handle, current_stream(), C.byref(desc), step, grad_scale, n, ptrs(params), ptrs(out), arr(*grad_ptrs),
+        ptrs(m), ptrs(v), lens))
     return out
 
 
