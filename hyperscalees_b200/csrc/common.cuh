@@ -25,7 +25,7 @@ struct DeviceTables {
     // inputs the host libm does not round correctly (reported by hses_ctx_calibration_info)
     uint64_t n_log_flips = 0, n_cos_flips = 0;
     // generator jump tables: entry k advances the state by 2^k steps
-    uint64_t* jump_pow2 = nullptr;  // kJumpLevels matrices
+    uint64_t* jump_tabs = nullptr;  // see jump_by: 16 matrices for each of kJumpLevels / 4 digits
     // lane tables (see lane_jump): lane l goes 4 l or 16 l normals (two steps each) ahead
     uint64_t *jump_lane4 = nullptr, *jump_lane16 = nullptr;
     // one int per device: kernels with bounded waits record here why they gave up
@@ -163,14 +163,14 @@ int solver_step_multi(hses_ctx* ctx, cudaStream_t st, const hses_solver* solver,
 // (offset a multiple of four; the last four may run past cnt).  The states of runs of 512 (128 when there is little to
 // do) come from the power-of-two tables, one per thread side by side, those of a warp's lanes inside a run from a lane
 // table.  state_s: room for max(32, ceil(cnt / 512)) states; cal: staged (stage_cal), the call synchronises.
-constexpr int kStreamCoarse = 4096;   // from here on sixteen normals per thread and table round keep 256 threads busy
+constexpr int kStreamCoarse = 2048;   // from here on sixteen normals per thread and table round keep half a block busy
 template <class Emit>
-__device__ __forceinline__ void stream_fill(const NoiseCal& cal, const uint64_t* __restrict__ pow2,
+__device__ __forceinline__ void stream_fill(const NoiseCal& cal, const uint64_t* __restrict__ jump,
                                             const uint64_t* __restrict__ lane4, const uint64_t* __restrict__ lane16,
                                             uint64_t s0, uint64_t pos0, int cnt, uint64_t* state_s, Emit emit) {
     const bool coarse = cnt >= kStreamCoarse;
     const int chn = coarse ? 16 : 4, run = 32 * chn, runs = (cnt + run - 1) / run, lane = threadIdx.x & 31;
-    for (int e = threadIdx.x; e < runs; e += blockDim.x) state_s[e] = jump_by(pow2, s0, 2ull * (pos0 + (uint64_t)e * run));
+    for (int e = threadIdx.x; e < runs; e += blockDim.x) state_s[e] = jump_by(jump, s0, 2ull * (pos0 + (uint64_t)e * run));
     __syncthreads();
     for (int e = threadIdx.x >> 5; e < runs; e += blockDim.x >> 5) {
         const int off = e * run + lane * chn;

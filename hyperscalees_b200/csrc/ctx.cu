@@ -149,16 +149,22 @@ static int build_tables(DeviceTables& t) {
     HSES_CUDA(cudaMalloc(&t.status_word, sizeof(int)));
     HSES_CUDA(cudaMemset(t.status_word, 0, sizeof(int)));
 
-    // jump tables T^(2^k)
+    // jump tables T^(d * 16^k)
     {
-        std::vector<uint64_t> host((size_t)kJumpLevels * kJumpWords);
-        BitMat m = step_matrix();
-        for (int k = 0; k < kJumpLevels; ++k) {
-            nibble_table(m, host.data() + (size_t)k * kJumpWords);
-            m = compose(m, m);
+        constexpr int digits = kJumpLevels / 4;
+        std::vector<uint64_t> host((size_t)digits * 16 * kJumpWords);
+        BitMat unit = step_matrix();
+        for (int k = 0; k < digits; ++k) {
+            BitMat m;
+            for (int j = 0; j < 64; ++j) m.col[j] = 1ull << j;   // identity
+            for (int d = 0; d < 16; ++d) {
+                nibble_table(m, host.data() + (size_t)(16 * k + d) * kJumpWords);
+                m = compose(unit, m);
+            }
+            unit = m;
         }
-        HSES_CUDA(cudaMalloc(&t.jump_pow2, host.size() * sizeof(uint64_t)));
-        HSES_CUDA(cudaMemcpy(t.jump_pow2, host.data(), host.size() * sizeof(uint64_t),
+        HSES_CUDA(cudaMalloc(&t.jump_tabs, host.size() * sizeof(uint64_t)));
+        HSES_CUDA(cudaMemcpy(t.jump_tabs, host.data(), host.size() * sizeof(uint64_t),
                              cudaMemcpyHostToDevice));
     }
 

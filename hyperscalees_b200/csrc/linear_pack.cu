@@ -568,7 +568,7 @@ int run_pack_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
             int rc = resolve_factor_cache(g, &f.cache_a, &f.cache_b);
             if (rc != HSES_OK) return rc;
         }
-        f.pow2 = ctx->t.jump_pow2;
+        f.jump = ctx->t.jump_tabs;
         f.lane4 = ctx->t.jump_lane4;
         f.lane16 = ctx->t.jump_lane16;
         f.cal = ctx->cal();
@@ -583,8 +583,6 @@ int run_pack_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
         f.a = g.a;
         f.row_a0 = g.factor_order == 1 ? 0 : g.k;
         f.row_b0 = g.factor_order == 1 ? g.a : 0;
-        const int seg = std::max(8, std::min(512, PK_SEG / g.rank & ~7));
-        f.seg_a = f.seg_b = seg;
         f.bn = p.bn;
         f.n_chunks = p.n_chunks;
         f.kb = p.kb;
@@ -593,7 +591,7 @@ int run_pack_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
         f.bhi = half_at(p.o_bhi);
         f.blo = half_at(p.o_blo);
         f.aimg = reinterpret_cast<__nv_bfloat16*>(ws + p.o_aimg);
-        segs = (g.k + seg - 1) / seg + (g.a + seg - 1) / seg;
+        segs = plan_segments(f, ctx->sm_count);
     }
     auto prepare = [&](auto nj_c, auto rpw_c) -> int {
         constexpr int NJ = decltype(nj_c)::value, RPW = decltype(rpw_c)::value;

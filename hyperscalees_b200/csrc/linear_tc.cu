@@ -83,7 +83,7 @@ struct TcArgs {
     float* out;
     int64_t out_stride;
     float* pot;
-    const uint64_t* pow2; // T^(2^k) tables
+    const uint64_t* jump; // T^(2^k) tables
     const uint64_t* hop;  // generator advance from the end of one item of a warp to its next one
     const int* x_lo_flag; // 0 when every lo half of the split x is zero (x exactly representable in fp16)
     const float* cache_a; // cached raw A rows (pair, a, rank) from the call's first pair on, or NULL
@@ -456,7 +456,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
             uint64_t a_state = 0;
             if (!src) {
                 uint64_t s0 = noise_seed(g.key, g.true_epoch, pair) | 1ull;
-                a_state = jump_by(g.pow2, s0, 2ull * ((uint64_t)rt * (uint64_t)(g.row_a0 + it0 * IT::ROWS + n_local) + (uint64_t)qoff));
+                a_state = jump_by(g.jump, s0, 2ull * ((uint64_t)rt * (uint64_t)(g.row_a0 + it0 * IT::ROWS + n_local) + (uint64_t)qoff));
             }
             for (int it = it0; it < items_per_tile; it += GENS) {
                 const uint32_t item = tile_no * (uint32_t)items_per_tile + (uint32_t)it;
@@ -591,7 +591,7 @@ constexpr int LT_ROWS = 64;
 constexpr int LT_KB = 256;
 template <int RANK_G>
 __global__ void __launch_bounds__(LT_THREADS, 2)
-lowrank_t_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, const uint64_t* __restrict__ hop_kb,
+lowrank_t_kernel(NoiseCal cal, const uint64_t* __restrict__ jump, const uint64_t* __restrict__ hop_kb,
                  uint64_t key, int32_t true_epoch, int32_t first_thread, const float* __restrict__ x,
                  int64_t x_stride, int t_steps, int64_t n_pop, int bm, int k, float* __restrict__ t,
                  __half* __restrict__ xhi, __half* __restrict__ xlo, float* __restrict__ inv_scale,
@@ -772,7 +772,7 @@ lowrank_t_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, const uint64_t
     uint64_t sb = 0;
     if (!cache_b) {
         sb = noise_seed(key, true_epoch, pair) | 1ull;
-        sb = jump_by(pow2, sb, 2ull * (uint64_t)rank_true * (uint64_t)(row_b0 + tid));   // row_b0: first input-side row
+        sb = jump_by(jump, sb, 2ull * (uint64_t)rank_true * (uint64_t)(row_b0 + tid));   // row_b0: first input-side row
     }
     // cached raw B rows of this pair, (k, rank) row-major like the block in shared memory
     // (ranks 1..3: rank_true values per row, the remaining columns of the block are zero)
@@ -889,7 +889,7 @@ __device__ __forceinline__ float4 apply_x_op(float4 v, int x_op) {
 // 32 apart, then read consecutive rows, eight of them covering all banks.
 template <int RANK_G, int NJ, int RPR, bool HALF>
 __global__ void __launch_bounds__(LT_THREADS, 2)
-lowrank_t_rows_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, const uint64_t* __restrict__ lane4,
+lowrank_t_rows_kernel(NoiseCal cal, const uint64_t* __restrict__ jump, const uint64_t* __restrict__ lane4,
                       const uint64_t* __restrict__ lane16,
                       uint64_t key, int32_t true_epoch, int32_t first_thread, const float* __restrict__ x,
                       int64_t x_stride, int t_steps, int64_t n_pop, int bm, int k, float* __restrict__ t,
@@ -956,7 +956,7 @@ lowrank_t_rows_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, const uin
             for (int kr = tid; kr < k; kr += LT_THREADS) bsm4[stored_row(kr)] = make_float4(0.f, 0.f, 0.f, 0.f);
             __syncthreads();
         }
-        stream_fill(cal, pow2, lane4, lane16, s0, pos0, k * rank_true, state_s, [&](int off, float (&z)[4]) {
+        stream_fill(cal, jump, lane4, lane16, s0, pos0, k * rank_true, state_s, [&](int off, float (&z)[4]) {
             if (rank_true < 4) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -1132,7 +1132,7 @@ lowrank_t_rows_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, const uin
 // the pieces.  The block kernel walks such a row four values per lane and trip.
 template <int RANK_G>
 __global__ void __launch_bounds__(LT_THREADS, 2)
-lowrank_t_long_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, const uint64_t* __restrict__ lane4,
+lowrank_t_long_kernel(NoiseCal cal, const uint64_t* __restrict__ jump, const uint64_t* __restrict__ lane4,
                       const uint64_t* __restrict__ lane16,
                       uint64_t key, int32_t true_epoch, int32_t first_thread, const float* __restrict__ x,
                       int64_t x_stride, int t_steps, int64_t n_pop, int bm, int k, float* __restrict__ t,
@@ -1201,7 +1201,7 @@ lowrank_t_long_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, const uin
             for (int kr = tid; kr < k; kr += LT_THREADS) bsm4[stored_row(kr)] = make_float4(0.f, 0.f, 0.f, 0.f);
             __syncthreads();
         }
-        stream_fill(cal, pow2, lane4, lane16, s0, pos0, k * rank_true, state_s, [&](int off, float (&z)[4]) {
+        stream_fill(cal, jump, lane4, lane16, s0, pos0, k * rank_true, state_s, [&](int off, float (&z)[4]) {
             if (rank_true < 4) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -1599,7 +1599,7 @@ int run_tensor_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
     ta.out = g.out;
     ta.out_stride = g.out_row_stride;
     ta.pot = g.lif ? g.potentials : nullptr;
-    ta.pow2 = ctx->t.jump_pow2;
+    ta.jump = ctx->t.jump_tabs;
     ta.cal = ctx->cal();
     ta.status = ctx->t.status_word;
     ta.hop = nullptr;
@@ -1618,7 +1618,7 @@ int run_tensor_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
         HSES_KERNEL(ctx, st, "lowrank_t");
 #define HSES_LT(RG)                                                                                          \
     lowrank_t_kernel<RG><<<lt_grid, LT_THREADS, 0, st>>>(                                            \
-        ctx->cal(), ctx->t.jump_pow2, hop127, g.key, ta.true_epoch, g.first_thread, g.x, g.x_row_stride,     \
+        ctx->cal(), ctx->t.jump_tabs, hop127, g.key, ta.true_epoch, g.first_thread, g.x, g.x_row_stride,     \
         g.t_steps, g.n_pop, g.bm, g.k, sc.t, sc.xhi, sc.xlo, sc.rs, cache_b, sc.lo_flag, one_pass, g.rank, g.factor_order == 1 ? g.a : 0, \
         reuse_split ? 1 : 0)
         dim3 lt_grid((unsigned)pairs, (unsigned)((2 * (int64_t)g.bm * g.t_steps + LT_ROWS - 1) / LT_ROWS));
@@ -1631,7 +1631,7 @@ int run_tensor_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
         HSES_CUDA(cudaFuncSetAttribute(lowrank_t_rows_kernel<RG, NJ, RPR, HALF>,                              \
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));                  \
         lowrank_t_rows_kernel<RG, NJ, RPR, HALF><<<HALF ? lt_grid2 : lt_grid, LT_THREADS, b_bytes, st>>>(     \
-            ctx->cal(), ctx->t.jump_pow2, ctx->t.jump_lane4, ctx->t.jump_lane16, g.key, ta.true_epoch, g.first_thread, g.x, g.x_row_stride, \
+            ctx->cal(), ctx->t.jump_tabs, ctx->t.jump_lane4, ctx->t.jump_lane16, g.key, ta.true_epoch, g.first_thread, g.x, g.x_row_stride, \
             g.t_steps, g.n_pop, g.bm, g.k, sc.t, sc.xhi, sc.xlo, sc.rs, cache_b, sc.lo_flag, one_pass, g.rank, \
             g.factor_order == 1 ? g.a : 0, reuse_split ? 1 : 0, groups, g.x_op);                                      \
     } while (0)
@@ -1660,7 +1660,7 @@ int run_tensor_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
         HSES_CUDA(cudaFuncSetAttribute(lowrank_t_long_kernel<RG>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                        65536));                                                               \
         lowrank_t_long_kernel<RG><<<lt_grid, LT_THREADS, b_bytes, st>>>(                                      \
-            ctx->cal(), ctx->t.jump_pow2, ctx->t.jump_lane4, ctx->t.jump_lane16, g.key, ta.true_epoch, g.first_thread, g.x, g.x_row_stride, \
+            ctx->cal(), ctx->t.jump_tabs, ctx->t.jump_lane4, ctx->t.jump_lane16, g.key, ta.true_epoch, g.first_thread, g.x, g.x_row_stride, \
             g.t_steps, g.n_pop, g.bm, g.k, sc.t, sc.xhi, sc.xlo, sc.rs, cache_b, sc.lo_flag, one_pass, g.rank, \
             g.factor_order == 1 ? g.a : 0, reuse_split ? 1 : 0, 1, g.x_op);                                           \
     } while (0)

@@ -11,19 +11,19 @@ namespace hses {
 // chunk with a jump of 2*kChunk*chunk_index generator steps.
 constexpr int kChunk = 16;
 
-__global__ void normal_fill_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, uint64_t seed,
+__global__ void normal_fill_kernel(NoiseCal cal, const uint64_t* __restrict__ jump, uint64_t seed,
                                    float* __restrict__ out, size_t n) {
     size_t chunk = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     size_t begin = chunk * kChunk;
     if (begin >= n) return;
-    uint64_t s = jump_by(pow2, seed | 1ull, 2ull * begin);
+    uint64_t s = jump_by(jump, seed | 1ull, 2ull * begin);
     size_t end = begin + kChunk < n ? begin + kChunk : n;
     for (size_t i = begin; i < end; ++i) out[i] = normal1(s, cal);
 }
 
 // One thread per (member, row of the (a+b, r) block).  Rows [0,b) are B, rows
 // [b,a+b) are A (eggroll.rs:98-101).
-__global__ void lora_factors_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, uint64_t key,
+__global__ void lora_factors_kernel(NoiseCal cal, const uint64_t* __restrict__ jump, uint64_t key,
                                     int32_t true_epoch, const int32_t* __restrict__ thread_ids,
                                     int32_t first_thread, int64_t n_members, int rank, int a, int b,
                                     float base_sigma, int layout, float* __restrict__ A,
@@ -36,7 +36,7 @@ __global__ void lora_factors_kernel(NoiseCal cal, const uint64_t* __restrict__ p
     int32_t tid = thread_ids ? thread_ids[member] : first_thread + (int32_t)member;
     float scale = (tid % 2 == 0) ? base_sigma : -base_sigma;  // sign * base_sigma
     uint64_t s = noise_seed(key, true_epoch, tid / 2) | 1ull;
-    s = jump_by(pow2, s, 2ull * (uint64_t)rank * (uint64_t)row);
+    s = jump_by(jump, s, 2ull * (uint64_t)rank * (uint64_t)row);
     int m = is_a ? row - b : row;
     int dim = is_a ? a : b;
     float* dst = is_a ? A : B;
@@ -50,7 +50,7 @@ __global__ void lora_factors_kernel(NoiseCal cal, const uint64_t* __restrict__ p
     }
 }
 
-__global__ void dense_noise_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, uint64_t key,
+__global__ void dense_noise_kernel(NoiseCal cal, const uint64_t* __restrict__ jump, uint64_t key,
                                    int32_t true_epoch, const int32_t* __restrict__ thread_ids,
                                    int32_t first_thread, int64_t n_members, int len,
                                    float base_sigma, float* __restrict__ out) {
@@ -60,7 +60,7 @@ __global__ void dense_noise_kernel(NoiseCal cal, const uint64_t* __restrict__ po
     int32_t tid = thread_ids ? thread_ids[member] : first_thread + (int32_t)member;
     float scale = (tid % 2 == 0) ? base_sigma : -base_sigma;
     uint64_t s = noise_seed(key, true_epoch, tid / 2) | 1ull;
-    s = jump_by(pow2, s, 2ull * (uint64_t)begin);
+    s = jump_by(jump, s, 2ull * (uint64_t)begin);
     int end = begin + kChunk < len ? begin + kChunk : len;
     for (int i = begin; i < end; ++i) out[(size_t)member * len + i] = fmul(normal1(s, cal), scale);
 }
@@ -69,7 +69,7 @@ __global__ void dense_noise_kernel(NoiseCal cal, const uint64_t* __restrict__ po
 // threads stride over the antithetic pairs, then reduce in a fixed order so
 // that every rank obtains the same bits.
 constexpr int kDenseThreads = 1024;  // few blocks (one per chunk of a leaf): all the parallelism is in the block
-__global__ void es_update_dense_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, uint64_t key,
+__global__ void es_update_dense_kernel(NoiseCal cal, const uint64_t* __restrict__ jump, uint64_t key,
                                        int32_t true_epoch, int32_t first_pair, int64_t n_pairs,
                                        int len, float sigma, float out_scale,
                                        const float* __restrict__ fitness, float* __restrict__ grad) {
@@ -84,7 +84,7 @@ __global__ void es_update_dense_kernel(NoiseCal cal, const uint64_t* __restrict_
         // member 2p has sign +1, member 2p+1 sign -1 (eggroll.rs:60-65)
         float w = fmul(fitness[2 * p] - fitness[2 * p + 1], sigma);
         uint64_t s = noise_seed(key, true_epoch, first_pair + (int32_t)p) | 1ull;
-        s = jump_by(pow2, s, 2ull * (uint64_t)begin);
+        s = jump_by(jump, s, 2ull * (uint64_t)begin);
 #pragma unroll
         for (int i = 0; i < kChunk; ++i)
             if (i < cnt) acc[i] = fmaf(w, normal1(s, cal), acc[i]);
@@ -105,7 +105,7 @@ __global__ void es_update_dense_kernel(NoiseCal cal, const uint64_t* __restrict_
 // stream; CTA (pair, piece) makes kPfPiece normals of it.  Bound by instruction issue (about a hundred per normal).
 constexpr int kPfPiece = 8192;
 __global__ void __launch_bounds__(256)
-pair_factors_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, const uint64_t* __restrict__ lane4,
+pair_factors_kernel(NoiseCal cal, const uint64_t* __restrict__ jump, const uint64_t* __restrict__ lane4,
                     const uint64_t* __restrict__ lane16, uint64_t key, int32_t true_epoch, int32_t first_pair, int64_t na,
                     int64_t nb, const float* __restrict__ pair_weight, float* __restrict__ A, float* __restrict__ B) {
     __shared__ CalTab tab;
@@ -119,7 +119,7 @@ pair_factors_kernel(NoiseCal cal, const uint64_t* __restrict__ pow2, const uint6
     const int split = (int)min((int64_t)cnt, max((int64_t)0, nb - e0));   // values of this piece that belong to B
     const bool vec = ((reinterpret_cast<uintptr_t>(dst_b) | reinterpret_cast<uintptr_t>(dst_a)) & 15) == 0 && (split & 3) == 0 &&
                      (cnt & 3) == 0;
-    stream_fill(cal, pow2, lane4, lane16, noise_seed(key, true_epoch, first_pair + (int32_t)p) | 1ull, (uint64_t)e0, cnt, state_s,
+    stream_fill(cal, jump, lane4, lane16, noise_seed(key, true_epoch, first_pair + (int32_t)p) | 1ull, (uint64_t)e0, cnt, state_s,
                 [&](int off, float (&z)[4]) {
                     if (vec) {
                         const bool is_a = off >= split;
@@ -148,7 +148,7 @@ int launch_pair_factors(hses_ctx* ctx, cudaStream_t stream, uint64_t key, int32_
     HSES_REQUIRE(pairs >= 1 && pairs < (1ll << 31), "pair count out of range");
     dim3 grid((unsigned)pairs, (unsigned)pieces);
     HSES_KERNEL(ctx, stream, "pair_factors");
-    pair_factors_kernel<<<grid, 256, 0, stream>>>(ctx->cal(), ctx->t.jump_pow2, ctx->t.jump_lane4, ctx->t.jump_lane16, key,
+    pair_factors_kernel<<<grid, 256, 0, stream>>>(ctx->cal(), ctx->t.jump_tabs, ctx->t.jump_lane4, ctx->t.jump_lane16, key,
                                                   true_epoch, first_pair, na, nb, pair_weight, A, B);
     HSES_LAUNCH_CHECK();
     return HSES_OK;
@@ -200,7 +200,7 @@ int hses_normal_fill(hses_ctx* ctx, hses_stream stream, uint64_t seed, float* ou
     size_t chunks = (n + kChunk - 1) / kChunk;
     unsigned blocks = (unsigned)((chunks + 127) / 128);
     HSES_KERNEL(ctx, as_stream(stream), "normal_fill");
-    normal_fill_kernel<<<blocks, 128, 0, as_stream(stream)>>>(ctx->cal(), ctx->t.jump_pow2, seed, out, n);
+    normal_fill_kernel<<<blocks, 128, 0, as_stream(stream)>>>(ctx->cal(), ctx->t.jump_tabs, seed, out, n);
     HSES_LAUNCH_CHECK();
     return HSES_OK;
 }
@@ -221,7 +221,7 @@ int hses_lora_factors(hses_ctx* ctx, hses_stream stream, uint64_t key, int32_t e
     dim3 grid((unsigned)n_members, (unsigned)((rows + 127) / 128));
     HSES_KERNEL(ctx, as_stream(stream), "lora_factors");
     lora_factors_kernel<<<grid, 128, 0, as_stream(stream)>>>(
-        ctx->cal(), ctx->t.jump_pow2, key, true_epoch_of(epoch, noise_reuse), thread_ids,
+        ctx->cal(), ctx->t.jump_tabs, key, true_epoch_of(epoch, noise_reuse), thread_ids,
         first_thread, n_members, rank, a, b, base_sigma, layout, A, B);
     HSES_LAUNCH_CHECK();
     return HSES_OK;
@@ -241,7 +241,7 @@ int hses_dense_noise(hses_ctx* ctx, hses_stream stream, uint64_t key, int32_t ep
     dim3 grid((unsigned)n_members, (unsigned)((chunks + 63) / 64));
     HSES_KERNEL(ctx, as_stream(stream), "dense_noise");
     dense_noise_kernel<<<grid, 64, 0, as_stream(stream)>>>(
-        ctx->cal(), ctx->t.jump_pow2, key, true_epoch_of(epoch, noise_reuse), thread_ids,
+        ctx->cal(), ctx->t.jump_tabs, key, true_epoch_of(epoch, noise_reuse), thread_ids,
         first_thread, n_members, len, base_sigma, out);
     HSES_LAUNCH_CHECK();
     return HSES_OK;
@@ -262,7 +262,7 @@ int hses_es_update_dense(hses_ctx* ctx, hses_stream stream, uint64_t key, int32_
     int blocks = (len + kChunk - 1) / kChunk;
     HSES_KERNEL(ctx, as_stream(stream), "es_update_dense");
     chain_launch(es_update_dense_kernel, blocks, kDenseThreads, 0, as_stream(stream),
-        ctx->cal(), ctx->t.jump_pow2, key, true_epoch_of(epoch, noise_reuse), first_thread / 2,
+        ctx->cal(), ctx->t.jump_tabs, key, true_epoch_of(epoch, noise_reuse), first_thread / 2,
         n / 2, len, sigma, out_scale, fitness, grad);
     HSES_LAUNCH_CHECK();
     return HSES_OK;

@@ -5,13 +5,15 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 #include "tc_common.cuh"
 
 namespace hses {
 namespace pack {
 
 constexpr int PK_EXP_B = 11;       // B * 2^11: |normal| < 6 keeps it below 2^14
-constexpr int PK_SEG = 4096;       // normals of a factor segment
+constexpr int PK_SEG = 8192;       // normals of a factor segment, at most
 
 // Which row of the call a packed row is.
 struct RowMap {
@@ -160,14 +162,14 @@ __device__ __forceinline__ void split_rows(const SplitJob& j, const RowMap& map,
 }
 struct FactorJob {
     const float *cache_a, *cache_b;   // raw (pairs, a, r) and (pairs, k, r), or NULL: regenerate
-    const uint64_t *pow2, *lane4, *lane16;
+    const uint64_t *jump, *lane4, *lane16;
     NoiseCal cal;
     uint64_t key;
     int32_t true_epoch, first_pair;
     int64_t pairs;
     int r, r16, k, kp, a;
     int row_a0, row_b0;               // first output-side and input-side row of a pair's stream block
-    int seg_b, seg_a;                 // rows per segment (multiples of 8)
+    int seg;                          // rows per segment (a multiple of 8)
     int bn, n_chunks, kb;             // output columns per chunk, chunks, rank values per block of A's image
     float base_sigma;
     const float* col_scale;           // 2^-e of W's rows
@@ -175,78 +177,101 @@ struct FactorJob {
     __nv_bfloat16* aimg;              // (pairs, chunk, r16 / kb, part 3, kb / 8, bn, 8)
 };
 
+// Segments of a pair's k + a rows of normals: as long as shared memory allows (a segment's start is a chain of tables that
+// its block waits for), shorter where that leaves SMs without four of them.  In stream order a segment may hold the end of
+// B and the start of A; else B's segments come first, then A's.  1000 members of 784-300-100, rank 6: 49 us; 512 rows of
+// one factor at a time, four normals to a thread 64 us; 16 pairs are fastest in short segments.
+inline int plan_segments(FactorJob& f, int sms) {
+    const int64_t normals = f.pairs * (int64_t)(f.k + f.a) * f.r;
+    const int want = (int)std::max<int64_t>(512, std::min<int64_t>(PK_SEG, normals / (4 * (int64_t)sms)));
+    f.seg = std::max(8, std::min(2048, (want / f.r) & ~7));
+    return f.row_b0 == 0 ? (f.k + f.a + f.seg - 1) / f.seg : (f.k + f.seg - 1) / f.seg + (f.a + f.seg - 1) / f.seg;
+}
 // Segment `seg` of pair `p`: its normals into shared memory (from the cache, or stream_fill), then to the operand layout.
 __device__ __forceinline__ void factor_segment(const FactorJob& f, int64_t p, int seg, float* buf, CalTab& tab, uint64_t* state_s) {
-    const int tid = threadIdx.x;
-    const int nseg_b = (f.k + f.seg_b - 1) / f.seg_b;
-    const bool is_b = seg < nseg_b;
-    const int row0 = is_b ? seg * f.seg_b : (seg - nseg_b) * f.seg_a;
-    const int nrows = is_b ? min(f.seg_b, f.k - row0) : min(f.seg_a, f.a - row0);
-    const int cnt = nrows * f.r;
+    const int tid = threadIdx.x, step = f.seg;
+    int b0, nb, a0, na;                                       // first row and rows of B and of A in this segment
+    if (f.row_b0 == 0) {
+        const int c0 = seg * step, c1 = min(c0 + step, f.k + f.a);
+        b0 = min(c0, f.k), nb = min(c1, f.k) - b0;
+        a0 = max(c0 - f.k, 0), na = max(c1 - f.k, 0) - a0;
+    } else {
+        const int nseg_b = (f.k + step - 1) / step;
+        const bool is_b = seg < nseg_b;
+        b0 = is_b ? seg * step : f.k, nb = is_b ? min(step, f.k - b0) : 0;
+        a0 = is_b ? 0 : (seg - nseg_b) * step, na = is_b ? 0 : min(step, f.a - a0);
+    }
     if (f.cache_b) {
         chain_wait();
-        const float* src = is_b ? f.cache_b + ((size_t)p * f.k + row0) * f.r : f.cache_a + ((size_t)p * f.a + row0) * f.r;
-        if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-            for (int i = tid; i < cnt / 4; i += blockDim.x)
-                *reinterpret_cast<float4*>(buf + 4 * i) = __ldg(reinterpret_cast<const float4*>(src) + i);
-            for (int i = (cnt & ~3) + tid; i < cnt; i += blockDim.x) buf[i] = __ldg(src + i);
-        } else {
-            for (int i = tid; i < cnt; i += blockDim.x) buf[i] = __ldg(src + i);
-        }
+        auto fetch = [&](float* dst, const float* src, int cnt) {
+            if (((reinterpret_cast<uintptr_t>(src) | (uintptr_t)(4 * (dst - buf))) & 15) == 0) {
+                for (int i = tid; i < cnt / 4; i += blockDim.x)
+                    *reinterpret_cast<float4*>(dst + 4 * i) = __ldg(reinterpret_cast<const float4*>(src) + i);
+                for (int i = (cnt & ~3) + tid; i < cnt; i += blockDim.x) dst[i] = __ldg(src + i);
+            } else {
+                for (int i = tid; i < cnt; i += blockDim.x) dst[i] = __ldg(src + i);
+            }
+        };
+        fetch(buf, f.cache_b + ((size_t)p * f.k + b0) * f.r, nb * f.r);
+        fetch(buf + nb * f.r, f.cache_a + ((size_t)p * f.a + a0) * f.r, na * f.r);
     } else {
         NoiseCal cal = f.cal;
         stage_cal(cal, tab);
-        const uint64_t first = (uint64_t)f.r * (uint64_t)(row0 + (is_b ? f.row_b0 : f.row_a0));
-        stream_fill(cal, f.pow2, f.lane4, f.lane16, noise_seed(f.key, f.true_epoch, f.first_pair + (int32_t)p) | 1ull, first, cnt,
-                    state_s, [&](int off, float (&z)[4]) {
+        const uint64_t first = (uint64_t)f.r * (uint64_t)(nb ? b0 + f.row_b0 : a0 + f.row_a0);
+        stream_fill(cal, f.jump, f.lane4, f.lane16, noise_seed(f.key, f.true_epoch, f.first_pair + (int32_t)p) | 1ull, first,
+                    (nb + na) * f.r, state_s, [&](int off, float (&z)[4]) {
                         *reinterpret_cast<float4*>(buf + off) = make_float4(z[0], z[1], z[2], z[3]);
                     });
         chain_wait();   // the normals need nothing of the kernels before
     }
     __syncthreads();
-    if (is_b) {
+    if (nb) {
         // eight consecutive k of one rank column per thread: 4 such pieces x 8 columns per warp
-        const int kend = min(f.kp - row0, f.seg_b);           // the padding of the last segment's rows is zero
-        const int ng = (kend + 7) >> 3;
+        const int kend = b0 + nb == f.k ? f.kp - b0 : nb;     // the padding of the last segment's rows is zero
+        const int ng = (kend + 7) >> 3, qb = f.r16 >> 3;
         const float sc = (float)(1 << PK_EXP_B);
         for (int idx = tid; idx < ((ng + 3) & ~3) * f.r16; idx += blockDim.x) {
             const int blk = idx >> 5, l = idx & 31;
-            const int qb = f.r16 >> 3;
             const int q = (blk % qb) * 8 + (l & 7), g = (blk / qb) * 4 + (l >> 3);
             if (g >= ng) continue;
-            float v[8];
+            uint2 h0 = make_uint2(0, 0), h1 = h0, l0 = h0, l1 = h0;
+            if (q < f.r) {
+                float v[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                v[j] = (q < f.r && g * 8 + j < nrows) ? buf[(g * 8 + j) * f.r + q] : 0.0f;
-            uint2 h0, h1, l0, l1;
-            uint32_t nz = 0;
-            split4(make_float4(v[0], v[1], v[2], v[3]), sc, h0, l0, nz);
-            split4(make_float4(v[4], v[5], v[6], v[7]), sc, h1, l1, nz);
-            const size_t o = ((size_t)p * f.r16 + q) * f.kp + row0 + g * 8;
+                for (int j = 0; j < 8; ++j) v[j] = g * 8 + j < nb ? buf[(g * 8 + j) * f.r + q] : 0.0f;
+                uint32_t nz = 0;
+                split4(make_float4(v[0], v[1], v[2], v[3]), sc, h0, l0, nz);
+                split4(make_float4(v[4], v[5], v[6], v[7]), sc, h1, l1, nz);
+            }
+            const size_t o = ((size_t)p * f.r16 + q) * f.kp + b0 + g * 8;
             *reinterpret_cast<uint4*>(f.bhi + o) = make_uint4(h0.x, h0.y, h1.x, h1.y);
             *reinterpret_cast<uint4*>(f.blo + o) = make_uint4(l0.x, l0.y, l1.x, l1.y);
         }
-    } else {
-        for (int idx = tid; idx < nrows * (f.r16 >> 3); idx += blockDim.x) {
-            const int g = idx / nrows, i = idx - g * nrows;   // rank piece, row of the segment
-            const int n = row0 + i, c = n / f.bn, nn = n - c * f.bn;
-            const uint32_t e = 254u - (__float_as_uint(__ldg(f.col_scale + n)) >> 23);   // exponent field of 2^+e
-            const float sc = __fmul_rn(f.base_sigma, __uint_as_float(e << 23)) * (1.0f / (1 << PK_EXP_B));
-            uint32_t w[3][4];
+    }
+    if (na) {
+        const float* src = buf + nb * f.r;
+        for (int idx = tid; idx < na * (f.r16 >> 3); idx += blockDim.x) {
+            const int g = idx / na, i = idx - g * na;         // rank piece, row of the segment
+            const int n = a0 + i, c = n / f.bn, nn = n - c * f.bn;
+            uint32_t w[3][4] = {};
+            if (g * 8 < f.r) {
+                const uint32_t e = 254u - (__float_as_uint(__ldg(f.col_scale + n)) >> 23);   // exponent field of 2^+e
+                const float sc = __fmul_rn(f.base_sigma, __uint_as_float(e << 23)) * (1.0f / (1 << PK_EXP_B));
 #pragma unroll
-            for (int j = 0; j < 8; j += 2) {
-                float v[2];
+                for (int j = 0; j < 8; j += 2) {
+                    float v[2];
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int q = g * 8 + j + h;
-                    v[h] = q < f.r ? __fmul_rn(buf[i * f.r + q], sc) : 0.0f;
-                }
+                    for (int h = 0; h < 2; ++h) {
+                        const int q = g * 8 + j + h;
+                        v[h] = q < f.r ? __fmul_rn(src[i * f.r + q], sc) : 0.0f;
+                    }
 #pragma unroll
-                for (int part = 0; part < 3; ++part) {
-                    const __nv_bfloat162 b = __floats2bfloat162_rn(v[0], v[1]);
-                    w[part][j >> 1] = *reinterpret_cast<const uint32_t*>(&b);
-                    v[0] -= __bfloat162float(b.x);
-                    v[1] -= __bfloat162float(b.y);
+                    for (int part = 0; part < 3; ++part) {
+                        const __nv_bfloat162 b = __floats2bfloat162_rn(v[0], v[1]);
+                        w[part][j >> 1] = *reinterpret_cast<const uint32_t*>(&b);
+                        v[0] -= __bfloat162float(b.x);
+                        v[1] -= __bfloat162float(b.y);
+                    }
                 }
             }
             const int kblk = (g * 8) / f.kb, gi = g - kblk * (f.kb >> 3);

@@ -171,10 +171,11 @@ HSES_HD uint64_t jump_apply(const uint64_t* __restrict__ tab, uint64_t x) {
     return r;
 }
 
-// tabs[k] advances the state by unit*2^k steps; n is in units.
+// Table 16 k + d advances the state by d * 16^k steps: a start state is a chain of dependent tables, one per non-zero
+// hexadecimal digit of its position (with one per set bit the chain was twice as long).
 HSES_HD uint64_t jump_by(const uint64_t* __restrict__ tabs, uint64_t x, uint64_t n) {
-    for (int k = 0; n != 0; ++k, n >>= 1)
-        if (n & 1) x = jump_apply(tabs + (size_t)k * kJumpWords, x);
+    for (int k = 0; n != 0; ++k, n >>= 4)
+        if (n & 15) x = jump_apply(tabs + (size_t)(16 * k + (int)(n & 15)) * kJumpWords, x);
     return x;
 }
 

@@ -569,7 +569,7 @@ struct ReadoutArgs {
     int32_t first_pair;
     const float *cache_a, *cache_b;
     NoiseCal cal;
-    const uint64_t *pow2, *lane4, *lane16;
+    const uint64_t *jump, *lane4, *lane16;
     uint64_t key;
     int32_t true_epoch;
     float base_sigma, gain;
@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(256, 4) snn_readout_kernel(const __grid_consta
             const int cnt = nb + na;
             for (int base = 0; base < cnt; base += 32768) {
                 __syncthreads();
-                stream_fill(cal, g.pow2, g.lane4, g.lane16,
+                stream_fill(cal, g.jump, g.lane4, g.lane16,
                             noise_seed(g.key, g.true_epoch, g.first_pair + (int32_t)p) | 1ull, (uint64_t)base,
                             min(32768, cnt - base), state_s, [&](int off, float (&z)[4]) {
 #pragma unroll
@@ -1009,7 +1009,7 @@ int run_snn_fused(hses_ctx* ctx, cudaStream_t st, const hses_snn_model* m, const
                 int rc = resolve_factor_cache(la, &f.cache_a, &f.cache_b);
                 if (rc != HSES_OK) return rc;
             }
-            f.pow2 = ctx->t.jump_pow2;
+            f.jump = ctx->t.jump_tabs;
             f.lane4 = ctx->t.jump_lane4;
             f.lane16 = ctx->t.jump_lane16;
             f.cal = ctx->cal();
@@ -1024,7 +1024,6 @@ int run_snn_fused(hses_ctx* ctx, cudaStream_t st, const hses_snn_model* m, const
             f.a = m->dims[l + 1];
             f.row_a0 = f.k;
             f.row_b0 = 0;
-            f.seg_a = f.seg_b = std::max(8, std::min(512, (PK_SEG / p->rank) & ~7));
             f.bn = q.bn;
             f.n_chunks = q.n_chunks;
             f.kb = q.r16;
@@ -1033,7 +1032,7 @@ int run_snn_fused(hses_ctx* ctx, cudaStream_t st, const hses_snn_model* m, const
             f.bhi = half_at(q.o_bhi);
             f.blo = half_at(q.o_blo);
             f.aimg = reinterpret_cast<__nv_bfloat16*>(ws + q.o_aimg);
-            jobs.segs[l] = (f.k + f.seg_b - 1) / f.seg_b + (f.a + f.seg_a - 1) / f.seg_a;
+            jobs.segs[l] = plan_segments(f, ctx->sm_count);
             jobs.block0[l] = blocks;
             blocks += s.pairs * jobs.segs[l];
         }
@@ -1121,7 +1120,7 @@ int run_snn_fused(hses_ctx* ctx, cudaStream_t st, const hses_snn_model* m, const
     o.first_pair = p->first_thread / 2;
     if (pert) {
         o.cal = ctx->cal();
-        o.pow2 = ctx->t.jump_pow2;
+        o.jump = ctx->t.jump_tabs;
         o.lane4 = ctx->t.jump_lane4;
         o.lane16 = ctx->t.jump_lane16;
         o.key = m->keys[hidden];

@@ -48,7 +48,7 @@ struct UmMat {
 };
 struct UmArgs {
     int n;
-    const uint64_t *pow2, *lane4, *lane16;
+    const uint64_t *jump, *lane4, *lane16;
     NoiseCal cal;
     int32_t true_epoch, first_pair;   // first_pair: of this chunk
     int64_t pair_off;                 // pairs of the call before this chunk
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(256, 4) update_operands_kernel(const __grid_co
             const uint64_t pos = (uint64_t)r * (uint64_t)((is_a ? m.b : 0) + row0 + (wide ? sg : 0)) +
                                  (wide ? (uint64_t)(kb % g.rkb) * 64u : 0u) + (uint64_t)c * run;
             const uint64_t s0 = noise_seed(m.key, g.true_epoch, g.first_pair + (int32_t)pair) | 1ull;
-            seg_state[e] = jump_by(g.pow2, s0, 2ull * pos);
+            seg_state[e] = jump_by(g.jump, s0, 2ull * pos);
         }
     }
     // eight consecutive K values of a row per thread; eight lanes fill a 128-byte row of the image
@@ -458,7 +458,7 @@ int run_update_multi(hses_ctx* ctx, cudaStream_t st, const UpdateMultiItem* item
     uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)c.workspace + 255) & ~(uintptr_t)255);
     UmArgs g{};
     g.n = n;
-    g.pow2 = ctx->t.jump_pow2;
+    g.jump = ctx->t.jump_tabs;
     g.lane4 = ctx->t.jump_lane4;
     g.lane16 = ctx->t.jump_lane16;
     g.cal = ctx->cal();
