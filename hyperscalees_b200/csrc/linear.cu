@@ -372,10 +372,10 @@ size_t hses_perturbed_linear_workspace_bytes(const hses_linear_args* g) {
     // the tensor path always needs room for the split weights, the general path
     // only needs scratch when it perturbs
     if (g->n_groups > 1 || g->x_op != HSES_X_NONE) return tensor_path_supports(*g) ? tensor_path_workspace_bytes(*g) : 0;
-    if (prefers_small_path(*g)) return small_path_workspace_bytes(*g);
+    if (prefers_small_path(*g)) return 0;
     if ((g->algo == HSES_ALGO_AUTO || g->algo == HSES_ALGO_TENSOR) && tensor_path_supports(*g))
         return tensor_path_workspace_bytes(*g);
-    if (g->algo == HSES_ALGO_AUTO && small_path_supports(*g)) return small_path_workspace_bytes(*g);
+    if (g->algo == HSES_ALGO_AUTO && small_path_supports(*g)) return 0;
     if ((g->algo == HSES_ALGO_AUTO || g->algo == HSES_ALGO_PAIR) && pair_path_supports(*g))
         return pair_path_workspace_bytes(*g);
     if (g->algo == HSES_ALGO_AUTO && pack_path_supports(*g)) return pack_path_workspace_bytes(*g);
@@ -441,7 +441,7 @@ int hses_perturbed_linear(hses_ctx* ctx, hses_stream stream, const hses_linear_a
         }
         return run_tensor_path(ctx, as_stream(stream), *g);
     }
-    if (prefers_small_path(*g)) return run_small_path(ctx, as_stream(stream), *g);
+    if (prefers_small_path(*g)) return run_small_path(ctx, as_stream(stream), g, 1, false);
     bool tc_ok = tensor_path_supports(*g);
     if (g->algo == HSES_ALGO_TENSOR && !tc_ok) {
         set_error("hses_perturbed_linear: the tensor-core path does not cover this shape");
@@ -449,7 +449,7 @@ int hses_perturbed_linear(hses_ctx* ctx, hses_stream stream, const hses_linear_a
     }
     if (g->algo == HSES_ALGO_TENSOR || (g->algo == HSES_ALGO_AUTO && tc_ok))
         return run_tensor_path(ctx, as_stream(stream), *g);
-    if (g->algo == HSES_ALGO_AUTO && small_path_supports(*g)) return run_small_path(ctx, as_stream(stream), *g);
+    if (g->algo == HSES_ALGO_AUTO && small_path_supports(*g)) return run_small_path(ctx, as_stream(stream), g, 1, false);
     bool pair_ok = pair_path_supports(*g);
     if (g->algo == HSES_ALGO_PAIR && !pair_ok) {
         set_error("hses_perturbed_linear: the per-pair path does not cover this shape");
@@ -459,6 +459,55 @@ int hses_perturbed_linear(hses_ctx* ctx, hses_stream stream, const hses_linear_a
         return run_pair_path(ctx, as_stream(stream), *g);
     if (g->algo == HSES_ALGO_AUTO && pack_path_supports(*g)) return run_pack_path(ctx, as_stream(stream), *g);
     return run_simt(ctx, as_stream(stream), *g);
+}
+
+// How many of the first layers run in one launch: narrow ones that read the same rows, as many as fit.
+static int joins(const hses_linear_args* args, int32_t n) {
+    int run = 0;
+    while (run < n && prefers_small_path(args[run]) && args[run].out_half == nullptr && small_path_joins(args, run + 1)) ++run;
+    return run;
+}
+
+size_t hses_perturbed_linear_group_workspace_bytes(const hses_linear_args* args, int32_t n, int32_t mean_steps) {
+    if (args == nullptr || n < 1) return 0;
+    size_t most = 0, currents = 0;
+    for (int i = 0; i < n; ++i) {
+        if (joins(args + i, 1)) continue;
+        most = std::max(most, hses_perturbed_linear_workspace_bytes(args + i));
+        currents = std::max(currents, (size_t)args[i].t_steps * args[i].n_pop * args[i].bm * args[i].a * sizeof(float));
+    }
+    return (most + 255) / 256 * 256 + (mean_steps ? currents : 0);
+}
+
+int hses_perturbed_linear_group(hses_ctx* ctx, hses_stream stream, const hses_linear_args* args, int32_t n, int32_t mean_steps) {
+    HSES_REQUIRE(ctx != nullptr && args != nullptr && n >= 1, "NULL pointer or no layers");
+    for (int i = 0; mean_steps && i < n; ++i)
+        HSES_REQUIRE(args[i].lif == 0 && args[i].out_half == nullptr, "the mean over the steps is taken of currents");
+    for (int i = 0; i < n; ++i) {
+        int rc = check_args(args + i);
+        if (rc != HSES_OK) return rc;
+    }
+    const size_t head = hses_perturbed_linear_group_workspace_bytes(args, n, 0);
+    for (int i = 0; i < n; ++i) {
+        if (const int run = joins(args + i, n - i)) {
+            int rc = run_small_path(ctx, as_stream(stream), args + i, run, mean_steps != 0);
+            if (rc != HSES_OK) return rc;
+            i += run - 1;
+            continue;
+        }
+        hses_linear_args g = args[i];
+        if (mean_steps) {
+            HSES_REQUIRE(g.workspace != nullptr && g.workspace_bytes >= hses_perturbed_linear_group_workspace_bytes(args, n, 1),
+                         "workspace too small; see hses_perturbed_linear_group_workspace_bytes");
+            g.out = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(g.workspace) + head);
+            g.out_row_stride = g.a;
+        }
+        int rc = hses_perturbed_linear(ctx, stream, &g);
+        if (rc == HSES_OK && mean_steps)
+            rc = hses_time_mean(ctx, stream, g.out, g.t_steps, g.n_pop * g.bm, g.a, g.a, args[i].out, args[i].out_row_stride);
+        if (rc != HSES_OK) return rc;
+    }
+    return HSES_OK;
 }
 
 }  // extern "C"

@@ -17,11 +17,12 @@ bool pair_path_fuses_scan(const hses_linear_args& g);   // lif == 2 is finished 
 size_t pair_path_workspace_bytes(const hses_linear_args& g);
 int run_pair_path(hses_ctx* ctx, cudaStream_t stream, const hses_linear_args& g);
 
-// Narrow layers (k, a <= 64, rank <= 16; linear_small.cu): persistent CTAs keep W in shared memory and
+// Narrow layers (k, a <= 64, rank <= 16; linear_small.cu): persistent CTAs keep W in registers and
 // walk over pairs.  Taken by HSES_ALGO_AUTO only.
+// Several layers over the same x run in one launch when small_path_joins says so.
 bool small_path_supports(const hses_linear_args& g);
-size_t small_path_workspace_bytes(const hses_linear_args& g);
-int run_small_path(hses_ctx* ctx, cudaStream_t stream, const hses_linear_args& g);
+bool small_path_joins(const hses_linear_args* args, int n);
+int run_small_path(hses_ctx* ctx, cudaStream_t stream, const hses_linear_args* args, int n, bool mean);
 
 // Any other shape on the tensor cores (linear_pack.cu): rows packed per antithetic pair, ragged widths and
 // pitches, ranks up to 128.  Taken by HSES_ALGO_AUTO only.

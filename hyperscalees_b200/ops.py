@@ -259,6 +259,46 @@ def perturbed_linear(x: torch.Tensor, param: torch.Tensor, *, n_pop: int, bm: in
     return (out, pot) if want_potentials else out
 
 
+def perturbed_linear_group(x: torch.Tensor, params: Sequence[torch.Tensor], keys: Sequence[int], *, n_pop: int, bm: int,
+                           t_steps: int = 1, sigma: float, rank: int, epoch: int = 0, first_thread: int = 0,
+                           noise_reuse: int = 0, caches: Optional[Sequence[Optional["FactorCache"]]] = None,
+                           outs: Optional[Sequence[torch.Tensor]] = None, mean_steps: bool = False):
+    """perturbed_linear of several parameters over the same x, with the same results; narrow layers in one launch.
+    mean_steps: the mean over the t_steps of each result, (n_pop*bm, a)."""
+    _check(x, "x")
+    rows, k, xs = _rows_2d(x, "x")
+    if rows != t_steps * n_pop * bm:
+        raise ValueError(f"x has {rows} rows, expected t_steps*n_pop*bm = {t_steps * n_pop * bm}")
+    n = len(params)
+    if mean_steps:
+        rows = n_pop * bm
+    if outs is None:
+        outs = [torch.empty((rows, p.shape[0]), dtype=torch.float32, device=x.device) for p in params]
+    g = (_lib.LinearArgs * n)()
+    for i, (p, key, out) in enumerate(zip(params, keys, outs)):
+        _check(p, "param", ndim=2)
+        _check(out, "out", ndim=2)
+        a, k2 = p.shape
+        if k2 != k or tuple(out.shape) != (rows, a):
+            raise ValueError("param must be (a, k) with k = x's last dim, out (rows, a)")
+        c = g[i]
+        c.x, c.t_steps, c.n_pop, c.bm, c.k, c.x_row_stride = x.data_ptr(), t_steps, n_pop, bm, k, xs
+        c.param, c.a, c.param_row_stride = p.data_ptr(), a, p.stride(0) if a > 1 else max(p.stride(0), k)
+        c.sigma, c.rank, c.key, c.epoch = sigma, rank, key & _U64, epoch
+        c.first_thread, c.noise_reuse, c.perturb = first_thread, noise_reuse, 1
+        c.tau_m, c.v_th, c.out_scale, c.n_groups = 20.0, 0.3, 1.0, 1
+        c.out, c.out_row_stride = out.data_ptr(), out.stride(0) if rows > 1 else max(out.stride(0), a)
+        if caches is not None and caches[i] is not None:
+            c.cache = C.pointer(caches[i].desc)
+    L = _lib.load()
+    need = int(L.hses_perturbed_linear_group_workspace_bytes(g, n, int(mean_steps)))
+    ws = _workspace(x.device, need)
+    for i in range(n if need else 0):
+        g[i].workspace, g[i].workspace_bytes = ws.data_ptr(), need
+    _lib.check(L.hses_perturbed_linear_group(get_context(x.device).handle, current_stream(), g, n, int(mean_steps)))
+    return outs
+
+
 def time_mean(x: torch.Tensor) -> torch.Tensor:
     """x (T, n, h) pitched -> dense (n, h) mean over T."""
     _check(x, "x", ndim=3)

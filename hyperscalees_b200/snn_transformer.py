@@ -114,6 +114,20 @@ class SnnTransformer:
         y = ops.perturbed_linear(x, w, n_pop=n, bm=tokens, t_steps=t_steps, perturb=perturb, out=out, **kw)
         return y
 
+    def nn_group(self, idxs: Sequence[int], x: torch.Tensor, ws: Sequence[torch.Tensor], noise: Optional[TrainNoise],
+                 outs: Optional[Sequence[torch.Tensor]] = None, t_steps: int = 1, mean_steps: bool = False):
+        """nn of several parameters over the same x; mean_steps: the mean over t_steps of each, (n * tokens, out)."""
+        n, tokens = x.shape[-3], x.shape[-2]
+        if noise is None or any(noise.mm_indices is not None and i not in noise.mm_indices for i in idxs):
+            ys = [self.nn(i, x, w, noise, out=None if outs is None else outs[j], t_steps=t_steps)
+                  for j, (i, w) in enumerate(zip(idxs, ws))]
+            return [ops.time_mean(y.view(t_steps, n * tokens, -1)) for y in ys] if mean_steps else ys
+        caches = None if noise.caches is None else [noise.caches.get(i) for i in idxs]
+        return ops.perturbed_linear_group(x, ws, [noise.base_keys[i] for i in idxs], n_pop=n, bm=tokens, t_steps=t_steps,
+                                          sigma=noise.sigma, rank=noise.rank, epoch=noise.epoch,
+                                          first_thread=noise.first_thread, noise_reuse=noise.noise_reuse, caches=caches,
+                                          outs=outs, mean_steps=mean_steps)
+
     def build_caches(self, noise: TrainNoise, n: int) -> dict:
         """The chunk's factors of every MM parameter, generated once (what the reference trainer does
         with `batched_lora_noise` before the forward and the gradient einsum of a chunk,
@@ -134,11 +148,9 @@ class SnnTransformer:
         T, n, in_dim = x.shape
         nt, tin, d = self.num_tokens, self.token_in_dim, self.d_model
         xt = x.reshape(T, n, nt, tin)
-        rates = []
-        for idx, w in ((0, self.in_q), (1, self.in_k), (2, self.in_v)):
-            proj = self.nn(idx, xt, w, noise, t_steps=T)                 # (T*n*nt, d): every step in one launch
-            mean = ops.time_mean(proj.view(T, n * nt, d))                # sum over steps times 1/T
-            rates.append(ops.rate_encode(mean, self.proj_gain))
+        # every step and all three projections in one launch, their means over the steps out
+        means = self.nn_group((0, 1, 2), xt, (self.in_q, self.in_k, self.in_v), noise, t_steps=T, mean_steps=True)
+        rates = [ops.rate_encode(mean, self.proj_gain) for mean in means]
         return ((rates[0] + rates[1] + rates[2]) / 3.0).view(n, nt, d)
 
     # ---- forward_batched, snn_transformer.rs:345-413 ----
@@ -160,13 +172,10 @@ class SnnTransformer:
         for b, blk in enumerate(self.blocks):
             base = self.block_base(b)
             xh = xh.contiguous()
-            for h in range(H):
-                # head h's projections land in columns [h*hd, (h+1)*hd) of the shared buffers,
-                # which is the layout the attention kernel reads and the concat the reference builds
-                sl = slice(h * hd, (h + 1) * hd)
-                self.nn(base + 3 * h, xh, blk["q"][h], noise, out=qb.view(n * nt, d)[:, sl])
-                self.nn(base + 3 * h + 1, xh, blk["k"][h], noise, out=kb.view(n * nt, d)[:, sl])
-                self.nn(base + 3 * h + 2, xh, blk["v"][h], noise, out=vb.view(n * nt, d)[:, sl])
+            # head h's projections land in columns [h*hd, (h+1)*hd) of the shared buffers,
+            # which is the layout the attention kernel reads and the concat the reference builds
+            outs = [buf.view(n * nt, d)[:, h * hd:(h + 1) * hd] for h in range(H) for buf in (qb, kb, vb)]
+            self.nn_group(range(base, base + 3 * H), xh, [blk[c][h] for h in range(H) for c in "qkv"], noise, outs=outs)
             concat = ops.spiking_attention(qb, kb, vb, H, mode=2, tau_m=self.tau_a, g_inh=self.g_inh,
                                            n_iter=self.n_iter, beta_per_seq=beta)
             attn = self.nn(base + 3 * H, concat, blk["o"], noise).view(n, nt, d)

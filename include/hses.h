@@ -260,6 +260,13 @@ typedef struct {
 /* Scratch the call needs for these shapes and this algo (0 is possible). */
 size_t hses_perturbed_linear_workspace_bytes(const hses_linear_args* args);
 int hses_perturbed_linear(hses_ctx* ctx, hses_stream stream, const hses_linear_args* args);
+/* n calls whose outputs do not overlap, with the same results as n calls of hses_perturbed_linear; narrow layers
+ * (k, a <= 64, rank <= 16) that read the same x with the same noise arguments run in one launch.  They may share
+ * one workspace of the size the query gives.  mean_steps: out receives the mean over the t_steps (hses_time_mean of
+ * the call's result), n_pop*bm rows. */
+size_t hses_perturbed_linear_group_workspace_bytes(const hses_linear_args* args /*host, n*/, int32_t n, int32_t mean_steps);
+int hses_perturbed_linear_group(hses_ctx* ctx, hses_stream stream, const hses_linear_args* args /*host, n*/, int32_t n,
+                                int32_t mean_steps);
 
 /* ---- mean firing rate over the time axis, spikes.mean_dim(0) of snn.rs:278:
  *      x (T, n, h) pitched -> out (n, h) with its own pitch. ---------------- */
