@@ -342,6 +342,10 @@ static bool prefers_small_path(const hses_linear_args& g) {
     return (int64_t)2 * g.bm * g.t_steps <= 256;
 }
 
+static bool prefers_rows_path(const hses_linear_args& g) {
+    return g.algo == HSES_ALGO_AUTO && g.out_half == nullptr && !prefers_small_path(g) && rows_path_supports(g);
+}
+
 // does the call end in the per-pair kernel with the scan inside it (the one kernel that writes out_half itself)?
 static bool ends_in_pair_scan(const hses_linear_args& g) {
     if (g.lif != 2) return false;
@@ -371,6 +375,7 @@ size_t hses_perturbed_linear_workspace_bytes(const hses_linear_args* g) {
     }
     // the tensor path always needs room for the split weights, the general path
     // only needs scratch when it perturbs
+    if (prefers_rows_path(*g)) return rows_path_workspace_bytes(*g);
     if (g->n_groups > 1 || g->x_op != HSES_X_NONE) return tensor_path_supports(*g) ? tensor_path_workspace_bytes(*g) : 0;
     if (prefers_small_path(*g)) return 0;
     if ((g->algo == HSES_ALGO_AUTO || g->algo == HSES_ALGO_TENSOR) && tensor_path_supports(*g))
@@ -423,6 +428,7 @@ int hses_perturbed_linear(hses_ctx* ctx, hses_stream stream, const hses_linear_a
         return hses_lif_scan(ctx, stream, g->out, g->t_steps, g->n_pop * g->bm, g->a, g->out_row_stride, nullptr,
                              g->tau_m, g->v_th, g->reset_mode, g->out);
     }
+    if (prefers_rows_path(*g)) return run_rows_path(ctx, as_stream(stream), *g, RowsPost{});
     if (g->x_op != HSES_X_NONE) {
         // an activation on the input: only where the prepass of the tensor-core path can apply it on the fly
         HSES_REQUIRE(g->x_op == HSES_X_RELU_SQUARE, "unknown x_op");

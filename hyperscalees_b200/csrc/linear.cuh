@@ -24,6 +24,17 @@ bool small_path_supports(const hses_linear_args& g);
 bool small_path_joins(const hses_linear_args* args, int n);
 int run_small_path(hses_ctx* ctx, cudaStream_t stream, const hses_linear_args* args, int n, bool mean);
 
+// Layers with many rows per member and weights that fit shared memory (linear_rows.cu).  Taken by HSES_ALGO_AUTO only.
+enum RowsPostKind { ROWS_PLAIN = 0, ROWS_SWISH = 1, ROWS_ADD = 2, ROWS_LIF_RATE = 3 };
+struct RowsPost {          // what follows the layer: nothing, swish, out += y, the firing rate of constant currents
+    int kind, steps;
+    float leak, v_th;
+    int reset;
+};
+bool rows_path_supports(const hses_linear_args& g);
+size_t rows_path_workspace_bytes(const hses_linear_args& g);
+int run_rows_path(hses_ctx* ctx, cudaStream_t stream, const hses_linear_args& g, const RowsPost& post);
+
 // Any other shape on the tensor cores (linear_pack.cu): rows packed per antithetic pair, ragged widths and
 // pitches, ranks up to 128.  Taken by HSES_ALGO_AUTO only.
 bool pack_path_supports(const hses_linear_args& g);

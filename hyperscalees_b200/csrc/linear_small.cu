@@ -18,10 +18,14 @@
 
 #include "common.cuh"
 #include "linear.cuh"
+#include "pack.cuh"
 
 namespace hses {
 
 namespace {
+
+using pack::Parts;
+using pack::split2;
 
 constexpr int SP_ROWS = 32;          // rows staged at a time
 constexpr int SP_MAXK = 64, SP_MAXA = 64, SP_MAXR = 16;
@@ -69,21 +73,6 @@ __device__ __forceinline__ void copy_async(void* dst, const void* src) {
 __device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// two values as three bf16 pairs whose sums are the values (24 bits)
-struct Parts {
-    uint32_t p[3];
-};
-__device__ __forceinline__ Parts split2(float a, float b) {
-    Parts r;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-        r.p[i] = *reinterpret_cast<const uint32_t*>(&h);
-        a -= __uint_as_float(r.p[i] << 16);
-        b -= __uint_as_float(r.p[i] & 0xffff0000u);
-    }
-    return r;
-}
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])

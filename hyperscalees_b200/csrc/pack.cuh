@@ -15,6 +15,22 @@ namespace pack {
 constexpr int PK_EXP_B = 11;       // B * 2^11: |normal| < 6 keeps it below 2^14
 constexpr int PK_SEG = 8192;       // normals of a factor segment, at most
 
+// two values as three bf16 pairs whose sums are the values (24 bits)
+struct Parts {
+    uint32_t p[3];
+};
+__device__ __forceinline__ Parts split2(float a, float b) {
+    Parts r;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+        r.p[i] = *reinterpret_cast<const uint32_t*>(&h);
+        a -= __uint_as_float(r.p[i] << 16);
+        b -= __uint_as_float(r.p[i] & 0xffff0000u);
+    }
+    return r;
+}
+
 // Which row of the call a packed row is.
 struct RowMap {
     int packed;          // 0: row p is row p; 2: p = sample * t_steps + step is row step * n_pop + sample; 1: pairs, see below

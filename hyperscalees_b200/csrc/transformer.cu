@@ -109,7 +109,7 @@ __global__ void lif_rate_kernel(const float* __restrict__ cur, int64_t n, int T_
 __global__ void swish_kernel(const float* __restrict__ x, int64_t n, float* __restrict__ out) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t n4 = n >> 2;
-    auto f = [](float v) { return __fmul_rn(v, __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-v)))); };
+    auto f = [](float v) { return swish_of(v); };
     if (i < n4) {
         const float4 v = reinterpret_cast<const float4*>(x)[i];
         reinterpret_cast<float4*>(out)[i] = make_float4(f(v.x), f(v.y), f(v.z), f(v.w));
