@@ -21,7 +21,8 @@ EXPORTS = [
     "hses_noise_seed", "hses_normal_fill", "hses_lora_factors",
     "hses_dense_noise", "hses_poisson_encode", "hses_poisson_encode_dual", "hses_lif_scan",
     "hses_perturbed_linear_workspace_bytes", "hses_perturbed_linear",
-    "hses_perturbed_linear_group_workspace_bytes", "hses_perturbed_linear_group", "hses_time_mean", "hses_fitness",
+    "hses_perturbed_linear_group_workspace_bytes", "hses_perturbed_linear_group",
+    "hses_perturbed_linear_fuses_post", "hses_perturbed_linear_post", "hses_time_mean", "hses_fitness",
     "hses_peer_window_bytes", "hses_peer_alloc", "hses_peer_open", "hses_peer_close", "hses_peer_free",
     "hses_fitness_publish", "hses_fitness_wait", "hses_fitness_exchange",
     "hses_member_mean", "hses_convert_fitnesses", "hses_es_update_workspace_bytes",
@@ -136,6 +137,8 @@ def load():
     L.hses_perturbed_linear_workspace_bytes.restype = sz
     L.hses_perturbed_linear_workspace_bytes.argtypes = [C.POINTER(LinearArgs)]
     L.hses_perturbed_linear.argtypes = [vp, vp, C.POINTER(LinearArgs)]
+    L.hses_perturbed_linear_fuses_post.argtypes = [C.POINTER(LinearArgs)]
+    L.hses_perturbed_linear_post.argtypes = [vp, vp, C.POINTER(LinearArgs), i32, i32]
     L.hses_perturbed_linear_group_workspace_bytes.restype = sz
     L.hses_perturbed_linear_group_workspace_bytes.argtypes = [C.POINTER(LinearArgs), i32, i32]
     L.hses_perturbed_linear_group.argtypes = [vp, vp, C.POINTER(LinearArgs), i32, i32]

@@ -235,7 +235,7 @@ __device__ __forceinline__ float sample_fitness(const float* row, int classes, i
 #endif
 #if defined(__CUDACC__)
 // x * sigmoid(x)
-__device__ __forceinline__ float swish_of(float v) { return __fmul_rn(v, __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-v)))); }
+__device__ __forceinline__ float swish_of(float v) { return __fmul_rn(v, __frcp_rn(__fadd_rn(1.0f, expf(-v)))); }
 #endif
 // lif_step (hyperscalees-models/src/snn.rs:53-65): charge, threshold, reset; returns the spike
 __device__ __forceinline__ float lif_update(float& v, float cur, float leak, float v_th, int reset) {
@@ -245,12 +245,6 @@ __device__ __forceinline__ float lif_update(float& v, float cur, float leak, flo
     float s = c >= v_th ? 1.0f : 0.0f;
     v = reset == HSES_RESET_HARD ? __fmul_rn(c, __fadd_rn(-s, 1.0f)) : __fsub_rn(c, __fmul_rn(s, v_th));
     return s;
-}
-// firing rate of a neuron under a constant current
-__device__ __forceinline__ float lif_rate_of(float current, int steps, float leak, float v_th, int reset) {
-    float v = 0.0f, s = 0.0f;
-    for (int t = 0; t < steps; ++t) s = __fadd_rn(s, lif_update(v, current, leak, v_th, reset));
-    return __fdiv_rn(s, (float)steps);
 }
 
 

@@ -467,6 +467,26 @@ int hses_perturbed_linear(hses_ctx* ctx, hses_stream stream, const hses_linear_a
     return run_simt(ctx, as_stream(stream), *g);
 }
 
+int hses_perturbed_linear_fuses_post(const hses_linear_args* g) {
+    return g != nullptr && check_args(g) == HSES_OK && prefers_rows_path(*g) ? 1 : 0;
+}
+
+int hses_perturbed_linear_post(hses_ctx* ctx, hses_stream stream, const hses_linear_args* g, int32_t post, int32_t steps) {
+    HSES_REQUIRE(ctx != nullptr, "ctx is NULL");
+    int rc = check_args(g);
+    if (rc != HSES_OK) return rc;
+    HSES_REQUIRE(post >= HSES_POST_SWISH && post <= HSES_POST_LIF_RATE, "unknown post");
+    HSES_REQUIRE(post != HSES_POST_LIF_RATE || (steps >= 1 && g->tau_m != 0.0f &&
+                                                (g->reset_mode == HSES_RESET_HARD || g->reset_mode == HSES_RESET_SUBTRACT)),
+                 "bad firing-rate arguments");
+    if (!prefers_rows_path(*g)) {
+        set_error("hses_perturbed_linear_post: the call does not take the path that fuses it");
+        return HSES_ERR_UNSUPPORTED;
+    }
+    const float leak = post == HSES_POST_LIF_RATE ? 1.0f / g->tau_m : 0.0f;
+    return run_rows_path(ctx, as_stream(stream), *g, RowsPost{post, steps, leak, g->v_th, g->reset_mode});
+}
+
 // How many of the first layers run in one launch: narrow ones that read the same rows, as many as fit.
 static int joins(const hses_linear_args* args, int32_t n) {
     int run = 0;

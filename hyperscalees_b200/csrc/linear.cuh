@@ -25,7 +25,6 @@ bool small_path_joins(const hses_linear_args* args, int n);
 int run_small_path(hses_ctx* ctx, cudaStream_t stream, const hses_linear_args* args, int n, bool mean);
 
 // Layers with many rows per member and weights that fit shared memory (linear_rows.cu).  Taken by HSES_ALGO_AUTO only.
-enum RowsPostKind { ROWS_PLAIN = 0, ROWS_SWISH = 1, ROWS_ADD = 2, ROWS_LIF_RATE = 3 };
 struct RowsPost {          // what follows the layer: nothing, swish, out += y, the firing rate of constant currents
     int kind, steps;
     float leak, v_th;

@@ -37,9 +37,10 @@ struct RowsFactors {
     NoiseCal cal;
     uint64_t key;
     int32_t true_epoch, first_pair;
-    int r, r16, k, kb, a, groups, order;     // kb: 64-wide blocks of k; order 1: A's rows come first in the stream
+    int r, rg, k, kb, a, groups, order;      // rg: a group's share of t's columns; kb: 64-wide blocks of k; order 1: A's rows
+                                             // come first in the stream
     float base_sigma;
-    uint8_t *bimg, *aimg;                    // per pair: (kb, part, groups * r16 rows, 128 B); (group, part, r16 / 8, a / G, 8)
+    uint8_t *bimg, *aimg;                    // per pair: (kb, part, groups * rg rows, 128 B); (slab, part, 2, outputs of a slab, 8)
     size_t b_bytes, a_bytes;
 };
 
@@ -89,8 +90,8 @@ __global__ void __launch_bounds__(256) rows_factors_kernel(const __grid_constant
         chain_wait();
     }
     __syncthreads();
-    for (int e = tid; e < f.kb * f.r16 * 8; e += 256) {       // eight k of one rank value
-        const int q = (e >> 3) % f.r16, blk = (e >> 3) / f.r16, c = e & 7, row = gi * f.r16 + q;
+    for (int e = tid; e < f.kb * f.rg * 8; e += 256) {        // eight k of one rank value
+        const int q = (e >> 3) % f.rg, blk = (e >> 3) / f.rg, c = e & 7, row = gi * f.rg + q;
         uint32_t v[3][4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -101,15 +102,17 @@ __global__ void __launch_bounds__(256) rows_factors_kernel(const __grid_constant
         }
 #pragma unroll
         for (int part = 0; part < 3; ++part)
-            *reinterpret_cast<uint4*>(f.bimg + p * f.b_bytes + ((size_t)(blk * 3 + part) * G * f.r16 + row) * 128 +
+            *reinterpret_cast<uint4*>(f.bimg + p * f.b_bytes + ((size_t)(blk * 3 + part) * G * f.rg + row) * 128 +
                                       ((c ^ (row & 7)) << 4)) = make_uint4(v[part][0], v[part][1], v[part][2], v[part][3]);
     }
-    for (int e = tid; e < ag * (f.r16 >> 3); e += 256) {      // eight rank values of one output
-        const int n = e % ag, g8 = e / ag;
+    // s·A: slabs of 16 of t's columns; with rank <= 8 two groups share a slab, each with zeros in the other's half
+    const int gs = 16 / f.rg, slab = gi / gs, own = gi % gs, sn = gs * ag;
+    for (int e = tid; e < ag * 2; e += 256) {                 // eight rank values of one output
+        const int n = e % ag, g8 = e / ag, q0 = gs == 2 ? (g8 == own ? 0 : r) : g8 * 8;
         uint32_t v[3][4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int q = g8 * 8 + 2 * j;
+            const int q = q0 + 2 * j;
             const Parts s = split2(q < r ? __fmul_rn(A[n * r + q], f.base_sigma) : 0.0f,
                                    q + 1 < r ? __fmul_rn(A[n * r + q + 1], f.base_sigma) : 0.0f);
 #pragma unroll
@@ -117,8 +120,7 @@ __global__ void __launch_bounds__(256) rows_factors_kernel(const __grid_constant
         }
 #pragma unroll
         for (int part = 0; part < 3; ++part)
-            *reinterpret_cast<uint4*>(f.aimg + p * f.a_bytes +
-                                      (((size_t)(gi * 3 + part) * (f.r16 >> 3) + g8) * ag + n) * 16) =
+            *reinterpret_cast<uint4*>(f.aimg + p * f.a_bytes + (((size_t)(slab * 3 + part) * 2 + g8) * sn + own * ag + n) * 16) =
                 make_uint4(v[part][0], v[part][1], v[part][2], v[part][3]);
     }
 }
@@ -126,7 +128,8 @@ __global__ void __launch_bounds__(256) rows_factors_kernel(const __grid_constant
 struct RowsArgs {
     const float* x;
     int64_t x_stride;
-    int k, kb, a, groups, r16, nt;           // nt: groups * r16
+    int k, kb, a, slabs, nt;                 // nt: columns of t, 16 per slab
+    int merged;                              // B lies behind W's rows: one product gives y and t
     int64_t n_pop, pairs;
     int t_steps, bm;
     int tps;                                 // tiles per pair and step
@@ -178,18 +181,36 @@ struct Turn {
         }
     }
 };
+// hses_lif_rate of 16 currents: the steps outside, so that 16 chains run side by side; the division by a power of two is a
+// product with the same result
+template <bool HARD>
+__device__ __forceinline__ void lif_rates(float (&v)[2][8], const RowsPost& post) {
+    float m[16], s[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) m[j] = s[j] = 0.0f;
+    for (int t = 0; t < post.steps; ++t)
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            s[j] = __fadd_rn(s[j], lif_update(m[j], v[j >> 3][j & 7], post.leak, post.v_th, HARD ? HSES_RESET_HARD : HSES_RESET_SUBTRACT));
+    const float n = (float)post.steps, inv = 1.0f / n;
+    const bool pow2 = (post.steps & (post.steps - 1)) == 0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j >> 3][j & 7] = pow2 ? __fmul_rn(s[j], inv) : __fdiv_rn(s[j], n);
+}
 __device__ __forceinline__ void store8f(float* p, const float (&v)[8]) {
     asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]),
                  "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
                  : "memory");
 }
 
+template <int POST>
 __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_kernel(const __grid_constant__ RowsArgs g) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* wsm = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t* xsm = wsm + g.w_bytes;                           // [buf][part 3][128 rows][128 B]
-    uint8_t* bsm = xsm + (size_t)g.xbufs * 3 * LR_PART;       // [buf] B's image
-    uint8_t* asm_ = bsm + (size_t)g.fbufs * g.b_bytes;        // [buf] A's image
+    const uint32_t w_tile = (uint32_t)(g.a + (g.merged ? g.nt : 0)) * 128;   // of one block of k and part
+    uint8_t* xsm = wsm + g.kb * 3 * w_tile;                   // [buf][part 3][128 rows][128 B]
+    uint8_t* bsm = xsm + (size_t)g.xbufs * 3 * LR_PART;       // [buf] B's image, unless merged
+    uint8_t* asm_ = bsm + (g.merged ? 0 : (size_t)g.fbufs * g.b_bytes);      // [buf] A's image
     uint8_t* tsm = asm_ + (size_t)g.fbufs * g.a_bytes;        // t: [part 3][nt / 8][128][8] bf16
     const int t_part = g.nt * LR_TILE * 2;
     __shared__ uint64_t wfull, xfull[2], xempty[2], ffull[2], fempty[2], tfull[2], tempty[2], tacc, tready;
@@ -230,7 +251,8 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_kernel(const __grid
     if (warp == 1) {
         if (lane == 0) {
             mbar_expect_tx(&wfull, g.w_bytes);
-            for (uint32_t o = 0; o < g.w_bytes; o += 16384) bulk_load(wsm + o, g.wimg + o, min(16384u, g.w_bytes - o), &wfull);
+            for (int i = 0; i < g.kb * 3; ++i)
+                bulk_load(wsm + (size_t)i * w_tile, g.wimg + (size_t)i * g.a * 128, (uint32_t)g.a * 128, &wfull);
             Walk w = start;
             Turn f{0, 0};
             bool ok = true, fresh = true;
@@ -239,7 +261,12 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_kernel(const __grid
                     ok = mbar_wait(&fempty[f.b], f.ph ^ 1, abort_flag, g.status, 1);
                     if (!ok) break;
                     mbar_expect_tx(&ffull[f.b], g.b_bytes + g.a_bytes);
-                    bulk_load(bsm + (size_t)f.b * g.b_bytes, g.bimg + (size_t)w.pair * g.b_bytes, g.b_bytes, &ffull[f.b]);
+                    const uint8_t* src = g.bimg + (size_t)w.pair * g.b_bytes;
+                    if (g.merged)
+                        for (int j = 0; j < g.kb * 3; ++j)
+                            bulk_load(wsm + (size_t)j * w_tile + g.a * 128, src + (size_t)j * g.nt * 128, (uint32_t)g.nt * 128, &ffull[f.b]);
+                    else
+                        bulk_load(bsm + (size_t)f.b * g.b_bytes, src, g.b_bytes, &ffull[f.b]);
                     bulk_load(asm_ + (size_t)f.b * g.a_bytes, g.aimg + (size_t)w.pair * g.a_bytes, g.a_bytes, &ffull[f.b]);
                     f.next(g.fbufs);
                 }
@@ -254,12 +281,12 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_kernel(const __grid
                 }
         }
     } else if (warp == 0) {
-        const uint32_t idesc = make_idesc_bf16(g.a), idesc_t = make_idesc_bf16(g.nt), idesc_u = make_idesc_bf16(g.a / g.groups);
+        const int sn = g.a / g.slabs;                         // outputs of a slab
+        const uint32_t idesc = make_idesc_bf16(g.a + (g.merged ? g.nt : 0)), idesc_t = make_idesc_bf16(g.nt), idesc_u = make_idesc_bf16(sn);
         const uint64_t dx0 = make_smem_desc(xsm), dw0 = make_smem_desc(wsm), db0 = make_smem_desc(bsm);
-        const uint64_t dt0 = make_plain_desc(tsm, LR_TILE * 16), da0 = make_plain_desc(asm_, g.a / g.groups * 16);
-        const uint32_t w_part = (uint32_t)g.a * 128 >> 4, b_part = (uint32_t)g.nt * 128 >> 4, x_part = LR_PART >> 4;
-        const int ag = g.a / g.groups;
-        const uint32_t a_part = (uint32_t)(g.r16 * ag * 2) >> 4, a_group = 3 * a_part;
+        const uint64_t dt0 = make_plain_desc(tsm, LR_TILE * 16), da0 = make_plain_desc(asm_, sn * 16);
+        const uint32_t w_part = w_tile >> 4, b_part = (uint32_t)g.nt * 128 >> 4, x_part = LR_PART >> 4;
+        const uint32_t a_part = (uint32_t)(16 * sn * 2) >> 4, a_slab = 3 * a_part;
         bool ok = __all_sync(0xffffffffu, mbar_wait(&wfull, 0, abort_flag, g.status, 2));
         Walk w = start;
         Turn x{0, 0}, f{0, 0}, acc{0, 0};
@@ -286,12 +313,14 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_kernel(const __grid
                 for (int ks = 0; ks < ksteps; ++ks) {         // 16 values = 32 bytes along k; smallest terms first
                     const uint64_t xd = dx + 2 * ks, wd = dw + 2 * ks, bb = dbk + 2 * ks;
                     const uint32_t more = (kb | ks) != 0;
-                    umma_f16_warp(du, xd + 2 * x_part, bb, idesc_t, more);
-                    umma_f16_warp(du, xd, bb + 2 * b_part, idesc_t, 1);
-                    umma_f16_warp(du, xd + x_part, bb + b_part, idesc_t, 1);
-                    umma_f16_warp(du, xd + x_part, bb, idesc_t, 1);
-                    umma_f16_warp(du, xd, bb + b_part, idesc_t, 1);
-                    umma_f16_warp(du, xd, bb, idesc_t, 1);
+                    if (!g.merged) {
+                        umma_f16_warp(du, xd + 2 * x_part, bb, idesc_t, more);
+                        umma_f16_warp(du, xd, bb + 2 * b_part, idesc_t, 1);
+                        umma_f16_warp(du, xd + x_part, bb + b_part, idesc_t, 1);
+                        umma_f16_warp(du, xd + x_part, bb, idesc_t, 1);
+                        umma_f16_warp(du, xd, bb + b_part, idesc_t, 1);
+                        umma_f16_warp(du, xd, bb, idesc_t, 1);
+                    }
                     umma_f16_warp(d, xd + 2 * x_part, wd, idesc, more);
                     umma_f16_warp(d, xd, wd + 2 * w_part, idesc, 1);
                     umma_f16_warp(d, xd + x_part, wd + w_part, idesc, 1);
@@ -307,9 +336,9 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_kernel(const __grid
             if (!ok) break;
             tc_fence_after();
             const uint32_t t1 = (uint32_t)t_part >> 4;
-            for (int gi = 0; gi < g.groups; ++gi) {
-                const uint64_t t = dt0 + (uint64_t)(gi * (g.r16 >> 3) * 128), a = da + (uint64_t)(gi * a_group);
-                const uint32_t u = du + (uint32_t)(gi * ag);
+            for (int sl = 0; sl < g.slabs; ++sl) {
+                const uint64_t t = dt0 + (uint64_t)(sl * 2 * 128), a = da + (uint64_t)(sl * a_slab);
+                const uint32_t u = du + (uint32_t)(sl * sn);
                 umma_f16_warp(u, t + 2 * t1, a, idesc_u, 0);
                 umma_f16_warp(u, t, a + 2 * a_part, idesc_u, 1);
                 umma_f16_warp(u, t + t1, a + a_part, idesc_u, 1);
@@ -376,7 +405,7 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_kernel(const __grid
     } else if (warp < 14) {
         // ---------------------------------------------------------------- t to operand layout
         const int q4 = warp & 3, gt = q4 * 32 + lane;         // TMEM quadrant, row of the tile
-        const uint32_t lane_base = tmem + ((uint32_t)(q4 * 32) << 16) + 256;
+        const uint32_t lane_base = tmem + ((uint32_t)(q4 * 32) << 16) + (g.merged ? g.a : 256);
         Walk w = start;
         Turn acc{0, 0};
         for (int i = 0; i < count; ++i, w.next(g), acc.next(g.tbufs)) {
@@ -411,10 +440,21 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_kernel(const __grid
         Turn acc{0, 0};
         for (int i = 0; i < count; ++i, w.next(g), acc.next(g.tbufs)) {
             const int b = acc.b, cnt = w.rows(g);
-            const int64_t row0 = w.row0(g);
+            float* orow = g.out + (size_t)(w.row0(g) + gt) * g.out_stride;
+            // the residual's values of a block of columns are asked for one block ahead
+            float4 old[4];
+            const bool add = POST == HSES_POST_ADD && gt < cnt;
+            auto fetch = [&](int cb) {
+                if (!add || cb >= g.a) return;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float* o = orow + cb + 4 * j;
+                    old[j] = g.wide_out ? *reinterpret_cast<const float4*>(o) : make_float4(o[0], o[1], o[2], o[3]);
+                }
+            };
+            fetch(eh * 16);
             if (!__all_sync(0xffffffffu, mbar_wait(&tfull[b], acc.ph, abort_flag, g.status, 9))) break;
             tc_fence_after();
-            float* orow = g.out + (size_t)(row0 + gt) * g.out_stride;
             for (int cb = eh * 16; cb < g.a; cb += 32) {
                 uint32_t y[2][8], u[2][8];
 #pragma unroll
@@ -423,29 +463,37 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_kernel(const __grid
                     tmem_ld8_issue(lane_base + b * 128 + 256 + cb + 8 * h, u[h]);
                 }
                 tmem_ld_wait();
+                float v[2][8];
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        v[h][j] = __fmul_rn(__fadd_rn(__uint_as_float(y[h][j]), __uint_as_float(u[h][j])), gain);
+                if (POST == HSES_POST_SWISH) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j >> 3][j & 7] = swish_of(v[j >> 3][j & 7]);
+                } else if (POST == HSES_POST_LIF_RATE) {
+                    if (g.post.reset == HSES_RESET_HARD) lif_rates<true>(v, g.post);
+                    else lif_rates<false>(v, g.post);
+                }
+                if (add) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        float* p = &v[j >> 1][(j & 1) * 4];
+                        p[0] = __fadd_rn(old[j].x, p[0]), p[1] = __fadd_rn(old[j].y, p[1]);
+                        p[2] = __fadd_rn(old[j].z, p[2]), p[3] = __fadd_rn(old[j].w, p[3]);
+                    }
+                    fetch(cb + 32);
+                }
                 if (gt < cnt) {
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        float v[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            v[j] = __fmul_rn(__fadd_rn(__uint_as_float(y[h][j]), __uint_as_float(u[h][j])), gain);
-                        if (g.post.kind == ROWS_ADD) {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) v[j] = __fadd_rn(orow[cb + 8 * h + j], v[j]);
-                        } else if (g.post.kind == ROWS_SWISH) {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) v[j] = swish_of(v[j]);
-                        } else if (g.post.kind == ROWS_LIF_RATE) {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                v[j] = lif_rate_of(v[j], g.post.steps, g.post.leak, g.post.v_th, g.post.reset);
-                        }
+                        float* o = orow + cb + 8 * h;
                         if (g.wide_out) {
-                            store8f(orow + cb + 8 * h, v);
+                            store8f(o, v[h]);
                         } else {
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) orow[cb + 8 * h + j] = v[j];
+                            for (int j = 0; j < 8; ++j) o[j] = v[h][j];
                         }
                     }
                 }
@@ -464,7 +512,7 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_kernel(const __grid
 
 struct RowsPlan {
     bool ok;
-    int kb, r16, xbufs, fbufs, smem;
+    int kb, rg, nt, merged, xbufs, fbufs, tbufs, smem;
     int64_t pairs;
     uint32_t w_bytes, b_bytes, a_bytes;
     size_t o_b, o_a, bytes;
@@ -484,16 +532,21 @@ RowsPlan plan_rows(const hses_linear_args& g) {
     if (tiles < plan_sm_count()) return p;
     p.pairs = g.n_pop / 2;
     p.kb = (g.k + 63) / 64;
-    p.r16 = 16;
-    const int nt = G * p.r16;
+    p.rg = G % 2 == 0 && g.rank <= 8 ? 8 : 16;
+    const int nt = p.nt = G * p.rg;
+    // With a few tiles per pair B may wait for the pair before: it lies behind W and one product makes y and t (a product of
+    // 16 columns costs the tensor core about what one of 64 does)
+    p.merged = g.a + nt <= 256 && tiles / p.pairs >= 4;
+    p.tbufs = g.a + (p.merged ? nt : 0) <= 128 ? 2 : 1;
     p.w_bytes = (uint32_t)p.kb * 3 * g.a * 128;
     p.b_bytes = (uint32_t)p.kb * 3 * nt * 128;
-    p.a_bytes = (uint32_t)3 * p.r16 * g.a * 2;
+    p.a_bytes = (uint32_t)3 * 16 * g.a * 2;
     const int fixed = 1024 + (int)p.w_bytes + 3 * nt * 256;
     for (int bufs = 3; bufs >= 0; --bufs) {       // x's parts, then the factors in two buffers, where they fit
         p.xbufs = bufs & 2 ? 2 : 1;
         p.fbufs = bufs & 1 ? 2 : 1;
-        p.smem = fixed + p.xbufs * 3 * LR_PART + p.fbufs * (int)(p.b_bytes + p.a_bytes);
+        if (p.merged) p.fbufs = 1;
+        p.smem = fixed + p.xbufs * 3 * LR_PART + (int)p.b_bytes * p.fbufs + (int)p.a_bytes * p.fbufs;
         if (p.smem <= LR_SMEM - 1024) break;
         if (bufs == 0) return p;
     }
@@ -532,7 +585,7 @@ int run_rows_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g, con
     f.true_epoch = true_epoch_of(g.epoch, g.noise_reuse);
     f.first_pair = g.first_thread / 2;
     f.r = g.rank;
-    f.r16 = p.r16;
+    f.rg = p.rg;
     f.k = g.k;
     f.kb = p.kb;
     f.a = g.a;
@@ -563,9 +616,9 @@ int run_rows_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g, con
     a.k = g.k;
     a.kb = p.kb;
     a.a = g.a;
-    a.groups = G;
-    a.r16 = p.r16;
-    a.nt = G * p.r16;
+    a.nt = p.nt;
+    a.slabs = p.nt / 16;
+    a.merged = p.merged;
     a.n_pop = g.n_pop;
     a.pairs = p.pairs;
     a.t_steps = g.t_steps;
@@ -580,7 +633,7 @@ int run_rows_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g, con
     a.a_bytes = p.a_bytes;
     a.xbufs = p.xbufs;
     a.fbufs = p.fbufs;
-    a.tbufs = g.a <= 128 ? 2 : 1;
+    a.tbufs = p.tbufs;
     a.out = g.out;
     a.out_stride = g.out_row_stride;
     a.wide_out = ((uintptr_t)g.out & 31u) == 0 && g.out_row_stride % 8 == 0;
@@ -588,9 +641,12 @@ int run_rows_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g, con
     a.out_scale_ptr = g.out_scale_ptr;
     a.post = post;
     a.status = ctx->t.status_word;
-    HSES_CUDA(cudaFuncSetAttribute(linear_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem));
+    auto kernel = post.kind == HSES_POST_SWISH ? linear_rows_kernel<HSES_POST_SWISH>
+                  : post.kind == HSES_POST_ADD ? linear_rows_kernel<HSES_POST_ADD>
+                  : post.kind == HSES_POST_LIF_RATE ? linear_rows_kernel<HSES_POST_LIF_RATE> : linear_rows_kernel<0>;
+    HSES_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem));
     HSES_KERNEL(ctx, st, "linear_rows");
-    chain_launch(linear_rows_kernel, (unsigned)std::min<int64_t>(a.tiles, ctx->sm_count), LR_THREADS, p.smem, st, a);
+    chain_launch(kernel, (unsigned)std::min<int64_t>(a.tiles, ctx->sm_count), LR_THREADS, p.smem, st, a);
     HSES_LAUNCH_CHECK();
     return HSES_OK;
 }

@@ -190,7 +190,7 @@ def perturbed_linear(x: torch.Tensor, param: torch.Tensor, *, n_pop: int, bm: in
                      algo: int = ALGO_AUTO, cache: Optional["FactorCache"] = None, precision: int = 0,
                      tmm: bool = False, x_half: Optional[torch.Tensor] = None,
                      out_half: Optional[torch.Tensor] = None, reuse_x_split: bool = False, n_groups: int = 1,
-                     x_relu_square: bool = False):
+                     x_relu_square: bool = False, post: Optional[str] = None, post_steps: int = 0):
     """do_mm over a population (+ optional LIF step).  x: (..., k) with
     t_steps*n_pop*bm rows; param: (a, k).  Returns out (rows, a) and, if asked,
     the charged potentials.  With `cache` the factors are read from it instead of
@@ -200,8 +200,13 @@ def perturbed_linear(x: torch.Tensor, param: torch.Tensor, *, n_pop: int, bm: in
     calls that path does not take this way, by one pass of its own before the call.
     n_groups: `param` stacks that many parameters of equal shape along its rows, each with its own noise;
     `cache` must then be a GroupedFactorCache over them and `key` its key (tensor-core path only).
+    post: what follows the layer, in the same pass where the path allows it: "swish"; "add": out += y (out must be
+    given); "lif_rate": the firing rate of post_steps LIF steps (tau_m, v_th, reset_mode) under the current y.
     reuse_x_split: the previous call on this device and stream had the same x and the same shapes
     (another projection of the same activation): its operand split of x is taken as it stands."""
+    if post is not None and (post not in ("swish", "add", "lif_rate") or lif or want_potentials or
+                             (post == "add" and out is None)):
+        raise ValueError("post is swish, add (with out) or lif_rate, of a layer's currents")
     _check(x, "x")
     _check(param, "param", ndim=2)
     rows, k, xs = _rows_2d(x, "x")
@@ -255,8 +260,23 @@ def perturbed_linear(x: torch.Tensor, param: torch.Tensor, *, n_pop: int, bm: in
     g.workspace = ws.data_ptr() if ws is not None else None
     g.workspace_bytes = need
     ctx = get_context(x.device)
+    if post is not None and not L.hses_perturbed_linear_fuses_post(C.byref(g)):
+        y = out
+        if post == "add":   # the layer needs an output of its own
+            y = torch.empty((rows, a), dtype=torch.float32, device=x.device)
+            g.out, g.out_row_stride = y.data_ptr(), a
+        _lib.check(L.hses_perturbed_linear(ctx.handle, current_stream(), C.byref(g)))
+        if post == "add":
+            return add_inplace(out, y)
+        return swish(y, out=y) if post == "swish" else lif_rate(y, post_steps, tau_m, v_th, reset_mode, out=y)
+    if post is not None:
+        _lib.check(L.hses_perturbed_linear_post(ctx.handle, current_stream(), C.byref(g), _POSTS[post], post_steps))
+        return out
     _lib.check(L.hses_perturbed_linear(ctx.handle, current_stream(), C.byref(g)))
     return (out, pot) if want_potentials else out
+
+
+_POSTS = {"swish": 1, "add": 2, "lif_rate": 3}
 
 
 def perturbed_linear_group(x: torch.Tensor, params: Sequence[torch.Tensor], keys: Sequence[int], *, n_pop: int, bm: int,

@@ -96,7 +96,8 @@ class SpikingLM:
         return 2 + len(self.blocks) * (3 * self.num_heads + 3)
 
     def nn(self, idx: int, x: torch.Tensor, w: torch.Tensor, n: int, rows_per_member: int,
-           noise: Optional[LmNoise], out: Optional[torch.Tensor] = None, same_x: bool = False) -> torch.Tensor:
+           noise: Optional[LmNoise], out: Optional[torch.Tensor] = None, same_x: bool = False,
+           post: Optional[str] = None) -> torch.Tensor:
         """same_x: the call right before this one projected the same x with a matrix of the same shape (the
         per-head Q/K/V of a block): the tensor-core path keeps that call's fp16 operand split of x."""
         kw = {}
@@ -111,18 +112,19 @@ class SpikingLM:
                 kw["cache"] = ops.FactorCache(noise.base_keys[idx], noise.epoch, noise.noise_reuse, noise.rank, a, k,
                                               n // 2, first_pair=noise.first_thread // 2, device=self.device)
         return ops.perturbed_linear(x, w, n_pop=n, bm=rows_per_member, perturb=noise is not None, out=out,
-                                    reuse_x_split=same_x, **kw)
+                                    reuse_x_split=same_x, post=post, **kw)
 
     def nn_heads(self, idxs, x: torch.Tensor, ws, n: int, rows_per_member: int, noise: Optional[LmNoise],
                  out: torch.Tensor, same_x: bool) -> bool:
         """The per-head projections `ws` (parameters idxs) of one x in ONE call: the heads' matrices stacked
         along the rows, every head with its own noise, columns [h*hd, (h+1)*hd) of `out` for head h.  x is
-        read once instead of once per head.  Returns False when the shapes do not allow it (the caller then
+        read once instead of once per head; `out` receives the firing rates of the currents.  Returns False when the shapes do not allow it (the caller then
         projects head by head)."""
         hd = ws[0].shape[0]
+        rate = dict(post="lif_rate", post_steps=self.T, tau_m=self.tau_m, v_th=self.v_th)
         if noise is None:
             ops.perturbed_linear(x, torch.cat(list(ws), 0), n_pop=n, bm=rows_per_member, perturb=False, out=out,
-                                 reuse_x_split=same_x)
+                                 reuse_x_split=same_x, **rate)
             return True
         groupable = (noise.first_thread % 2 == 0 and n % 2 == 0 and noise.rank in (1, 2, 3, 4, 8, 16) and
                      (hd % 32 == 0 or (hd % 16 == 0 and noise.rank >= 8)))
@@ -135,7 +137,7 @@ class SpikingLM:
         ops.perturbed_linear(x, torch.cat(list(ws), 0), n_pop=n, bm=rows_per_member, sigma=noise.sigma,
                              rank=noise.rank, key=grouped.key, epoch=noise.epoch, first_thread=noise.first_thread,
                              noise_reuse=noise.noise_reuse, cache=grouped, n_groups=len(ws), out=out,
-                             reuse_x_split=same_x)
+                             reuse_x_split=same_x, **rate)
         return True
 
     def forward_population(self, ids: torch.Tensor, noise: Optional[LmNoise] = None) -> torch.Tensor:
@@ -173,15 +175,14 @@ class SpikingLM:
                     self.nn(base + 3 * h, x, blk["q"][h], n, rpm, noise, out=qc[:, sl], same_x=h > 0)
                     self.nn(base + 3 * h + 1, x, blk["k"][h], n, rpm, noise, out=kc[:, sl], same_x=True)
                     self.nn(base + 3 * h + 2, x, blk["v"][h], n, rpm, noise, out=vc[:, sl], same_x=True)
-            # LIF over T steps on the constant currents, firing rates in place
-            for buf in (qc, kc, vc):
-                ops.lif_rate(buf, self.T, self.tau_m, self.v_th, out=buf)
+                # LIF over T steps on the constant currents, firing rates in place
+                for buf in (qc, kc, vc):
+                    ops.lif_rate(buf, self.T, self.tau_m, self.v_th, out=buf)
             attn = ops.spiking_attention(qc.view(n * seqs, L, d), kc.view(n * seqs, L, d), vc.view(n * seqs, L, d), H,
                                          mode=3, beta_per_seq=beta)
-            ops.add_inplace(x, self.nn(base + 3 * H, attn.view(rows, d), blk["o"], n, rpm, noise))
-            ff1 = self.nn(base + 3 * H + 1, x, blk["ff1"], n, rpm, noise)
-            ops.swish(ff1, out=ff1)
-            ops.add_inplace(x, self.nn(base + 3 * H + 2, ff1, blk["ff2"], n, rpm, noise))
+            self.nn(base + 3 * H, attn.view(rows, d), blk["o"], n, rpm, noise, out=x, post="add")
+            ff1 = self.nn(base + 3 * H + 1, x, blk["ff1"], n, rpm, noise, post="swish")
+            self.nn(base + 3 * H + 2, ff1, blk["ff2"], n, rpm, noise, out=x, post="add")
             del attn, ff1
         return self.nn(self.out_param_index(), x, self.out, n, rpm, noise)
 

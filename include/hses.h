@@ -260,6 +260,13 @@ typedef struct {
 /* Scratch the call needs for these shapes and this algo (0 is possible). */
 size_t hses_perturbed_linear_workspace_bytes(const hses_linear_args* args);
 int hses_perturbed_linear(hses_ctx* ctx, hses_stream stream, const hses_linear_args* args);
+/* hses_perturbed_linear and what follows it in one pass: swish y * sigmoid(y), the residual out += y, or the firing rate
+ * of `steps` LIF steps (tau_m, v_th and reset_mode of args) under the constant current y (hses_lif_rate).  For calls that
+ * hses_perturbed_linear_fuses_post answers 1 for (many rows per member, weights within shared memory); others return
+ * HSES_ERR_UNSUPPORTED and take the separate entry points. */
+enum { HSES_POST_SWISH = 1, HSES_POST_ADD = 2, HSES_POST_LIF_RATE = 3 };
+int hses_perturbed_linear_fuses_post(const hses_linear_args* args);
+int hses_perturbed_linear_post(hses_ctx* ctx, hses_stream stream, const hses_linear_args* args, int32_t post, int32_t steps);
 /* n calls whose outputs do not overlap, with the same results as n calls of hses_perturbed_linear; narrow layers
  * (k, a <= 64, rank <= 16) that read the same x with the same noise arguments run in one launch.  They may share
  * one workspace of the size the query gives.  mean_steps: out receives the mean over the t_steps (hses_time_mean of

@@ -50,3 +50,20 @@ def test_grouped_heads_take_the_rows_path(hs):
     for i, (w, c) in enumerate(zip(ws, caches)):
         one = ops.perturbed_linear(x, w, n_pop=n_pop, bm=bm, sigma=0.2, rank=rank, key=20 + i, cache=c)
         assert torch.equal(y[:, i * hd:(i + 1) * hd], one)
+
+
+@pytest.mark.parametrize("bm,a", [(1024, 64), (20, 48)])   # fused, and as two calls
+@pytest.mark.parametrize("post", ["swish", "add", "lif_rate"])
+def test_post_matches_the_separate_calls(hs, post, bm, a):
+    from hyperscalees_b200 import ops
+    n_pop, k = 40, 64
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(n_pop, bm, k, device="cuda", generator=g)
+    w = torch.randn(a, k, device="cuda", generator=g) / 8
+    kw = dict(n_pop=n_pop, bm=bm, sigma=0.2, rank=8, key=20, tau_m=2.0, v_th=0.3)
+    y = ops.perturbed_linear(x, w, **kw)
+    acc = torch.randn(n_pop * bm, a, device="cuda", generator=g)
+    want = {"swish": lambda: ops.swish(y), "add": lambda: ops.add_inplace(acc.clone(), y),
+            "lif_rate": lambda: ops.lif_rate(y, 5, 2.0, 0.3)}[post]()
+    got = ops.perturbed_linear(x, w, post=post, post_steps=5, out=acc if post == "add" else None, **kw)
+    assert torch.equal(got, want)
