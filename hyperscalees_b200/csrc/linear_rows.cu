@@ -137,6 +137,7 @@ struct RowsArgs {
     const uint8_t *wimg, *bimg, *aimg;
     uint32_t w_bytes, b_bytes, a_bytes;
     int xbufs, fbufs, tbufs;                 // buffers of x's parts, of the factors, accumulators
+    int chunk, chunks;                       // outputs at a time: all, or 128 (one block of k) in two accumulators
     float* out;
     int64_t out_stride;
     int wide_out;                            // 32-byte aligned rows
@@ -282,7 +283,7 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_kernel(const __grid
         }
     } else if (warp == 0) {
         const int sn = g.a / g.slabs;                         // outputs of a slab
-        const uint32_t idesc = make_idesc_bf16(g.a + (g.merged ? g.nt : 0)), idesc_t = make_idesc_bf16(g.nt), idesc_u = make_idesc_bf16(sn);
+        const uint32_t idesc_t = make_idesc_bf16(g.nt), idesc_u = make_idesc_bf16(sn);
         const uint64_t dx0 = make_smem_desc(xsm), dw0 = make_smem_desc(wsm), db0 = make_smem_desc(bsm);
         const uint64_t dt0 = make_plain_desc(tsm, LR_TILE * 16), da0 = make_plain_desc(asm_, sn * 16);
         const uint32_t w_part = w_tile >> 4, b_part = (uint32_t)g.nt * 128 >> 4, x_part = LR_PART >> 4;
@@ -291,62 +292,87 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_kernel(const __grid
         Walk w = start;
         Turn x{0, 0}, f{0, 0}, acc{0, 0};
         bool fresh = true;
-        for (int i = 0; i < count && ok; ++i, acc.next(g.tbufs)) {
+        const int row_units = 128 * 128 >> 4;                 // a chunk's rows of W, in units of a descriptor's address
+        const uint32_t t1 = (uint32_t)t_part >> 4;
+        // the rank term of outputs n0 .. n1-1 and the accumulator's hand-over
+        auto rank_term = [&](int b, int fb, int n0, int n1) {
+            const uint32_t u0 = tmem + 256 + (uint32_t)(b * 128);
+            const uint64_t da = da0 + (uint64_t)(fb * (g.a_bytes >> 4));
+            for (int sl = n0 / sn; sl * sn < n1; ++sl) {      // a slab's outputs in this chunk: all of them, or 128
+                const uint64_t t = dt0 + (uint64_t)(sl * 2 * 128);
+                const uint64_t a = da + (uint64_t)(sl * a_slab + max(0, n0 - sl * sn));
+                const uint32_t u = u0 + (uint32_t)max(0, sl * sn - n0), id = sn > g.chunk ? make_idesc_bf16(n1 - n0) : idesc_u;
+                umma_f16_warp(u, t + 2 * t1, a, id, 0);
+                umma_f16_warp(u, t, a + 2 * a_part, id, 1);
+                umma_f16_warp(u, t + t1, a + a_part, id, 1);
+                umma_f16_warp(u, t + t1, a, id, 1);
+                umma_f16_warp(u, t, a + a_part, id, 1);
+                umma_f16_warp(u, t, a, id, 1);
+            }
+            umma_commit_warp(&tfull[b]);
+        };
+        for (int i = 0; i < count && ok; ++i) {
             if (fresh) {
                 ok = __all_sync(0xffffffffu, mbar_wait(&ffull[f.b], f.ph, abort_flag, g.status, 3));
                 if (!ok) break;
             }
-            const int fb = __shfl_sync(0xffffffffu, f.b, 0), b = __shfl_sync(0xffffffffu, acc.b, 0);
-            ok = __all_sync(0xffffffffu, mbar_wait(&tempty[b], acc.ph ^ 1, abort_flag, g.status, 4));
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t d = tmem + (uint32_t)(b * 128), du = d + 256;
-            const uint64_t db = db0 + (uint64_t)(fb * (g.b_bytes >> 4)), da = da0 + (uint64_t)(fb * (g.a_bytes >> 4));
-            for (int kb = 0; kb < g.kb; ++kb, x.next(g.xbufs)) {
-                const int xb = __shfl_sync(0xffffffffu, x.b, 0);
-                ok = __all_sync(0xffffffffu, mbar_wait(&xfull[xb], x.ph, abort_flag, g.status, 5));
+            const int fb = __shfl_sync(0xffffffffu, f.b, 0);
+            const uint64_t db = db0 + (uint64_t)(fb * (g.b_bytes >> 4));
+            int b0 = 0;
+            for (int ch = 0; ch < g.chunks && ok; ++ch, acc.next(g.tbufs)) {
+                const int b = __shfl_sync(0xffffffffu, acc.b, 0), n = min(g.chunk, g.a - ch * g.chunk);
+                ok = __all_sync(0xffffffffu, mbar_wait(&tempty[b], acc.ph ^ 1, abort_flag, g.status, 4));
                 if (!ok) break;
                 tc_fence_after();
-                const uint64_t dx = dx0 + (uint64_t)(xb * 3 * x_part), dw = dw0 + (uint64_t)(kb * 3 * w_part),
-                               dbk = db + (uint64_t)(kb * 3 * b_part);
-                const int ksteps = min(4, (g.k - kb * 64 + 15) / 16);
-                for (int ks = 0; ks < ksteps; ++ks) {         // 16 values = 32 bytes along k; smallest terms first
-                    const uint64_t xd = dx + 2 * ks, wd = dw + 2 * ks, bb = dbk + 2 * ks;
-                    const uint32_t more = (kb | ks) != 0;
-                    if (!g.merged) {
-                        umma_f16_warp(du, xd + 2 * x_part, bb, idesc_t, more);
-                        umma_f16_warp(du, xd, bb + 2 * b_part, idesc_t, 1);
-                        umma_f16_warp(du, xd + x_part, bb + b_part, idesc_t, 1);
-                        umma_f16_warp(du, xd + x_part, bb, idesc_t, 1);
-                        umma_f16_warp(du, xd, bb + b_part, idesc_t, 1);
-                        umma_f16_warp(du, xd, bb, idesc_t, 1);
+                const uint32_t d = tmem + (uint32_t)(b * 128), du = d + 256;
+                const uint32_t idesc = make_idesc_bf16(n + (g.merged ? g.nt : 0));
+                const bool with_t = ch == 0 && !g.merged;
+                for (int kb = 0; kb < g.kb; ++kb) {
+                    const int xb = __shfl_sync(0xffffffffu, x.b, 0);
+                    if (ch == 0) {
+                        ok = __all_sync(0xffffffffu, mbar_wait(&xfull[xb], x.ph, abort_flag, g.status, 5));
+                        if (!ok) break;
+                        tc_fence_after();
                     }
-                    umma_f16_warp(d, xd + 2 * x_part, wd, idesc, more);
-                    umma_f16_warp(d, xd, wd + 2 * w_part, idesc, 1);
-                    umma_f16_warp(d, xd + x_part, wd + w_part, idesc, 1);
-                    umma_f16_warp(d, xd + x_part, wd, idesc, 1);
-                    umma_f16_warp(d, xd, wd + w_part, idesc, 1);
-                    umma_f16_warp(d, xd, wd, idesc, 1);
+                    const uint64_t dx = dx0 + (uint64_t)(xb * 3 * x_part), dbk = db + (uint64_t)(kb * 3 * b_part),
+                                   dw = dw0 + (uint64_t)(kb * 3 * w_part + ch * row_units);
+                    const int ksteps = min(4, (g.k - kb * 64 + 15) / 16);
+                    for (int ks = 0; ks < ksteps; ++ks) {     // 16 values = 32 bytes along k; smallest terms first
+                        const uint64_t xd = dx + 2 * ks, wd = dw + 2 * ks, bb = dbk + 2 * ks;
+                        const uint32_t more = (kb | ks) != 0;
+                        if (with_t) {
+                            umma_f16_warp(du, xd + 2 * x_part, bb, idesc_t, more);
+                            umma_f16_warp(du, xd, bb + 2 * b_part, idesc_t, 1);
+                            umma_f16_warp(du, xd + x_part, bb + b_part, idesc_t, 1);
+                            umma_f16_warp(du, xd + x_part, bb, idesc_t, 1);
+                            umma_f16_warp(du, xd, bb + b_part, idesc_t, 1);
+                            umma_f16_warp(du, xd, bb, idesc_t, 1);
+                        }
+                        umma_f16_warp(d, xd + 2 * x_part, wd, idesc, more);
+                        umma_f16_warp(d, xd, wd + 2 * w_part, idesc, 1);
+                        umma_f16_warp(d, xd + x_part, wd + w_part, idesc, 1);
+                        umma_f16_warp(d, xd + x_part, wd, idesc, 1);
+                        umma_f16_warp(d, xd, wd + w_part, idesc, 1);
+                        umma_f16_warp(d, xd, wd, idesc, 1);
+                    }
+                    if (ch + 1 == g.chunks) {
+                        umma_commit_warp(&xempty[xb]);
+                        x.next(g.xbufs);
+                    }
                 }
-                umma_commit_warp(&xempty[xb]);
+                if (!ok) break;
+                if (ch == 0) {
+                    umma_commit_warp(&tacc);
+                    b0 = b;
+                }
             }
             if (!ok) break;
-            umma_commit_warp(&tacc);
+            // t's way to shared memory and back, while the second chunk's products run
             ok = __all_sync(0xffffffffu, mbar_wait(&tready, i & 1, abort_flag, g.status, 6));
             if (!ok) break;
             tc_fence_after();
-            const uint32_t t1 = (uint32_t)t_part >> 4;
-            for (int sl = 0; sl < g.slabs; ++sl) {
-                const uint64_t t = dt0 + (uint64_t)(sl * 2 * 128), a = da + (uint64_t)(sl * a_slab);
-                const uint32_t u = du + (uint32_t)(sl * sn);
-                umma_f16_warp(u, t + 2 * t1, a, idesc_u, 0);
-                umma_f16_warp(u, t, a + 2 * a_part, idesc_u, 1);
-                umma_f16_warp(u, t + t1, a + a_part, idesc_u, 1);
-                umma_f16_warp(u, t + t1, a, idesc_u, 1);
-                umma_f16_warp(u, t, a + a_part, idesc_u, 1);
-                umma_f16_warp(u, t, a, idesc_u, 1);
-            }
-            umma_commit_warp(&tfull[b]);
+            rank_term(b0, fb, 0, g.chunk);
+            if (g.chunks == 2) rank_term(b0 ^ 1, fb, g.chunk, g.a);
             fresh = w.next(g);
             if (fresh) {
                 umma_commit_warp(&fempty[fb]);
@@ -408,13 +434,15 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_kernel(const __grid
         const uint32_t lane_base = tmem + ((uint32_t)(q4 * 32) << 16) + (g.merged ? g.a : 256);
         Walk w = start;
         Turn acc{0, 0};
-        for (int i = 0; i < count; ++i, w.next(g), acc.next(g.tbufs)) {
+        for (int i = 0; i < count; ++i, w.next(g)) {
+            const int b = acc.b;                              // the accumulator of the tile's first chunk
+            for (int ch = 0; ch < g.chunks; ++ch) acc.next(g.tbufs);
             const bool odd = w.first() + gt >= g.bm;          // the odd member of a pair has A negated
             if (!__all_sync(0xffffffffu, mbar_wait(&tacc, i & 1, abort_flag, g.status, 8))) break;
             tc_fence_after();
             for (int c8 = 0; c8 < g.nt / 8; ++c8) {
                 uint32_t tv[8];
-                tmem_ld8(lane_base + acc.b * 128 + c8 * 8, tv);
+                tmem_ld8(lane_base + b * 128 + c8 * 8, tv);
                 Parts s[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -438,29 +466,30 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_kernel(const __grid
         const float gain = g.out_scale_ptr ? *g.out_scale_ptr : g.out_scale;
         Walk w = start;
         Turn acc{0, 0};
-        for (int i = 0; i < count; ++i, w.next(g), acc.next(g.tbufs)) {
-            const int b = acc.b, cnt = w.rows(g);
+        for (int i = 0; i < count * g.chunks; ++i, acc.next(g.tbufs)) {
+            const int b = acc.b, cnt = w.rows(g), ch = g.chunks == 2 ? i & 1 : 0, c_lo = ch * g.chunk, c_hi = min(c_lo + g.chunk, g.a);
             float* orow = g.out + (size_t)(w.row0(g) + gt) * g.out_stride;
             // the residual's values of a block of columns are asked for one block ahead
             float4 old[4];
             const bool add = POST == HSES_POST_ADD && gt < cnt;
             auto fetch = [&](int cb) {
-                if (!add || cb >= g.a) return;
+                if (!add || cb >= c_hi) return;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const float* o = orow + cb + 4 * j;
                     old[j] = g.wide_out ? *reinterpret_cast<const float4*>(o) : make_float4(o[0], o[1], o[2], o[3]);
                 }
             };
-            fetch(eh * 16);
+            fetch(c_lo + eh * 16);
+            if (ch + 1 == g.chunks) w.next(g);
             if (!__all_sync(0xffffffffu, mbar_wait(&tfull[b], acc.ph, abort_flag, g.status, 9))) break;
             tc_fence_after();
-            for (int cb = eh * 16; cb < g.a; cb += 32) {
+            for (int cb = c_lo + eh * 16; cb < c_hi; cb += 32) {
                 uint32_t y[2][8], u[2][8];
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    tmem_ld8_issue(lane_base + b * 128 + cb + 8 * h, y[h]);
-                    tmem_ld8_issue(lane_base + b * 128 + 256 + cb + 8 * h, u[h]);
+                    tmem_ld8_issue(lane_base + b * 128 + cb - c_lo + 8 * h, y[h]);
+                    tmem_ld8_issue(lane_base + b * 128 + 256 + cb - c_lo + 8 * h, u[h]);
                 }
                 tmem_ld_wait();
                 float v[2][8];
@@ -512,7 +541,7 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_kernel(const __grid
 
 struct RowsPlan {
     bool ok;
-    int kb, rg, nt, merged, xbufs, fbufs, tbufs, smem;
+    int kb, rg, nt, merged, xbufs, fbufs, tbufs, chunk, smem;
     int64_t pairs;
     uint32_t w_bytes, b_bytes, a_bytes;
     size_t o_b, o_a, bytes;
@@ -536,19 +565,20 @@ RowsPlan plan_rows(const hses_linear_args& g) {
     const int nt = p.nt = G * p.rg;
     // With a few tiles per pair B may wait for the pair before: it lies behind W and one product makes y and t (a product of
     // 16 columns costs the tensor core about what one of 64 does)
-    p.merged = g.a + nt <= 256 && tiles / p.pairs >= 4;
-    p.tbufs = g.a + (p.merged ? nt : 0) <= 128 ? 2 : 1;
+    p.merged = g.a + nt <= (p.kb == 1 ? 128 : 256) && tiles / p.pairs >= 4;
+    // more than 128 outputs: two accumulators of 128 in turn while x's only block of k is there, else one of 256
+    const int sn = g.a / (nt / 16);
+    p.chunk = g.a > 128 && p.kb == 1 && (sn == g.a || 128 % sn == 0) ? 128 : g.a;
+    p.tbufs = p.chunk + (p.merged ? nt : 0) <= 128 ? 2 : 1;
     p.w_bytes = (uint32_t)p.kb * 3 * g.a * 128;
     p.b_bytes = (uint32_t)p.kb * 3 * nt * 128;
     p.a_bytes = (uint32_t)3 * 16 * g.a * 2;
-    const int fixed = 1024 + (int)p.w_bytes + 3 * nt * 256;
-    for (int bufs = 3; bufs >= 0; --bufs) {       // x's parts, then the factors in two buffers, where they fit
+    for (int bufs = 3;; --bufs) {                 // x's parts, then the factors in two buffers, where they fit
+        if (bufs < 0) return p;
         p.xbufs = bufs & 2 ? 2 : 1;
-        p.fbufs = bufs & 1 ? 2 : 1;
-        if (p.merged) p.fbufs = 1;
-        p.smem = fixed + p.xbufs * 3 * LR_PART + (int)p.b_bytes * p.fbufs + (int)p.a_bytes * p.fbufs;
+        p.fbufs = bufs & 1 && !p.merged ? 2 : 1;
+        p.smem = 1024 + (int)p.w_bytes + 3 * nt * 256 + p.xbufs * 3 * LR_PART + p.fbufs * (int)(p.b_bytes + p.a_bytes);
         if (p.smem <= LR_SMEM - 1024) break;
-        if (bufs == 0) return p;
     }
     size_t o = (p.w_bytes + 255) / 256 * 256;
     p.o_b = o;
@@ -634,6 +664,8 @@ int run_rows_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g, con
     a.xbufs = p.xbufs;
     a.fbufs = p.fbufs;
     a.tbufs = p.tbufs;
+    a.chunk = p.chunk;
+    a.chunks = (g.a + p.chunk - 1) / p.chunk;
     a.out = g.out;
     a.out_stride = g.out_row_stride;
     a.wide_out = ((uintptr_t)g.out & 31u) == 0 && g.out_row_stride % 8 == 0;
