@@ -73,6 +73,7 @@ struct SplitJob {
     __half *hi, *lo;
     float* inv_scale;
     int* lo_flag;
+    int fixed;           // hi: multiples of 8 (11 bits of the row's largest value): sums over spikes are exact
 };
 
 // values e .. e+3 of a row of k values; past the end: 0
@@ -100,9 +101,10 @@ __device__ __forceinline__ float warp_max(float m) {
 __device__ __forceinline__ float max4(float m, float4 v) {
     return fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
 }
-__device__ __forceinline__ void split4(float4 v, float s, uint2& h2, uint2& l2, uint32_t& nz) {
+__device__ __forceinline__ void split4(float4 v, float s, uint2& h2, uint2& l2, uint32_t& nz, bool fixed = false) {
     const float x0 = v.x * s, x1 = v.y * s, x2 = v.z * s, x3 = v.w * s;
-    const __half2 h01 = __floats2half2_rn(x0, x1), h23 = __floats2half2_rn(x2, x3);
+    const auto grid = [&](float x) { return fixed ? rintf(x * 0.125f) * 8.0f : x; };
+    const __half2 h01 = __floats2half2_rn(grid(x0), grid(x1)), h23 = __floats2half2_rn(grid(x2), grid(x3));
     const float2 b01 = __half22float2(h01), b23 = __half22float2(h23);
     const __half2 l01 = __floats2half2_rn(x0 - b01.x, x1 - b01.y), l23 = __floats2half2_rn(x2 - b23.x, x3 - b23.y);
     h2 = make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
@@ -147,7 +149,7 @@ __device__ __forceinline__ void split_rows(const SplitJob& j, const RowMap& map,
                 const int c = lane + 32 * i;
                 if (c < n4) {
                     uint2 h2, l2;
-                    split4(v[r][i], s, h2, l2, nz);
+                    split4(v[r][i], s, h2, l2, nz, j.fixed);
                     dh[c] = h2;
                     dl[c] = l2;
                 }
@@ -167,7 +169,7 @@ __device__ __forceinline__ void split_rows(const SplitJob& j, const RowMap& map,
         uint2* dl = reinterpret_cast<uint2*>(j.lo + (size_t)p0 * j.kp);
         for (int c = lane; c < n4; c += 32) {
             uint2 h2, l2;
-            split4(load4(row, 4 * c, j.k, j.vec), s, h2, l2, nz);
+            split4(load4(row, 4 * c, j.k, j.vec), s, h2, l2, nz, j.fixed);
             dh[c] = h2;
             dl[c] = l2;
         }

@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(256) snn_factors_kernel(const __grid_constant_
 // ------------------------------------------------------------------------- hidden layer
 struct LayerArgs {
     int T, spt;              // steps, samples per tile; (T - 1) * spt and spt rounded up to 8 fit `rows`
+    int exact;               // 128 rows: the products with W's lo half in an accumulator of their own (see make_plan)
     int rows;                // 128: two accumulators in turn; 192, 256: one, W and the factors read less often
     int64_t n;               // samples
     int64_t tiles;
@@ -175,6 +176,7 @@ struct Ring {
     }
 };
 struct Scan {
+    uint32_t lo;             // accumulator of the lo products, or 0: in y
     uint32_t y, u;           // TMEM address of sample 0's first step in the accumulators of the product and of the rank term
     int T, spt, cnt;         // samples of the tile
     bool live;
@@ -190,13 +192,14 @@ struct Scan {
 // these warps, and a loop over the steps: unrolled for a known T the same work was bound by fetching instructions.
 template <bool PERT, bool HARD>
 __device__ __forceinline__ void scan8(const Scan& c, int sb) {
-    uint32_t ny[8], nu[8];
+    uint32_t ny[8], nu[8], nl[8] = {};
     float v[8], sum[8];
     const int left = c.cnt - sb;                                // samples of this block, uniform
 #pragma unroll
     for (int s = 0; s < 8; ++s) v[s] = sum[s] = 0.0f;
     auto load = [&](int t) {
         tmem_ld8_issue(c.y + t * c.spt + sb, ny);
+        if (c.lo) tmem_ld8_issue(c.lo + t * c.spt + sb, nl);
         if (PERT) tmem_ld8_issue(c.u + t * c.spt + sb, nu);
     };
     load(0);
@@ -208,7 +211,8 @@ __device__ __forceinline__ void scan8(const Scan& c, int sb) {
         tmem_ld_wait();
 #pragma unroll
         for (int s = 0; s < 8; ++s) {                           // the scales are powers of two: exact
-            const float y = __uint_as_float(ny[s]);
+            float y = __uint_as_float(ny[s]);
+            if (c.lo) y = __fadd_rn(y, __uint_as_float(nl[s]));
             cur[s] = __fmul_rn(PERT ? __fadd_rn(y, __uint_as_float(nu[s])) : y, c.cs);
         }
         load(min(t + 1, c.T - 1));
@@ -253,7 +257,7 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
     const uint32_t w_tx = (uint32_t)g.bn * 128, b_bytes = (uint32_t)g.nt * 128;
     const int W_HI = g.rows * 128, W_LO = W_HI + SL_OPERAND, B_HI = W_LO + SL_OPERAND;
     uint8_t* tparts = smem + (size_t)g.stages * g.stage_bytes;   // t: [part 3][nt / 8][rows][8] bf16
-    const int part_bytes = g.nt * g.rows * 2, bufs = !PERT || g.rows == 128 ? 2 : 1;
+    const int part_bytes = g.nt * g.rows * 2, bufs = !PERT || (g.rows == 128 && !g.exact) ? 2 : 1;
     __shared__ uint64_t full[SL_MAX_STAGES], empty[SL_MAX_STAGES], tfull[2], tempty[2], tacc, tready;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag_s;
@@ -284,6 +288,7 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
     __syncthreads();
     tc_fence_after();
     chain_next();
+    // exact: the product at 0, its lo part 128 (without noise 256) further, the rank term at 256, t at 384.  Else:
     // Columns 0-255: accumulators of the product, `rows` each (without noise up to 511).  The same from 256: the rank term,
     // whose columns hold t (a part of 128 columns per 128 rows) until it has been read.
     const uint32_t tmem = tmem_slot;
@@ -389,8 +394,9 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
                 ok = __all_sync(0xffffffffu, mbar_wait(&tempty[b], ph ^ 1, abort_flag, g.status, 2));
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t d = tmem + (uint32_t)(b * g.rows), tmem_u = d + 256;
-                uint32_t tc_col = tmem_u;                     // accumulator and k-blocks left of t's current sum
+                const uint32_t d = tmem + (uint32_t)(b * g.rows), dl = !g.exact ? d : d + (PERT ? 128 : 256);
+                const uint32_t tmem_u = d + 256;
+                uint32_t tc_col = g.exact ? tmem + 384 : tmem_u;                     // accumulator and k-blocks left of t's current sum
                 int tc_left = tc_len;
                 for (int kb = 0; kb < g.k_blocks && ok; ++kb)
                     for (int part = 0; part < x_parts; ++part, ring.next(g.stages)) {
@@ -404,8 +410,8 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
                         {
 #pragma unroll
                             for (int ks = 0; ks < 4; ++ks) {       // 16 fp16 = 32 bytes along k
-                                if (!part) umma_f16_warp(d, dwl + 2 * ks, dx + 2 * ks, idesc, ks ? 1u : more);
-                                umma_f16_warp(d, dwh + 2 * ks, dx + 2 * ks, idesc, 1);
+                                if (!part) umma_f16_warp(dl, dwl + 2 * ks, dx + 2 * ks, idesc, ks ? 1u : more);
+                                umma_f16_warp(part ? dl : d, dwh + 2 * ks, dx + 2 * ks, idesc, !g.exact || part || kb || ks);
                             }
                             if (with_t) {
                                 // t: B's halves side by side, in sums of a few k-blocks each
@@ -473,7 +479,7 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
             tile_of(mt, s0, cnt, p0, nd);
             const int b = bufs == 2 ? (int)(acc_it & 1) : 0;
             acc_it += g.n_chunks * (grp + 1) / g.groups - g.n_chunks * grp / g.groups;
-            const uint32_t t0 = tmem + ((uint32_t)(q4 * 32) << 16) + 256 + b * g.rows + (tall ? eh * 128 : 0);
+            const uint32_t t0 = tmem + ((uint32_t)(q4 * 32) << 16) + (g.exact ? 384 : 256 + b * g.rows) + (tall ? eh * 128 : 0);
             const int64_t s = s0 + sm;
             const bool odd = ((s / g.bm) & 1) != 0;           // the odd member of a pair has A negated
             const int d = step < g.T && sm < cnt ? (int)(s / g.spp - p0) : -1;
@@ -535,7 +541,7 @@ snn_layer_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_consta
                 const int n = c * g.bn + gt;
                 const bool live = gt < g.bn && n < g.a;
                 if (c * g.bn + q4 * 32 < g.a && q4 * 32 < g.bn) {
-                    const Scan sc{lane_base + b * g.rows, lane_base + 256 + b * g.rows, g.T, g.spt, cnt, live, live ? __ldg(g.col_scale + n) : 0.0f,
+                    const Scan sc{g.exact ? lane_base + b * g.rows + (PERT ? 128 : 256) : 0, lane_base + b * g.rows, lane_base + 256 + b * g.rows, g.T, g.spt, cnt, live, live ? __ldg(g.col_scale + n) : 0.0f,
                                   g.leak, g.v_th, x_lo ? g.row_scale + s0 * g.T : nullptr,
                                   g.out_half ? g.out_half + (size_t)s0 * g.T * g.out_pitch + n : nullptr, g.out_pitch,
                                   g.count ? g.count + (size_t)s0 * g.a + n : nullptr, g.a};
@@ -708,7 +714,7 @@ __global__ void __launch_bounds__(256, 4) snn_readout_kernel(const __grid_consta
 
 // ---------------------------------------------------------------------------- host side
 struct LayerPlan {
-    int rows, spt, ppt, tpp, nt, r16, bn, n_chunks, groups, kp, ap, stages, stage_bytes, smem;
+    int exact, rows, spt, ppt, tpp, nt, r16, bn, n_chunks, groups, kp, ap, stages, stage_bytes, smem;
     int64_t tiles;
     size_t o_whi, o_wlo, o_cs, o_bhi, o_blo, o_aimg;
 };
@@ -720,6 +726,25 @@ struct SnnPlan {
     bool ro_members;                 // the readout's blocks hold whole members
     size_t o_x, o_xlo, o_rs, o_h[2], o_rate, o_flag, o_per, bytes;
 };
+
+// would the layer's product run on linear_tc?
+bool on_linear_tc(const hses_snn_model* m, const hses_pop_args* p, int l) {
+    hses_linear_args g{};
+    g.x = g.param = reinterpret_cast<const float*>(0x100);
+    g.out = reinterpret_cast<float*>(0x100);
+    g.t_steps = p->T;
+    g.n_pop = p->n_pop;
+    g.bm = p->bm;
+    g.k = m->dims[l];
+    g.a = m->dims[l + 1];
+    g.x_row_stride = g.param_row_stride = g.k;
+    g.out_row_stride = g.a;
+    g.rank = p->rank;
+    g.first_thread = p->first_thread;
+    g.perturb = p->perturb;
+    g.out_scale = 1.0f;
+    return tensor_path_supports(g);
+}
 
 SnnPlan make_plan(const hses_snn_model* m, const hses_pop_args* p) {
     SnnPlan s{};
@@ -752,12 +777,16 @@ SnnPlan make_plan(const hses_snn_model* m, const hses_pop_args* p) {
         q.n_chunks = (a + 127) / 128;
         q.bn = ((a + q.n_chunks - 1) / q.n_chunks + 15) & ~15;
         if (pert) q.r16 = (r + 15) & ~15;
+        // The tensor core truncates as it adds up; from the second block of k on a neuron near its threshold may decide otherwise.  Shapes
+        // that linear_tc has no tile for were always fp32 multiply-adds and keep that accuracy: W's hi half on a fixed
+        // grid, whose sums over spikes are exact, its lo half in an accumulator of its own.
+        q.exact = k > 64 && !on_linear_tc(m, p, l);
         // Samples per tile and groups of chunks: the cheapest by a model of the kernel in cycles (measured at 784 -> 128 and
         // 128 -> 128, T = 8, rank 4).  Loads: 35 bytes per cycle reach an SM when all of them load; products: 8192 flop per
         // cycle; the rank term's way through shared memory and back: 2600; scan: 20 per row.  Tiles of 128 rows overlap the
         // scan with the next tile's products, taller ones read W less often.
         int64_t best = -1;
-        for (int rows = 256; rows >= 128; rows -= 64)
+        for (int rows = q.exact ? 128 : 256; rows >= 128; rows -= 64)
             for (int cap = rows / p->T; cap >= 1; cap -= std::max(1, cap / 16)) {
                 if ((p->T - 1) * cap + ((cap + 7) & ~7) > rows) continue;   // the scan reads eight columns at a time
                 LayerPlan t = q;
@@ -792,7 +821,7 @@ SnnPlan make_plan(const hses_snn_model* m, const hses_pop_args* p) {
                 const int64_t rank = pert ? 2600 + (int64_t)std::max(1, t.ppt) * q.r16 / 16 * 6 * used / 2 : 0;
                 const int64_t block = std::max(load, mma) + (t.stages == 2 ? std::min(load, mma) / 2 : 0);   // two hide less
                 const int64_t front = (k + 63) / 64 * block + rank, scan = 600 + 20 * (int64_t)used;
-                const int64_t chunk = pert && rows > 128 ? front + scan : std::max(front, scan);
+                const int64_t chunk = pert && (rows > 128 || q.exact) ? front + scan : std::max(front, scan);
                 for (int gr = 1; gr <= q.n_chunks; ++gr) {
                     const int64_t waves = (t.tiles * gr + sms - 1) / sms;
                     const int64_t cost = waves * ((q.n_chunks + gr - 1) / gr) * chunk + front + scan - chunk;
@@ -943,7 +972,7 @@ int run_snn_fused(hses_ctx* ctx, cudaStream_t st, const hses_snn_model* m, const
             const LayerPlan& q = s.l[l];
             const int vec = ((uintptr_t)m->weights[l] & 15u) == 0 && m->weight_strides[l] % 4 == 0;
             jobs.j[l] = SplitJob{m->weights[l], m->weight_strides[l], m->dims[l + 1], m->dims[l], q.kp, vec, half_at(q.o_whi),
-                                 half_at(q.o_wlo), float_at(q.o_cs), nullptr};
+                                 half_at(q.o_wlo), float_at(q.o_cs), nullptr, q.exact};
             jobs.block0[l] = blocks;
             blocks += (m->dims[l + 1] + rpb - 1) / rpb;
         }
@@ -1050,6 +1079,7 @@ int run_snn_fused(hses_ctx* ctx, cudaStream_t st, const hses_snn_model* m, const
         a.T = p->T;
         a.spt = q.spt;
         a.rows = q.rows;
+        a.exact = q.exact;
         a.k_blocks = (m->dims[l] + 63) / 64;
         a.nt = q.nt;
         if (pert) {
