@@ -14,6 +14,11 @@
 //                              stream or read from a cache, as B (K-major fp16 hi + lo, fixed scale 2^11)
 //                              and A (three bf16 parts, scaled by s and by the scale of W's row)
 //   launch 3  linear_pack      persistent, ten warps: TMA producer, MMA issuer, eight epilogue warps
+//
+// linear_pack waits for its copies more than for the L2 (31 %), DRAM or the tensor pipe (below 30 %): what counts is the
+// bytes in flight, so the store buffer holds 16 rows, which leaves room for a third stage at 128 columns, t takes no more
+// columns than there are pairs, and the operands' rows start at a 128-byte line.  1022 members x 36 rows, 500 -> 250,
+// rank 8: 108 us with two stages, 97 with three, 90 with aligned rows.
 // Products of x, W and B are hi*hi + hi*lo + lo*hi in fp16 (2^-21 relative residue); t and A are split into
 // three bf16 parts (24 bits, six products): bf16 has the exponent range of fp32, so that the rank-r term
 // can be accumulated on top of the main product in its scale.  No multicast, no cluster launch; every wait
@@ -39,8 +44,8 @@ constexpr int PK_BK = 64;          // fp16 values per k-block (one 128-byte swiz
 constexpr int PK_THREADS = 320;    // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
 constexpr int PK_MAX_STAGES = 6;
 constexpr int PK_SMEM_LIMIT = 232448;
-constexpr int PK_TR_PITCH = 17;    // staged 32 x 16 output block of an epilogue warp
-constexpr int PK_TR_BYTES = 8 * 32 * PK_TR_PITCH * 4;
+constexpr int PK_TR_PITCH = 17;    // staged 16 x 16 output block of an epilogue warp
+constexpr int PK_TR_BYTES = 8 * 16 * PK_TR_PITCH * 4;
 
 template <int NJ, int RPW>
 __global__ void __launch_bounds__(256) pack_split_kernel(SplitJob j, RowMap map, int* clear) {
@@ -145,15 +150,14 @@ linear_pack_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_cons
 
     if (warp == 0) {
         if (lane == 0) {
-            uint32_t it = 0;
+            Ring ring{0, 0};
             bool ok = true;
             const bool skip_xlo = *g.x_lo_flag == 0;
             auto slot = [&](uint32_t bytes) -> uint8_t* {
-                const int s = it % g.stages;
-                ok = mbar_wait(&empty[s], ((it / g.stages) & 1) ^ 1, abort_flag, g.status, 1);
+                ok = mbar_wait(&empty[ring.s], ring.ph ^ 1, abort_flag, g.status, 1);
                 if (!ok) return nullptr;
-                mbar_expect_tx(&full[s], bytes);
-                return smem + (size_t)s * g.stage_bytes;
+                mbar_expect_tx(&full[ring.s], bytes);
+                return smem + (size_t)ring.s * g.stage_bytes;
             };
             for (int64_t u = blockIdx.x; u < units && ok; u += gridDim.x) {
                 const int64_t mt = u / g.groups;
@@ -163,10 +167,10 @@ linear_pack_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_cons
                 int nd = 0;
                 if (PERT) {
                     nd = pairs_of(mt, p0);
-                    for (int kb = 0; kb < g.k_blocks; ++kb, ++it) {
+                    for (int kb = 0; kb < g.k_blocks; ++kb, ring.next(g.stages)) {
                         uint8_t* st = slot((skip_xlo ? 1 : 2) * X_BYTES + 2 * b_bytes);
                         if (!ok) break;
-                        uint64_t* bar = &full[it % g.stages];
+                        uint64_t* bar = &full[ring.s];
                         tma_load_2d(st, &tm_xhi, kb * PK_BK, (int)(mt * PK_TILE), bar);
                         if (!skip_xlo) tma_load_2d(st + X_BYTES, &tm_xlo, kb * PK_BK, (int)(mt * PK_TILE), bar);
                         tma_load_2d(st + 2 * X_BYTES, &tm_bhi, kb * PK_BK, (int)(p0 * g.r16), bar);
@@ -174,10 +178,10 @@ linear_pack_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_cons
                     }
                 }
                 for (int c = c0; c < c1 && ok; ++c) {
-                    for (int kb = 0; kb < g.k_blocks; ++kb, ++it) {
+                    for (int kb = 0; kb < g.k_blocks; ++kb, ring.next(g.stages)) {
                         uint8_t* st = slot((skip_xlo ? 1 : 2) * X_BYTES + 2 * w_bytes);
                         if (!ok) break;
-                        uint64_t* bar = &full[it % g.stages];
+                        uint64_t* bar = &full[ring.s];
                         tma_load_2d(st, &tm_xhi, kb * PK_BK, (int)(mt * PK_TILE), bar);
                         if (!skip_xlo) tma_load_2d(st + X_BYTES, &tm_xlo, kb * PK_BK, (int)(mt * PK_TILE), bar);
                         tma_load_2d(st + 2 * X_BYTES, &tm_whi, kb * PK_BK, c * g.bn, bar);
@@ -185,12 +189,12 @@ linear_pack_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_cons
                     }
                     if (PERT) {
                         const uint32_t bytes = 3u * g.kb * g.bn * 2;
-                        for (int i = 0; i < nd * nkb && ok; ++i, ++it) {
+                        for (int i = 0; i < nd * nkb && ok; ++i, ring.next(g.stages)) {
                             uint8_t* st = slot(bytes);
                             if (!ok) break;
                             const int d = i / nkb, kblk = i - d * nkb;
                             const size_t img = (((size_t)(p0 + d) * g.n_chunks + c) * nkb + kblk) * 3 * g.kb * g.bn;
-                            bulk_load(st, g.aimg + img, bytes, &full[it % g.stages]);
+                            bulk_load(st, g.aimg + img, bytes, &full[ring.s]);
                         }
                     }
                 }
@@ -205,87 +209,82 @@ linear_pack_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_cons
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = make_idesc(g.bn), idesc_t = make_idesc(PERT ? g.nt : 16), idesc_u = make_idesc_bf16(g.bn);
-            uint32_t it = 0, acc_it = 0, unit_no = 0;
-            bool ok = true;
-            const bool skip_xlo = *g.x_lo_flag == 0;
-            auto arrive = [&]() -> uint8_t* {
-                const int s = it % g.stages;
-                ok = mbar_wait(&full[s], (it / g.stages) & 1, abort_flag, g.status, 3);
-                if (!ok) return nullptr;
+        // the whole warp runs the loop, so that addresses and descriptors stay warp-uniform; an elected lane issues (one
+        // lane in a branch of its own took about 128 cycles per product, twice what the tensor core does)
+        const uint32_t idesc = make_idesc(g.bn), idesc_t = make_idesc(PERT ? g.nt : 16), idesc_u = make_idesc_bf16(g.bn);
+        const uint64_t desc0 = make_smem_desc(smem), desc_step = (uint64_t)(g.stage_bytes >> 4);
+        const uint64_t plain0 = make_plain_desc(smem, g.bn * 16), plain_t = make_plain_desc(tpp, PK_TILE * 16);
+        const uint32_t a1 = (uint32_t)g.kb * g.bn * 2 >> 4, t1 = (uint32_t)part_bytes >> 4;   // one part of an image block, of t
+        uint32_t acc_it = 0, unit_no = 0;
+        Ring ring{0, 0};
+        bool ok = true;
+        const bool skip_xlo = *g.x_lo_flag == 0;
+        auto arrive = [&]() -> bool {
+            ok = __all_sync(0xffffffffu, mbar_wait(&full[ring.s], ring.ph, abort_flag, g.status, 3));
+            if (ok) tc_fence_after();
+            return ok;
+        };
+        // three fp16 passes over one k-block
+        auto three = [&](uint32_t d, uint32_t bytes, uint32_t id, bool first) {
+            const uint64_t xh = desc0 + __shfl_sync(0xffffffffu, ring.s, 0) * desc_step, xl = xh + (X_BYTES >> 4);
+            const uint64_t wh = xl + (X_BYTES >> 4), wl = wh + (bytes >> 4);
+#pragma unroll
+            for (int ks = 0; ks < PK_BK / 16; ++ks) {             // 16 fp16 = 32 bytes along k
+                const uint32_t acc = !(first && ks == 0);
+                if (!skip_xlo) umma_f16_warp(d, xl + 2 * ks, wh + 2 * ks, id, acc);
+                umma_f16_warp(d, xh + 2 * ks, wl + 2 * ks, id, skip_xlo ? acc : 1u);
+                umma_f16_warp(d, xh + 2 * ks, wh + 2 * ks, id, 1);
+            }
+            umma_commit_warp(&empty[ring.s]);
+        };
+        for (int64_t u = blockIdx.x; u < units && ok; u += gridDim.x, ++unit_no) {
+            const int64_t mt = u / g.groups;
+            const int grp = (int)(u - mt * g.groups);
+            const int c0 = g.n_chunks * grp / g.groups, c1 = g.n_chunks * (grp + 1) / g.groups;
+            int64_t p0 = 0;
+            int nd = 0;
+            if (PERT) {
+                nd = pairs_of(mt, p0);
+                for (int kb = 0; kb < g.k_blocks; ++kb, ring.next(g.stages)) {
+                    if (!arrive()) break;
+                    three(tmem + 256, (uint32_t)b_bytes, idesc_t, kb == 0);
+                }
+                if (!ok) break;
+                umma_commit_warp(&tacc);
+            }
+            for (int c = c0; c < c1 && ok; ++c, ++acc_it) {
+                const int b = acc_it & 1;
+                ok = __all_sync(0xffffffffu, mbar_wait(&tempty[b], ((acc_it >> 1) & 1) ^ 1, abort_flag, g.status, 2));
+                if (!ok) break;
                 tc_fence_after();
-                return smem + (size_t)s * g.stage_bytes;
-            };
-            // three fp16 passes over one k-block
-            auto three = [&](uint32_t d, uint8_t* st, int bytes, uint32_t id, bool first) {
-                const uint64_t dxh = make_smem_desc(st), dxl = make_smem_desc(st + X_BYTES);
-                const uint64_t dwh = make_smem_desc(st + 2 * X_BYTES), dwl = make_smem_desc(st + 2 * X_BYTES + bytes);
-#pragma unroll
-                for (int ks = 0; ks < PK_BK / 16; ++ks) {
-                    const uint64_t off = (uint64_t)(ks * 32 >> 4);
-                    const uint32_t acc = !(first && ks == 0);
-                    if (!skip_xlo) umma_f16(d, dxl + off, dwh + off, id, acc);
-                    umma_f16(d, dxh + off, dwl + off, id, skip_xlo ? acc : 1u);
-                    umma_f16(d, dxh + off, dwh + off, id, 1);
+                const uint32_t d = tmem + (uint32_t)(b * 128);
+                for (int kb = 0; kb < g.k_blocks; ++kb, ring.next(g.stages)) {
+                    if (!arrive()) break;
+                    three(d, (uint32_t)w_bytes, idesc, kb == 0);
                 }
-            };
-            for (int64_t u = blockIdx.x; u < units && ok; u += gridDim.x, ++unit_no) {
-                const int64_t mt = u / g.groups;
-                const int grp = (int)(u - mt * g.groups);
-                const int c0 = g.n_chunks * grp / g.groups, c1 = g.n_chunks * (grp + 1) / g.groups;
-                int64_t p0 = 0;
-                int nd = 0;
-                if (PERT) {
-                    nd = pairs_of(mt, p0);
-                    for (int kb = 0; kb < g.k_blocks; ++kb, ++it) {
-                        uint8_t* st = arrive();
-                        if (!ok) break;
-                        three(tmem + 256, st, b_bytes, idesc_t, kb == 0);
-                        umma_commit(&empty[it % g.stages]);
-                    }
+                if (PERT && ok) {
+                    if (c == c0) ok = __all_sync(0xffffffffu, mbar_wait(&tready, unit_no & 1, abort_flag, g.status, 4));
                     if (!ok) break;
-                    umma_commit(&tacc);
-                }
-                for (int c = c0; c < c1 && ok; ++c, ++acc_it) {
-                    const int b = acc_it & 1;
-                    if (!mbar_wait(&tempty[b], ((acc_it >> 1) & 1) ^ 1, abort_flag, g.status, 2)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t d = tmem + (uint32_t)(b * 128);
-                    for (int kb = 0; kb < g.k_blocks; ++kb, ++it) {
-                        uint8_t* st = arrive();
-                        if (!ok) break;
-                        three(d, st, w_bytes, idesc, kb == 0);
-                        umma_commit(&empty[it % g.stages]);
-                    }
-                    if (PERT && ok) {
-                        if (c == c0 && !mbar_wait(&tready, unit_no & 1, abort_flag, g.status, 4)) { ok = false; break; }
-                        tc_fence_after();
-                        const uint32_t abytes = (uint32_t)g.kb * g.bn * 2;   // one part of an image block
-                        for (int i = 0; i < nd * nkb; ++i, ++it) {
-                            uint8_t* st = arrive();
-                            if (!ok) break;
-                            const int dd = i / nkb, kblk = i - dd * nkb;
+                    for (int dd = 0; dd < nd && ok; ++dd)
+                        for (int kblk = 0; kblk < nkb; ++kblk, ring.next(g.stages)) {
+                            if (!arrive()) break;
+                            const uint64_t da0 = plain0 + __shfl_sync(0xffffffffu, ring.s, 0) * desc_step;
                             for (int ks = 0; ks < g.kb / 16; ++ks) {
-                                const int col8 = (dd * g.r16 + kblk * g.kb + ks * 16) >> 3;
-                                uint64_t dt[3], da[3];
-#pragma unroll
-                                for (int part = 0; part < 3; ++part) {
-                                    dt[part] = make_plain_desc(tpp + part * part_bytes + col8 * (PK_TILE * 16), PK_TILE * 16);
-                                    da[part] = make_plain_desc(st + part * abytes + ks * 2 * g.bn * 16, g.bn * 16);
-                                }
-                                umma_f16(d, dt[2], da[0], idesc_u, 1);
-                                umma_f16(d, dt[0], da[2], idesc_u, 1);
-                                umma_f16(d, dt[1], da[1], idesc_u, 1);
-                                umma_f16(d, dt[1], da[0], idesc_u, 1);
-                                umma_f16(d, dt[0], da[1], idesc_u, 1);
-                                umma_f16(d, dt[0], da[0], idesc_u, 1);
+                                const uint64_t dt = plain_t + (uint64_t)(((dd * g.r16 + kblk * g.kb + ks * 16) >> 3) * PK_TILE);
+                                const uint64_t da = da0 + (uint64_t)(ks * 2 * g.bn);
+                                umma_f16_warp(d, dt + 2 * t1, da, idesc_u, 1);
+                                umma_f16_warp(d, dt, da + 2 * a1, idesc_u, 1);
+                                umma_f16_warp(d, dt + t1, da + a1, idesc_u, 1);
+                                umma_f16_warp(d, dt + t1, da, idesc_u, 1);
+                                umma_f16_warp(d, dt, da + a1, idesc_u, 1);
+                                umma_f16_warp(d, dt, da, idesc_u, 1);
                             }
-                            umma_commit(&empty[it % g.stages]);
+                            umma_commit_warp(&empty[ring.s]);
                         }
-                    }
-                    if (ok) umma_commit(&tfull[b]);
                 }
+                if (ok) umma_commit_warp(&tfull[b]);
+                __syncwarp();
             }
         }
     } else {
@@ -295,7 +294,7 @@ linear_pack_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_cons
         const float gain = g.out_scale_ptr ? *g.out_scale_ptr : g.out_scale;
         const bool wide = (reinterpret_cast<uintptr_t>(g.out) & 31) == 0 && (g.out_stride & 7) == 0 && (g.a & 7) == 0 &&
                           (!g.pot || (reinterpret_cast<uintptr_t>(g.pot) & 31) == 0);
-        float* my_tr = tr + (warp - 2) * 32 * PK_TR_PITCH;
+        float* my_tr = tr + (warp - 2) * 16 * PK_TR_PITCH;
         uint32_t acc_it = 0, unit_no = 0;
         bool ok = true;
         for (int64_t u = blockIdx.x; u < units && ok; u += gridDim.x, ++unit_no) {
@@ -380,25 +379,30 @@ linear_pack_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_cons
                             }
                         }
                     } else if (g.staged_stores) {
-                        // rows that start anywhere: through shared memory, so that sixteen lanes write sixteen
-                        // neighbouring values of a row
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) my_tr[lane * PK_TR_PITCH + j] = v[j];
-                        __syncwarp();
+                        // rows that start anywhere: through shared memory, 16 rows at a time, so that sixteen lanes
+                        // write sixteen neighbouring values of a row
                         const int col = lane & 15;
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const int row = 2 * i + (lane >> 4);
-                            const int64_t Rr = __shfl_sync(0xffffffffu, R, row);
-                            const bool vr = __shfl_sync(0xffffffffu, (int)valid, row) != 0;
-                            const float x = my_tr[row * PK_TR_PITCH + col];
-                            if (vr && n0 + col < g.a) {
-                                const size_t o = (size_t)Rr * g.out_stride + n0 + col;
-                                if (g.pot) g.pot[o] = x;
-                                g.out[o] = g.lif ? (x >= g.v_th ? 1.0f : 0.0f) : x;
+                        for (int h = 0; h < 2; ++h) {
+                            if ((lane >> 4) == h) {
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) my_tr[col * PK_TR_PITCH + j] = v[j];
                             }
+                            __syncwarp();
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) {
+                                const int row = 2 * i + (lane >> 4);
+                                const int64_t Rr = __shfl_sync(0xffffffffu, R, h * 16 + row);
+                                const bool vr = __shfl_sync(0xffffffffu, (int)valid, h * 16 + row) != 0;
+                                const float x = my_tr[row * PK_TR_PITCH + col];
+                                if (vr && n0 + col < g.a) {
+                                    const size_t o = (size_t)Rr * g.out_stride + n0 + col;
+                                    if (g.pot) g.pot[o] = x;
+                                    g.out[o] = g.lif ? (x >= g.v_th ? 1.0f : 0.0f) : x;
+                                }
+                            }
+                            __syncwarp();
                         }
-                        __syncwarp();
                     } else if (valid) {
 #pragma unroll
                         for (int j = 0; j < 16; ++j)
@@ -425,7 +429,7 @@ linear_pack_kernel(const __grid_constant__ CUtensorMap tm_xhi, const __grid_cons
 // ------------------------------------------------------------------------------ host side
 struct PackPlan {
     bool ok;
-    int rp, rb, r16, nt, kb, kp, bn, n_chunks, groups;
+    int rp, rb, r16, nt, kb, kp, pitch, bn, n_chunks, groups;
     int64_t pairs, rows, m_tiles;
     int stages, stage_bytes, staged, smem;
     size_t o_xhi, o_xlo, o_whi, o_wlo, o_rs, o_cs, o_bhi, o_blo, o_aimg, o_flag, bytes;
@@ -435,6 +439,7 @@ PackPlan plan_pack(const hses_linear_args& g) {
     PackPlan p{};
     const int64_t rows_nat = (int64_t)g.t_steps * g.n_pop * g.bm;
     p.kp = (g.k + 7) & ~7;
+    p.pitch = (g.k + PK_BK - 1) / PK_BK * PK_BK;   // a box row of 128 bytes is one line of memory, not parts of two
     p.n_chunks = (g.a + 127) / 128;
     p.bn = ((g.a + p.n_chunks - 1) / p.n_chunks + 15) & ~15;
     p.n_chunks = (g.a + p.bn - 1) / p.bn;
@@ -450,10 +455,10 @@ PackPlan plan_pack(const hses_linear_args& g) {
         if (rp > (1 << 30)) return p;
         p.rp = (int)rp;
         p.rb = p.rp / 32;
-        const int nd = p.rp == 32 ? 4 : p.rp % 128 == 0 ? 1 : 2;
-        p.nt = nd * p.r16;
-        p.kb = std::min(p.r16, 64);
         p.pairs = ((int64_t)g.first_thread + g.n_pop - 1) / 2 - g.first_thread / 2 + 1;
+        const int nd = p.rp == 32 ? 4 : p.rp % 128 == 0 ? 1 : 2;
+        p.nt = (int)std::min<int64_t>(nd, p.pairs) * p.r16;
+        p.kb = std::min(p.r16, 64);
         p.rows = p.pairs * p.rp;
     }
     if (p.rows >= (1ll << 31) - 256) return p;
@@ -483,7 +488,7 @@ PackPlan plan_pack(const hses_linear_args& g) {
         o += (bytes + 255) / 256 * 256;
         return at;
     };
-    const size_t nx = (size_t)p.rows * p.kp * 2, nw = (size_t)g.a * p.kp * 2;
+    const size_t nx = (size_t)p.rows * p.pitch * 2, nw = (size_t)g.a * p.pitch * 2;
     p.o_xhi = take(nx);
     p.o_xlo = take(nx);
     p.o_whi = take(nw);
@@ -492,7 +497,7 @@ PackPlan plan_pack(const hses_linear_args& g) {
     p.o_cs = take((size_t)g.a * 4);
     p.o_flag = take(4);
     if (g.perturb) {
-        const size_t nb = (size_t)p.pairs * p.r16 * p.kp * 2;
+        const size_t nb = (size_t)p.pairs * p.r16 * p.pitch * 2;
         p.o_bhi = take(nb);
         p.o_blo = take(nb);
         p.o_aimg = take((size_t)p.pairs * p.n_chunks * p.r16 * 3 * p.bn * 2);
@@ -502,14 +507,14 @@ PackPlan plan_pack(const hses_linear_args& g) {
     return p;
 }
 
-int encode_rows(CUtensorMap* map, const void* base, int64_t rows, int cols, int box_rows) {
+int encode_rows(CUtensorMap* map, const void* base, int64_t rows, int cols, int pitch, int box_rows) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) {
         set_error("cuTensorMapEncodeTiled is not available from the driver");
         return HSES_ERR_CUDA;
     }
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+    cuuint64_t strides[1] = {(cuuint64_t)pitch * 2};
     cuuint32_t box[2] = {(cuuint32_t)PK_BK, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
@@ -555,9 +560,9 @@ int run_pack_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
     plain.rows = g.a;
 
     const SplitJob jw{g.param, g.param_row_stride, g.a, g.k, p.kp, vec_ok(g.param, g.param_row_stride),
-                      half_at(p.o_whi), half_at(p.o_wlo), cs, nullptr};
+                      half_at(p.o_whi), half_at(p.o_wlo), cs, nullptr, 0, p.pitch};
     SplitJob jx{g.x, g.x_row_stride, p.rows, g.k, p.kp, vec_ok(g.x, g.x_row_stride),
-                half_at(p.o_xhi), half_at(p.o_xlo), reinterpret_cast<float*>(ws + p.o_rs), flag};
+                half_at(p.o_xhi), half_at(p.o_xlo), reinterpret_cast<float*>(ws + p.o_rs), flag, 0, p.pitch};
     // a caller-provided fp16 copy of an x that is exact in fp16 is the operand as it stands
     const bool x_ready = !g.perturb && g.x_half != nullptr && ((uintptr_t)g.x_half & 15u) == 0 && p.kp == g.k;
 
@@ -580,6 +585,7 @@ int run_pack_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
         f.r16 = p.r16;
         f.k = g.k;
         f.kp = p.kp;
+        f.pitch = p.pitch;
         f.a = g.a;
         f.row_a0 = g.factor_order == 1 ? 0 : g.k;
         f.row_b0 = g.factor_order == 1 ? g.a : 0;
@@ -651,15 +657,16 @@ int run_pack_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
     a.staged_stores = p.staged;
     a.status = ctx->t.status_word;
     CUtensorMap mx, mxl, mw, mwl, mb, mbl;
+    const int xpitch = x_ready ? p.kp : p.pitch;
     const void* xhi = x_ready ? g.x_half : static_cast<const void*>(jx.hi);
-    rc = encode_rows(&mx, xhi, p.rows, p.kp, PK_TILE);
-    if (rc == HSES_OK) rc = encode_rows(&mxl, x_ready ? g.x_half : static_cast<const void*>(jx.lo), p.rows, p.kp, PK_TILE);
-    if (rc == HSES_OK) rc = encode_rows(&mw, jw.hi, g.a, p.kp, p.bn);
-    if (rc == HSES_OK) rc = encode_rows(&mwl, jw.lo, g.a, p.kp, p.bn);
+    rc = encode_rows(&mx, xhi, p.rows, p.kp, xpitch, PK_TILE);
+    if (rc == HSES_OK) rc = encode_rows(&mxl, x_ready ? g.x_half : static_cast<const void*>(jx.lo), p.rows, p.kp, xpitch, PK_TILE);
+    if (rc == HSES_OK) rc = encode_rows(&mw, jw.hi, g.a, p.kp, p.pitch, p.bn);
+    if (rc == HSES_OK) rc = encode_rows(&mwl, jw.lo, g.a, p.kp, p.pitch, p.bn);
     mb = mw;
     mbl = mwl;
-    if (rc == HSES_OK && g.perturb) rc = encode_rows(&mb, f.bhi, p.pairs * p.r16, p.kp, p.nt);
-    if (rc == HSES_OK && g.perturb) rc = encode_rows(&mbl, f.blo, p.pairs * p.r16, p.kp, p.nt);
+    if (rc == HSES_OK && g.perturb) rc = encode_rows(&mb, f.bhi, p.pairs * p.r16, p.kp, p.pitch, p.nt);
+    if (rc == HSES_OK && g.perturb) rc = encode_rows(&mbl, f.blo, p.pairs * p.r16, p.kp, p.pitch, p.nt);
     if (rc != HSES_OK) return rc;
     const int64_t units = p.m_tiles * p.groups;
     const unsigned grid = (unsigned)std::min<int64_t>(units, ctx->sm_count);

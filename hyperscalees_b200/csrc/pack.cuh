@@ -68,12 +68,13 @@ struct SplitJob {
     const float* src;
     int64_t stride;
     int64_t rows;
-    int k, kp;           // values per row, row pitch of the operand (multiple of 8, padded with zeros)
+    int k, kp;           // values per row, of the operand (multiple of 8, padded with zeros)
     int vec;             // rows are 16-byte aligned
     __half *hi, *lo;
     float* inv_scale;
     int* lo_flag;
     int fixed;           // hi: multiples of 8 (11 bits of the row's largest value): sums over spikes are exact
+    int pitch;           // values from one row of the operand to the next; 0: kp
 };
 
 // values e .. e+3 of a row of k values; past the end: 0
@@ -119,7 +120,7 @@ __device__ __forceinline__ void split_rows(const SplitJob& j, const RowMap& map,
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t p0 = (block * (blockDim.x >> 5) + warp) * RPW;
     uint32_t nz = 0;
-    const int n4 = j.kp >> 2;
+    const int n4 = j.kp >> 2, pitch = j.pitch ? j.pitch : j.kp;
     if (NJ > 0) {
         float4 v[RPW][NJ > 0 ? NJ : 1];
         bool valid[RPW];
@@ -142,8 +143,8 @@ __device__ __forceinline__ void split_rows(const SplitJob& j, const RowMap& map,
             const int e = scale_exponent(warp_max(m));
             const float s = __uint_as_float((uint32_t)(127 + e) << 23);
             if (lane == 0) j.inv_scale[p0 + r] = __uint_as_float((uint32_t)(127 - e) << 23);
-            uint2* dh = reinterpret_cast<uint2*>(j.hi + (size_t)(p0 + r) * j.kp);
-            uint2* dl = reinterpret_cast<uint2*>(j.lo + (size_t)(p0 + r) * j.kp);
+            uint2* dh = reinterpret_cast<uint2*>(j.hi + (size_t)(p0 + r) * pitch);
+            uint2* dl = reinterpret_cast<uint2*>(j.lo + (size_t)(p0 + r) * pitch);
 #pragma unroll
             for (int i = 0; i < NJ; ++i) {
                 const int c = lane + 32 * i;
@@ -165,8 +166,8 @@ __device__ __forceinline__ void split_rows(const SplitJob& j, const RowMap& map,
         const int e = scale_exponent(warp_max(m));
         const float s = __uint_as_float((uint32_t)(127 + e) << 23);
         if (lane == 0) j.inv_scale[p0] = __uint_as_float((uint32_t)(127 - e) << 23);
-        uint2* dh = reinterpret_cast<uint2*>(j.hi + (size_t)p0 * j.kp);
-        uint2* dl = reinterpret_cast<uint2*>(j.lo + (size_t)p0 * j.kp);
+        uint2* dh = reinterpret_cast<uint2*>(j.hi + (size_t)p0 * pitch);
+        uint2* dl = reinterpret_cast<uint2*>(j.lo + (size_t)p0 * pitch);
         for (int c = lane; c < n4; c += 32) {
             uint2 h2, l2;
             split4(load4(row, 4 * c, j.k, j.vec), s, h2, l2, nz, j.fixed);
@@ -191,7 +192,8 @@ struct FactorJob {
     int bn, n_chunks, kb;             // output columns per chunk, chunks, rank values per block of A's image
     float base_sigma;
     const float* col_scale;           // 2^-e of W's rows
-    __half *bhi, *blo;                // (pairs, r16, kp)
+    __half *bhi, *blo;                // (pairs, r16, kp), rows pitch values apart (0: kp)
+    int pitch;
     __nv_bfloat16* aimg;              // (pairs, chunk, r16 / kb, part 3, kb / 8, bn, 8)
 };
 
@@ -261,7 +263,7 @@ __device__ __forceinline__ void factor_segment(const FactorJob& f, int64_t p, in
                 split4(make_float4(v[0], v[1], v[2], v[3]), sc, h0, l0, nz);
                 split4(make_float4(v[4], v[5], v[6], v[7]), sc, h1, l1, nz);
             }
-            const size_t o = ((size_t)p * f.r16 + q) * f.kp + b0 + g * 8;
+            const size_t o = ((size_t)p * f.r16 + q) * (f.pitch ? f.pitch : f.kp) + b0 + g * 8;
             *reinterpret_cast<uint4*>(f.bhi + o) = make_uint4(h0.x, h0.y, h1.x, h1.y);
             *reinterpret_cast<uint4*>(f.blo + o) = make_uint4(l0.x, l0.y, l1.x, l1.y);
         }

@@ -164,17 +164,6 @@ struct LayerArgs {
 };
 constexpr int SL_OPERAND = 128 * 128;    // bytes of 128 rows x 64 values: x, W hi, W lo
 
-// the stage in turn and the parity of its use; counting beats a division per stage
-struct Ring {
-    int s;
-    uint32_t ph;
-    __device__ __forceinline__ void next(int stages) {
-        if (++s == stages) {
-            s = 0;
-            ph ^= 1;
-        }
-    }
-};
 struct Scan {
     uint32_t lo;             // accumulator of the lo products, or 0: in y
     uint32_t y, u;           // TMEM address of sample 0's first step in the accumulators of the product and of the rank term
