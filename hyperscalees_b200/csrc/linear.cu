@@ -417,13 +417,14 @@ int hses_perturbed_linear(hses_ctx* ctx, hses_stream stream, const hses_linear_a
         const bool takes_pair = (g->algo == HSES_ALGO_PAIR && pair_ok2) ||
                                 (g->algo == HSES_ALGO_AUTO && !tensor_path_supports(*g) && pair_ok2);
         if (takes_pair && pair_path_fuses_scan(*g))
-            return run_pair_path(ctx, as_stream(stream), *g);   // the scan runs in that kernel's last phase
+            return run_pair_path(ctx, as_stream(stream), *g, true);   // the scan runs in that kernel's last phase
         // elsewhere: the currents go to `out` and are scanned in place
         hses_linear_args h = *g;
         h.lif = 0;
         h.out_scale = 1.0f;
         h.out_scale_ptr = nullptr;
-        rc = hses_perturbed_linear(ctx, stream, &h);
+        rc = takes_pair && !prefers_small_path(h) && !prefers_rows_path(h) ? run_pair_path(ctx, as_stream(stream), h, true)
+                                                                            : hses_perturbed_linear(ctx, stream, &h);
         if (rc != HSES_OK) return rc;
         return hses_lif_scan(ctx, stream, g->out, g->t_steps, g->n_pop * g->bm, g->a, g->out_row_stride, nullptr,
                              g->tau_m, g->v_th, g->reset_mode, g->out);
@@ -462,7 +463,7 @@ int hses_perturbed_linear(hses_ctx* ctx, hses_stream stream, const hses_linear_a
         return HSES_ERR_UNSUPPORTED;
     }
     if (g->algo == HSES_ALGO_PAIR || (g->algo == HSES_ALGO_AUTO && pair_ok))
-        return run_pair_path(ctx, as_stream(stream), *g);
+        return run_pair_path(ctx, as_stream(stream), *g, false);
     if (g->algo == HSES_ALGO_AUTO && pack_path_supports(*g)) return run_pack_path(ctx, as_stream(stream), *g);
     return run_simt(ctx, as_stream(stream), *g);
 }

@@ -15,7 +15,8 @@ int run_tensor_path(hses_ctx* ctx, cudaStream_t stream, const hses_linear_args& 
 bool pair_path_supports(const hses_linear_args& g);
 bool pair_path_fuses_scan(const hses_linear_args& g);   // lif == 2 is finished inside the per-pair kernel
 size_t pair_path_workspace_bytes(const hses_linear_args& g);
-int run_pair_path(hses_ctx* ctx, cudaStream_t stream, const hses_linear_args& g);
+// scanned: the rows are currents that a LIF scan turns into spikes
+int run_pair_path(hses_ctx* ctx, cudaStream_t stream, const hses_linear_args& g, bool scanned);
 
 // Narrow layers (k, a <= 64, rank <= 16; linear_small.cu): persistent CTAs keep W in registers and
 // walk over pairs.  Taken by HSES_ALGO_AUTO only.

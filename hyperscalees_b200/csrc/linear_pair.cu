@@ -548,9 +548,14 @@ size_t pair_path_workspace_bytes(const hses_linear_args& g) {
     return base + up256((size_t)chunk_pairs_of(g, pairs) * (g.a + g.k) * g.rank * sizeof(float));
 }
 
-int run_pair_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g) {
+int run_pair_path(hses_ctx* ctx, cudaStream_t st, const hses_linear_args& g, bool scanned) {
     // 1. clean product of all rows
     hses_linear_args b = base_call(g);
+    // Under a scan a potential at its threshold spikes or not, and with one sample per member a spike decides a member's
+    // fitness.  Shapes without a linear_tc tile were always fp32 multiply-adds there and stay that: the three-pass product
+    // of linear_pack, whose sums the tensor core truncates, moved one of 31246 members in some runs and gained nothing
+    // beside the pairs' factors (784-36-132-51-10, rank 96: 6.18 ms with either).
+    if (scanned && !tensor_path_supports(b) && !small_path_supports(b)) b.algo = HSES_ALGO_SIMT;
     size_t base_bytes = up256(hses_perturbed_linear_workspace_bytes(&b));
     size_t need = pair_path_workspace_bytes(g);
     HSES_REQUIRE(need == 0 || (g.workspace != nullptr && g.workspace_bytes >= need &&
