@@ -533,10 +533,12 @@ int vec_ok(const void* p, int64_t stride) { return ((uintptr_t)p & 15u) == 0 && 
 
 bool pack_path_supports(const hses_linear_args& g) {
     if (g.n_groups > 1 || g.x_op != HSES_X_NONE || g.lif == 2) return false;
-    // Narrow layers with a rank above 64 and a few rows per pair: a pair takes a whole tile and 128 columns of t, mostly
-    // padding.  15623 pairs of two rows, 51 -> 10, rank 96: operands and product 1.18 ms, fp32 multiply-adds 0.67 ms.
-    if (g.perturb && g.rank > 64 && g.k <= 64 && g.a <= 64 && (int64_t)2 * g.bm * g.t_steps <= 16) return false;
-    return plan_pack(g).ok;
+    const PackPlan p = plan_pack(g);
+    // Pairs of one or two rows (four or eight at wide ranks) fill a sixteenth of their slice, and once the tiles are more
+    // than one wave the padding costs more than fp32 multiply-adds do: 2123 pairs of two rows, 288 -> 49, rank 1: 110 us
+    // against 49; 15623 pairs of two rows, 51 -> 10, rank 96: 1.18 ms against 0.67.
+    if (g.perturb && p.m_tiles > plan_sm_count() && p.rows >= 16 * p.pairs * 2 * g.bm * g.t_steps) return false;
+    return p.ok;
 }
 
 size_t pack_path_workspace_bytes(const hses_linear_args& g) { return plan_pack(g).bytes; }

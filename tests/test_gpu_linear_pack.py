@@ -81,18 +81,23 @@ def test_packed_path_pitched_operands(hs, oracle):
     assert torch.isnan(ob[:, 3 + a:]).all() and torch.isnan(ob[:, :3]).all()
 
 
-@pytest.mark.parametrize("bm,k,a,rank,packed", [(1, 51, 10, 96, False), (8, 64, 64, 65, False), (9, 51, 10, 96, True),
-                                               (1, 51, 10, 64, None), (1, 65, 10, 96, True)])
-def test_narrow_layers_of_wide_rank_with_few_rows(hs, oracle, bm, k, a, rank, packed):
-    """A pair of a few rows would take a whole tile: such layers stay on fp32 multiply-adds."""
+@pytest.mark.parametrize("n_pop,bm,k,a,rank,packed", [
+    (1300, 1, 70, 19, 3, False),    # two rows of 32, more tiles than SMs
+    (1300, 2, 70, 19, 3, True),     # four rows of 32
+    (40, 1, 70, 19, 3, True),       # one wave
+    (400, 1, 51, 10, 96, False),    # two rows of 128
+])
+def test_pairs_of_few_rows(hs, oracle, n_pop, bm, k, a, rank, packed):
+    """Many pairs of a row or two per member would be mostly padding: they stay on fp32 multiply-adds."""
     from hyperscalees_b200 import core, ops
     ctx = core.get_context(0)
     g = np.random.default_rng(k + rank)
-    x = g.standard_normal((1, 6, bm, k)).astype(np.float32)
+    x = g.standard_normal((1, n_pop, bm, k)).astype(np.float32)
     w = (g.standard_normal((a, k)) / np.sqrt(k)).astype(np.float32)
-    got, names = launched(ctx, lambda: ops.perturbed_linear(dev(x), dev(w), n_pop=6, bm=bm, t_steps=1, sigma=0.5, rank=rank,
-                                                            key=KEY, epoch=3, first_thread=0, noise_reuse=1))
-    want = oracle_mm(oracle, x, w, 0.5, rank, KEY, 3, 0, 1, acc64=True)
-    assert packed is None or ("linear_pack" in names) == packed
-    assert np.abs(got.cpu().numpy() - want).max() <= 2e-5 * max(np.abs(want).max(), 1.0)
+    got, names = launched(ctx, lambda: ops.perturbed_linear(dev(x), dev(w), n_pop=n_pop, bm=bm, t_steps=1, sigma=0.5,
+                                                            rank=rank, key=KEY, epoch=3, first_thread=0, noise_reuse=1))
+    assert ("linear_pack" in names) == packed
+    rows = slice(n_pop - 6, n_pop)
+    want = oracle_mm(oracle, x[:, rows], w, 0.5, rank, KEY, 3, n_pop - 6, 1, acc64=True)
+    assert np.abs(got.cpu().numpy().reshape(x.shape[:3] + (a,))[:, rows] - want.reshape(1, 6, bm, a)).max() <= 2e-5 * max(np.abs(want).max(), 1.0)
     assert ctx.device_status() == 0
