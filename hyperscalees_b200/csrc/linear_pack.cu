@@ -534,11 +534,18 @@ int vec_ok(const void* p, int64_t stride) { return ((uintptr_t)p & 15u) == 0 && 
 bool pack_path_supports(const hses_linear_args& g) {
     if (g.n_groups > 1 || g.x_op != HSES_X_NONE || g.lif == 2) return false;
     const PackPlan p = plan_pack(g);
-    // Pairs of one or two rows (four or eight at wide ranks) fill a sixteenth of their slice, and once the tiles are more
-    // than one wave the padding costs more than fp32 multiply-adds do: 2123 pairs of two rows, 288 -> 49, rank 1: 110 us
-    // against 49; 15623 pairs of two rows, 51 -> 10, rank 96: 1.18 ms against 0.67.
-    if (g.perturb && p.m_tiles > plan_sm_count() && p.rows >= 16 * p.pairs * 2 * g.bm * g.t_steps) return false;
-    return p.ok;
+    if (!p.ok || !g.perturb || p.m_tiles <= plan_sm_count()) return p.ok;
+    // Beyond one wave, pairs of a few rows (2 .. 10 of a 32-row slice) may be so much padding that fp32 multiply-adds are
+    // the faster ones.  Both in microseconds, fitted to 4246 members of 1 .. 5 rows, 288 -> 49 at rank 1 (110 here, 49 .. 73
+    // there), 1000 -> 900 at rank 3 (735; 308 .. 1372), 300 -> 200 at rank 28 (215; 197 .. 397), and to 1246 members,
+    // 302 -> 200 at rank 50 (147; 330): steps of a block of k in waves of tiles, bytes of padded rows and factors and
+    // launches; multiply-adds at 13 T/s and the rank term, which grows with the rank and a pair's rows.
+    const double R = 2.0 * g.bm * g.t_steps, k = g.k, a = g.a;
+    const double waves = (double)((p.m_tiles + plan_sm_count() - 1) / plan_sm_count());
+    const double pack = 39 + waves * (p.n_chunks + 1) * ((g.k + PK_BK - 1) / PK_BK) + 1.6e-6 * p.rows * k +
+                        2.5e-6 * p.pairs * p.r16 * (k + a);
+    const double fp32 = 25 + p.pairs * R * k * a / 13e6 + g.rank * R;
+    return pack < fp32;
 }
 
 size_t pack_path_workspace_bytes(const hses_linear_args& g) { return plan_pack(g).bytes; }

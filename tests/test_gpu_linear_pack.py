@@ -83,9 +83,11 @@ def test_packed_path_pitched_operands(hs, oracle):
 
 @pytest.mark.parametrize("n_pop,bm,k,a,rank,packed", [
     (1300, 1, 70, 19, 3, False),    # two rows of 32, more tiles than SMs
-    (1300, 2, 70, 19, 3, True),     # four rows of 32
+    (1300, 2, 70, 19, 3, False),    # four rows of 32
+    (1300, 6, 150, 300, 28, True),  # twelve rows of 32, a wider rank
     (40, 1, 70, 19, 3, True),       # one wave
-    (400, 1, 51, 10, 96, False),    # two rows of 128
+    (400, 1, 51, 10, 96, True),     # two rows of 128, two waves
+    (12000, 1, 51, 10, 96, False),  # many
 ])
 def test_pairs_of_few_rows(hs, oracle, n_pop, bm, k, a, rank, packed):
     """Many pairs of a row or two per member would be mostly padding: they stay on fp32 multiply-adds."""
